@@ -185,6 +185,12 @@ int pcg_eri_class_nout(int cls);
  * single precision (for quartets below the mixed-precision Schwarz threshold). */
 int pcg_eri_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                   int ntask, double *store, int fp32, void *stream);
+/* The same with the first nheavy tasks (a prefix: lists are ordered by decreasing
+ * primitive-quartet count) spread over 16 lanes each, for quartets of many primitives that
+ * would outlast the launch on one lane.  The blocks are the same up to the order of their
+ * primitive sums; fp32 != 0 ignores nheavy. */
+int pcg_eri_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
+                        int ntask, int nheavy, double *store, int fp32, void *stream);
 
 /* Schwarz factor Q[pair] = sqrt(max (mn|mn)) from diagonal blocks of a diagonal class. */
 int pcg_schwarz_class(int cls, const int *tasks, int ntask, const double *store, double *Q,
@@ -216,6 +222,12 @@ int pcg_digest_class_u(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pai
  * the screened store of each grid value. */
 int pcg_scattering_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                          int ntask, double S, double *store, void *stream);
+/* fac[i] for every primitive pair: what it contributes to each scattering integral's
+ * prefactor, K (sqrt(pi)/(2 zeta))^{1/2} exp(-S^2/(4 zeta)); formed once per S. */
+int pcg_scattering_factors(int npp, const double *zeta, const double *K, double S, double *fac, void *stream);
+/* pcg_scattering_class from those factors, with nheavy as in pcg_eri_class_split. */
+int pcg_scattering_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const double *fac,
+                               const int *tasks, int ntask, int nheavy, double S, double *store, void *stream);
 /* Co-density digestion for non-orthogonal CI (Methods/noci.py:243-300 evaluates
  * hartree_fock.py:345-347 on the non-symmetric co-densities of Lowdin-paired
  * determinants): nd densities W, consecutive nbf x nbf row-major blocks; per density

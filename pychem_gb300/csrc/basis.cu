@@ -29,6 +29,29 @@ static void boys_host(int mmax, double T, double* F) {
   for (int m = mmax; m > 0; --m) F[m - 1] = (2.0 * T * F[m] + e) / (2 * m - 1);
 }
 
+// z^-m j_m(z), m = 0 .. mmax (z <= 10 < mmax): the power series for the two highest
+// orders, where nothing cancels, and f_{m-1} = (2m+1) f_m - z^2 f_{m+1} downwards
+static void bessel_host(int mmax, double z, double* f) {
+  const long double x = 0.5L * z * z;
+  long double up[2];
+  for (int m = mmax; m <= mmax + 1; ++m) {
+    long double term = 1.0L;
+    for (int k = 1; k <= m; ++k) term /= 2 * k + 1;
+    long double acc = term;
+    for (int k = 1; fabsl(term) > 1e-22L * fabsl(acc); ++k) {
+      term *= -x / ((long double)k * (2 * m + 2 * k + 1));
+      acc += term;
+    }
+    up[m - mmax] = acc;
+  }
+  for (int m = mmax; m >= 0; --m) {
+    f[m] = (double)up[0];
+    const long double lower = (2 * m + 1) * up[0] - 2.0L * x * up[1];
+    up[1] = up[0];
+    up[0] = lower;
+  }
+}
+
 static DeviceState g_dev[16];
 
 DeviceState* pcg_state() {
@@ -41,35 +64,67 @@ int pcg_ensure_boys(BoysTable* out) {
   DeviceState* st = pcg_state();
   if (!st) { pcg_set_error("no CUDA device"); return PCG_ERR_CUDA; }
   if (!st->boys_c) {
-    const int nm = BOYS_M + BOYS_K;
-    std::vector<double> c((size_t)BOYS_NP * BOYS_M * BOYS_K), ex(BOYS_NP);
-    std::vector<float> cf((size_t)BOYS_NP * BOYS_M * BOYS_KF), exf(BOYS_NP);
+    std::vector<TaylorRow> c((size_t)BOYS_M * BOYS_NP);
+    std::vector<double> ex(BOYS_NP);
+    std::vector<float> cf((size_t)BOYS_NPF * BOYS_M * BOYS_KF), exf(BOYS_NPF);
     double F[64], fact[BOYS_K];
     fact[0] = 1.0;
     for (int k = 1; k < BOYS_K; ++k) fact[k] = fact[k - 1] * k;
     for (int p = 0; p < BOYS_NP; ++p) {
-      double T = (double)p / BOYS_INV_H;
-      boys_host(nm, T, F);
+      const double T = (double)p / BOYS_INV_H;
+      boys_host(BOYS_M + BOYS_K, T, F);
       for (int m = 0; m < BOYS_M; ++m) {
-        for (int k = 0; k < BOYS_K; ++k) c[((size_t)p * BOYS_M + m) * BOYS_K + k] = F[m + k] / fact[k];
-        for (int k = 0; k < BOYS_KF; ++k) cf[((size_t)p * BOYS_M + m) * BOYS_KF + k] = (float)(F[m + k] / fact[k]);
+        TaylorRow& r = c[(size_t)m * BOYS_NP + p];
+        for (int k = 0; k < 4; ++k) r.c[k] = F[m + k] / fact[k];
+        for (int k = 4; k < BOYS_K; ++k) r.t[k - 4] = (float)(F[m + k] / fact[k]);
+        r.t[3] = 0.0f;
       }
       ex[p] = exp(-T);
-      exf[p] = (float)ex[p];
+      if (p % (BOYS_INV_H / BOYS_INV_HF) == 0) {
+        const int q = p / (BOYS_INV_H / BOYS_INV_HF);
+        for (int m = 0; m < BOYS_M; ++m)
+          for (int k = 0; k < BOYS_KF; ++k) cf[((size_t)q * BOYS_M + m) * BOYS_KF + k] = (float)(F[m + k] / fact[k]);
+        exf[q] = (float)ex[p];
+      }
     }
-    double *dc = nullptr, *dex = nullptr;
-    float *dcf = nullptr, *dexf = nullptr;
-    PCG_CUDA(cudaMalloc(&dc, c.size() * sizeof(double)));
-    PCG_CUDA(cudaMalloc(&dex, ex.size() * sizeof(double)));
-    PCG_CUDA(cudaMalloc(&dcf, cf.size() * sizeof(float)));
-    PCG_CUDA(cudaMalloc(&dexf, exf.size() * sizeof(float)));
-    PCG_CUDA(cudaMemcpy(dc, c.data(), c.size() * sizeof(double), cudaMemcpyHostToDevice));
-    PCG_CUDA(cudaMemcpy(dex, ex.data(), ex.size() * sizeof(double), cudaMemcpyHostToDevice));
-    PCG_CUDA(cudaMemcpy(dcf, cf.data(), cf.size() * sizeof(float), cudaMemcpyHostToDevice));
-    PCG_CUDA(cudaMemcpy(dexf, exf.data(), exf.size() * sizeof(float), cudaMemcpyHostToDevice));
-    st->boys_c = dc; st->boys_ex = dex; st->boys_cf = dcf; st->boys_exf = dexf;
+    // j_m(z) / z^m about x_p = p / 64, x = z^2 / 2: its derivative in x is -j_{m+1}(z) / z^{m+1},
+    // so the rows have the Boys rows' form
+    std::vector<TaylorRow> bj((size_t)BOYS_M * BESSEL_NP);
+    std::vector<double2> sc(SINCOS_NP);
+    for (int p = 0; p < BESSEL_NP; ++p) {
+      bessel_host(BOYS_M + BOYS_K, sqrt(2.0 * p / BOYS_INV_H), F);
+      for (int m = 0; m < BOYS_M; ++m) {
+        TaylorRow& r = bj[(size_t)m * BESSEL_NP + p];
+        for (int k = 0; k < 4; ++k) r.c[k] = F[m + k] / fact[k];
+        for (int k = 4; k < BOYS_K; ++k) r.t[k - 4] = (float)(F[m + k] / fact[k]);
+        r.t[3] = 0.0f;
+      }
+    }
+    for (int p = 0; p < SINCOS_NP; ++p) sc[p] = make_double2(sin((double)p / BOYS_INV_H), cos((double)p / BOYS_INV_H));
+    auto upload = [](auto** dst, const auto& v) {
+      const size_t bytes = v.size() * sizeof(v[0]);
+      cudaError_t e = cudaMalloc((void**)dst, bytes);
+      return e != cudaSuccess ? e : cudaMemcpy((void*)*dst, v.data(), bytes, cudaMemcpyHostToDevice);
+    };
+    DeviceState n;
+    PCG_CUDA(upload(&n.boys_c, c));
+    PCG_CUDA(upload(&n.boys_ex, ex));
+    PCG_CUDA(upload(&n.boys_cf, cf));
+    PCG_CUDA(upload(&n.boys_exf, exf));
+    PCG_CUDA(upload(&n.bessel, bj));
+    PCG_CUDA(upload(&n.sincos, sc));
+    *st = n;
   }
   out->c = st->boys_c; out->ex = st->boys_ex; out->cf = st->boys_cf; out->exf = st->boys_exf;
+  return PCG_OK;
+}
+
+int pcg_ensure_bessel(BesselTable* out) {
+  BoysTable bt;
+  if (int rc = pcg_ensure_boys(&bt)) return rc;
+  DeviceState* st = pcg_state();
+  out->c = st->bessel;
+  out->sc = st->sincos;
   return PCG_OK;
 }
 

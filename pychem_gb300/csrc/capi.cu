@@ -99,8 +99,21 @@ int pcg_eri_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, c
   BoysTable bt;
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
-  return pcg_launch_eri(cls, to_dev(basis), to_dev(pairs), bt, (const int2*)tasks, ntask, store, fp32 ? 1 : 0,
-                        0.0f, nullptr, (cudaStream_t)stream);
+  return pcg_launch_eri(cls, to_dev(pairs), bt, (const int2*)tasks, ntask, 0, store, fp32 ? 1 : 0,
+                        (cudaStream_t)stream);
+}
+
+int pcg_eri_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const int* tasks, int ntask,
+                        int nheavy, double* store, int fp32, void* stream) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || ntask < 0 || nheavy < 0 || nheavy > ntask) {
+    pcg_set_error("pcg_eri_class_split: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  BoysTable bt;
+  int rc = pcg_ensure_boys(&bt);
+  if (rc) return rc;
+  return pcg_launch_eri(cls, to_dev(pairs), bt, (const int2*)tasks, ntask, nheavy, store, fp32 ? 1 : 0,
+                        (cudaStream_t)stream);
 }
 
 int pcg_schwarz_class(int cls, const int* tasks, int ntask, const double* store, double* Q, void* stream) {
@@ -139,7 +152,30 @@ int pcg_scattering_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* p
     pcg_set_error("pcg_scattering_class: bad arguments");
     return PCG_ERR_ARG;
   }
-  return pcg_launch_scattering(cls, to_dev(pairs), (const int2*)tasks, ntask, S, store, (cudaStream_t)stream);
+  BesselTable bt;
+  if (int rc = pcg_ensure_bessel(&bt)) return rc;
+  return pcg_launch_scattering(cls, to_dev(pairs), bt, nullptr, (const int2*)tasks, ntask, 0, S, store,
+                               (cudaStream_t)stream);
+}
+
+int pcg_scattering_factors(int npp, const double* zeta, const double* K, double S, double* fac, void* stream) {
+  if (npp < 0 || (npp > 0 && (!zeta || !K || !fac)) || !(S >= 0.0)) {
+    pcg_set_error("pcg_scattering_factors: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  return pcg_launch_scattering_factors(npp, zeta, K, S, fac, (cudaStream_t)stream);
+}
+
+int pcg_scattering_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const double* fac,
+                               const int* tasks, int ntask, int nheavy, double S, double* store, void* stream) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || !fac || ntask < 0 || nheavy < 0 || nheavy > ntask || !(S >= 0.0)) {
+    pcg_set_error("pcg_scattering_class_split: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  BesselTable bt;
+  if (int rc = pcg_ensure_bessel(&bt)) return rc;
+  return pcg_launch_scattering(cls, to_dev(pairs), bt, fac, (const int2*)tasks, ntask, nheavy, S, store,
+                               (cudaStream_t)stream);
 }
 
 int pcg_digest_class_co(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const int* tasks, int ntask,

@@ -21,73 +21,108 @@ void pcg_set_cuda_error(cudaError_t e, const char* what);
 void pcg_set_error(const char* msg);
 
 // ----------------------------------------------------------------------------------
-// Boys function F_m(T).  Grid T_p = p / 16 for T < BOYS_TMAX; per grid point the
-// rows c[m][k] = F_{m+k}(T_p) / k! (k < BOYS_K) and exp(-T_p).  F_m(T) is the Taylor
-// series about the nearest grid point (|dT| <= 1/32), truncation < 2e-17 relative for
-// BOYS_K = 8.  Lower orders come from the downward recursion
-//   F_{m-1} = (2T F_m + exp(-T)) / (2m - 1),
-// exp(-T) from the same grid.  Beyond BOYS_TMAX: F_0 = sqrt(pi/T)/2 and the upward
-// recursion F_{m+1} = (2m+1) F_m / (2T) (exp(-T) < 1e-20 there).
+// Boys function F_m(T), T < BOYS_TMAX: the Taylor series about the nearest grid point
+// T_p = p / 64, with d = T_p - T (|d| <= 1/128): F_m(T) = sum_k F_{m+k}(T_p) d^k / k!.
+// The FP64 pipe of this GPU issues 2 lanes per clock and SM, 1/64 of the FP32 and
+// integer rates, so an integral kernel's time is its count of FP64 instructions and the
+// series is arranged to need few of them: the terms d^4 .. d^6, below 2e-10 of the sum,
+// are summed in FP32 (their rounding is 1e-17 of the sum), and grid index, grid point and
+// the conversions between the two precisions are integer operations.  A row of the
+// table holds four doubles and three floats (48 bytes, three 16-byte loads), truncation
+// 2e-18.  Order m costs 4 FP64 instructions (the 16-point grid with eight FP64 terms: 7, and
+// 5 more for the argument).  Orders up to 2 are each read from the table; above, the lower ones come
+// from the downward recursion F_{m-1} = (2T F_m + exp(-T)) / (2m - 1), exp(-T) from the
+// same grid.  Beyond BOYS_TMAX: F_0 = sqrt(pi/T)/2 and the upward recursion
+// F_{m+1} = (2m+1) F_m / (2T) (exp(-T) < 1e-20 there).
+// The single-precision variant keeps a grid of 16 points per unit and BOYS_KF terms.
 // ----------------------------------------------------------------------------------
-#define BOYS_INV_H 16
 #define BOYS_TMAX 48.0
+#define BOYS_TMAX_HI 0x40480000  // high word of 48.0
+#define BOYS_INV_H 64
 #define BOYS_NP (48 * BOYS_INV_H + 1)
-#define BOYS_K 8
 #define BOYS_M (PCG_MAXLT + 1)
+#define BOYS_K 7
+#define BOYS_INV_HF 16
+#define BOYS_NPF (48 * BOYS_INV_HF + 1)
 #define BOYS_KF 5  // terms for the single-precision variant
 
-struct BoysTable {
-  const double* c;    // [BOYS_NP][BOYS_M][BOYS_K]
-  const double* ex;   // [BOYS_NP]
-  const float* cf;    // [BOYS_NP][BOYS_M][BOYS_KF]
-  const float* exf;   // [BOYS_NP]
+// Taylor row of a function of one variable about a grid point: c_0 .. c_3 and c_4 .. c_6
+struct __align__(16) TaylorRow {
+  double c[4];
+  float t[4];
 };
 
-// Reciprocal square root by Newton-Raphson refinement of the single-precision
-// estimate: y <- y (3 - x y^2) / 2, quadratic convergence; two steps reach double
-// precision from rsqrtf's ~2^-23 relative error.
-__device__ __forceinline__ double nr_rsqrt(double x) {
-  double y = (double)rsqrtf((float)x);
-  double h = 0.5 * x;
-  y = y * fma(-h * y, y, 1.5);
-  y = y * fma(-h * y, y, 1.5);
-  return y;
+struct BoysTable {
+  const TaylorRow* c;  // [BOYS_M][BOYS_NP]
+  const double* ex;    // exp(-T_p), [BOYS_NP]
+  const float* cf;     // [BOYS_NPF][BOYS_M][BOYS_KF]
+  const float* exf;    // [BOYS_NPF]
+};
+
+// Tables of the j0(S r12) fundamentals: rows of z^-m j_m(z) over x = z^2 / 2 < 50, and
+// (sin, cos) at z_p = p / 64 up to z = 100
+#define BESSEL_NP (50 * BOYS_INV_H + 1)
+#define SINCOS_NP (100 * BOYS_INV_H + 1)
+struct BesselTable {
+  const TaylorRow* c;  // [BOYS_M][BESSEL_NP]
+  const double2* sc;   // [SINCOS_NP]
+};
+
+// Double to float and back by integer operations (the conversion instructions use the
+// FP64 pipe).  to_float truncates; magnitudes below 2^-126 become (nearly) 0.
+// to_double of 0 is 2^-127, far below anything that it is added to here.
+__device__ __forceinline__ float bits_to_float(double x) {
+  const int hi = __double2hiint(x);
+  const int m = max((hi & 0x7fffffff) - (896 << 20), 0);
+  return __int_as_float((hi & 0x80000000) | __funnelshift_l(__double2loint(x), m, 3));
+}
+__device__ __forceinline__ double bits_to_double(float x) {
+  const unsigned u = __float_as_uint(x);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
 }
 
-// Reciprocal by Newton-Raphson: y <- y (2 - x y), two steps from the float estimate.
-__device__ __forceinline__ double nr_rcp(double x) {
-  double y = (double)(1.0f / (float)x);
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  return y;
+// Reciprocal square root: the hardware's FP64 estimate (about 20 bits) and one
+// third-order step y <- y (1 + e/2 + 3 e^2/8), e = 1 - x y^2, whose remainder 5 e^3 / 16 is
+// below 2^-58: 5 FP64 instructions.
+__device__ __forceinline__ double nr_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// c_0 + c_1 d + ... + c_6 d^6 from a row; df = d in single precision
+__device__ __forceinline__ double taylor_row(const TaylorRow* row, double d, float df) {
+  const double2 a = __ldg((const double2*)row), b = __ldg((const double2*)row + 1);
+  const float4 t = __ldg((const float4*)row + 2);
+  const float x = df * fmaf(df, fmaf(df, t.z, t.y), t.x);
+  return fma(fma(fma(b.y + bits_to_double(x), d, b.x), d, a.y), d, a.x);
+}
+
+// nearest point of a grid of 64 per unit to T in [0, 2^15): its index, and d = T_p - T
+__device__ __forceinline__ int taylor_point(double T, double& d, float& df) {
+  const float r = fmaf(bits_to_float(T), 64.0f, 12582912.0f);   // 1.5 * 2^23: rounds to an integer
+  d = bits_to_double((r - 12582912.0f) * 0.015625f) - T;
+  df = bits_to_float(d);
+  return __float_as_int(r) - 0x4B400000;
 }
 
 template <int L>
 __device__ __forceinline__ void boys_eval(const BoysTable& bt, double T, double* F) {
-  if (T < BOYS_TMAX) {
-    // nearest grid point without conversions: adding 1.5 * 2^52 rounds T * 16 to an
-    // integer held in the low mantissa bits
-    const double r = fma(T, (double)BOYS_INV_H, 6755399441055744.0);
-    const int p = __double2loint(r);
-    const double d = (r - 6755399441055744.0) * (1.0 / BOYS_INV_H) - T;  // -(T - T_p)
-    const double* row = bt.c + ((size_t)p * BOYS_M + L) * BOYS_K;
-    double f = __ldg(row + BOYS_K - 1);
+  if (__double2hiint(T) < BOYS_TMAX_HI) {
+    double d;
+    float df;
+    const int p = taylor_point(T, d, df);
+    if (L <= 2) {
 #pragma unroll
-    for (int k = BOYS_K - 2; k >= 0; --k) f = fma(f, d, __ldg(row + k));
-    F[L] = f;
-    if (L > 0) {
-      // exp(-T) = exp(-T_p) * sum_k d^k / k!
-      double e = 1.0 / 5040.0;
-      e = fma(e, d, 1.0 / 720.0);
-      e = fma(e, d, 1.0 / 120.0);
-      e = fma(e, d, 1.0 / 24.0);
-      e = fma(e, d, 1.0 / 6.0);
-      e = fma(e, d, 0.5);
-      e = fma(e, d, 1.0);
-      e = fma(e, d, 1.0);
-      e *= __ldg(bt.ex + p);
+      for (int m = 0; m <= L; ++m) F[m] = taylor_row(bt.c + m * BOYS_NP + p, d, df);
+    } else {
+      F[L] = taylor_row(bt.c + L * BOYS_NP + p, d, df);
+      // exp(-T) = exp(-T_p) (1 + d (1 + d/2 + d^2 (1/6 + ...)))
+      const float x = df * fmaf(df, fmaf(df, 1.0f / 720.0f, 1.0f / 120.0f), 1.0f / 24.0f);
+      const double u = fma(fma(1.0 / 6.0 + bits_to_double(x), d, 0.5), d, 1.0);
+      const double ep = __ldg(bt.ex + p);
+      const double e = fma(ep * d, u, ep);
       const double t2 = 2.0 * T;
 #pragma unroll
       for (int m = L; m > 0; --m) F[m - 1] = fma(t2, F[m], e) * (1.0 / (2 * m - 1));
@@ -106,8 +141,8 @@ __device__ __forceinline__ void boys_eval(const BoysTable& bt, double T, double*
 template <int L>
 __device__ __forceinline__ void boys_eval_f(const BoysTable& bt, float T, float* F) {
   if (T < (float)BOYS_TMAX) {
-    const int p = __float2int_rn(T * BOYS_INV_H);
-    const float d = (float)p * (1.0f / BOYS_INV_H) - T;
+    const int p = __float2int_rn(T * BOYS_INV_HF);
+    const float d = (float)p * (1.0f / BOYS_INV_HF) - T;
     const float* row = bt.cf + ((size_t)p * BOYS_M + L) * BOYS_KF;
     float f = __ldg(row + BOYS_KF - 1);
 #pragma unroll

@@ -2,12 +2,13 @@
 #include "eri_kernels.cuh"
 
 int pcg_launch_eri_g3(int cls, const DevPairsExt& pr, const BoysTable& bt, const int2* tasks, int ntask,
-                      double* store, int precision, cudaStream_t s) {
+                      int nheavy, double* store, int precision, cudaStream_t s) {
   const int threads = 128, blocks = (ntask + threads - 1) / threads;
+  const EriRange rg = eri_range(ntask, nheavy);
   if (precision == 0) {
     switch (cls) {
-      case 18: k_eri<Eri2220><<<blocks, threads, 0, s>>>(pr, bt, tasks, ntask, store); break;
-      case 19: k_eri<Eri2221><<<blocks, threads, 0, s>>>(pr, bt, tasks, ntask, store); break;
+      case 18: k_eri<Eri2220><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, bt, tasks, rg, store); break;
+      case 19: k_eri<Eri2221><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, bt, tasks, rg, store); break;
       default: return PCG_ERR_ARG;
     }
   } else {

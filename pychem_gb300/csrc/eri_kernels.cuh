@@ -12,56 +12,120 @@ struct PQf {
   float PAx, PAy, PAz, WPx, WPy, WPz, QCx, QCy, QCz, WQx, WQy, WQz, oo2z, oo2e, oo2ze, rz, re;
 };
 
+// The tasks of one launch.  Tasks [0, nheavy) -- a prefix: the lists are sorted by
+// decreasing primitive-quartet count -- are shared by 2^lgh lanes each, the others by 2^lgl
+// lanes; a lane takes every 2^lg-th primitive quartet, and the partial sums are added by
+// shuffles.  A quartet of two oxygen 1s pairs has 36 x 36 primitive quartets, about a
+// millisecond on one lane, so without the split it ends long after the rest of its launch.
+// stride: distance of a block's elements in the store.
+struct EriRange {
+  int ntask, nheavy, lgh, lgl, stride;
+};
+
+// heavy tasks (as counted by the caller) get 16 lanes; the others as many as leave no more
+// than about 40,000 lanes: two warps a scheduler fill the FP64 pipe
+static inline EriRange eri_range(int ntask, int nheavy) {
+  EriRange r;
+  r.ntask = r.stride = ntask;
+  r.nheavy = nheavy < 0 ? 0 : (nheavy > ntask ? ntask : nheavy);
+  r.lgh = 4;
+  r.lgl = 0;
+  while (r.lgl < 4 && ((long long)(ntask - r.nheavy) << (r.lgl + 1)) <= 40000) ++r.lgl;
+  return r;
+}
+static inline unsigned eri_blocks(const EriRange& r, int threads) {
+  // the heavy part is rounded up to whole warps
+  const long long heavy = (((long long)r.nheavy << r.lgh) + 31) / 32 * 32;
+  return (unsigned)((heavy + ((long long)(r.ntask - r.nheavy) << r.lgl) + threads - 1) / threads);
+}
+
+// This lane's task, its place among the lanes of the task, and log2 of their number; lanes
+// past the end take part in the shuffles on the last task with no primitive quartet.
+struct EriLane {
+  int t, g, lg;
+  bool on;
+};
+__device__ __forceinline__ EriLane eri_lane(const EriRange& r) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long heavy = (((long long)r.nheavy << r.lgh) + 31) / 32 * 32;
+  EriLane l;
+  long long t;
+  if (x < heavy) {
+    l.lg = r.lgh;
+    t = x >> l.lg;
+    l.on = t < r.nheavy;
+  } else {
+    l.lg = r.lgl;
+    t = r.nheavy + ((x - heavy) >> l.lg);
+    l.on = t < r.ntask;
+  }
+  l.g = (int)(threadIdx.x & ((1u << l.lg) - 1));
+  l.t = l.on ? (int)t : r.ntask - 1;
+  return l;
+}
+
+// sums of acc over the lanes of a task (every lane of the warp takes part, with the same lg)
+template <int N, class T>
+__device__ __forceinline__ void eri_lane_sum(T* acc, int lg) {
+  for (int o = 1; o < (1 << lg); o <<= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+}
+
 template <class C>
-__global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, BoysTable bt, const int2* __restrict__ tasks,
-                                             int ntask, double* __restrict__ store) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntask) return;
+__global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, BoysTable bt, const int2* __restrict__ tasks, EriRange rg,
+                                             double* __restrict__ store) {
+  const EriLane ln = eri_lane(rg);
+  const int t = ln.t;
   const int2 tk = tasks[t];
-  const int i0 = __ldg(pr.p.ppoff + tk.x), i1 = i0 + __ldg(pr.p.npp_of + tk.x);
-  const int j0 = __ldg(pr.p.ppoff + tk.y), j1 = j0 + __ldg(pr.p.npp_of + tk.y);
+  const int i0 = __ldg(pr.p.ppoff + tk.x), j0 = __ldg(pr.p.ppoff + tk.y), nj = __ldg(pr.p.npp_of + tk.y);
+  const int nq = ln.on ? __ldg(pr.p.npp_of + tk.x) * nj : 0;
   double acc[C::NACC];
 #pragma unroll
   for (int k = 0; k < C::NACC; ++k) acc[k] = 0.0;
-  for (int i = i0; i < i1; ++i) {
-    const double zeta = __ldg(pr.p.zeta + i);
-    const double Px = __ldg(pr.p.P + 3 * i), Py = __ldg(pr.p.P + 3 * i + 1), Pz = __ldg(pr.p.P + 3 * i + 2);
-    const double Kp = __ldg(pr.p.K + i);
-    PQd q;
-    q.PAx = __ldg(pr.p.PA + 3 * i);
-    q.PAy = __ldg(pr.p.PA + 3 * i + 1);
-    q.PAz = __ldg(pr.p.PA + 3 * i + 2);
-    q.oo2z = __ldg(pr.oo2z + i);
-    for (int j = j0; j < j1; ++j) {
-      const double eta = __ldg(pr.p.zeta + j);
-      const double PQx = Px - __ldg(pr.p.P + 3 * j);
-      const double PQy = Py - __ldg(pr.p.P + 3 * j + 1);
-      const double PQz = Pz - __ldg(pr.p.P + 3 * j + 2);
-      const double rs = nr_rsqrt(zeta + eta);
-      const double izpe = rs * rs;
-      const double rho = zeta * eta * izpe;
-      const double T = rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
-      double F[C::L + 1];
-      boys_eval<C::L>(bt, T, F);
-      const double pre = Kp * __ldg(pr.p.K + j) * rs;
-#pragma unroll
-      for (int m = 0; m <= C::L; ++m) F[m] *= pre;
-      const double wp = -eta * izpe, wq = zeta * izpe;
-      q.WPx = wp * PQx; q.WPy = wp * PQy; q.WPz = wp * PQz;
-      q.WQx = wq * PQx; q.WQy = wq * PQy; q.WQz = wq * PQz;
-      q.QCx = __ldg(pr.p.PA + 3 * j);
-      q.QCy = __ldg(pr.p.PA + 3 * j + 1);
-      q.QCz = __ldg(pr.p.PA + 3 * j + 2);
-      q.oo2e = __ldg(pr.oo2z + j);
-      q.oo2ze = 0.5 * izpe;
-      q.rz = eta * izpe;
-      q.re = zeta * izpe;
-      C::prim(q, F, acc);
+  int i = i0 - 1, jj = ln.g + nj;      // jj: ket primitive plus the bra steps not yet taken
+  double zeta = 0.0, Px = 0.0, Py = 0.0, Pz = 0.0, Kp = 0.0;
+  PQd q;
+  for (int n = ln.g; n < nq; n += 1 << ln.lg, jj += 1 << ln.lg) {
+    if (jj >= nj) {
+      do { jj -= nj; ++i; } while (jj >= nj);
+      zeta = __ldg(pr.p.zeta + i);
+      Px = __ldg(pr.p.P + 3 * i); Py = __ldg(pr.p.P + 3 * i + 1); Pz = __ldg(pr.p.P + 3 * i + 2);
+      Kp = __ldg(pr.p.K + i);
+      q.PAx = __ldg(pr.p.PA + 3 * i);
+      q.PAy = __ldg(pr.p.PA + 3 * i + 1);
+      q.PAz = __ldg(pr.p.PA + 3 * i + 2);
+      q.oo2z = __ldg(pr.oo2z + i);
     }
+    const int j = j0 + jj;
+    const double eta = __ldg(pr.p.zeta + j);
+    const double PQx = Px - __ldg(pr.p.P + 3 * j);
+    const double PQy = Py - __ldg(pr.p.P + 3 * j + 1);
+    const double PQz = Pz - __ldg(pr.p.P + 3 * j + 2);
+    const double rs = nr_rsqrt(zeta + eta);
+    const double izpe = rs * rs;
+    q.rz = eta * izpe;
+    const double T = zeta * q.rz * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
+    double F[C::L + 1];
+    boys_eval<C::L>(bt, T, F);
+    const double pre = Kp * __ldg(pr.p.K + j) * rs;
+#pragma unroll
+    for (int m = 0; m <= C::L; ++m) F[m] *= pre;
+    q.re = zeta * izpe;
+    q.WPx = -q.rz * PQx; q.WPy = -q.rz * PQy; q.WPz = -q.rz * PQz;
+    q.WQx = q.re * PQx; q.WQy = q.re * PQy; q.WQz = q.re * PQz;
+    q.QCx = __ldg(pr.p.PA + 3 * j);
+    q.QCy = __ldg(pr.p.PA + 3 * j + 1);
+    q.QCz = __ldg(pr.p.PA + 3 * j + 2);
+    q.oo2e = __ldg(pr.oo2z + j);
+    q.oo2ze = 0.5 * izpe;
+    C::prim(q, F, acc);
   }
+  eri_lane_sum<C::NACC>(acc, ln.lg);
+  if (ln.g != 0 || !ln.on) return;
   const double ABx = __ldg(pr.p.AB + 3 * tk.x), ABy = __ldg(pr.p.AB + 3 * tk.x + 1), ABz = __ldg(pr.p.AB + 3 * tk.x + 2);
   const double CDx = __ldg(pr.p.AB + 3 * tk.y), CDy = __ldg(pr.p.AB + 3 * tk.y + 1), CDz = __ldg(pr.p.AB + 3 * tk.y + 2);
-  C::finish(acc, ABx, ABy, ABz, CDx, CDy, CDz, [&](int k, double v) { store[(size_t)k * ntask + t] = v; });
+  C::finish(acc, ABx, ABy, ABz, CDx, CDy, CDz, [&](int k, double v) { store[(size_t)k * rg.stride + t] = v; });
 }
 
 // Single-precision variant for quartets whose Schwarz bound is below the mixed

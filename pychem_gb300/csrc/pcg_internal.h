@@ -5,14 +5,17 @@
 #include "common.cuh"
 
 struct DeviceState {
-  double* boys_c = nullptr;
+  TaylorRow* boys_c = nullptr;
   double* boys_ex = nullptr;
   float* boys_cf = nullptr;
   float* boys_exf = nullptr;
+  TaylorRow* bessel = nullptr;
+  double2* sincos = nullptr;
 };
 
 DeviceState* pcg_state();
 int pcg_ensure_boys(BoysTable* out);
+int pcg_ensure_bessel(BesselTable* out);
 
 int pcg_launch_pair_data(const DevBasis& b, int npair, const int* pA, const int* pB, const int* ppoff,
                          double* AB, double* zeta, double* P, double* PA, double* K, float* Kf, double* oo2z,
@@ -30,22 +33,22 @@ struct DevPairsExt {
   const double* oo2z;  // 1/(2 zeta) per primitive pair
 };
 
-int pcg_launch_eri(int cls, const DevBasis& b, const DevPairsExt& pr, const BoysTable& bt, const int2* tasks,
-                   int ntask, double* store, int precision, float fp32_below, const double* qpair,
-                   cudaStream_t s);
+int pcg_launch_eri(int cls, const DevPairsExt& pr, const BoysTable& bt, const int2* tasks, int ntask, int nheavy,
+                   double* store, int precision, cudaStream_t s);
 int pcg_launch_pair_data_f32(int npp, const double* zeta, const double* PA, const double* oo2z, const float* Kf,
                              float* pf8, cudaStream_t s);
 int pcg_launch_pair_ao(const DevBasis& b, int npair, const int* pA, const int* pB, int* ao4, cudaStream_t s);
-int pcg_launch_eri_s0(int cls, const DevPairsExt& pr, const int2* tasks, int ntask, double S, double* store,
-                      cudaStream_t s);
-int pcg_launch_eri_s1(int cls, const DevPairsExt& pr, const int2* tasks, int ntask, double S, double* store,
-                      cudaStream_t s);
-int pcg_launch_eri_s2(int cls, const DevPairsExt& pr, const int2* tasks, int ntask, double S, double* store,
-                      cudaStream_t s);
-int pcg_launch_eri_s3(int cls, const DevPairsExt& pr, const int2* tasks, int ntask, double S, double* store,
-                      cudaStream_t s);
-int pcg_launch_scattering(int cls, const DevPairsExt& pr, const int2* tasks, int ntask, double S, double* store,
-                          cudaStream_t s);
+int pcg_launch_eri_s0(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
+                      int ntask, int nheavy, double S, double* store, cudaStream_t s);
+int pcg_launch_eri_s1(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
+                      int ntask, int nheavy, double S, double* store, cudaStream_t s);
+int pcg_launch_eri_s2(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
+                      int ntask, int nheavy, double S, double* store, cudaStream_t s);
+int pcg_launch_eri_s3(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
+                      int ntask, int nheavy, double S, double* store, cudaStream_t s);
+int pcg_launch_scattering(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
+                          int ntask, int nheavy, double S, double* store, cudaStream_t s);
+int pcg_launch_scattering_factors(int npp, const double* zeta, const double* K, double S, double* fac, cudaStream_t s);
 int pcg_launch_digest(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                       const double* store, const double* D, double* G, cudaStream_t s);
 int pcg_launch_digest_u(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,

@@ -18,6 +18,10 @@ from ._lib import BasisT, PairsT
 
 INTEGRAL_THRESHOLD = 1.0e-8   # Data/constants.py:31
 N_SPHER = [1, 3, 5]
+# primitive quartets from which a shell quartet is shared by 16 lanes: with one lane the 1,296
+# of two oxygen 1s pairs take longer than the rest of a mid-size molecule's launch, and from
+# 128 on each of 16 lanes still has eight or more to sum
+HEAVY = 128
 
 
 def _ptr(t):
@@ -40,7 +44,7 @@ def pair_colmap(n, pmap, device):
     return cm
 
 
-def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None):
+def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None, info=None):
     """Screened canonical quartet plan (Methods/hartree_fock.py:241-312: the quartet
     loop, the Schwarz test Q_ab Q_cd > threshold, and the diagonal quartet that is
     always computed), with tensor operations on Q's device.
@@ -62,7 +66,8 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None):
     the diagonal flag; row r covers tasks [off[r], off[r+1]).  With kind_work (work
     per pair of each kind, e.g. its primitive-pair count) the buckets run in
     decreasing work per quartet, so a launch's heaviest CTAs start first and the light
-    ones fill its tail."""
+    ones fill its tail.  info (a dict) receives per (class, part) the number of tasks and
+    of those, a prefix, whose work is at least HEAVY (0 without kind_work)."""
     dev = Q.device
     nk = int(class_table.shape[0])
     o = torch.sort(-Q, stable=True).indices
@@ -82,6 +87,7 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None):
         key = (int(w.max()) - w) * (nk * nk * npair) + key
     ro = torch.sort(key).indices
     pos, kk, kb = pos[ro], kk[ro], kb[ro]
+    heavy = (w[ro] >= HEAVY).to(torch.int64) if kind_work is not None else torch.zeros_like(pos)
     qb = Qs[pos]
     key = kk * nmol + ms[pos]
     lo = torch.searchsorted(seg_key, key, right=False)
@@ -118,19 +124,24 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None):
     plan = []
     ncls = int(class_table.max()) + 1 if class_table.numel() else 0
     for part, n, qs, dg in (("64", c64 + diag, lo, diag), ("32", cnt - c64, lo + c64, torch.zeros_like(diag))):
-        # rows grouped by class (a stable sort keeps each class's rows in order), the
-        # class sizes read back once per part
+        # rows grouped by class (a stable sort keeps each class's rows in order); the class
+        # sizes, tasks and heavy tasks read back once per part
         key = torch.where(n > 0, cls_row, torch.full_like(cls_row, ncls))
         order = torch.sort(key, stable=True).indices
-        counts = torch.bincount(key, minlength=ncls + 1)[:ncls].tolist()
+        cols = [torch.bincount(key, minlength=ncls + 1)]
+        cols += [torch.bincount(key, weights=x.to(torch.float64), minlength=ncls + 1).to(torch.int64)
+                 for x in (n, n * heavy)]
+        counts, tasks, heavies = torch.stack(cols).tolist()
         start = 0
-        for cls, c in enumerate(counts):
+        for cls, c in enumerate(counts[:ncls]):
             if c == 0:
                 continue
             sel = order[start:start + c]
             start += c
             off = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), torch.cumsum(n[sel], 0)])
             plan.append((cls, part, bra[sel], off, qs[sel], dg[sel]))
+            if info is not None:
+                info[(cls, part)] = (tasks[cls], heavies[cls])
     return plan, o
 
 
@@ -155,6 +166,7 @@ class GpuEngine:
         self._build_pairs()
         self.S = self.H = None
         self.classes = {}
+        self.heavy = {}
         self.stats = {}
 
     # ---------------------------------------------------------------------------------
@@ -277,78 +289,50 @@ class GpuEngine:
     # Methods/properties.py:20-23); schwarz(), build_tasks() and compute_eris() follow it
     scattering = None
 
-    def _eri(self, cls, tasks, ntask, store, fp32, pairs=None):
-        pairs = self.pairs_t if pairs is None else pairs
+    def _eri(self, cls, tasks, ntask, store, fp32, nheavy=0, factors=None):
+        """Blocks of one task list; its first nheavy tasks have HEAVY or more primitive
+        quartets.  factors: _scattering_factors() of this pass (scattering operator)."""
         if self.scattering is not None:
             if fp32:
                 raise ValueError("scattering integrals are FP64 only")
-            _lib.call("pcg_scattering_class", cls, ctypes.byref(self.basis_t), ctypes.byref(pairs),
-                      _ptr(tasks), ntask, float(self.scattering), _ptr(store), _stream())
+            _lib.call("pcg_scattering_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
+                      _ptr(factors), _ptr(tasks), ntask, nheavy, float(self.scattering), _ptr(store), _stream())
             return
-        _lib.call("pcg_eri_class", cls, ctypes.byref(self.basis_t), ctypes.byref(pairs), _ptr(tasks), ntask,
-                  _ptr(store), 1 if fp32 else 0, _stream())
+        _lib.call("pcg_eri_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(tasks),
+                  ntask, nheavy, _ptr(store), 1 if fp32 else 0, _stream())
 
-    # bra primitive pairs per task in the Schwarz pass
-    schwarz_slice = 4
-
-    def _sliced_pairs(self, ids, nslice):
-        """A pair table of len(ids) * nslice bra slices -- slice s of pair k covers its
-        kept primitive pairs [s * schwarz_slice, (s + 1) * schwarz_slice) -- followed by
-        the len(ids) whole pairs, sharing the primitive arrays (device tensors kept in
-        the returned tuple)."""
-        p, ch = self.pd, self.schwarz_slice
-        idt = torch.as_tensor(ids, dtype=torch.int64).to(self.dev)
-        sl = torch.arange(nslice, dtype=torch.int64, device=self.dev)
-        rep = lambda x: torch.cat([x.repeat_interleave(nslice, dim=0), x])
-        off, cnt = p["ppoff"][idt].to(torch.int64), p["npp"][idt].to(torch.int64)
-        s_off = (off[:, None] + sl[None, :] * ch).reshape(-1)
-        s_cnt = (cnt[:, None] - sl[None, :] * ch).clamp(0, ch).reshape(-1)
-        keep = dict(A=rep(p["A"][idt]).contiguous(), B=rep(p["B"][idt]).contiguous(),
-                    AB=rep(p["AB"].view(-1, 3)[idt]).reshape(-1).contiguous(),
-                    ppoff=torch.cat([s_off, off]).to(torch.int32), npp=torch.cat([s_cnt, cnt]).to(torch.int32))
-        t = PairsT()
-        ctypes.memmove(ctypes.addressof(t), ctypes.addressof(self.pairs_t), ctypes.sizeof(PairsT))
-        t.npair = len(ids) * (nslice + 1)
-        for k, f in (("A", "A"), ("B", "B"), ("ppoff", "ppoff"), ("npp", "npp_of"), ("AB", "AB")):
-            setattr(t, f, keep[k].data_ptr())
-        t.ao4 = None
-        return t, keep
+    def _scattering_factors(self):
+        if self.scattering is None:
+            return None
+        fac = torch.empty_like(self.pd["K"])
+        _lib.call("pcg_scattering_factors", fac.numel(), _ptr(self.pd["zeta"]), _ptr(self.pd["K"]),
+                  float(self.scattering), _ptr(fac), _stream())
+        return fac
 
     def schwarz(self):
-        """Q[pair] = sqrt(max (mn|mn)) over the diagonal quartets (ab|ab).  A diagonal
-        quartet of many primitive pairs (the oxygen 1s pair: 36, so 1,296 primitive
-        quartets) would run long on one thread, so the bra's kept primitive pairs are
-        split into slices of schwarz_slice, each slice one task against the whole ket
-        pair; the slices' integrals (linear in the primitive sum) are added in a fixed
-        order before the maximum."""
+        """Q[pair] = sqrt(max (mn|mn)) over the diagonal quartets (ab|ab), the pairs of
+        each class in decreasing order of their kept primitives: the quartets of HEAVY or
+        more primitive quartets (an oxygen 1s pair has 36 x 36) get several lanes each."""
         Q = torch.zeros(self.npair, dtype=torch.float64, device=self.dev)
         pc = pair_class(self.h_pairs["lA"], self.h_pairs["lB"])
-        self.diag_blocks = {}
+        factors = self._scattering_factors()
         npp = self.h_npp
-        for c in np.unique(pc):
-            ids = np.nonzero(pc == c)[0].astype(np.int32)
-            # heaviest pairs first: the warps run uniform primitive loops and the long
-            # quartets start early
-            ids = ids[np.argsort(-npp[ids], kind="stable")]
-            la, lb = int(self.h_pairs["lA"][ids[0]]), int(self.h_pairs["lB"][ids[0]])
-            cls = _lib.load().pcg_eri_class_id(la, lb, la, lb)
-            m = len(ids)
-            nout = _lib.load().pcg_eri_class_nout(cls)
-            nslice = 1 if self.scattering is not None else max(1, -(-int(npp[ids].max()) // self.schwarz_slice))
-            if nslice == 1:
-                tasks = self._t(np.stack([ids, ids], axis=1))
-                store = torch.empty(nout * m, dtype=torch.float64, device=self.dev)
-                self._eri(cls, tasks, m, store, False)
-            else:
-                pairs, keep = self._sliced_pairs(ids, nslice)
-                vt = np.stack([np.arange(m * nslice), m * nslice + np.repeat(np.arange(m), nslice)], axis=1)
-                vtasks = self._t(vt.astype(np.int32))
-                part = torch.empty(nout * m * nslice, dtype=torch.float64, device=self.dev)
-                self._eri(cls, vtasks, m * nslice, part, False, pairs=pairs)
-                store = part.view(nout, m, nslice).sum(dim=2).contiguous()
-                tasks = self._t(np.stack([ids, ids], axis=1))
-                del keep
-            _lib.call("pcg_schwarz_class", cls, _ptr(tasks), m, _ptr(store), _ptr(Q), _stream())
+        lib = _lib.load()
+        # the tasks of every class in one upload
+        order = np.lexsort((-npp, pc))
+        tasks = self._t(np.repeat(order.astype(np.int32), 2))
+        starts = np.searchsorted(pc[order], np.arange(pair_class(2, 2) + 2))
+        for c in range(len(starts) - 1):
+            lo, hi = int(starts[c]), int(starts[c + 1])
+            if lo == hi:
+                continue
+            la, lb = int(self.h_pairs["lA"][order[lo]]), int(self.h_pairs["lB"][order[lo]])
+            cls = lib.pcg_eri_class_id(la, lb, la, lb)
+            part = tasks[2 * lo:2 * hi]
+            store = torch.empty(lib.pcg_eri_class_nout(cls) * (hi - lo), dtype=torch.float64, device=self.dev)
+            n = npp[order[lo:hi]]
+            self._eri(cls, part, hi - lo, store, False, int(np.count_nonzero(n * n >= HEAVY)), factors)
+            _lib.call("pcg_schwarz_class", cls, _ptr(part), hi - lo, _ptr(store), _ptr(Q), _stream())
         self.Q = Q
         return Q
 
@@ -373,13 +357,15 @@ class GpuEngine:
                 ct[i, j] = lib.pcg_eri_class_id(int(kl[i, 0]), int(kl[i, 1]), int(kl[j, 0]), int(kl[j, 1]))
         mol, nmol = self._pair_molecule()
         work = torch.as_tensor([k[1] for k in self.kinds], dtype=torch.int64, device=dev)
+        info = {}
         plan, ket_list = plan_quartets(self.Q, torch.as_tensor(self.pair_kind, dtype=torch.int64, device=dev), mol,
                                        nmol, torch.as_tensor(ct, device=dev), float(self.threshold),
-                                       float(self.fp32_below), kind_work=work)
-        totals = torch.stack([x[3][-1] for x in plan]).cpu().tolist() if plan else []
+                                       float(self.fp32_below), kind_work=work, info=info)
         ket32 = ket_list.to(torch.int32)
         self.classes = {}
-        for (cls, part, bra, off, qs, dg), total in zip(plan, totals):
+        self.heavy = {key: heavy for key, (_, heavy) in info.items()}
+        for cls, part, bra, off, qs, dg in plan:
+            total = info[(cls, part)][0]
             tasks = torch.empty(int(total) * 2, dtype=torch.int32, device=dev)
             # named so that the int32 copies outlive the launch that reads them
             bra32, qs32, dg32 = bra.to(torch.int32), qs.to(torch.int32), dg.to(torch.int32)
@@ -416,11 +402,12 @@ class GpuEngine:
     def compute_eris(self):
         """Compute every screened quartet block into the in-core class stores."""
         self.stores = {}
+        factors = self._scattering_factors()
         for cls, rec in self.classes.items():
             nout = _lib.load().pcg_eri_class_nout(cls)
             for part, (tasks, n) in rec.items():
                 store = torch.empty(nout * n, dtype=torch.float64, device=self.dev)
-                self._eri(cls, tasks, n, store, part == "32")
+                self._eri(cls, tasks, n, store, part == "32", min(n, self.heavy.get((cls, part), 0)), factors)
                 self.stores[(cls, part)] = store
         return self.stores
 
