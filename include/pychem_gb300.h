@@ -349,19 +349,43 @@ int pcg_jacobi_eigh(int batch, int n, const double *A, double *w, void *V, int f
 /* Learned initial guess (no upstream counterpart; upstream's guesses are the core
  * Hamiltonian and MO files, Methods/hartree_fock.py:35-57).  Dense-layer kernels:
  * C[m][n] (+)= sum_k A[m*sam + k*sak] B[k*sbk + n*sbn] with FP32 A, FP32 or BF16 B
- * (b_bf16), FP32 accumulation, optional epilogue Z = C + bias, C = silu(Z) (act = 1);
+ * (b_bf16), FP32 accumulation, optional epilogue Z = C + bias, C = silu(Z) (act = 1) or, reading
+ * Z, C *= silu'(Z) (act = 2);
  * G *= silu'(Z); column sums; masked squared error (dY = 2 (Y - T) mask * inv_count,
  * loss += sum of squares * inv_count); Adam on FP32 master weights with an optional
  * BF16 copy (bias-corrected by step). */
 int pcg_mlp_gemm(int M, int N, int K, const float *A, long long sam, long long sak, const void *B,
                  int b_bf16, long long sbk, long long sbn, float *C, int ldc, int accumulate,
                  const float *bias, float *Z, int act, void *stream);
+/* The weight gradient dW = A^T G (K x N) of a layer from its input A (M x K) and output
+ * gradient G (M x N), both row-major, and the bias gradient db = column sums of G; the
+ * workspace (16-byte aligned) holds partial sums over ranges of rows. */
+size_t pcg_mlp_wgrad_workspace(int M, int K, int N);
+int pcg_mlp_wgrad(int M, int K, int N, const float *A, const float *G, float *dW, float *db, void *workspace,
+                  size_t ws_bytes, void *stream);
+/* Nonzero once a GEMM's wait has given up on this device; synchronises the stream. */
+int pcg_mlp_status(void *stream);
 int pcg_mlp_dsilu(long long n, float *dY, const float *Z, void *stream);
 int pcg_mlp_colsum(int M, int N, const float *G, float *db, void *stream);
 int pcg_mlp_mse(long long n, const float *Y, const float *T, const float *mask, float inv_count,
                 float *dY, float *loss, void *stream);
 int pcg_mlp_adam(long long n, float *w, const float *g, float *m, float *v, void *w_bf16, float lr,
                  float b1, float b2, float eps, int step, void *stream);
+/* pcg_mlp_mse with 1 / max(*count, 1) of a device value as the factor. */
+int pcg_mlp_mse_counted(long long n, const float *Y, const float *T, const float *mask, const float *count,
+                        float *dY, float *loss, void *stream);
+/* One Adam step of up to PCG_ADAM_MAX tensors in one launch (w_bf16 may be null). */
+#define PCG_ADAM_MAX 16
+typedef struct {
+  long long n[PCG_ADAM_MAX];
+  float *w[PCG_ADAM_MAX];
+  const float *g[PCG_ADAM_MAX];
+  float *m[PCG_ADAM_MAX];
+  float *v[PCG_ADAM_MAX];
+  void *w_bf16[PCG_ADAM_MAX];
+} pcg_adam_t;
+int pcg_mlp_adam_all(int ntensor, const pcg_adam_t *tensors, float lr, float b1, float b2, float eps, int step,
+                     void *stream);
 
 /* Arithmetic-throughput probe (measurement support, no upstream counterpart): blocks x
  * threads threads each run 8 independent FMA chains of `iters` steps in FP64 (fp32 = 0)

@@ -36,6 +36,14 @@ class PairsT(ctypes.Structure):
                 ("pf8", c_void_p)]
 
 
+ADAM_MAX = 16
+
+
+class AdamT(ctypes.Structure):
+    _fields_ = [("n", c_longlong * ADAM_MAX), ("w", c_void_p * ADAM_MAX), ("g", c_void_p * ADAM_MAX),
+                ("m", c_void_p * ADAM_MAX), ("v", c_void_p * ADAM_MAX), ("w_bf16", c_void_p * ADAM_MAX)]
+
+
 # name -> argtypes (all return int status unless listed in _RESTYPES)
 _SIGS = {
     "pcg_version": [],
@@ -82,6 +90,12 @@ _SIGS = {
     "pcg_fma_probe": [c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "pcg_mlp_gemm": [c_int, c_int, c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_longlong,
                      c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
+    "pcg_mlp_wgrad_workspace": [c_int, c_int, c_int],
+    "pcg_mlp_wgrad": [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_size_t, c_void_p],
+    "pcg_mlp_status": [c_void_p],
+    "pcg_mlp_mse_counted": [c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    "pcg_mlp_adam_all": [c_int, ctypes.POINTER(AdamT), ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                         c_int, c_void_p],
     "pcg_mlp_dsilu": [c_longlong, c_void_p, c_void_p, c_void_p],
     "pcg_mlp_colsum": [c_int, c_int, c_void_p, c_void_p, c_void_p],
     "pcg_mlp_mse": [c_longlong, c_void_p, c_void_p, c_void_p, ctypes.c_float, c_void_p, c_void_p, c_void_p],
@@ -113,15 +127,16 @@ _SIGS = {
 LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_schwarz_class", "pcg_expand_tasks",
              "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
              "pcg_dgemm", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
-             "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_adam",
+             "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_mse_counted", "pcg_mlp_adam", "pcg_mlp_adam_all",
              "pcg_shellpair_quantities", "pcg_two_electron_bound", "pcg_two_electron_fundamentals",
              "pcg_two_electron_vrr", "pcg_two_electron_contract", "pcg_two_electron_hrr",
              "pcg_one_electron_fundamentals", "pcg_one_electron_vrr", "pcg_one_electron_hrr",
              "pcg_one_electron_kinetic", "pcg_one_electron_contract"}
 launch_count = 0
-_RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t}
+_RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
+             "pcg_mlp_wgrad_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4}
+MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_mlp_wgrad": 2}
 
 _lib = None
 

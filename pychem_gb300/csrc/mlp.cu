@@ -1,25 +1,45 @@
 // Kernels of the learned initial-guess network: dense layers with BF16 weights and
 // FP32 accumulation, SiLU activation, masked squared-error loss and Adam.
 //
-// One tiled GEMM serves the forward pass and both backward products:
+// One tensor-core GEMM (tcgen05) serves the forward pass and both backward products:
 //   C[m][n] (+)= sum_k A(m, k) B(k, n),  A(m, k) = A[m*sam + k*sak] (FP32),
-//   B(k, n) = B[k*sbk + n*sbn] (FP32 or BF16), C row-major with ldc,
-// with an optional epilogue Z = C + bias, C = silu(Z).  64x64 output tiles, K in
-// steps of 16 through shared memory, 256 threads with a 4x4 micro-tile each.
+//   B(k, n) = B[k*sbk + n*sbn] (FP32 or BF16), C row-major with ldc.
+// FP32 operands keep all their bits: x = x0 + x1 + x2 with BF16 terms of 8 bits each (the
+// top 16 bits of x, of what is left, and the rest), so a product with a BF16 weight is three
+// exact BF16 products and one of two FP32 operands the eight with p + q <= 3 (the others are
+// below 2^-32 of it).  The tensor core truncates each FP32 partial sum, so a long chain in
+// one accumulator drifts (5e-7 of the result at K = 256, more than FP32 cores lose): the
+// leading products x0 y0 go round three accumulators in tensor memory and the corrections have
+// a fourth, added once at the end.
+//
+// A CTA owns a 128 x 64 tile; eight producer warps load 32 columns of K at a time (16-byte
+// loads where the operand is contiguous along k and aligned, coalesced along m or n where it
+// is contiguous there), split and store them K-major and 64-byte swizzled through three
+// stages, one thread issues the MMAs.  64 columns give 132 CTAs at 4,097 rows x 256, one
+// wave of the 152 SMs; the split of A is repeated for each of the 4 column tiles, which costs
+// less than idle SMs.  The weight gradient contracts over the rows: its few output tiles
+// (8 for 256 x 256) are split along the rows into partial sums, as many as fill the GPU,
+// added in a fixed order by a second kernel; the bias gradient is summed by the same producers.
+// 10,989 rows, 256 x 256: 1.5 ms with 16 CTAs of a 64 x 64 FP32-core GEMM.
 #include <cuda_bf16.h>
 #include <math.h>
 
 #include "../../include/pychem_gb300.h"
 #include "common.cuh"
 #include "pcg_internal.h"
+#include "umma.cuh"
 
-#define MT 64
-#define KT 16
+#define ML_BM 128
+#define ML_BN 64
+#define ML_BK 32
+#define ML_PROD 256
+#define ML_THREADS (ML_PROD + 32)
+#define ML_STAGES 3
+#define ML_WAIT (1u << 24)
 
-template <typename TB>
-__device__ __forceinline__ float ldb_(const TB* p) { return (float)*p; }
-template <>
-__device__ __forceinline__ float ldb_<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+// set when a wait of the GEMM gave up (its tile is then not written); read by
+// pcg_mlp_status
+static __device__ int g_mlp_err;
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + __expf(-z)); }
 __device__ __forceinline__ float dsilu(float z) {
@@ -27,63 +47,285 @@ __device__ __forceinline__ float dsilu(float z) {
   return s * (1.0f + z * (1.0f - s));
 }
 
-template <typename TB>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A, long long sam,
-                                              long long sak, const TB* __restrict__ B, long long sbk, long long sbn,
-                                              float* __restrict__ C, int ldc, int accumulate,
-                                              const float* __restrict__ bias, float* __restrict__ Z, int act) {
-  __shared__ float As[KT][MT + 4];
-  __shared__ float Bs[KT][MT + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m0 = blockIdx.y * MT, n0 = blockIdx.x * MT;
-  float acc[4][4];
+// high halves of two words as one BF16 pair (first in the low half)
+__device__ __forceinline__ unsigned pack_hi(unsigned a, unsigned b) { return __byte_perm(a, b, 0x7632); }
+
+// the three BF16 terms of eight floats; an infinity or NaN is its first term alone
+__device__ __forceinline__ void split3(const float (&x)[8], uint4 (&s)[3]) {
+  unsigned h[3][8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  for (int k0 = 0; k0 < K; k0 += KT) {
-    for (int idx = threadIdx.x; idx < KT * MT; idx += 256) {
-      // A tile: consecutive threads along m when sam == 1, else along k
-      int kk, mm;
-      if (sam == 1) { mm = idx % MT; kk = idx / MT; } else { kk = idx % KT; mm = idx / KT; }
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < K) ? A[(long long)m * sam + (long long)k * sak] : 0.0f;
-      int kb, nn;
-      if (sbn == 1) { nn = idx % MT; kb = idx / MT; } else { kb = idx % KT; nn = idx / KT; }
-      const int n = n0 + nn, k2 = k0 + kb;
-      Bs[kb][nn] = (n < N && k2 < K) ? ldb_<TB>(B + (long long)k2 * sbk + (long long)n * sbn) : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < KT; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int j = 0; j < 8; ++j) {
+    const unsigned u = __float_as_uint(x[j]);
+    const bool finite = (u & 0x7f800000u) != 0x7f800000u;
+    const unsigned quiet = !finite && (u << 9) ? 0x00400000u : 0u;     // a NaN stays one
+    const float r1 = finite ? x[j] - __uint_as_float(u & 0xffff0000u) : 0.0f;
+    const unsigned u1 = __float_as_uint(r1);
+    const float r2 = r1 - __uint_as_float(u1 & 0xffff0000u);
+    h[0][j] = u | quiet;
+    h[1][j] = u1;
+    h[2][j] = __float_as_uint(r2);
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
+  for (int p = 0; p < 3; ++p)
+    s[p] = make_uint4(pack_hi(h[p][0], h[p][1]), pack_hi(h[p][2], h[p][3]), pack_hi(h[p][4], h[p][5]),
+                      pack_hi(h[p][6], h[p][7]));
+}
+
+// eight consecutive k of one row of an operand, zero outside; vec: contiguous along k with
+// 16-byte aligned rows (k is a multiple of 8)
+__device__ __forceinline__ void load8(const float* __restrict__ p, long long sr, long long sk, long long r, long long R,
+                                      int k, int K, bool vec, float (&v)[8]) {
+  if (r < R && vec && k + 8 <= K) {
+    const float4 a = __ldg((const float4*)(p + r * sr + k)), b = __ldg((const float4*)(p + r * sr + k) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      float* c = C + (long long)m * ldc + n;
-      if (accumulate) v += *c;
-      if (bias) v += bias[n];
-      if (Z) Z[(long long)m * ldc + n] = v;
-      if (act) v = silu(v);
-      *c = v;
+    for (int j = 0; j < 8; ++j) v[j] = (r < R && k + j < K) ? __ldg(p + r * sr + (k + j) * sk) : 0.0f;
+  }
+}
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* __restrict__ p, long long sr, long long sk, long long r,
+                                       long long R, int k, int K, bool vec) {
+  const unsigned short* u = (const unsigned short*)p;
+  if (r < R && vec && k + 8 <= K) return __ldg((const uint4*)(u + r * sr + k));
+  unsigned h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = (r < R && k + j < K) ? (unsigned)__ldg(u + r * sr + (k + j) * sk) : 0u;
+  return make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+}
+
+// one item of a tile of `rows` rows x 4 groups of eight k: consecutive threads along the
+// groups of a row, or along the rows where those are contiguous in memory
+__device__ __forceinline__ void tile_item(int t, int rows, bool along_rows, int& r, int& g) {
+  if (along_rows) { r = t % rows; g = t / rows; } else { r = t >> 2; g = t & 3; }
+}
+
+template <bool BF>
+struct MlCfg {
+  static constexpr int SB = BF ? 1 : 3;            // BF16 terms of B
+  static constexpr int AT = ML_BM * ML_BK * 2;     // bytes of one term of the A tile
+  static constexpr int BT = ML_BN * ML_BK * 2;
+  static constexpr int STAGE = 3 * AT + SB * BT;
+  static constexpr int SMEM = ML_STAGES * STAGE + 2048;   // 1 KB alignment slack, barriers
+};
+
+struct MlArgs {
+  int M, N, K;
+  const float* A;
+  long long sam, sak;
+  const void* B;
+  long long sbk, sbn;
+  float* C;
+  int ldc, accumulate;
+  const float* bias;
+  float* Z;
+  int act;                 // 1: C = silu(C), pre-activation to Z; 2: C *= silu'(Z)
+  int splits;              // > 1: partial sums of a range of K to C + split * M * N, ldc = N
+  float* colsum;           // partial sums of B over k per split (wgrad), or null
+};
+
+template <bool BF>
+__global__ void __launch_bounds__(ML_THREADS, 2) k_gemm(const MlArgs a) {
+  using Cfg = MlCfg<BF>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sm = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = (uint64_t*)(sm + ML_STAGES * Cfg::STAGE);     // full[3], empty[3], done
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * ML_STAGES + 1);
+  volatile int* abort_s = (volatile int*)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ntn = (a.N + ML_BN - 1) / ML_BN;
+  const int m0 = (int)(blockIdx.x / ntn) * ML_BM, n0 = (int)(blockIdx.x % ntn) * ML_BN;
+  const int nall = (a.K + ML_BK - 1) / ML_BK;
+  const int c0 = (int)((long long)nall * blockIdx.y / a.splits), c1 = (int)((long long)nall * (blockIdx.y + 1) / a.splits);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < ML_STAGES; ++i) {
+      mbar_init(&bars[i], ML_PROD);
+      mbar_init(&bars[ML_STAGES + i], 1);
     }
+    mbar_init(&bars[2 * ML_STAGES], 1);
+    *abort_s = 0;
+    mbar_fence_init();
+  }
+  if (warp == ML_PROD / 32) tmem_alloc(tmem_slot, 4 * ML_BN);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp < ML_PROD / 32) {
+    const int t = threadIdx.x;
+    const bool a_rows = a.sam == 1 && a.sak != 1, b_rows = a.sbn == 1 && a.sbk != 1;
+    const bool a_vec = a.sak == 1 && a.sam % 4 == 0 && ((uintptr_t)a.A & 15) == 0;
+    const bool b_vec = a.sbk == 1 && a.sbn % (BF ? 8 : 4) == 0 && ((uintptr_t)a.B & 15) == 0;
+    int ra[2], ga[2], rb, gb;
+    tile_item(t, ML_BM, a_rows, ra[0], ga[0]);
+    tile_item(t + ML_PROD, ML_BM, a_rows, ra[1], ga[1]);
+    tile_item(t, ML_BN, b_rows, rb, gb);
+    float csum = 0.0f;
+    bool ok = true;
+    for (int c = c0; c < c1; ++c) {
+      const int it = c - c0, st = it % ML_STAGES, k0 = c * ML_BK;
+      float va[2][8], vb[8];
+      uint4 wb;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        load8(a.A, a.sam, a.sak, (long long)m0 + ra[u], a.M, k0 + 8 * ga[u], a.K, a_vec, va[u]);
+      if (BF) wb = load8((const __nv_bfloat16*)a.B, a.sbn, a.sbk, (long long)n0 + rb, a.N, k0 + 8 * gb, a.K, b_vec);
+      else load8((const float*)a.B, a.sbn, a.sbk, (long long)n0 + rb, a.N, k0 + 8 * gb, a.K, b_vec, vb);
+      if (it >= ML_STAGES && !mbar_wait(&bars[ML_STAGES + st], (it / ML_STAGES + 1) & 1, ML_WAIT, abort_s)) {
+        ok = false;
+        break;
+      }
+      uint8_t* at = sm + st * Cfg::STAGE;
+      uint8_t* bt = at + 3 * Cfg::AT;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint4 s[3];
+        split3(va[u], s);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *(uint4*)(at + p * Cfg::AT + sw64_offset(ra[u], ga[u])) = s[p];
+      }
+      if (BF) {
+        *(uint4*)(bt + sw64_offset(rb, gb)) = wb;
+      } else {
+        uint4 s[3];
+        split3(vb, s);
+#pragma unroll
+        for (int p = 0; p < Cfg::SB; ++p) *(uint4*)(bt + p * Cfg::BT + sw64_offset(rb, gb)) = s[p];
+        if (a.colsum) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) csum += vb[j];
+        }
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&bars[st]);
+    }
+    if (!ok) { *abort_s = 1; atomicExch(&g_mlp_err, 1); }
+    if (ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s)) {
+      tc_fence_after();
+      const int m = m0 + 32 * (warp & 3) + lane;
+      const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+      float* C = a.C + (a.splits > 1 ? (long long)blockIdx.y * a.M * a.N : 0ll);
+      const bool cvec = a.ldc % 4 == 0 && ((uintptr_t)C & 15) == 0 && (!a.Z || ((uintptr_t)a.Z & 15) == 0);
+#pragma unroll 1
+      for (int cb = 8 * (warp >> 2); cb < ML_BN; cb += 16) {
+        // the accumulators in use: three only from three K steps of 16 on
+        const int lead = min(3, (c1 - c0) * (ML_BK / 16));
+        float v[8], w[8], u[8], x3[8];
+        tmem_ld8(trow + cb, v);
+        tmem_ld8(trow + ML_BN + cb, u);
+        tmem_ld8(trow + 2 * ML_BN + cb, x3);
+        tmem_ld8(trow + 3 * ML_BN + cb, w);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          w[j] += lead > 2 ? x3[j] : 0.0f;
+          v[j] += u[j];
+        }
+        const int n = n0 + cb;
+        if (m >= a.M || n >= a.N) continue;
+        const long long o = (long long)m * a.ldc + n;
+        const bool full = cvec && n + 8 <= a.N;
+        float z[8];
+        if (a.act == 2) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) z[j] = n + j < a.N ? a.Z[o + j] : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const bool in = n + j < a.N;
+          float x = v[j] + w[j];
+          if (a.accumulate && in) x += C[o + j];
+          if (a.bias && in) x += __ldg(a.bias + n + j);
+          if (a.act == 2) x *= dsilu(z[j]);
+          else z[j] = x;
+          v[j] = a.act == 1 ? silu(x) : x;
+        }
+        if (full) {
+          if (a.Z && a.act != 2) {
+            *(float4*)(a.Z + o) = make_float4(z[0], z[1], z[2], z[3]);
+            *(float4*)(a.Z + o + 4) = make_float4(z[4], z[5], z[6], z[7]);
+          }
+          *(float4*)(C + o) = make_float4(v[0], v[1], v[2], v[3]);
+          *(float4*)(C + o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (n + j < a.N) {
+              if (a.Z && a.act != 2) a.Z[o + j] = z[j];
+              C[o + j] = v[j];
+            }
+        }
+      }
+      if (a.colsum && m0 == 0) {
+        // the MMAs have read the last tiles, so the stages are free for the four groups' sums
+        float* red = (float*)sm;
+        red[gb * ML_BN + rb] = csum;
+        asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
+        if (t < ML_BN && n0 + t < a.N)
+          a.colsum[(long long)blockIdx.y * a.N + n0 + t] =
+              (red[t] + red[ML_BN + t]) + (red[2 * ML_BN + t] + red[3 * ML_BN + t]);
+      }
+    } else {
+      *abort_s = 1;
+      atomicExch(&g_mlp_err, 1);
+      if (a.colsum && m0 == 0) asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
+    }
+  } else if (lane == 0) {
+    const uint32_t idesc = idesc_bf16_f32(ML_BM, ML_BN);
+    bool ok = true;
+    unsigned have = 0;       // accumulators that hold a sum; 3: the corrections
+    for (int it = 0; it < c1 - c0; ++it) {
+      const int st = it % ML_STAGES;
+      if (!mbar_wait(&bars[st], (it / ML_STAGES) & 1, ML_WAIT, abort_s)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t xa = smem_u32(sm + st * Cfg::STAGE), xb = xa + 3 * Cfg::AT;
+#pragma unroll
+      for (int kk = 0; kk < ML_BK / 16; ++kk) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int q = 0; q < Cfg::SB; ++q) {
+            if (p + q > 3) continue;
+            const int acc = p + q == 0 ? (it * (ML_BK / 16) + kk) % 3 : 3;
+            umma_bf16(tmem + acc * ML_BN, sdesc_k_sw64(xa + p * Cfg::AT + kk * 32),
+                      sdesc_k_sw64(xb + q * Cfg::BT + kk * 32), idesc, (have >> acc) & 1u);
+            have |= 1u << acc;
+          }
+      }
+      umma_commit(&bars[ML_STAGES + st]);
+    }
+    umma_commit(&bars[2 * ML_STAGES]);
+    if (!ok) {
+      *abort_s = 1;
+      atomicExch(&g_mlp_err, 2);
+      volatile int keep_waiting = 0;
+      mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, &keep_waiting);   // drain before tensor memory is freed
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == ML_PROD / 32) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem, 4 * ML_BN);
+  }
+}
+
+// dW = sum of the partial products, db = sum of the partial column sums, splits in order
+__global__ void k_wgrad_sum(long long len, int N, int splits, const float* __restrict__ part,
+                            const float* __restrict__ cpart, float* __restrict__ dW, float* __restrict__ db) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < len) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) s += __ldg(part + k * len + i);
+    dW[i] = s;
+  } else if (i < len + N) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) s += __ldg(cpart + (long long)k * N + (i - len));
+    db[i - len] = s;
   }
 }
 
@@ -93,37 +335,55 @@ __global__ void k_dsilu(long long n, float* __restrict__ dY, const float* __rest
   if (i < n) dY[i] *= dsilu(Z[i]);
 }
 
-// column sums: db[n] = sum_m G[m][n]
-__global__ void k_colsum(int M, int N, const float* __restrict__ G, float* __restrict__ db) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
+// column sums: db[n] = sum_m G[m][n]; one block per 32 columns, 32 rows at a time
+__global__ void __launch_bounds__(1024) k_colsum(int M, int N, const float* __restrict__ G, float* __restrict__ db) {
+  __shared__ float red[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, n = blockIdx.x * 32 + tx;
   float s = 0.0f;
-  for (int m = 0; m < M; ++m) s += G[(long long)m * N + n];
-  db[n] = s;
+  if (n < N)
+    for (int m = ty; m < M; m += 32) s += __ldg(G + (long long)m * N + n);
+  red[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && n < N) {
+    float t = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) t += red[k][tx];
+    db[n] = t;
+  }
 }
 
-// masked squared error: loss partial sums and dY = 2 (Y - T) mask / count
-__global__ void k_mse(long long n, const float* __restrict__ Y, const float* __restrict__ T,
-                      const float* __restrict__ mask, float inv_count, float* __restrict__ dY,
-                      float* __restrict__ loss) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// masked squared error: loss partial sums and dY = 2 (Y - T) mask / count, count from
+// *cnt (a device value) when given.  One atomic per block.
+__global__ void __launch_bounds__(256) k_mse(long long n, const float* __restrict__ Y, const float* __restrict__ T,
+                                             const float* __restrict__ mask, float inv_count,
+                                             const float* __restrict__ cnt, float* __restrict__ dY,
+                                             float* __restrict__ loss) {
+  const float inv = cnt ? (float)(1.0 / fmax((double)*cnt, 1.0)) : inv_count;
   float l = 0.0f;
-  if (i < n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float d = (Y[i] - T[i]) * mask[i];
-    dY[i] = 2.0f * d * inv_count;
-    l = d * d * inv_count;
+    dY[i] = 2.0f * d * inv;
+    l += d * d * inv;
   }
   for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
+  __shared__ float red[8];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) l += red[k];
+    atomicAdd(loss, l);
+  }
 }
 
-// Adam on FP32 master weights, refreshing the BF16 copy used by the GEMMs
-__global__ void k_adam(long long n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
+// Adam on FP32 master weights, refreshing the BF16 copy used by the GEMMs; all tensors of
+// a network in one launch (blockIdx.y: the tensor)
+__global__ void k_adam(pcg_adam_t ts, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int k = blockIdx.y;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
+  if (i >= ts.n[k]) return;
+  float *w = ts.w[k], *m = ts.m[k], *v = ts.v[k];
+  __nv_bfloat16* wb = (__nv_bfloat16*)ts.w_bf16[k];
+  const float gi = ts.g[k][i];
   const float mi = b1 * m[i] + (1.0f - b1) * gi;
   const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
   m[i] = mi;
@@ -133,20 +393,63 @@ __global__ void k_adam(long long n, float* __restrict__ w, const float* __restri
   if (wb) wb[i] = __float2bfloat16_rn(wi);
 }
 
+template <bool BF>
+static int run_gemm(const MlArgs& a, cudaStream_t s) {
+  const long long tiles = (long long)((a.M + ML_BM - 1) / ML_BM) * ((a.N + ML_BN - 1) / ML_BN);
+  if (tiles > 0x7fffffffLL) { pcg_set_error("pcg_mlp_gemm: too many tiles for one launch"); return PCG_ERR_UNSUPPORTED; }
+  PCG_CUDA(cudaFuncSetAttribute(k_gemm<BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, MlCfg<BF>::SMEM));
+  k_gemm<BF><<<dim3((unsigned)tiles, a.splits), ML_THREADS, MlCfg<BF>::SMEM, s>>>(a);
+  PCG_CUDA(cudaGetLastError());
+  return PCG_OK;
+}
+
 extern "C" int pcg_mlp_gemm(int M, int N, int K, const float* A, long long sam, long long sak, const void* B,
                             int b_bf16, long long sbk, long long sbn, float* C, int ldc, int accumulate,
                             const float* bias, float* Z, int act, void* stream) {
-  if (M < 1 || N < 1 || K < 1 || !A || !B || !C) { pcg_set_error("pcg_mlp_gemm: bad arguments"); return PCG_ERR_ARG; }
-  dim3 grid((N + MT - 1) / MT, (M + MT - 1) / MT);
-  cudaStream_t s = (cudaStream_t)stream;
-  if (b_bf16)
-    k_gemm<__nv_bfloat16><<<grid, 256, 0, s>>>(M, N, K, A, sam, sak, (const __nv_bfloat16*)B, sbk, sbn, C, ldc,
-                                               accumulate, bias, Z, act);
-  else
-    k_gemm<float><<<grid, 256, 0, s>>>(M, N, K, A, sam, sak, (const float*)B, sbk, sbn, C, ldc, accumulate, bias, Z,
-                                       act);
+  if (M < 1 || N < 1 || K < 1 || !A || !B || !C || (act == 2 && !Z)) {
+    pcg_set_error("pcg_mlp_gemm: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  const MlArgs a = {M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, accumulate, bias, Z, act, 1, nullptr};
+  return b_bf16 ? run_gemm<true>(a, (cudaStream_t)stream) : run_gemm<false>(a, (cudaStream_t)stream);
+}
+
+// row splits of the weight gradient: two CTAs an SM, but at least four 32-row steps each
+static int wgrad_splits(int M, int K, int N) {
+  const long long tiles = (long long)((K + ML_BM - 1) / ML_BM) * ((N + ML_BN - 1) / ML_BN);
+  const long long most = (M + 4 * ML_BK - 1) / (4 * ML_BK), want = (2 * 152 + tiles - 1) / tiles;
+  const long long k = want < most ? want : most;
+  return k < 1 ? 1 : (int)k;
+}
+
+extern "C" size_t pcg_mlp_wgrad_workspace(int M, int K, int N) {
+  if (M < 1 || K < 1 || N < 1) return 0;
+  return (size_t)wgrad_splits(M, K, N) * ((size_t)K * N + N) * sizeof(float);
+}
+
+extern "C" int pcg_mlp_wgrad(int M, int K, int N, const float* A, const float* G, float* dW, float* db, void* workspace,
+                             size_t ws_bytes, void* stream) {
+  if (M < 1 || K < 1 || N < 1 || !A || !G || !dW || !db) { pcg_set_error("pcg_mlp_wgrad: bad arguments"); return PCG_ERR_ARG; }
+  if (!workspace || ((size_t)workspace & 15) || ws_bytes < pcg_mlp_wgrad_workspace(M, K, N)) {
+    pcg_set_error("pcg_mlp_wgrad: workspace missing, misaligned or too small (query pcg_mlp_wgrad_workspace)");
+    return PCG_ERR_CAPACITY;
+  }
+  const int splits = wgrad_splits(M, K, N);
+  const long long len = (long long)K * N;
+  float* part = (float*)workspace;
+  float* cpart = part + splits * len;
+  MlArgs a = {K, N, M, A, 1, K, G, N, 1, part, N, 0, nullptr, nullptr, 0, splits, cpart};
+  if (int rc = run_gemm<false>(a, (cudaStream_t)stream)) return rc;
+  k_wgrad_sum<<<(unsigned)((len + N + 255) / 256), 256, 0, (cudaStream_t)stream>>>(len, N, splits, part, cpart, dW, db);
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
+}
+
+extern "C" int pcg_mlp_status(void* stream) {
+  int h = 0;
+  PCG_CUDA(cudaMemcpyFromSymbolAsync(&h, g_mlp_err, sizeof(int), 0, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  PCG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  return h;
 }
 
 extern "C" int pcg_mlp_dsilu(long long n, float* dY, const float* Z, void* stream) {
@@ -156,23 +459,47 @@ extern "C" int pcg_mlp_dsilu(long long n, float* dY, const float* Z, void* strea
 }
 
 extern "C" int pcg_mlp_colsum(int M, int N, const float* G, float* db, void* stream) {
-  k_colsum<<<(N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(M, N, G, db);
+  k_colsum<<<(N + 31) / 32, 1024, 0, (cudaStream_t)stream>>>(M, N, G, db);
+  PCG_CUDA(cudaGetLastError());
+  return PCG_OK;
+}
+
+static int run_mse(long long n, const float* Y, const float* T, const float* mask, float inv_count, const float* cnt,
+                   float* dY, float* loss, cudaStream_t s) {
+  const long long blocks = (n + 1023) / 1024;
+  k_mse<<<(unsigned)(blocks < 1 ? 1 : (blocks < 608 ? blocks : 608)), 256, 0, s>>>(n, Y, T, mask, inv_count, cnt, dY, loss);
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
 }
 
 extern "C" int pcg_mlp_mse(long long n, const float* Y, const float* T, const float* mask, float inv_count,
                            float* dY, float* loss, void* stream) {
-  k_mse<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(n, Y, T, mask, inv_count, dY, loss);
+  return run_mse(n, Y, T, mask, inv_count, nullptr, dY, loss, (cudaStream_t)stream);
+}
+
+extern "C" int pcg_mlp_mse_counted(long long n, const float* Y, const float* T, const float* mask, const float* count,
+                                   float* dY, float* loss, void* stream) {
+  if (!count) { pcg_set_error("pcg_mlp_mse_counted: no count"); return PCG_ERR_ARG; }
+  return run_mse(n, Y, T, mask, 0.0f, count, dY, loss, (cudaStream_t)stream);
+}
+
+extern "C" int pcg_mlp_adam_all(int ntensor, const pcg_adam_t* tensors, float lr, float b1, float b2, float eps,
+                                int step, void* stream) {
+  if (ntensor < 1 || ntensor > PCG_ADAM_MAX || !tensors) {
+    pcg_set_error("pcg_mlp_adam_all: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  long long most = 1;
+  for (int k = 0; k < ntensor; ++k) most = tensors->n[k] > most ? tensors->n[k] : most;
+  const float c1 = 1.0f / (1.0f - powf(b1, (float)step)), c2 = 1.0f / (1.0f - powf(b2, (float)step));
+  k_adam<<<dim3((unsigned)((most + 255) / 256), ntensor), 256, 0, (cudaStream_t)stream>>>(*tensors, lr, b1, b2, eps, c1, c2);
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
 }
 
 extern "C" int pcg_mlp_adam(long long n, float* w, const float* g, float* m, float* v, void* w_bf16, float lr,
                             float b1, float b2, float eps, int step, void* stream) {
-  const float c1 = 1.0f / (1.0f - powf(b1, (float)step)), c2 = 1.0f / (1.0f - powf(b2, (float)step));
-  k_adam<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(n, w, g, m, v, (__nv_bfloat16*)w_bf16, lr,
-                                                                        b1, b2, eps, c1, c2);
-  PCG_CUDA(cudaGetLastError());
-  return PCG_OK;
+  pcg_adam_t t = {};
+  t.n[0] = n; t.w[0] = w; t.g[0] = g; t.m[0] = m; t.v[0] = v; t.w_bf16[0] = w_bf16;
+  return pcg_mlp_adam_all(1, &t, lr, b1, b2, eps, step, stream);
 }

@@ -69,46 +69,51 @@ class PairMLP:
         """Gradients (dW, db) per layer for output gradient dY (M, NPARAM)."""
         M = dY.shape[0]
         G = dY.contiguous()
+        lib = _lib.load()
+        ws = torch.empty(max(lib.pcg_mlp_wgrad_workspace(M, k, n) for k, n in zip(self.dims, self.dims[1:])),
+                         dtype=torch.uint8, device=self.dev)
         grads = [None] * self.nlayers
         for k in reversed(range(self.nlayers)):
             K, N = self.dims[k], self.dims[k + 1]
-            A, Z = cache[k]
-            if Z is not None:
-                _lib.call("pcg_mlp_dsilu", M * N, _p(G), _p(Z), _s())
+            A = cache[k][0]
             dW = torch.empty(K, N, dtype=torch.float32, device=self.dev)
-            _lib.call("pcg_mlp_gemm", K, N, M, _p(A), 1, K, _p(G), 0, N, 1, _p(dW), N, 0, None, None, 0, _s())
             db = torch.empty(N, dtype=torch.float32, device=self.dev)
-            _lib.call("pcg_mlp_colsum", M, N, _p(G), _p(db), _s())
+            _lib.call("pcg_mlp_wgrad", M, K, N, _p(A), _p(G), _p(dW), _p(db), _p(ws), ws.numel(), _s())
             grads[k] = (dW, db)
             if k > 0:
+                # dA, times the derivative of the activation below it
+                Z = cache[k - 1][1]
                 dA = torch.empty(M, K, dtype=torch.float32, device=self.dev)
-                _lib.call("pcg_mlp_gemm", M, K, N, _p(G), N, 1, _p(self.Wb[k]), 1, 1, N, _p(dA), K, 0, None, None, 0,
-                          _s())
+                _lib.call("pcg_mlp_gemm", M, K, N, _p(G), N, 1, _p(self.Wb[k]), 1, 1, N, _p(dA), K, 0, None, _p(Z),
+                          2 if Z is not None else 0, _s())
                 G = dA
         return grads
 
     def loss_grad(self, Y, T, mask):
         n = Y.numel()
-        cnt = float(mask.sum())
         dY = torch.empty_like(Y)
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
-        _lib.call("pcg_mlp_mse", n, _p(Y), _p(T), _p(mask), ctypes.c_float(1.0 / max(cnt, 1.0)), _p(dY), _p(loss),
-                  _s())
+        count = mask.sum()
+        _lib.call("pcg_mlp_mse_counted", n, _p(Y), _p(T), _p(mask), _p(count), _p(dY), _p(loss), _s())
         return loss, dY
 
     def adam(self, grads, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1
+        rows = []
         for k, (dW, db) in enumerate(grads):
-            _lib.call("pcg_mlp_adam", self.W[k].numel(), _p(self.W[k]), _p(dW), _p(self.mW[k]), _p(self.vW[k]),
-                      _p(self.Wb[k]), ctypes.c_float(lr), ctypes.c_float(b1), ctypes.c_float(b2), ctypes.c_float(eps),
-                      self.step_count, _s())
-            _lib.call("pcg_mlp_adam", self.b[k].numel(), _p(self.b[k]), _p(db), _p(self.mb[k]), _p(self.vb[k]), None,
-                      ctypes.c_float(lr), ctypes.c_float(b1), ctypes.c_float(b2), ctypes.c_float(eps), self.step_count,
-                      _s())
+            rows.append((self.W[k], dW, self.mW[k], self.vW[k], self.Wb[k]))
+            rows.append((self.b[k], db, self.mb[k], self.vb[k], None))
+        for first in range(0, len(rows), _lib.ADAM_MAX):
+            part = rows[first:first + _lib.ADAM_MAX]
+            t = _lib.AdamT()
+            for j, (w, g, m, v, wb) in enumerate(part):
+                t.n[j], t.w[j], t.g[j], t.m[j], t.v[j] = w.numel(), w.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr()
+                t.w_bf16[j] = wb.data_ptr() if wb is not None else None
+            _lib.call("pcg_mlp_adam_all", len(part), ctypes.byref(t), lr, b1, b2, eps, self.step_count, _s())
 
     def predict(self, X):
         Y, _ = self.forward(X)
-        return Y * self.std + self.mean
+        return torch.addcmul(self.mean, Y, self.std)
 
     def state(self):
         d = {"dims": np.array(self.dims), "mean": self.mean.cpu().numpy(), "std": self.std.cpu().numpy()}
