@@ -196,6 +196,24 @@ int pcg_eri_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pa
 int pcg_schwarz_class(int cls, const int *tasks, int ntask, const double *store, double *Q,
                       void *stream);
 
+/* Screened canonical quartet lists of all classes (Methods/hartree_fock.py:241-312).  The
+ * pairs in order[] are sorted by (kind, molecule, A, B); kind k starts at position kind0[k],
+ * the pairs of kind k and molecule m at seg0[k * nmol + m] (seg0 has nkind * nmol + 1
+ * entries), mol[] by position.  Bucket b pairs bra kind bra_kind[b] with ket_kind[b] <= it;
+ * its rows, one per bra pair, start at row0[b].  Qs: Schwarz factors by position.  A row holds the kets
+ * with Q_bra Q_ket > thr (within one kind those up to the bra, and always the bra itself); with
+ * thr32 > 0 those at or below thr32 form a second, FP32 part.
+ * pcg_plan_count: cnt[0] = 0, cnt[r + 1] = tasks of row r, then cnt[nrow + r + 1] those of the FP32
+ * part when thr32 > 0.  pcg_plan_fill: the tasks {bra pair, ket pair} at the inclusive
+ * prefix sums off of cnt (off[r], and off[nrow + r] for the FP32 part). */
+typedef struct {
+  long long nrow;
+  int nbucket, nmol;
+  const int *row0, *bra_kind, *ket_kind, *kind0, *seg0, *order, *mol;
+} pcg_plan_t;
+int pcg_plan_count(const pcg_plan_t *plan, const double *Qs, double thr, double thr32, long long *cnt, void *stream);
+int pcg_plan_fill(const pcg_plan_t *plan, const double *Qs, double thr, double thr32, const long long *off, int *tasks,
+                  void *stream);
 /* Expand screened quartet rows into task pairs: row r pairs bra pair bra[r] with the
  * kets ket[qstart[r] + q] for q < off[r+1] - off[r] - diag[r], and with itself last
  * when diag[r]; its tasks are written at [off[r], off[r+1]) of out_tasks (int2). */

@@ -36,6 +36,12 @@ class PairsT(ctypes.Structure):
                 ("pf8", c_void_p)]
 
 
+class PlanT(ctypes.Structure):
+    _fields_ = [("nrow", c_longlong), ("nbucket", c_int), ("nmol", c_int), ("row0", c_void_p), ("bra_kind", c_void_p),
+                ("ket_kind", c_void_p), ("kind0", c_void_p), ("seg0", c_void_p), ("order", c_void_p),
+                ("mol", c_void_p)]
+
+
 ADAM_MAX = 16
 
 
@@ -71,6 +77,8 @@ _SIGS = {
     "pcg_eri_class_split": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_int, c_void_p,
                             c_int, c_void_p],
     "pcg_schwarz_class": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
+    "pcg_plan_count": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p],
+    "pcg_plan_fill": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p, c_void_p],
     "pcg_expand_tasks": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p],
     "pcg_digest_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
                          c_void_p, c_void_p, c_void_p],
@@ -124,7 +132,7 @@ _SIGS = {
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
 }
 # entry points that launch exactly one kernel of this library per call
-LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_schwarz_class", "pcg_expand_tasks",
+LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_schwarz_class", "pcg_plan_count", "pcg_plan_fill", "pcg_expand_tasks",
              "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
              "pcg_dgemm", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
              "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_mse_counted", "pcg_mlp_adam", "pcg_mlp_adam_all",

@@ -44,9 +44,10 @@ def pair_colmap(n, pmap, device):
     return cm
 
 
-def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None, info=None):
-    """Screened canonical quartet plan (Methods/hartree_fock.py:241-312: the quartet
-    loop, the Schwarz test Q_ab Q_cd > threshold, and the diagonal quartet that is
+def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None):
+    """The screened canonical quartet plan in tensor operations, the reference that the
+    planner's kernels (pcg_plan_count, pcg_plan_fill) are checked against
+    (Methods/hartree_fock.py:241-312: the quartet loop, the Schwarz test Q_ab Q_cd > threshold, and the diagonal quartet that is
     always computed), with tensor operations on Q's device.
 
     Q, kind, mol: per shell pair its Schwarz factor, kind index (kinds ordered by
@@ -66,8 +67,7 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None, i
     the diagonal flag; row r covers tasks [off[r], off[r+1]).  With kind_work (work
     per pair of each kind, e.g. its primitive-pair count) the buckets run in
     decreasing work per quartet, so a launch's heaviest CTAs start first and the light
-    ones fill its tail.  info (a dict) receives per (class, part) the number of tasks and
-    of those, a prefix, whose work is at least HEAVY (0 without kind_work)."""
+    ones fill its tail."""
     dev = Q.device
     nk = int(class_table.shape[0])
     o = torch.sort(-Q, stable=True).indices
@@ -87,7 +87,6 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None, i
         key = (int(w.max()) - w) * (nk * nk * npair) + key
     ro = torch.sort(key).indices
     pos, kk, kb = pos[ro], kk[ro], kb[ro]
-    heavy = (w[ro] >= HEAVY).to(torch.int64) if kind_work is not None else torch.zeros_like(pos)
     qb = Qs[pos]
     key = kk * nmol + ms[pos]
     lo = torch.searchsorted(seg_key, key, right=False)
@@ -124,24 +123,19 @@ def plan_quartets(Q, kind, mol, nmol, class_table, thr, thr32, kind_work=None, i
     plan = []
     ncls = int(class_table.max()) + 1 if class_table.numel() else 0
     for part, n, qs, dg in (("64", c64 + diag, lo, diag), ("32", cnt - c64, lo + c64, torch.zeros_like(diag))):
-        # rows grouped by class (a stable sort keeps each class's rows in order); the class
-        # sizes, tasks and heavy tasks read back once per part
+        # rows grouped by class (a stable sort keeps each class's rows in order), the
+        # class sizes read back once per part
         key = torch.where(n > 0, cls_row, torch.full_like(cls_row, ncls))
         order = torch.sort(key, stable=True).indices
-        cols = [torch.bincount(key, minlength=ncls + 1)]
-        cols += [torch.bincount(key, weights=x.to(torch.float64), minlength=ncls + 1).to(torch.int64)
-                 for x in (n, n * heavy)]
-        counts, tasks, heavies = torch.stack(cols).tolist()
+        counts = torch.bincount(key, minlength=ncls + 1)[:ncls].tolist()
         start = 0
-        for cls, c in enumerate(counts[:ncls]):
+        for cls, c in enumerate(counts):
             if c == 0:
                 continue
             sel = order[start:start + c]
             start += c
             off = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), torch.cumsum(n[sel], 0)])
             plan.append((cls, part, bra[sel], off, qs[sel], dg[sel]))
-            if info is not None:
-                info[(cls, part)] = (tasks[cls], heavies[cls])
     return plan, o
 
 
@@ -259,6 +253,7 @@ class GpuEngine:
         uniq, inv = np.unique(pc * mb + npp, return_inverse=True)
         self.kinds = [(int(c // mb), int(c % mb)) for c in uniq]
         self.pair_kind = np.asarray(inv).ravel().astype(np.int32)
+        self._plan_tables = None
 
     def compute_pair_data(self):
         """Primitive-pair data of every pair, the negligible primitive pairs dropped
@@ -337,42 +332,72 @@ class GpuEngine:
         return Q
 
     # ---------------------------------------------------------------------------------
-    def _pair_molecule(self):
-        """Molecule index of every shell pair (device int64) and the molecule count."""
-        return torch.zeros(self.npair, dtype=torch.int64, device=self.dev), 1
+    def _pair_molecules_host(self):
+        """Molecule index of every shell pair and the molecule count."""
+        return np.zeros(self.npair, dtype=np.int64), 1
+
+    def _plan(self):
+        """Tables of the quartet planner (pcg_plan_t): the pairs sorted by (kind, molecule,
+        A, B), and the buckets (bra kind, ket kind <= it) sorted by (class, decreasing
+        primitive quartets per task, bra kind, ket kind).  They follow from the pairs and
+        their kept primitives, not from the Schwarz factors.  Returns the struct and per
+        class its rows (first, end of the tasks of HEAVY or more, end)."""
+        if self._plan_tables is not None:
+            return self._plan_tables
+        nk = len(self.kinds)
+        kind = self.pair_kind.astype(np.int64)
+        mol, nmol = self._pair_molecules_host()
+        order = np.lexsort((self.h_pairs["B"], self.h_pairs["A"], mol, kind))
+        key = (kind * nmol + mol)[order]
+        seg0 = np.searchsorted(key, np.arange(nk * nmol + 1))
+        kind0 = seg0[::nmol]
+        pc, npp = np.array(self.kinds, dtype=np.int64).T
+        kb, kk = np.tril_indices(nk)
+        cls = pc[kb] * (pc[kb] + 1) // 2 + pc[kk]
+        work = npp[kb] * npp[kk]
+        o = np.lexsort((kk, kb, -work, cls))
+        kb, kk, cls, work = kb[o], kk[o], cls[o], work[o]
+        row0 = np.concatenate([[0], np.cumsum(np.diff(kind0)[kb])])
+        rows = {}
+        for c in np.unique(cls):
+            lo, hi = np.searchsorted(cls, [c, c + 1])
+            rows[int(c)] = (int(row0[lo]), int(row0[lo + np.count_nonzero(work[lo:hi] >= HEAVY)]), int(row0[hi]))
+        if row0[-1] > 0x7fffffff:
+            raise _lib.PcgError("too many rows for the quartet planner")
+        tabs = [x.astype(np.int32) for x in (row0, kb, kk, kind0, seg0, order, mol[order])]
+        buf = self._t(np.concatenate(tabs))
+        t = _lib.PlanT()
+        t.nrow, t.nbucket, t.nmol = int(row0[-1]), len(kb), nmol
+        at = 0
+        for name, x in zip(("row0", "bra_kind", "ket_kind", "kind0", "seg0", "order", "mol"), tabs):
+            setattr(t, name, buf.data_ptr() + 4 * at)
+            at += len(x)
+        self._plan_tables = (t, rows, buf, buf[at - 2 * len(order):at - len(order)])
+        return self._plan_tables
 
     def build_tasks(self):
-        """Screened canonical quartet lists per class and precision part, planned on the
-        GPU by plan_quartets() and expanded by the library (one launch per class and
-        part)."""
-        dev = self.dev
-        nk = len(self.kinds)
-        order = np.argsort(self.pair_kind, kind="stable")
-        first = order[np.searchsorted(self.pair_kind[order], np.arange(nk))]
-        kl = np.stack([self.h_pairs["lA"][first], self.h_pairs["lB"][first]], axis=1)
-        ct = np.full((nk, nk), -1, dtype=np.int64)
-        lib = _lib.load()
-        for i in range(nk):
-            for j in range(i + 1):
-                ct[i, j] = lib.pcg_eri_class_id(int(kl[i, 0]), int(kl[i, 1]), int(kl[j, 0]), int(kl[j, 1]))
-        mol, nmol = self._pair_molecule()
-        work = torch.as_tensor([k[1] for k in self.kinds], dtype=torch.int64, device=dev)
-        info = {}
-        plan, ket_list = plan_quartets(self.Q, torch.as_tensor(self.pair_kind, dtype=torch.int64, device=dev), mol,
-                                       nmol, torch.as_tensor(ct, device=dev), float(self.threshold),
-                                       float(self.fp32_below), kind_work=work, info=info)
-        ket32 = ket_list.to(torch.int32)
-        self.classes = {}
-        self.heavy = {key: heavy for key, (_, heavy) in info.items()}
-        for cls, part, bra, off, qs, dg in plan:
-            total = info[(cls, part)][0]
-            tasks = torch.empty(int(total) * 2, dtype=torch.int32, device=dev)
-            # named so that the int32 copies outlive the launch that reads them
-            bra32, qs32, dg32 = bra.to(torch.int32), qs.to(torch.int32), dg.to(torch.int32)
-            _lib.call("pcg_expand_tasks", bra.numel(), _ptr(bra32), _ptr(ket32), _ptr(off), _ptr(qs32), _ptr(dg32),
-                      int(total), _ptr(tasks), _stream())
-            self.classes.setdefault(cls, {})[part] = (tasks, int(total))
-        self.classes = dict(sorted(self.classes.items()))
+        """Screened canonical quartet lists per class and precision part (pcg_plan_count,
+        one prefix sum over the rows, pcg_plan_fill); the class boundaries are read back
+        once."""
+        plan, rows, _, order = self._plan()
+        thr, thr32 = float(self.threshold), float(self.fp32_below)
+        parts = 2 if thr32 > 0 else 1
+        n = plan.nrow
+        Qs = self.Q[order]
+        cnt = torch.empty(parts * n + 1, dtype=torch.int64, device=self.dev)
+        _lib.call("pcg_plan_count", ctypes.byref(plan), _ptr(Qs), thr, thr32, _ptr(cnt), _stream())
+        off = torch.cumsum(cnt, 0)
+        at = np.array([[p * n + r for r in rows[c]] for p in range(parts) for c in rows])
+        ends = off[self._t(at)].tolist()
+        total = ends[-1][2]
+        tasks = torch.empty(2 * total, dtype=torch.int32, device=self.dev)
+        _lib.call("pcg_plan_fill", ctypes.byref(plan), _ptr(Qs), thr, thr32, _ptr(off), _ptr(tasks), _stream())
+        self.classes, self.heavy = {}, {}
+        for part, lists in zip(("64", "32"), (ends[:len(rows)], ends[len(rows):])):
+            for cls, (lo, heavy, hi) in zip(rows, lists):
+                if hi > lo:
+                    self.classes.setdefault(cls, {})[part] = (tasks[2 * lo:2 * hi], hi - lo)
+                    self.heavy[(cls, part)] = heavy - lo
         self._task_stats()
         return self.classes
 

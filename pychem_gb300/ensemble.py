@@ -137,10 +137,8 @@ class EnsembleEngine(GpuEngine):
         self.S, self.H = S, H
         return S, H
 
-    def _pair_molecule(self):
-        if getattr(self, "_pair_mol_dev", None) is None:
-            self._pair_mol_dev = torch.as_tensor(self.pair_mol, dtype=torch.int64, device=self.dev)
-        return self._pair_mol_dev, self.B
+    def _pair_molecules_host(self):
+        return self.pair_mol.astype(np.int64), self.B
 
     # ---------------------------------------------------------------------------------
     def fock(self, D, out=None, G=None):
