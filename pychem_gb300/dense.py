@@ -14,14 +14,11 @@ import math
 import torch
 
 from . import _lib
+from ._stream import stream as _stream
 
 
 def _p(t):
     return ctypes.c_void_p(t.data_ptr())
-
-
-def _s():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _mat(t, trans):
@@ -46,7 +43,7 @@ def mm(A, B, ta=False, tb=False, out=None, alpha=1.0, beta=0.0):
         beta = 0.0
     sCb = out.stride(0) if out.dim() == 3 else 0
     _lib.call("pcg_dgemm", batch, M, N, K, float(alpha), _p(A), sAb, sAm, sAk, _p(B), sBb, sBk, sBn, float(beta),
-              _p(out), sCb, out.stride(-2), out.stride(-1), _s())
+              _p(out), sCb, out.stride(-2), out.stride(-1), _stream())
     return out
 
 
@@ -55,7 +52,7 @@ def oa_correction(S, R, nocc, mode, delta=None, E=None, lam=None):
     n = S.shape[0]
     E = torch.empty_like(S) if E is None else E
     _lib.call("pcg_oa_correction", n, nocc, mode, _p(delta) if delta is not None else None, _p(S), _p(R), _p(E),
-              _p(lam) if lam is not None else None, _s())
+              _p(lam) if lam is not None else None, _stream())
     return E
 
 
@@ -104,5 +101,5 @@ class DeviceDIIS:
     def step(self, F, R, Fx):
         """Store (F, R), solve, write the extrapolated Fock matrix into Fx."""
         _lib.call("pcg_diis_step", self.len, self.cap, _p(self.state), _p(F), _p(R), _p(self.focks), _p(self.resids),
-                  _p(self.Bm), _p(self.row), _p(self.coef), _p(Fx), _s())
+                  _p(self.Bm), _p(self.row), _p(self.coef), _p(Fx), _stream())
         return Fx

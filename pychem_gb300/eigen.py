@@ -18,15 +18,12 @@ import ctypes
 import torch
 
 from . import _lib, dense
+from ._stream import stream as _stream
 
 FP64_JACOBI_MAX_N = 136
 
 # counts of eigh calls by route (exact library solve, refinement, refinement rejected)
 stats = {"exact": 0, "refined": 0, "fallback": 0}
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def jacobi(A, fp32=False, max_sweeps=40, tol=None):

@@ -15,6 +15,7 @@ import torch
 
 from . import _lib
 from ._lib import BasisT, PairsT
+from ._stream import stream as _stream
 
 INTEGRAL_THRESHOLD = 1.0e-8   # Data/constants.py:31
 N_SPHER = [1, 3, 5]
@@ -26,10 +27,6 @@ HEAVY = 128
 
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else ctypes.c_void_p(0)
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def pair_class(la, lb):
@@ -518,11 +515,14 @@ class GpuEngine:
             sp = np.empty(nao2, dtype=np.int64)
             sp[(hi * (hi + 1) // 2 + lo)[ok]] = np.broadcast_to(np.arange(self.npair)[:, None], ok.shape)[ok]
             self._ao_shell_pair = (self.h_pairs, torch.as_tensor(sp, device=self.dev))
-        # shell pairs in some off-diagonal stored quartet (pcg_mark_pairs), no host round trip
-        used = torch.zeros(self.npair, dtype=torch.bool, device=self.dev)
-        for rec in self.classes.values():
-            for tasks, ntask in rec.values():
-                _lib.call("pcg_mark_pairs", _ptr(tasks), ntask, _ptr(used), _stream())
+        # a pair is in some off-diagonal stored quartet when its product with the largest
+        # Schwarz factor of the other pairs passes the screen (products are monotone)
+        if self.npair > 1:
+            top, at = torch.topk(self.Q, 2)
+            other = torch.where(torch.arange(self.npair, device=self.dev) == at[0], top[1], top[0])
+            used = self.Q * other > float(self.threshold)
+        else:
+            used = torch.zeros(1, dtype=torch.bool, device=self.dev)
         flag = used[self._ao_shell_pair[1]]
         rank = torch.cumsum(flag, 0, dtype=torch.int32)
         pmap = torch.where(flag, rank - 1, -1).to(torch.int32)

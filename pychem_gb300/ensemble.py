@@ -17,7 +17,8 @@ import torch
 
 from . import _lib, eigen
 from ._lib import BasisT
-from .engine import GpuEngine, _ptr, _stream, pair_class
+from ._stream import stream as _stream
+from .engine import GpuEngine, _ptr
 from .scf import SCFResult, diis_coefficients_batched
 
 PAD_DIAG = 1.0e3
@@ -35,28 +36,23 @@ class EnsembleEngine(GpuEngine):
     # ---------------------------------------------------------------------------------
     def _upload_basis(self):
         arrs = [m.arrays() for m in self.mols]
-        nsh = [len(a["sh_l"]) for a in arrs]
-        npr = [len(a["pr_exp"]) for a in arrs]
-        nat = [len(a["at_z"]) for a in arrs]
-        sh_off = np.concatenate([[0], np.cumsum(nsh)[:-1]])
-        pr_off = np.concatenate([[0], np.cumsum(npr)[:-1]])
-        at_off = np.concatenate([[0], np.cumsum(nat)[:-1]])
-        n2 = self.nmax * self.nmax
+        nsh = np.array([len(a["sh_l"]) for a in arrs])
+        npr = np.array([len(a["pr_exp"]) for a in arrs])
+        nat = np.array([len(a["at_z"]) for a in arrs])
+        sh_off, pr_off, at_off = (np.cumsum(k) - k for k in (nsh, npr, nat))
+        mols = np.arange(self.B)
+
+        def cat(name):
+            return np.concatenate([x[name] for x in arrs])
+
         a = dict(
-            sh_l=np.concatenate([x["sh_l"] for x in arrs]).astype(np.int32),
-            sh_nprim=np.concatenate([x["sh_nprim"] for x in arrs]).astype(np.int32),
-            sh_prim=np.concatenate([x["sh_prim"] + o for x, o in zip(arrs, pr_off)]).astype(np.int32),
-            sh_ao=np.concatenate([x["sh_ao"] for x in arrs]).astype(np.int32),
-            sh_atom=np.concatenate([x["sh_atom"] + o for x, o in zip(arrs, at_off)]).astype(np.int32),
-            sh_xyz=np.concatenate([x["sh_xyz"] for x in arrs]),
-            pr_exp=np.concatenate([x["pr_exp"] for x in arrs]),
-            pr_cc=np.concatenate([x["pr_cc"] for x in arrs]),
-            at_xyz=np.concatenate([x["at_xyz"] for x in arrs]),
-            at_z=np.concatenate([x["at_z"] for x in arrs]),
-            sh_blk=np.concatenate([np.full(k, m * n2, dtype=np.int64) for m, k in enumerate(nsh)]),
-            sh_at0=np.concatenate([np.full(k, o, dtype=np.int32) for k, o in zip(nsh, at_off)]),
-            sh_nat=np.concatenate([np.full(k, na, dtype=np.int32) for k, na in zip(nsh, nat)]),
-            sh_mol=np.concatenate([np.full(k, m, dtype=np.int32) for m, k in enumerate(nsh)]),
+            sh_l=cat("sh_l"), sh_nprim=cat("sh_nprim"),
+            sh_prim=(cat("sh_prim") + np.repeat(pr_off, nsh)).astype(np.int32), sh_ao=cat("sh_ao"),
+            sh_atom=(cat("sh_atom") + np.repeat(at_off, nsh)).astype(np.int32), sh_xyz=cat("sh_xyz"),
+            pr_exp=cat("pr_exp"), pr_cc=cat("pr_cc"), at_xyz=cat("at_xyz"), at_z=cat("at_z"),
+            sh_blk=np.repeat(mols * (self.nmax * self.nmax), nsh).astype(np.int64),
+            sh_at0=np.repeat(at_off, nsh).astype(np.int32), sh_nat=np.repeat(nat, nsh).astype(np.int32),
+            sh_mol=np.repeat(mols, nsh).astype(np.int32),
         )
         self.sh_off = sh_off
         self.h_basis = a
@@ -104,14 +100,19 @@ class EnsembleEngine(GpuEngine):
             self._full = None
 
     def _pair_index(self):
-        """Shell pairs a <= b inside each molecule (global shell indices)."""
-        ia_all, ib_all = [], []
-        for m, mol in enumerate(self.mols):
-            n = mol.NCgtf
-            ia, ib = np.triu_indices(n)
-            ia_all.append(ia + self.sh_off[m])
-            ib_all.append(ib + self.sh_off[m])
-        return np.concatenate(ia_all), np.concatenate(ib_all)
+        """Shell pairs a <= b inside each molecule (global shell indices), molecule by
+        molecule; molecules of one shell count are filled together."""
+        ns = np.array([m.NCgtf for m in self.mols])
+        count = ns * (ns + 1) // 2
+        start = np.cumsum(count) - count
+        ia, ib = np.empty((2, int(count.sum())), dtype=np.int64)
+        for n in np.unique(ns):
+            mols = np.nonzero(ns == n)[0]
+            i, j = np.triu_indices(n)
+            at = start[mols][:, None] + np.arange(len(i))[None, :]
+            ia[at] = self.sh_off[mols][:, None] + i
+            ib[at] = self.sh_off[mols][:, None] + j
+        return ia, ib
 
     def _build_pairs(self):
         a = self.h_basis

@@ -7,6 +7,7 @@ import numpy as np
 import torch
 
 from .. import _lib
+from .._stream import stream as _stream
 from .blocks import NFEAT, NPARAM
 
 DIMS = [NFEAT, 256, 256, 256, NPARAM]
@@ -14,10 +15,6 @@ DIMS = [NFEAT, 256, 256, 256, NPARAM]
 
 def _p(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
-
-
-def _s():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 class PairMLP:
@@ -60,7 +57,7 @@ class PairMLP:
             C = torch.empty(M, N, dtype=torch.float32, device=self.dev)
             Z = torch.empty(M, N, dtype=torch.float32, device=self.dev) if (keep and act) else None
             _lib.call("pcg_mlp_gemm", M, N, K, _p(A), K, 1, _p(self.Wb[k]), 1, N, 1, _p(C), N, 0, _p(self.b[k]),
-                      _p(Z), act, _s())
+                      _p(Z), act, _stream())
             cache.append((A, Z))
             A = C
         return A, cache
@@ -78,14 +75,14 @@ class PairMLP:
             A = cache[k][0]
             dW = torch.empty(K, N, dtype=torch.float32, device=self.dev)
             db = torch.empty(N, dtype=torch.float32, device=self.dev)
-            _lib.call("pcg_mlp_wgrad", M, K, N, _p(A), _p(G), _p(dW), _p(db), _p(ws), ws.numel(), _s())
+            _lib.call("pcg_mlp_wgrad", M, K, N, _p(A), _p(G), _p(dW), _p(db), _p(ws), ws.numel(), _stream())
             grads[k] = (dW, db)
             if k > 0:
                 # dA, times the derivative of the activation below it
                 Z = cache[k - 1][1]
                 dA = torch.empty(M, K, dtype=torch.float32, device=self.dev)
                 _lib.call("pcg_mlp_gemm", M, K, N, _p(G), N, 1, _p(self.Wb[k]), 1, 1, N, _p(dA), K, 0, None, _p(Z),
-                          2 if Z is not None else 0, _s())
+                          2 if Z is not None else 0, _stream())
                 G = dA
         return grads
 
@@ -94,7 +91,7 @@ class PairMLP:
         dY = torch.empty_like(Y)
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         count = mask.sum()
-        _lib.call("pcg_mlp_mse_counted", n, _p(Y), _p(T), _p(mask), _p(count), _p(dY), _p(loss), _s())
+        _lib.call("pcg_mlp_mse_counted", n, _p(Y), _p(T), _p(mask), _p(count), _p(dY), _p(loss), _stream())
         return loss, dY
 
     def adam(self, grads, lr, b1=0.9, b2=0.999, eps=1e-8):
@@ -109,7 +106,7 @@ class PairMLP:
             for j, (w, g, m, v, wb) in enumerate(part):
                 t.n[j], t.w[j], t.g[j], t.m[j], t.v[j] = w.numel(), w.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr()
                 t.w_bf16[j] = wb.data_ptr() if wb is not None else None
-            _lib.call("pcg_mlp_adam_all", len(part), ctypes.byref(t), lr, b1, b2, eps, self.step_count, _s())
+            _lib.call("pcg_mlp_adam_all", len(part), ctypes.byref(t), lr, b1, b2, eps, self.step_count, _stream())
 
     def predict(self, X):
         Y, _ = self.forward(X)

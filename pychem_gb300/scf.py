@@ -22,12 +22,14 @@ the AO->MO transforms run on the tcgen05 tensor cores with FP64 accuracy
 """
 import ctypes
 import math
+import threading
 import time
 
 import numpy as np
 import torch
 
 from . import _lib, eigen
+from ._stream import stream as _stream
 
 LINEAR_DEPENDENCE = 1.0e-6   # Data/constants.py:34
 
@@ -108,10 +110,12 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     kernels: Fock digestion, FP64 GEMMs (pcg_dgemm), the eigenvectors (Jacobi for the
     first exact_iters iterations, then refinement of the previous vectors that
     decouples the occupied space, checked, with the Jacobi route when the check
-    fails), the density C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc).  For
-    n > 136 (graph None or True) every iteration after the first exact_iters is one
-    CUDA graph replay followed by one read of six numbers (energy, density change,
-    refinement checks, commutator size)."""
+    fails; for n <= 136 the FP64 Jacobi kernel in every iteration), the density
+    C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc, n > 136).  With graph None or
+    True every iteration after the first exact_iters is one CUDA graph replay followed
+    by one read of six numbers (energy, density change, refinement checks, commutator
+    size): an iteration is 50 to 60 launches, which for a small molecule take 1 ms of
+    host time against 0.3 ms replayed."""
     from . import dense
     mol = engine.mol
     nocc = mol.NAlphaElectrons
@@ -122,7 +126,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     e_nuc = mol.nuclear_repulsion()
     n = engine.nbf
     big = n > eigen.FP64_JACOBI_MAX_N
-    use_graph = big if graph is None else (graph and big)
+    use_graph = graph is None or graph
     X = orthogonaliser(S)
     n2 = X.shape[1]
     mm = dense.mm
@@ -205,7 +209,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     scale = None
     for it in range(1, max_iter + 1):
         exact = it <= exact_iters or not big
-        if exact or not use_graph:
+        if it <= max(exact_iters, diis_start) or not use_graph:
             fock_and_diis(it > diis_start)
             if exact:
                 diag_exact()
@@ -223,17 +227,21 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
                 side, pool = _graph_stream_and_pool(dev)
                 side.wait_stream(torch.cuda.current_stream())
                 with torch.cuda.stream(side):
-                    g.capture_begin(pool=pool)
+                    # other threads may allocate and copy meanwhile
+                    g.capture_begin(pool=pool, capture_error_mode="thread_local")
                     try:
                         fock_and_diis(True)
-                        diag_refine()
+                        if exact:
+                            diag_exact()
+                        else:
+                            diag_refine()
                         density()
                     finally:
                         g.capture_end()
                 torch.cuda.current_stream().wait_stream(side)
                 # keeps the pool alive (its use count) until the next solve's capture;
                 # the graph it replaces returns its blocks to the pool
-                _LAST_GRAPH[dev] = g
+                _GRAPHS.last[dev] = g
                 per_replay = _lib_launches() - c0
                 if record:
                     phases["capture"] = time.perf_counter()
@@ -303,19 +311,28 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
                      converged=converged, history=history, fock_builds=it, diag_fallbacks=fallbacks)
 
 
-_GRAPH_POOLS = {}
-_LAST_GRAPH = {}
+class _Graphs(threading.local):
+    """Per thread and device: a capture stream with its memory pool, and the last
+    iteration graph (which keeps the pool in use).  Threads solve at the same time, so
+    they share neither."""
+
+    def __init__(self):
+        self.pools, self.last = {}, {}
+
+
+_GRAPHS = _Graphs()
 
 
 def _graph_stream_and_pool(dev):
-    """A capture stream and one memory pool per device for the SCF iteration graphs:
-    a new solve's capture takes its buffers from the pool, where the graph before the
+    """This thread's capture stream and memory pool for the SCF iteration graphs: a new
+    solve's capture takes its buffers from the pool, where the graph before the
     previous one left them (the previous graph is kept, never replayed again, until
     the capture that replaces it, so that the pool stays in use)."""
-    if dev not in _GRAPH_POOLS:
+    pools = _GRAPHS.pools
+    if dev not in pools:
         with torch.cuda.device(dev):
-            _GRAPH_POOLS[dev] = (torch.cuda.Stream(), torch.cuda.graph_pool_handle())
-    return _GRAPH_POOLS[dev]
+            pools[dev] = (torch.cuda.Stream(), torch.cuda.graph_pool_handle())
+    return pools[dev]
 
 
 def _lib_launches():
@@ -352,7 +369,7 @@ def ozaki_gemm_tc(X, Y, C, M, N, K, ldx, sY, sC, nslice=6, accumulate=False):
     ws = _tc_workspace(C.device, nbytes)
     _lib.call("pcg_ozaki_gemm_tc", M, N, K, ctypes.c_void_p(X.data_ptr()), ldx, ctypes.c_void_p(Y.data_ptr()),
               sY[0], sY[1], ctypes.c_void_p(C.data_ptr()), sC[0], sC[1], nslice, 1 if accumulate else 0,
-              ctypes.c_void_p(ws.data_ptr()), ws.numel(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+              ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream())
     return C
 
 
@@ -364,7 +381,7 @@ def ozaki_tc_status(dev):
     if ws is None:
         return 0
     return _lib.load().pcg_ozaki_tc_status(ctypes.c_void_p(ws.data_ptr()),
-                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+                                           _stream())
 
 
 def _pair_rows(n, dev):
@@ -437,7 +454,7 @@ def mp2_transform(eri, Co, Cv, gemm="tc", nslice=6, Co2=None, Cv2=None, timings=
     from .engine import pair_colmap
     cm = pair_colmap(n, pmap, dev)
     _lib.call("pcg_unpack_pairs", v * o, n, npair, ctypes.c_void_p(cm.data_ptr()), ctypes.c_void_p(T2p.data_ptr()),
-              ctypes.c_void_p(T2.data_ptr()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+              ctypes.c_void_p(T2.data_ptr()), _stream())
     del T2p
     T3 = quarter(T2, v * o * n, Co2, o2)
     del T2
@@ -477,7 +494,7 @@ def mp2_pair_sums(ovov, eo, ev):
     part = torch.empty(o * v, 2, dtype=torch.float64, device=ovov.device)
     vp = ctypes.c_void_p
     _lib.call("pcg_mp2_pair_sums", o, v, vp(X.data_ptr()), vp(eo.data_ptr()), vp(ev.data_ptr()), vp(part.data_ptr()),
-              vp(torch.cuda.current_stream().cuda_stream))
+              _stream())
     s = part.sum(0).tolist()
     return s[0], s[1]
 
