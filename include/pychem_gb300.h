@@ -232,6 +232,17 @@ int pcg_digest_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs
 int pcg_digest_class_u(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                        int ntask, const double *store, const double *Da, const double *Db, double *GJ,
                        double *GKa, double *GKb, void *stream);
+/* The digestion of all lists (class cls[q], tasks[q], ntask[q], stores[q]; the arrays are host
+ * memory): one launch a list, or one for all where the quartets are few. */
+int pcg_digest_lists(int nlist, const int *cls, const int *const *tasks, const int *ntask,
+                     const double *const *stores, const pcg_basis_t *basis, const pcg_pairs_t *pairs,
+                     const double *D, double *G, void *stream);
+int pcg_digest_lists_u(int nlist, const int *cls, const int *const *tasks, const int *ntask,
+                       const double *const *stores, const pcg_basis_t *basis, const pcg_pairs_t *pairs,
+                       const double *Da, const double *Db, double *GJ, double *GKa, double *GKb, void *stream);
+/* F_s = H + (GJ + GK_s + transpose) / 2 of both spins. */
+int pcg_fock_build_u(int n, const double *H, const double *GJ, const double *GKa, const double *GKb, double *Fa,
+                     double *Fb, void *stream);
 /* Electron-scattering integrals (ab|j0(S r12)|cd) of one class for a task list, same
  * store layout as pcg_eri_class (FP64): the operator of Methods/properties.py:20-23,
  * fundamentals of Methods/c_ints/two_electron_scattering.c:6-81 with z^-m j_m(z) by

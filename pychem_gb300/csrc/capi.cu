@@ -146,6 +146,44 @@ int pcg_digest_class_u(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pai
                              GKb, (cudaStream_t)stream);
 }
 
+static int check_lists(const char* msg, int nlist, const int* cls, const int* const* tasks, const int* ntask,
+                       const double* const* stores, const pcg_basis_t* basis, const pcg_pairs_t* pairs) {
+  bool ok = nlist >= 0 && basis && pairs && (nlist == 0 || (cls && tasks && ntask && stores));
+  for (int q = 0; ok && q < nlist; ++q)
+    ok = cls[q] >= 0 && cls[q] <= 20 && ntask[q] >= 0 && (ntask[q] == 0 || (tasks[q] && stores[q]));
+  if (!ok) { pcg_set_error(msg); return PCG_ERR_ARG; }
+  return PCG_OK;
+}
+
+int pcg_digest_lists(int nlist, const int* cls, const int* const* tasks, const int* ntask, const double* const* stores,
+                     const pcg_basis_t* basis, const pcg_pairs_t* pairs, const double* D, double* G, void* stream) {
+  if (int rc = check_lists("pcg_digest_lists: bad arguments", nlist, cls, tasks, ntask, stores, basis, pairs)) return rc;
+  if (!D || !G) { pcg_set_error("pcg_digest_lists: no density or accumulator"); return PCG_ERR_ARG; }
+  return pcg_launch_digest_lists(nlist, cls, tasks, ntask, stores, to_dev(basis), to_dev(pairs), D, G,
+                                 (cudaStream_t)stream);
+}
+
+int pcg_digest_lists_u(int nlist, const int* cls, const int* const* tasks, const int* ntask,
+                       const double* const* stores, const pcg_basis_t* basis, const pcg_pairs_t* pairs,
+                       const double* Da, const double* Db, double* GJ, double* GKa, double* GKb, void* stream) {
+  if (int rc = check_lists("pcg_digest_lists_u: bad arguments", nlist, cls, tasks, ntask, stores, basis, pairs)) return rc;
+  if (!Da || !Db || !GJ || !GKa || !GKb) {
+    pcg_set_error("pcg_digest_lists_u: no densities or accumulators");
+    return PCG_ERR_ARG;
+  }
+  return pcg_launch_digest_lists_u(nlist, cls, tasks, ntask, stores, to_dev(basis), to_dev(pairs), Da, Db, GJ, GKa,
+                                   GKb, (cudaStream_t)stream);
+}
+
+int pcg_fock_build_u(int n, const double* H, const double* GJ, const double* GKa, const double* GKb, double* Fa,
+                     double* Fb, void* stream) {
+  if (n < 1 || !H || !GJ || !GKa || !GKb || !Fa || !Fb) {
+    pcg_set_error("pcg_fock_build_u: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  return pcg_launch_fock_u(n, H, GJ, GKa, GKb, Fa, Fb, (cudaStream_t)stream);
+}
+
 int pcg_scattering_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const int* tasks, int ntask,
                          double S, double* store, void* stream) {
   if (cls < 0 || cls > 20 || !basis || !pairs || ntask < 0 || !(S >= 0.0)) {

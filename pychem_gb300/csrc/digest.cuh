@@ -1,0 +1,210 @@
+// Fock digestion kernels (closed shell and unrestricted) -- included by digest.cu and
+// digest_u.cu, one translation unit each so that the class instantiations compile in
+// parallel.
+//
+// For every stored quartet block, with the shell-level degeneracy d = (A!=B ? 2:1)
+// (C!=D ? 2:1)(AB!=CD ? 2:1) and v' = d (ab|cd),
+//   GJ_ab += D_cd v', GJ_cd += D_ab v',
+//   GK_ac -= D_bd v'/4, GK_bd -= D_ac v'/4, GK_ad -= D_bc v'/4, GK_bc -= D_ad v'/4.
+// Closed shell (S = 1): GJ = GK = G; the caller's F = H + (G + G^T)/2 equals H + 2J[D] - K[D]
+// with D the alpha density -- upstream's H + J[D_a + D_b] - K[D_a] (hartree_fock.py:345-355).
+// Unrestricted (S = 2): GJ from (D_a + D_b)/2 and one GK per spin, so that
+// F_s = H + sym(GJ + GK_s) = H + J[D_a + D_b] - K[D_s].  Co-densities W of non-orthogonal CI
+// (Methods/noci.py:243-300, hartree_fock.py:345-347 for non-symmetric densities) are the
+// unrestricted case with D_a = W and D_b = W^T, the D_a exchange blocks written transposed:
+// GK then holds G[W^T] + G[W]^T, J[W] = (GJ + GJ^T)/4 and K[W] = -GK/2 with K_ad = sum_bc
+// (ab|cd) W_cb; blockIdx.y selects the density.
+//
+// Bound: the FP64 pipe, six instructions an integral (0.48 ms for the 42 M integrals of
+// (H2O)16 / 6-31G), and the load/store queue, which one gather and one reduction a density
+// element and quartet fills (1.25 ms).  A thread therefore takes `run` consecutive quartets: lists
+// run through the kets (C, D) of one bra in order, so D_ab, D_ac, D_bc are loaded and G_ab,
+// G_ac, G_bc written once a run of equal (A, B) and C, and the lanes of a warp touch neighbouring
+// columns (run = 1, 2, 4, 8: 1.6, 1.1, 1.0, 1.2 ms).  All factors are powers of two and are
+// applied to exponents by integer operations, off the FP64 pipe.
+#pragma once
+#include "common.cuh"
+#include "pcg_internal.h"
+
+struct DigestArgs {
+  DevBasis b;
+  DevPairsExt pr;
+  const int2* tasks;
+  int ntask, run;              // quartets, and consecutive quartets per thread
+  const double* store;
+  const double* D[2];
+  double* GJ;
+  double* GK[2];
+  bool co;                     // co-densities: D[1] is D[0] transposed, GK[0] is written transposed
+  unsigned d0;                 // first density of the launch
+};
+
+// x 2^k, |k| <= 7, by its exponent; the few values near the ends of the range (and zero,
+// infinities, NaNs) take the exact route
+__device__ __forceinline__ double dg_scale(double x, int k) {
+  const int hi = __double2hiint(x);
+  const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+  if (e - 8u < 0x7e8u) return __hiloint2double(hi + (k << 20), __double2loint(x));
+  return e < 8u ? 0.0 : x * __hiloint2double((1023 + k) << 20, 0);
+}
+
+template <int R, int C>
+__device__ __forceinline__ void dg_load(const double* __restrict__ M, int r0, int c0, int n, double (&v)[R][C],
+                                        bool tr = false) {
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) v[i][j] = __ldg(M + (tr ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j));
+}
+// M += v 2^k, or -= if neg; clears v
+template <int R, int C>
+__device__ __forceinline__ void dg_add(double* __restrict__ M, int r0, int c0, int n, int k, bool neg,
+                                       double (&v)[R][C], bool tr = false) {
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      const double x = k ? dg_scale(v[i][j], k) : v[i][j];
+      atomicAdd(M + (tr ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j), neg ? -x : x);
+      v[i][j] = 0.0;
+    }
+}
+
+// the quartets of block blk: 128 threads of a.run consecutive ones
+template <int NA, int NB, int NC, int ND, int S>
+__device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) {
+  const long long first = ((long long)blk * blockDim.x + threadIdx.x) * a.run;
+  if (first >= a.ntask) return;
+  const int t1 = (int)(first + a.run < a.ntask ? first + a.run : a.ntask);
+  constexpr int JK = S == 2 ? -1 : 0;      // the J density is the sum of both spins: half of it
+  const int n = a.b.ld;
+  const bool co = S == 2 && a.co;
+  const long long dens = co ? (long long)(a.d0 + blockIdx.y) * n * n : 0;
+  int bra = -1, oa = 0, ob = 0, oc = -1;
+  long long o = dens;
+  bool sab = false;
+  double Jab[NA][NB], gab[NA][NB] = {};
+  double Dac[S][NA][NC], Dbc[S][NB][NC], gac[S][NA][NC] = {}, gbc[S][NB][NC] = {};
+  auto flush_c = [&]() {
+    if (oc < 0) return;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      dg_add(a.GK[s] + o, oa, oc, n, -2, true, gac[s], co && s == 0);
+      dg_add(a.GK[s] + o, ob, oc, n, -2, true, gbc[s], co && s == 0);
+    }
+  };
+  auto load_j = [&](int r0, int c0, auto& v) {
+    dg_load(a.D[0] + o, r0, c0, n, v);
+    if constexpr (S == 2) {
+      constexpr int R = sizeof(v) / sizeof(v[0]), C = sizeof(v[0]) / sizeof(double);
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) v[i][j] += __ldg(a.D[1] + o + (co ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j));
+    }
+  };
+  for (int t = (int)first; t < t1; ++t) {
+    const int2 tk = a.tasks[t];
+    int c, d;
+    bool scd;
+    int4 pb, pk;                       // (AO of A | (A == B) << 30, AO of B, block offset)
+    if (a.pr.p.ao4) {
+      pk = __ldg(a.pr.p.ao4 + tk.y);
+      c = pk.x & 0x3FFFFFFF; d = pk.y; scd = (pk.x >> 30) & 1;
+    } else {
+      const int C = __ldg(a.pr.p.A + tk.y), Dd = __ldg(a.pr.p.B + tk.y);
+      c = __ldg(a.b.sh_ao + C); d = __ldg(a.b.sh_ao + Dd); scd = C == Dd;
+    }
+    if (tk.x != bra) {
+      flush_c();
+      if (bra >= 0) dg_add(a.GJ + o, oa, ob, n, JK, false, gab);
+      bra = tk.x;
+      if (a.pr.p.ao4) {
+        pb = __ldg(a.pr.p.ao4 + bra);
+        oa = pb.x & 0x3FFFFFFF; ob = pb.y; sab = (pb.x >> 30) & 1;
+        o = dens + ((long long)(unsigned)pb.z | ((long long)pb.w << 32));
+      } else {
+        const int A = __ldg(a.pr.p.A + bra), B = __ldg(a.pr.p.B + bra);
+        o = dens + dev_blk(a.b, A);
+        oa = __ldg(a.b.sh_ao + A); ob = __ldg(a.b.sh_ao + B); sab = A == B;
+      }
+      load_j(oa, ob, Jab);
+      oc = -1;
+    }
+    if (c != oc) {
+      flush_c();
+      oc = c;
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        dg_load(a.D[s] + o, oa, oc, n, Dac[s], co && s == 1);
+        dg_load(a.D[s] + o, ob, oc, n, Dbc[s], co && s == 1);
+      }
+    }
+    const int deg = !sab + !scd + (tk.x != tk.y);      // log2 of the degeneracy
+    double Jcd[NC][ND], gcd[NC][ND] = {};
+    double Dad[S][NA][ND], Dbd[S][NB][ND], gad[S][NA][ND] = {}, gbd[S][NB][ND] = {};
+    load_j(oc, d, Jcd);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      dg_load(a.D[s] + o, oa, d, n, Dad[s], co && s == 1);
+      dg_load(a.D[s] + o, ob, d, n, Dbd[s], co && s == 1);
+    }
+    const double* st = a.store + t;
+#pragma unroll
+    for (int i = 0; i < NA; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+#pragma unroll
+          for (int l = 0; l < ND; ++l) {
+            const double v = dg_scale(__ldg(st + (size_t)(((i * NB + j) * NC + k) * ND + l) * a.ntask), deg);
+            gab[i][j] = fma(Jcd[k][l], v, gab[i][j]);
+            gcd[k][l] = fma(Jab[i][j], v, gcd[k][l]);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+              gac[s][i][k] = fma(Dbd[s][j][l], v, gac[s][i][k]);
+              gbd[s][j][l] = fma(Dac[s][i][k], v, gbd[s][j][l]);
+              gad[s][i][l] = fma(Dbc[s][j][k], v, gad[s][i][l]);
+              gbc[s][j][k] = fma(Dad[s][i][l], v, gbc[s][j][k]);
+            }
+          }
+    dg_add(a.GJ + o, oc, d, n, JK, false, gcd);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      dg_add(a.GK[s] + o, ob, d, n, -2, true, gbd[s], co && s == 0);
+      dg_add(a.GK[s] + o, oa, d, n, -2, true, gad[s], co && s == 0);
+    }
+  }
+  flush_c();
+  dg_add(a.GJ + o, oa, ob, n, JK, false, gab);
+}
+
+template <int NA, int NB, int NC, int ND, int S>
+__global__ void __launch_bounds__(128) k_digest(const DigestArgs a) {
+  digest_block<NA, NB, NC, ND, S>(a, blockIdx.x);
+}
+
+// consecutive quartets per thread: up to 4, fewer where that would leave less than 1,024
+// threads an SM
+static inline int digest_run(int ntask) {
+  const int r = ntask / (152 * 1024);
+  return r < 1 ? 1 : (r > 4 ? 4 : r);
+}
+
+template <int S>
+static int launch_digest(int cls, DigestArgs a, cudaStream_t s, unsigned ndens = 1) {
+  if (a.ntask <= 0) return PCG_OK;
+  a.run = digest_run(a.ntask);
+  const int threads = 128;
+  const unsigned blocks = (unsigned)(((long long)a.ntask + (long long)threads * a.run - 1) / ((long long)threads * a.run));
+  switch (cls) {
+#define X(id, na, nb, nc, nd) \
+  case id: k_digest<na, nb, nc, nd, S><<<dim3(blocks, ndens), threads, 0, s>>>(a); break;
+    PCG_SHAPE_CASES(X)
+#undef X
+    default: pcg_set_error("digestion: class id out of range"); return PCG_ERR_ARG;
+  }
+  PCG_CUDA(cudaGetLastError());
+  return PCG_OK;
+}

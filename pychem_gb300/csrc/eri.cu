@@ -1,5 +1,5 @@
-// Electron-repulsion integrals over Schwarz-screened shell quartets, Fock digestion
-// and dense expansion.
+// Electron-repulsion integrals over Schwarz-screened shell quartets and their dense
+// expansion.
 //
 // Upstream counterparts: Methods/integrals.py:427-555 (two_electron: fundamentals,
 // VRR, contraction, HRR, normalisation, spherical transform),
@@ -14,109 +14,6 @@
 // so writes here and reads in the digestion are coalesced across a warp.
 #include "common.cuh"
 #include "pcg_internal.h"
-
-// ----------------------------------------------------------------------------------
-// Fock digestion (closed shell): for every stored quartet block, with the shell-level
-// degeneracy d = (A!=B ? 2:1)(C!=D ? 2:1)(AB!=CD ? 2:1) and v' = d (ab|cd),
-//   G_ab += D_cd v', G_cd += D_ab v', G_ac -= D_bd v'/4, G_bd -= D_ac v'/4,
-//   G_ad -= D_bc v'/4, G_bc -= D_ad v'/4;
-// the caller symmetrises F = H + (G + G^T)/2, which equals H + 2J[D] - K[D] with D the
-// alpha density -- upstream's H + J[D_a + D_b] - K[D_a] (hartree_fock.py:345-355).
-// ----------------------------------------------------------------------------------
-template <int NA, int NB, int NC, int ND>
-__global__ void __launch_bounds__(128) k_digest(DevBasis b, DevPairsExt pr, const int2* __restrict__ tasks,
-                                                int ntask, const double* __restrict__ store,
-                                                const double* __restrict__ D, double* __restrict__ G) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntask) return;
-  const int2 tk = tasks[t];
-  int oa, ob, oc, od;
-  long long o;  // the four shells share one molecule block
-  bool sab, scd;
-  if (pr.p.ao4) {  // one 16-byte load per pair instead of the shell tables
-    const int4 pb = __ldg(pr.p.ao4 + tk.x), pk = __ldg(pr.p.ao4 + tk.y);
-    oa = pb.x & 0x3FFFFFFF; ob = pb.y; oc = pk.x & 0x3FFFFFFF; od = pk.y;
-    sab = (pb.x >> 30) & 1; scd = (pk.x >> 30) & 1;
-    o = (long long)(unsigned)pb.z | ((long long)pb.w << 32);
-  } else {
-    const int A = __ldg(pr.p.A + tk.x), B = __ldg(pr.p.B + tk.x);
-    const int C = __ldg(pr.p.A + tk.y), Dd = __ldg(pr.p.B + tk.y);
-    o = dev_blk(b, A);
-    oa = __ldg(b.sh_ao + A); ob = __ldg(b.sh_ao + B); oc = __ldg(b.sh_ao + C); od = __ldg(b.sh_ao + Dd);
-    sab = A == B; scd = C == Dd;
-  }
-  const int n = b.ld;
-  D += o;
-  G += o;
-  const double deg = (sab ? 1.0 : 2.0) * (scd ? 1.0 : 2.0) * (tk.x == tk.y ? 1.0 : 2.0);
-  double Dab[NA][NB], Dcd[NC][ND], Dac[NA][NC], Dbd[NB][ND], Dad[NA][ND], Dbc[NB][NC];
-  double gab[NA][NB], gcd[NC][ND], gac[NA][NC], gbd[NB][ND], gad[NA][ND], gbc[NB][NC];
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) { Dab[i][j] = __ldg(D + (size_t)(oa + i) * n + ob + j); gab[i][j] = 0.0; }
-#pragma unroll
-  for (int k = 0; k < NC; ++k)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) { Dcd[k][l] = __ldg(D + (size_t)(oc + k) * n + od + l); gcd[k][l] = 0.0; }
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int k = 0; k < NC; ++k) { Dac[i][k] = __ldg(D + (size_t)(oa + i) * n + oc + k); gac[i][k] = 0.0; }
-#pragma unroll
-  for (int j = 0; j < NB; ++j)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) { Dbd[j][l] = __ldg(D + (size_t)(ob + j) * n + od + l); gbd[j][l] = 0.0; }
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) { Dad[i][l] = __ldg(D + (size_t)(oa + i) * n + od + l); gad[i][l] = 0.0; }
-#pragma unroll
-  for (int j = 0; j < NB; ++j)
-#pragma unroll
-    for (int k = 0; k < NC; ++k) { Dbc[j][k] = __ldg(D + (size_t)(ob + j) * n + oc + k); gbc[j][k] = 0.0; }
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-      for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) {
-          const double v = deg * __ldg(store + (size_t)(((i * NB + j) * NC + k) * ND + l) * ntask + t);
-          const double vq = -0.25 * v;
-          gab[i][j] = fma(Dcd[k][l], v, gab[i][j]);
-          gcd[k][l] = fma(Dab[i][j], v, gcd[k][l]);
-          gac[i][k] = fma(Dbd[j][l], vq, gac[i][k]);
-          gbd[j][l] = fma(Dac[i][k], vq, gbd[j][l]);
-          gad[i][l] = fma(Dbc[j][k], vq, gad[i][l]);
-          gbc[j][k] = fma(Dad[i][l], vq, gbc[j][k]);
-        }
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) atomicAdd(G + (size_t)(oa + i) * n + ob + j, gab[i][j]);
-#pragma unroll
-  for (int k = 0; k < NC; ++k)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) atomicAdd(G + (size_t)(oc + k) * n + od + l, gcd[k][l]);
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int k = 0; k < NC; ++k) atomicAdd(G + (size_t)(oa + i) * n + oc + k, gac[i][k]);
-#pragma unroll
-  for (int j = 0; j < NB; ++j)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) atomicAdd(G + (size_t)(ob + j) * n + od + l, gbd[j][l]);
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int l = 0; l < ND; ++l) atomicAdd(G + (size_t)(oa + i) * n + od + l, gad[i][l]);
-#pragma unroll
-  for (int j = 0; j < NB; ++j)
-#pragma unroll
-    for (int k = 0; k < NC; ++k) atomicAdd(G + (size_t)(ob + j) * n + oc + k, gbc[j][k]);
-}
 
 // Dense N^4 store with the 8-fold permutational symmetry (hartree_fock.py:314-325).
 template <int NA, int NB, int NC, int ND>
@@ -391,21 +288,6 @@ int pcg_launch_scattering(int cls, const DevPairsExt& pr, const BesselTable& bt,
   if (cls <= 17) return pcg_launch_eri_s1(cls, pr, bt, fac, tasks, ntask, nheavy, S, store, s);
   if (cls <= 19) return pcg_launch_eri_s2(cls, pr, bt, fac, tasks, ntask, nheavy, S, store, s);
   return pcg_launch_eri_s3(cls, pr, bt, fac, tasks, ntask, nheavy, S, store, s);
-}
-
-int pcg_launch_digest(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
-                      const double* store, const double* D, double* G, cudaStream_t s) {
-  if (ntask <= 0) return PCG_OK;
-  const int threads = 128, blocks = (ntask + threads - 1) / threads;
-  switch (cls) {
-#define X(id, a, bb, c, d) \
-  case id: k_digest<a, bb, c, d><<<blocks, threads, 0, s>>>(b, pr, tasks, ntask, store, D, G); break;
-    PCG_SHAPE_CASES(X)
-#undef X
-    default: pcg_set_error("pcg_digest_class: class id out of range"); return PCG_ERR_ARG;
-  }
-  PCG_CUDA(cudaGetLastError());
-  return PCG_OK;
 }
 
 int pcg_launch_dense(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,

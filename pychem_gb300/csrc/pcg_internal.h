@@ -54,6 +54,14 @@ int pcg_launch_digest(int cls, const DevBasis& b, const DevPairsExt& pr, const i
 int pcg_launch_digest_u(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                         const double* store, const double* Da, const double* Db, double* GJ, double* GKa,
                         double* GKb, cudaStream_t s);
+int pcg_launch_digest_lists(int nlist, const int* cls, const int* const* tasks, const int* ntask,
+                            const double* const* stores, const DevBasis& b, const DevPairsExt& pr, const double* D,
+                            double* G, cudaStream_t s);
+int pcg_launch_digest_lists_u(int nlist, const int* cls, const int* const* tasks, const int* ntask,
+                              const double* const* stores, const DevBasis& b, const DevPairsExt& pr, const double* Da,
+                              const double* Db, double* GJ, double* GKa, double* GKb, cudaStream_t s);
+int pcg_launch_fock_u(int n, const double* H, const double* GJ, const double* GKa, const double* GKb, double* Fa,
+                      double* Fb, cudaStream_t s);
 int pcg_launch_digest_co(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                          const double* store, int nd, const double* W, double* GJ, double* GK, cudaStream_t s);
 int pcg_launch_dense_pairs(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,

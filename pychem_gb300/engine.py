@@ -444,6 +444,14 @@ class GpuEngine:
         return self
 
     # ---------------------------------------------------------------------------------
+    def _lists(self):
+        """The quartet lists and stores as the first five arguments of pcg_digest_lists."""
+        rows = [(cls, tasks, n, self.stores[(cls, part)]) for cls, rec in self.classes.items()
+                for part, (tasks, n) in rec.items()]
+        k = len(rows)
+        return (k, (ctypes.c_int * k)(*[r[0] for r in rows]), (ctypes.c_void_p * k)(*[r[1].data_ptr() for r in rows]),
+                (ctypes.c_int * k)(*[r[2] for r in rows]), (ctypes.c_void_p * k)(*[r[3].data_ptr() for r in rows]))
+
     def fock(self, D, out=None, G=None):
         """Closed-shell F = H + 2J[D] - K[D] for the alpha density D (nbf x nbf)."""
         n = self.nbf
@@ -452,10 +460,8 @@ class GpuEngine:
         else:
             G.zero_()
         D = D.contiguous()
-        for cls, rec in self.classes.items():
-            for part, (tasks, ntask) in rec.items():
-                _lib.call("pcg_digest_class", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(tasks),
-                          ntask, _ptr(self.stores[(cls, part)]), _ptr(D), _ptr(G), _stream())
+        _lib.call("pcg_digest_lists", *self._lists(), ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(D),
+                  _ptr(G), _stream())
         F = out if out is not None else torch.empty(n, n, dtype=torch.float64, device=self.dev)
         _lib.call("pcg_fock_build", n, _ptr(self.H), _ptr(G), _ptr(F), _stream())
         return F
@@ -465,13 +471,11 @@ class GpuEngine:
         n = self.nbf
         G = torch.zeros(3, n, n, dtype=torch.float64, device=self.dev)
         Da, Db = Da.contiguous(), Db.contiguous()
-        for cls, rec in self.classes.items():
-            for part, (tasks, ntask) in rec.items():
-                _lib.call("pcg_digest_class_u", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
-                          _ptr(tasks), ntask, _ptr(self.stores[(cls, part)]), _ptr(Da), _ptr(Db), _ptr(G[0]),
-                          _ptr(G[1]), _ptr(G[2]), _stream())
-        Ga, Gb = G[0] + G[1], G[0] + G[2]
-        return self.H + 0.5 * (Ga + Ga.T), self.H + 0.5 * (Gb + Gb.T)
+        _lib.call("pcg_digest_lists_u", *self._lists(), ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(Da),
+                  _ptr(Db), _ptr(G[0]), _ptr(G[1]), _ptr(G[2]), _stream())
+        Fa, Fb = torch.empty(2, n, n, dtype=torch.float64, device=self.dev).unbind(0)
+        _lib.call("pcg_fock_build_u", n, _ptr(self.H), _ptr(G[0]), _ptr(G[1]), _ptr(G[2]), _ptr(Fa), _ptr(Fb), _stream())
+        return Fa, Fb
 
     def coulomb_exchange(self, W):
         """J[W] and K[W] for general (not necessarily symmetric) co-densities W of shape

@@ -150,10 +150,8 @@ class EnsembleEngine(GpuEngine):
         else:
             G.zero_()
         D = D.contiguous()
-        for cls, rec in self.classes.items():
-            for part, (tasks, ntask) in rec.items():
-                _lib.call("pcg_digest_class", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(tasks),
-                          ntask, _ptr(self.stores[(cls, part)]), _ptr(D), _ptr(G), _stream())
+        _lib.call("pcg_digest_lists", *self._lists(), ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(D),
+                  _ptr(G), _stream())
         F = out if out is not None else torch.empty(self.B, n, n, dtype=torch.float64, device=self.dev)
         _lib.call("pcg_fock_build_batched", self.B, n, _ptr(self.H), _ptr(G), _ptr(F), _stream())
         return F
