@@ -267,6 +267,13 @@ int pcg_scattering_class_split(int cls, const pcg_basis_t *basis, const pcg_pair
 int pcg_digest_class_co(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                         int ntask, const double *store, int nd, const double *W, double *GJ, double *GK,
                         void *stream);
+/* The same matrices of nd co-densities from the dense integral tensor (n^4, every permutation):
+ * J[W]_ab = sum_cd (ab|cd) W_cd and K[W]_ad = sum_bc (ab|cd) W_cb, nd x n x n each, as
+ * products of packed densities with pair matrices (n <= 255, nd <= 65535; workspace 8-byte
+ * aligned). */
+size_t pcg_coulomb_exchange_workspace(int n, int nd);
+int pcg_coulomb_exchange(int n, int nd, const double *eri, const double *W, double *J, double *K, void *workspace,
+                         size_t ws_bytes, void *stream);
 int pcg_fock_build(int n, const double *H, const double *G, double *F, void *stream);
 /* Same for nblocks consecutive ld x ld blocks (an ensemble of molecules). */
 int pcg_fock_build_batched(int nblocks, int ld, const double *H, const double *G, double *F, void *stream);

@@ -96,6 +96,8 @@ _SIGS = {
                                    c_int, ctypes.c_double, c_void_p, c_void_p],
     "pcg_digest_class_co": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_void_p],
+    "pcg_coulomb_exchange_workspace": [c_int, c_int],
+    "pcg_coulomb_exchange": [c_int, c_int] + [c_void_p] * 5 + [ctypes.c_size_t, c_void_p],
     "pcg_fock_build": [c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_fock_build_batched": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_dense_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
@@ -147,9 +149,9 @@ LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_elect
              "pcg_one_electron_kinetic", "pcg_one_electron_contract"}
 launch_count = 0
 _RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
-             "pcg_mlp_wgrad_workspace": ctypes.c_size_t}
+             "pcg_mlp_wgrad_workspace": ctypes.c_size_t, "pcg_coulomb_exchange_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_mlp_wgrad": 2}
+MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_mlp_wgrad": 2, "pcg_coulomb_exchange": 4}
 
 _lib = None
 

@@ -23,6 +23,10 @@ N_SPHER = [1, 3, 5]
 # of two oxygen 1s pairs take longer than the rest of a mid-size molecule's launch, and from
 # 128 on each of 16 lanes still has eight or more to sum
 HEAVY = 128
+# co-density matrices by products with pair matrices: the dense tensor and the pair matrices
+# cost what the digestion of about 16 densities does, and take 1.2 GB at 96 functions
+COEXCHANGE_MIN = 16
+COEXCHANGE_MAX_N = 96
 
 
 def _ptr(t):
@@ -482,13 +486,27 @@ class GpuEngine:
         (nd, nbf, nbf): J_ab = sum_cd (ab|cd) W_cd, K_ad = sum_bc (ab|cd) W_cb
         (Methods/hartree_fock.py:345-347, applied by Methods/noci.py:261-318).
 
-        One pcg_digest_class_co launch per class part digests every density (blockIdx.y
-        selects it).  Per unique quartet the digestion accumulates one orientation of
-        each exchange block (G[M]_ad from M_bc and so on); the kernel adds G[W^T] and
-        G[W]^T, which together hold all eight index permutations: K[W] = -GK/2.  The
-        Coulomb buffer sees (W + W^T)/2, all that J depends on: J = (GJ + GJ^T)/4."""
+        From COEXCHANGE_MIN densities on, for molecules whose dense tensor is small, three
+        matrix products of the packed densities with pair matrices (pcg_coulomb_exchange).
+        Otherwise one pcg_digest_class_co launch per class part digests every density
+        (blockIdx.y selects it): per unique quartet the digestion accumulates one
+        orientation of each exchange block (G[M]_ad from M_bc and so on); the kernel adds
+        G[W^T] and G[W]^T, which together hold all eight index permutations: K[W] =
+        -GK/2.  The Coulomb buffer sees (W + W^T)/2, all that J depends on: J = (GJ +
+        GJ^T)/4."""
         W = W.contiguous()
-        nd = W.shape[0]
+        nd, n = W.shape[0], self.nbf
+        if nd >= COEXCHANGE_MIN and n <= COEXCHANGE_MAX_N:
+            lib = _lib.load()
+            eri = self.dense_eri()
+            J, K = torch.empty_like(W), torch.empty_like(W)
+            step = min(nd, 16384)
+            ws = torch.empty(lib.pcg_coulomb_exchange_workspace(n, step), dtype=torch.uint8, device=self.dev)
+            for k in range(0, nd, step):
+                w = W[k:k + step]
+                _lib.call("pcg_coulomb_exchange", n, w.shape[0], _ptr(eri), _ptr(w), _ptr(J[k:]), _ptr(K[k:]), _ptr(ws),
+                          ws.numel(), _stream())
+            return J, K
         GJ = torch.zeros_like(W)
         GK = torch.zeros_like(W)
         for cls, rec in self.classes.items():
