@@ -127,6 +127,10 @@ _SIGS = {
     "pcg_unpack_pairs": [c_longlong, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_dgemm": [c_int, c_int, c_int, c_int, c_double, c_void_p, c_longlong, c_longlong, c_longlong, c_void_p,
                   c_longlong, c_longlong, c_longlong, c_double, c_void_p, c_longlong, c_longlong, c_longlong, c_void_p],
+    "pcg_dgemm_sym": [c_int, c_int, c_double, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong,
+                      c_double, c_void_p, c_longlong, c_longlong, c_void_p],
+    "pcg_scf_stats": [c_int, c_int] + [c_void_p] * 9,
+    "pcg_projector_check": [c_int, c_int] + [c_void_p] * 4,
     "pcg_oa_correction": [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_diis_step": [c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_void_p],
@@ -141,7 +145,7 @@ _SIGS = {
 # entry points that launch exactly one kernel of this library per call
 LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_schwarz_class", "pcg_plan_count", "pcg_plan_fill", "pcg_expand_tasks",
              "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_digest_lists", "pcg_digest_lists_u", "pcg_fock_build_u", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
-             "pcg_dgemm", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
+             "pcg_dgemm", "pcg_dgemm_sym", "pcg_projector_check", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
              "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_mse_counted", "pcg_mlp_adam", "pcg_mlp_adam_all",
              "pcg_shellpair_quantities", "pcg_two_electron_bound", "pcg_two_electron_fundamentals",
              "pcg_two_electron_vrr", "pcg_two_electron_contract", "pcg_two_electron_hrr",
@@ -151,7 +155,7 @@ launch_count = 0
 _RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
              "pcg_mlp_wgrad_workspace": ctypes.c_size_t, "pcg_coulomb_exchange_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_mlp_wgrad": 2, "pcg_coulomb_exchange": 4}
+MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_coulomb_exchange": 4}
 
 _lib = None
 

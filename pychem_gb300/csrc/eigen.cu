@@ -30,6 +30,43 @@ __device__ __forceinline__ void rot_params(T app, T aqq, T apq, T& c, T& s) {
   s = t * c;
 }
 
+// The FP64 rotation without divisions or roots on the FP64 pipe (a chain of 60 dependent
+// instructions, longer than the rest of a small matrix's round): t = tan of the angle, the
+// smaller root of a t^2 + d t - a = 0 with a = apq, d = aqq - app, both scaled to order one by
+// their exponents; an FP32 root and two Newton steps in FP64 (relative errors 1e-7, 1e-14,
+// rounding), the slope's reciprocal in FP32.  c = (1 + t^2)^-1/2 to rounding keeps c^2 + s^2 = 1.
+__device__ __forceinline__ void rot_params(double app, double aqq, double apq, double& c, double& s) {
+  c = 1.0;
+  s = 0.0;
+  if (apq == 0.0) return;
+  double d = aqq - app, a = apq;
+  const int ed = (__double2hiint(d) >> 20) & 0x7ff, ea = (__double2hiint(a) >> 20) & 0x7ff;
+  const int e = max(ed, ea);
+  if (e >= 0x7fe || e == 0) {            // infinities, NaNs and subnormal pairs: the plain form
+    const double tau = d / (2.0 * a);
+    double t = fabs(tau) > 1e18 ? 0.5 / tau : (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+    c = 1.0 / sqrt(1.0 + t * t);
+    s = t * c;
+    return;
+  }
+  // exponents to [.., 1023]; what falls below 2^-1022 of the other is zero beside it
+  const int k = e - 1023;
+  d = ed > k ? __hiloint2double(__double2hiint(d) - (k << 20), __double2loint(d)) : 0.0;
+  if (ea <= k) return;
+  a = __hiloint2double(__double2hiint(a) - (k << 20), __double2loint(a));
+  const float df = bits_to_float(d), af = bits_to_float(a);
+  float tf = 2.0f * af / (fabsf(df) + sqrtf(fmaf(df, df, 4.0f * af * af)));
+  double t = bits_to_double(df < 0.0f ? -tf : tf);
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const double g = fma(a, t, d);                                  // a t + d
+    const double r = bits_to_double(1.0f / bits_to_float(fma(a, t, g)));   // 1 / (2 a t + d)
+    t = fma(-fma(g, t, -a), r, t);
+  }
+  c = nr_rsqrt(fma(t, t, 1.0));
+  s = t * c;
+}
+
 __device__ __forceinline__ int tri(int i, int j) {  // packed lower triangle, i >= j
   return i * (i + 1) / 2 + j;
 }
@@ -177,14 +214,14 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
   for (int idx = tid; idx < nrow * m; idx += nt) Vg[(size_t)b * sV + (size_t)r0 * m + idx] = V[idx];
 }
 
-// shared-memory plan of one launch: how many CTAs share a matrix, rows of V per CTA,
-// whether the block table fits, and the dynamic bytes
+// shared-memory plan of one launch: how many CTAs share a matrix (at least `least`), rows of V
+// per CTA, whether the block table fits, and the dynamic bytes
 template <typename T>
-static bool jacobi_plan(int m, int& split, int& rows_per, int& tab, size_t& bytes) {
+static bool jacobi_plan(int m, int least, int& split, int& rows_per, int& tab, size_t& bytes) {
   const size_t limit = 232448 - 5120;                // 227 KB less the static tables
   const size_t a_bytes = (size_t)((m * (m + 1) / 2 + 1) & ~1) * sizeof(T);
   const size_t tab_bytes = (size_t)(m / 2) * (m / 2 + 1) / 2 * sizeof(unsigned);
-  for (split = 1; split <= m; ++split) {
+  for (split = least; split <= m; ++split) {
     rows_per = (m + split - 1) / split;
     const size_t v_bytes = (size_t)(((size_t)rows_per * m + 1) & ~(size_t)1) * sizeof(T);
     if (a_bytes + v_bytes <= limit) {
@@ -215,18 +252,21 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
   const long long sA = (long long)n * n, sV = (long long)m * m, sw = n;
   // above n = 64 one CTA per SM is resident anyway (shared memory): 1024 threads
   const int threads = m <= 32 ? 128 : (m <= 64 ? 256 : 1024);
+  // A round updates m^2 / 8 blocks of A, in every CTA, and m^2 / 2 elements of V: while SMs are
+  // free, V's rows are shared by up to 16 CTAs (n = 208, FP32: 0.84 ms a sweep with 2 CTAs)
+  const int least = max(1, min(min(16, 152 / batch), m / 8));
   int split = 1, rows_per = m, tab = 0;
   size_t bytes = 0;
   if (!fp32) {
-    if (m / 2 > 68 || !jacobi_plan<double>(m, split, rows_per, tab, bytes) || split != 1) {
+    if (m / 2 > 68 || !jacobi_plan<double>(m, least, split, rows_per, tab, bytes)) {
       pcg_set_error("pcg_jacobi_eigh: FP64 variant needs n <= 136");
       return PCG_ERR_UNSUPPORTED;
     }
     PCG_CUDA(cudaFuncSetAttribute(k_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_jacobi<double><<<batch, threads, bytes, s>>>(n, m, 1, m, A, sA, (double*)V, sV, (const double*)V0, w, sw,
-                                                   max_sweeps, tol, info, tab);
+    k_jacobi<double><<<batch * split, threads, bytes, s>>>(n, m, split, rows_per, A, sA, (double*)V, sV,
+                                                           (const double*)V0, w, sw, max_sweeps, tol, info, tab);
   } else {
-    if (m / 2 > 167 || !jacobi_plan<float>(m, split, rows_per, tab, bytes)) {
+    if (m / 2 > 167 || !jacobi_plan<float>(m, least, split, rows_per, tab, bytes)) {
       pcg_set_error("pcg_jacobi_eigh: FP32 variant needs n <= 334");
       return PCG_ERR_UNSUPPORTED;
     }

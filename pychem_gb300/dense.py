@@ -29,9 +29,10 @@ def _mat(t, trans):
     return (c, r, sc, sr, sb) if trans else (r, c, sr, sc, sb)
 
 
-def mm(A, B, ta=False, tb=False, out=None, alpha=1.0, beta=0.0):
+def mm(A, B, ta=False, tb=False, out=None, alpha=1.0, beta=0.0, sym=False):
     """out = alpha op(A) op(B) + beta out for FP64 CUDA tensors (2-D, or 3-D batched with
-    the same batch), op = transpose when ta / tb."""
+    the same batch), op = transpose when ta / tb.  sym: the result is symmetric (2-D; half
+    of it is formed and mirrored)."""
     M, K, sAm, sAk, sAb = _mat(A, ta)
     K2, N, sBk, sBn, sBb = _mat(B, tb)
     if K != K2:
@@ -41,6 +42,12 @@ def mm(A, B, ta=False, tb=False, out=None, alpha=1.0, beta=0.0):
         shape = (batch, M, N) if (A.dim() == 3 or B.dim() == 3) else (M, N)
         out = torch.empty(shape, dtype=torch.float64, device=A.device)
         beta = 0.0
+    if sym:
+        if M != N or out.dim() != 2:
+            raise ValueError("mm: a symmetric product is one square matrix")
+        _lib.call("pcg_dgemm_sym", M, K, float(alpha), _p(A), sAm, sAk, _p(B), sBk, sBn, float(beta), _p(out),
+                  out.stride(0), out.stride(1), _stream())
+        return out
     sCb = out.stride(0) if out.dim() == 3 else 0
     _lib.call("pcg_dgemm", batch, M, N, K, float(alpha), _p(A), sAb, sAm, sAk, _p(B), sBb, sBk, sBn, float(beta),
               _p(out), sCb, out.stride(-2), out.stride(-1), _stream())
@@ -54,6 +61,14 @@ def oa_correction(S, R, nocc, mode, delta=None, E=None, lam=None):
     _lib.call("pcg_oa_correction", n, nocc, mode, _p(delta) if delta is not None else None, _p(S), _p(R), _p(E),
               _p(lam) if lam is not None else None, _stream())
     return E
+
+
+def projector_check(S, R, nocc, out=None):
+    """(max |R|, largest occupied-virtual element of S, max S_ii occupied - min S_jj
+    virtual) as a device vector."""
+    out = torch.empty(3, dtype=torch.float64, device=S.device) if out is None else out
+    _lib.call("pcg_projector_check", S.shape[0], nocc, _p(S), _p(R), _p(out), _stream())
+    return out
 
 
 def inv_sqrt(S, max_iter=60, tol=1e-13):

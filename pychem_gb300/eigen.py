@@ -97,8 +97,8 @@ def _rs(A, X, need_s=True):
     """R = I - X^T X and S = X^T A X on the library GEMM."""
     n = X.shape[-1]
     R = torch.eye(n, dtype=torch.float64, device=X.device)
-    dense.mm(X, X, ta=True, out=R, alpha=-1.0, beta=1.0)
-    S = dense.mm(X, dense.mm(A, X), ta=True) if need_s else None
+    dense.mm(X, X, ta=True, out=R, alpha=-1.0, beta=1.0, sym=True)
+    S = dense.mm(X, dense.mm(A, X), ta=True, sym=True) if need_s else None
     return R, S
 
 
@@ -150,9 +150,7 @@ def refine_projector(A, X, nocc, steps=2, check=False, ortho_steps=1):
     if not check:
         return lam, X
     R, S = _rs(A, X)
-    d = torch.diagonal(S)
-    chk = torch.stack([R.abs().amax(), S[:nocc, nocc:].abs().amax(), d[:nocc].amax() - d[nocc:].amin()])
-    return lam, X, chk
+    return lam, X, dense.projector_check(S, R, nocc)
 
 
 EXACT_BLOCK = 64    # exact_eigh finishes blocks up to this size with the FP64 Jacobi kernel

@@ -146,7 +146,9 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     F = torch.empty(n, n, dtype=torch.float64, device=dev)
     G = torch.empty(n, n, dtype=torch.float64, device=dev)
     Fp = torch.empty(n2, n2, dtype=torch.float64, device=dev)
+    P = torch.empty(n2, n2, dtype=torch.float64, device=dev)
     R = torch.empty(n2, n2, dtype=torch.float64, device=dev)
+    part = torch.empty(192, dtype=torch.float64, device=dev)
     Fx = torch.empty(n2, n2, dtype=torch.float64, device=dev)
     Q = torch.eye(n2, dtype=torch.float64, device=dev)
     C = torch.empty(n, n2, dtype=torch.float64, device=dev)
@@ -157,13 +159,10 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
 
     def fock_and_diis(use_diis):
         engine.fock(D, out=F, G=G)
-        mm(X, mm(F, X), ta=True, out=Fp)
-        P = mm(Dp, Fp)
-        torch.sub(P, P.T, out=R)
-        vals[0] = torch.sum(D * (H + F))
-        vals[1] = torch.sqrt(torch.mean((D - Dold) ** 2))
-        vals[5] = R.abs().amax()
-        Dold.copy_(D)
+        mm(X, mm(F, X), ta=True, out=Fp, sym=True)
+        mm(Dp, Fp, out=P)
+        _lib.call("pcg_scf_stats", n, n2, dense._p(P), dense._p(D), dense._p(H), dense._p(F), dense._p(Dold),
+                  dense._p(R), dense._p(part), dense._p(vals), _stream())
         if use_diis:
             diis.step(Fp, R, Fx)
         else:
@@ -174,8 +173,8 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
         if big:
             ozaki_gemm_tc(C, C, D, n, n, nocc, n2, (1, n2), (n, 1))      # D = C_occ C_occ^T
         else:
-            mm(C[:, :nocc], C[:, :nocc], tb=True, out=D)
-        mm(Q[:, :nocc], Q[:, :nocc], tb=True, out=Dp)
+            mm(C[:, :nocc], C[:, :nocc], tb=True, out=D, sym=True)
+        mm(Q[:, :nocc], Q[:, :nocc], tb=True, out=Dp, sym=True)
 
     def diag_exact():
         if big:
