@@ -170,9 +170,10 @@ extern "C" int pcg_dgemm(int batch, int M, int N, int K, double alpha, const dou
     return PCG_ERR_ARG;
   }
   if (M == 0 || N == 0) return PCG_OK;
-  // 32 x 32 tiles from two a SM on, where they waste no more than 8 x 8 ones do
+  // 32 x 32 tiles from two a SM on, for products long enough to fill their pipeline (a batch
+  // of 1,024 x 30 x 30 x 30: 77 us against 47 with 8 x 8 tiles)
   const long long tn = (N + DT_T - 1) / DT_T, tm = (M + DT_T - 1) / DT_T;
-  if (batch * tn * tm >= 304 && tm <= 65535 && 4LL * M * N >= 3LL * tm * tn * DT_T * DT_T) {
+  if (batch * tn * tm >= 304 && tm <= 65535 && M >= 64 && N >= 64 && K >= 64) {
     k_dgemm_tile<<<dim3((unsigned)tn, (unsigned)tm, batch), 64, 0, (cudaStream_t)stream>>>(
         M, N, K, alpha, A, sAb, sAm, sAk, B, sBb, sBk, sBn, beta, C, sCb, sCm, sCn);
     PCG_CUDA(cudaGetLastError());

@@ -20,7 +20,7 @@
 // element and quartet fills (1.25 ms).  A thread therefore takes `run` consecutive quartets: lists
 // run through the kets (C, D) of one bra in order, so D_ab, D_ac, D_bc are loaded and G_ab,
 // G_ac, G_bc written once a run of equal (A, B) and C, and the lanes of a warp touch neighbouring
-// columns (run = 1, 2, 4, 8: 1.6, 1.1, 1.0, 1.2 ms).  All factors are powers of two and are
+// columns (run = 1, 2, 4, 8: 1.64, 1.06, 0.92, 1.00 ms).  All factors are powers of two and are
 // applied to exponents by integer operations, off the FP64 pipe.
 #pragma once
 #include "common.cuh"
@@ -39,13 +39,14 @@ struct DigestArgs {
   unsigned d0;                 // first density of the launch
 };
 
-// x 2^k, |k| <= 7, by its exponent; the few values near the ends of the range (and zero,
-// infinities, NaNs) take the exact route
+// x 2^k, |k| <= 7, by its exponent; zero, infinities and NaNs stay what they are, below 2^-1015
+// is zero and beyond 2^1008 unscaled.  Selects, no branch: a branch an integral would keep the
+// loads of a block from being in flight together (1.6 times the time).
 __device__ __forceinline__ double dg_scale(double x, int k) {
-  const int hi = __double2hiint(x);
+  const int hi = __double2hiint(x), lo = __double2loint(x);
   const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  if (e - 8u < 0x7e8u) return __hiloint2double(hi + (k << 20), __double2loint(x));
-  return e < 8u ? 0.0 : x * __hiloint2double((1023 + k) << 20, 0);
+  const bool small = e < 8u, usual = e - 8u < 0x7e8u;
+  return __hiloint2double(small ? 0 : (usual ? hi + (k << 20) : hi), small ? 0 : lo);
 }
 
 template <int R, int C>
@@ -103,13 +104,20 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
         for (int j = 0; j < C; ++j) v[i][j] += __ldg(a.D[1] + o + (co ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j));
     }
   };
+  // the next quartet and its ket (AO of C | (C == D) << 30, AO of D, block offset) are loaded
+  // while this one is digested
+  int2 next = __ldg(a.tasks + (int)first);
+  int4 pn = a.pr.p.ao4 ? __ldg(a.pr.p.ao4 + next.y) : make_int4(0, 0, 0, 0);
   for (int t = (int)first; t < t1; ++t) {
-    const int2 tk = a.tasks[t];
+    const int2 tk = next;
+    const int4 pk = pn;
+    if (t + 1 < t1) {
+      next = __ldg(a.tasks + t + 1);
+      if (a.pr.p.ao4) pn = __ldg(a.pr.p.ao4 + next.y);
+    }
     int c, d;
     bool scd;
-    int4 pb, pk;                       // (AO of A | (A == B) << 30, AO of B, block offset)
     if (a.pr.p.ao4) {
-      pk = __ldg(a.pr.p.ao4 + tk.y);
       c = pk.x & 0x3FFFFFFF; d = pk.y; scd = (pk.x >> 30) & 1;
     } else {
       const int C = __ldg(a.pr.p.A + tk.y), Dd = __ldg(a.pr.p.B + tk.y);
@@ -120,7 +128,7 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
       if (bra >= 0) dg_add(a.GJ + o, oa, ob, n, JK, false, gab);
       bra = tk.x;
       if (a.pr.p.ao4) {
-        pb = __ldg(a.pr.p.ao4 + bra);
+        const int4 pb = __ldg(a.pr.p.ao4 + bra);
         oa = pb.x & 0x3FFFFFFF; ob = pb.y; sab = (pb.x >> 30) & 1;
         o = dens + ((long long)(unsigned)pb.z | ((long long)pb.w << 32));
       } else {

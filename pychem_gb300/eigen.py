@@ -1,9 +1,9 @@
 """Symmetric eigensolver for the SCF on the GPU (replaces numpy.linalg.eigh of
 ``Methods/hartree_fock.py:172-175,226``), on the library's own kernels only:
 
-* n <= 136: parallel cyclic Jacobi in FP64, one CTA per matrix (pcg_jacobi_eigh),
-  batched over any leading dimension.
-* larger n: the FP32 variant of the Jacobi kernel (FP32-accurate vectors, n <= 334),
+* batches with n <= 136, and single matrices of n <= 32: parallel cyclic Jacobi in FP64
+  (pcg_jacobi_eigh), one CTA per matrix in a batch.
+* single matrices of larger n: the FP32 variant of the Jacobi kernel (FP32-accurate vectors, n <= 334),
   then FP64 iterative refinement (T. Ogita and K. Aishima, "Iterative refinement for
   symmetric eigenvalue decomposition", Japan J. Indust. Appl. Math. 35 (2018)
   1007-1035, Algorithm 1) with the library's FP64 GEMM (pcg_dgemm) and correction
@@ -21,6 +21,10 @@ from . import _lib, dense
 from ._stream import stream as _stream
 
 FP64_JACOBI_MAX_N = 136
+# single matrices above this size go through FP32 Jacobi and FP64 refinement: an FP64 sweep of
+# one matrix is n - 1 rounds bound by one SM's FP64 pipe (an SCF iteration of 104 functions
+# took 3 to 6 ms in it, 0.9 ms refined)
+FP64_JACOBI_ONE_N = 32
 
 # counts of eigh calls by route (exact library solve, refinement, refinement rejected)
 stats = {"exact": 0, "refined": 0, "fallback": 0}
@@ -167,6 +171,13 @@ def _split_point(w, n, base=EXACT_BLOCK):
     return lo + int(torch.argmax(gaps))
 
 
+def _gap(w, s):
+    """Whether the ascending FP32-accurate spectrum w has a gap at s that its errors (about
+    1e-6 of the largest level) leave open."""
+    lo, hi, size = torch.stack([w[s - 1], w[s], w.abs().amax()]).tolist()
+    return hi - lo > 1e-5 * size
+
+
 def exact_eigh(A, X_prev=None, steps=4):
     """Eigenpairs of one symmetric A to FP64 accuracy on the library's kernels, by
     spectrum slicing (exact_eigh_many with one matrix)."""
@@ -226,19 +237,19 @@ def exact_eigh_many(As, X_prevs=None, steps=4):
     for r, (a, B) in enumerate(roots):
         n = a.shape[0]
         V = V32[r, :n, :n]
-        if n <= EXACT_BLOCK:
-            V = orthonormalize(V)       # FP32-orthonormal -> FP64 (parts get it from refinement)
+        V = orthonormalize(V)           # FP32-orthonormal -> FP64
         todo.append((r, a, B, w32[r, :n], V))
     leaves = []
     while todo:
         r, a, B, w, V = todo.pop()
         n = a.shape[0]
-        if n <= EXACT_BLOCK:
-            # the part in the basis V, where it is nearly diagonal
+        s = _split_point(w, n) if n > EXACT_BLOCK else 0
+        if n <= EXACT_BLOCK or (n <= FP64_JACOBI_MAX_N and not _gap(w, s)):
+            # the part in the basis V, where it is nearly diagonal; a cluster that leaves no gap
+            # to slice at stays whole where the FP64 kernel takes it
             Ap = dense.mm(V, dense.mm(a, V), ta=True)
             leaves.append((r, 0.5 * (Ap + Ap.T), V if B is None else dense.mm(B, V)))
             continue
-        s = _split_point(w, n)
         _, V = refine_projector(a, V, s, steps=steps)
         for blk in (V[:, :s], V[:, s:]):
             Ab = dense.mm(blk, dense.mm(a, blk), ta=True)
@@ -257,16 +268,27 @@ def exact_eigh_many(As, X_prevs=None, steps=4):
     return [_sort(torch.cat(wl), torch.cat(vl, dim=1)) for wl, vl in parts]
 
 
+def _eigh_scaled(A, X_prev):
+    """exact_eigh of A times a power of two that brings its largest element to order one
+    (its FP32 stage has FP32's range)."""
+    e = torch.frexp(A.abs().amax()).exponent.clamp(-1020, 1020)
+    w, V = exact_eigh(torch.ldexp(A, -e), X_prev)
+    return torch.ldexp(w, e), V
+
+
 def eigh(A, X_prev=None, refine_steps=2, exact=True, check_tol=1e-10, nocc=None):
     """Ascending eigenvalues and eigenvectors of symmetric FP64 A (..., n, n).
 
-    n <= 136: batched FP64 Jacobi (exact to rounding; the small-molecule ensemble).
-    Larger n (one matrix): exact=True or no X_prev -- spectrum slicing (exact_eigh);
+    n <= 136 in a batch, n <= 32 alone or while the stream is captured: FP64 Jacobi
+    (exact to rounding).  One matrix of n <= 136: spectrum slicing (exact_eigh) on the matrix
+    scaled to order one.  Larger n (one matrix): exact=True or no X_prev -- spectrum slicing (exact_eigh);
     otherwise refinement from X_prev (consecutive SCF iterations): with nocc, only the
     occupied-space projector is converged (checked: orthonormal, decoupled, gapped;
     else the exact route); without nocc, full refinement (checked for orthogonality,
     else the exact route)."""
     n = A.shape[-1]
+    if FP64_JACOBI_ONE_N < n <= FP64_JACOBI_MAX_N and A.dim() == 2 and not torch.cuda.is_current_stream_capturing():
+        return _eigh_scaled(A, X_prev)
     if n <= FP64_JACOBI_MAX_N:
         if X_prev is not None:
             shape = A.shape

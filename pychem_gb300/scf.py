@@ -43,11 +43,12 @@ def orthogonaliser(S, canonical=False):
     do not depend on the choice of X; otherwise the canonical route."""
     from . import dense
     n = S.shape[0]
-    if not canonical and n > eigen.FP64_JACOBI_MAX_N:
+    if not canonical and n > eigen.FP64_JACOBI_ONE_N:
         X, ok = dense.inv_sqrt(S)
         if ok:
             # power iteration on X^2 = S^-1, on the device; the host reads the result once
-            v = torch.ones(n, 1, dtype=S.dtype, device=S.device) / math.sqrt(n)
+            # (a start without the molecule's symmetry, which would hide some vectors)
+            v = torch.cos(1.7 * torch.arange(1, n + 1, dtype=S.dtype, device=S.device)).unsqueeze(1)
             for _ in range(16):
                 w = dense.mm(X, dense.mm(X, v))
                 nrm = torch.linalg.vector_norm(w)
@@ -110,7 +111,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     kernels: Fock digestion, FP64 GEMMs (pcg_dgemm), the eigenvectors (Jacobi for the
     first exact_iters iterations, then refinement of the previous vectors that
     decouples the occupied space, checked, with the Jacobi route when the check
-    fails; for n <= 136 the FP64 Jacobi kernel in every iteration), the density
+    fails; for n <= 32 the FP64 Jacobi kernel in every iteration), the density
     C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc, n > 136).  With graph None or
     True every iteration after the first exact_iters is one CUDA graph replay followed
     by one read of six numbers (energy, density change, refinement checks, commutator
@@ -125,10 +126,11 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     dev = S.device
     e_nuc = mol.nuclear_repulsion()
     n = engine.nbf
-    big = n > eigen.FP64_JACOBI_MAX_N
     use_graph = graph is None or graph
     X = orthogonaliser(S)
     n2 = X.shape[1]
+    # refined vectors instead of a Jacobi solve an iteration (with both spaces to decouple)
+    big = n > eigen.FP64_JACOBI_ONE_N and 0 < nocc < n2
     mm = dense.mm
 
     # static buffers (the CUDA graph reads and writes these addresses)
@@ -170,7 +172,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
 
     def density():
         mm(X, Q, out=C)
-        if big:
+        if n > eigen.FP64_JACOBI_MAX_N:
             ozaki_gemm_tc(C, C, D, n, n, nocc, n2, (1, n2), (n, 1))      # D = C_occ C_occ^T
         else:
             mm(C[:, :nocc], C[:, :nocc], tb=True, out=D, sym=True)
@@ -181,12 +183,13 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
             # a few FP32 Jacobi sweeps put the occupied space well inside the HOMO-LUMO
             # gap; the projector refinement does the rest in FP64
             _, V = eigen.eigh32_own(Fx, Q if have_q[0] else None, tol=1e-4, max_sweeps=5)
-            _, V = eigen.refine_projector(Fx, V, nocc, steps=3)
+            _, V, chk = eigen.refine_projector(Fx, V, nocc, steps=3, check=True)
+            vals[2:5] = chk
         else:
             _, V = eigen.eigh(Fx, X_prev=Q if have_q[0] else None)
+            vals[2:5] = 0.0
         Q.copy_(V)
         have_q[0] = True
-        vals[2:5] = 0.0
 
     def diag_refine():
         _, V, chk = eigen.refine_projector(Fx, Q, nocc, steps=2, check=True)
@@ -250,7 +253,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
         if record and it <= 2:
             phases["iteration%d" % it] = time.perf_counter()
         E = float(host[0]) + e_nuc
-        if not exact:
+        if not exact or (big and n <= eigen.FP64_JACOBI_MAX_N):
             if scale is None:
                 scale = max(float(Fx.abs().amax()), 1.0)
             # the refined occupied space need only be as good as the SCF itself: Q stays
@@ -261,16 +264,21 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
             ok = host[2] <= 1e-10 and host[3] <= ov_tol and host[4] < 0.0
             if not ok:
                 # refinement not yet converged (a large step early on): more steps from
-                # where it stopped, then the Jacobi route
+                # where it stopped, then the Jacobi route (for n <= 136 the FP64 kernel, at
+                # once when there is no gap between the spaces)
                 fallbacks += 1
-                for _ in range(4):
+                jacobi64 = n <= eigen.FP64_JACOBI_MAX_N
+                rounds = 0 if jacobi64 and not (np.isfinite(host[2:5]).all() and host[4] < 0.0) else 4
+                for _ in range(rounds):
                     _, V, chk = eigen.refine_projector(Fx, Q, nocc, steps=3, check=True, ortho_steps=2)
                     Q.copy_(V)
                     c = chk.cpu().numpy()
                     if c[0] <= 1e-10 and c[1] <= ov_tol and c[2] < 0.0:
                         ok = True
                         break
-                if not ok:
+                if not ok and jacobi64:
+                    Q.copy_(eigen.eigh(Fx.unsqueeze(0))[1][0])
+                elif not ok:
                     diag_exact()
                 density()
         if E_old is not None:
@@ -285,20 +293,27 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
                 break
         E_old = E
     # orbitals of the final Fock matrix, exact (including inside near-degenerate
-    # clusters) for MP2's denominators: for n > 136 the occupied and virtual blocks of
+    # clusters) for MP2's denominators: for n > 32 the occupied and virtual blocks of
     # the refined vectors are decoupled once more and each block is diagonalised
-    # exactly (spectrum slicing inside blocks above 136)
+    # exactly (spectrum slicing inside blocks above 64)
     if record:
         torch.cuda.synchronize()
         phases["loop"] = time.perf_counter()
     Ff = mm(X, mm(F, X), ta=True)
+    split = big
     if big:
-        _, V = eigen.refine_projector(Ff, Q, nocc, steps=2)
+        _, V, chk = eigen.refine_projector(Ff, Q, nocc, steps=2, check=True)
+        if n <= eigen.FP64_JACOBI_MAX_N:
+            c = chk.cpu().numpy()
+            split = c[0] <= 1e-10 and c[1] <= 1e-8 * max(scale or 1.0, 1.0) and c[2] < 0.0
+    if split:
         blks = (V[:, :nocc], V[:, nocc:])
         Abs = [mm(blk, mm(Ff, blk), ta=True) for blk in blks]
         res = eigen.exact_eigh_many([0.5 * (Ab + Ab.T) for Ab in Abs])
         eps = torch.cat([wb for wb, _ in res])
         Qf = torch.cat([mm(blk, Ub) for blk, (_, Ub) in zip(blks, res)], dim=1)
+    elif n <= eigen.FP64_JACOBI_MAX_N:
+        eps, Qf = (t[0] for t in eigen.eigh(Ff.unsqueeze(0)))
     else:
         eps, Qf = eigen.eigh(Ff, exact=True)
     Cf = mm(X, Qf)

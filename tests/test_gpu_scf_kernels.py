@@ -94,3 +94,72 @@ def test_fp32_jacobi_shared_matrix(n, batch):
     size = float(A.abs().amax()) * n ** 0.5
     assert float((V.transpose(1, 2) @ V - torch.eye(n, **F64)).abs().max()) < 1e-4
     assert float((A @ V - V * w.unsqueeze(1)).abs().max()) < 1e-4 * size
+
+
+@pytest.mark.parametrize("n", [32, 33, 52, 64, 65, 104, 136])
+@pytest.mark.parametrize("scale", [1.0, 1e-150, 1e150])
+def test_one_matrix(n, scale):
+    """Both sides of the sizes where a single matrix changes route; a cluster of equal levels."""
+    from pychem_gb300 import eigen
+    Q, _ = torch.linalg.qr(torch.randn(n, n, generator=_gen(n), **F64))
+    lam = torch.linspace(-2.0, 5.0, n, **F64)
+    lam[: n // 4] = -20.0
+    A = (Q * lam) @ Q.T
+    A = 0.5 * (A + A.T)
+    for X in (None, Q):
+        w, V = eigen.eigh(A * scale, X_prev=X)
+        w = w / scale
+        assert float((w - lam).abs().max()) < 2e-11
+        assert float((A @ V - V * w).abs().max()) < 2e-11
+        assert float((V.T @ V - torch.eye(n, **F64)).abs().max()) < 1e-13
+    w, V = eigen.eigh(torch.zeros(n, n, **F64))
+    assert float(w.abs().max()) == 0.0 and float((V.T @ V - torch.eye(n, **F64)).abs().max()) < 1e-13
+
+
+@pytest.mark.parametrize("atoms", [6, 8])
+def test_rhf_without_virtual_orbitals(atoms):
+    """Every orbital occupied (neon atoms in a minimal basis, 30 and 40 functions)."""
+    from pychem_gb300.engine import GpuEngine
+    from pychem_gb300.molecule import Molecule
+    from pychem_gb300.scf import rhf
+    one = rhf(GpuEngine(Molecule([["NE", 10.0, 0.0, 0.0, 0.0]], "STO-3G")).prepare()).E
+    r = rhf(GpuEngine(Molecule([["NE", 10.0, 30.0 * k, 0.0, 0.0] for k in range(atoms)], "STO-3G")).prepare())
+    assert r.converged and abs(r.E - atoms * one) < 1e-7
+
+
+@pytest.mark.parametrize("n", [40, 65, 100, 136])
+def test_one_matrix_without_gaps(n):
+    """Multiples of the identity, and clusters wider than a part of the sliced spectrum."""
+    from pychem_gb300 import eigen
+    Q, _ = torch.linalg.qr(torch.randn(n, n, generator=_gen(n), **F64))
+    for lam in (torch.ones(n, **F64), torch.cat([torch.zeros(n - 3, **F64), torch.ones(3, **F64)]),
+                1.0 + 1e-9 * torch.arange(n, **F64)):
+        A = (Q * lam) @ Q.T
+        A = 0.5 * (A + A.T)
+        w, V = eigen.eigh(A)
+        assert float((w - lam).abs().max()) < 1e-12
+        assert float((A @ V - V * w).abs().max()) < 1e-12
+        assert float((V.T @ V - torch.eye(n, **F64)).abs().max()) < 1e-13
+
+
+def test_rhf_without_a_gap():
+    """A square of hydrogen atoms (degenerate frontier orbitals) among distant helium atoms, 36
+    functions: the route with refined vectors gives the Jacobi route's energies."""
+    from pychem_gb300 import eigen
+    from pychem_gb300.engine import GpuEngine
+    from pychem_gb300.molecule import Molecule
+    from pychem_gb300.scf import rhf
+    coords = [["H", 1.0, x, y, 0.0] for x in (0.0, 1.2) for y in (0.0, 1.2)]
+    coords += [["HE", 2.0, 6.0 + 3.0 * k, 0.0, 0.0] for k in range(14)]
+    eng = GpuEngine(Molecule(coords, "6-31G")).prepare()
+    assert eng.nbf > eigen.FP64_JACOBI_ONE_N
+    got = rhf(eng, max_iter=60)
+    old = eigen.FP64_JACOBI_ONE_N
+    eigen.FP64_JACOBI_ONE_N = eigen.FP64_JACOBI_MAX_N
+    try:
+        want = rhf(eng, max_iter=60)
+    finally:
+        eigen.FP64_JACOBI_ONE_N = old
+    assert bool(torch.isfinite(got.eps).all()) and bool(torch.isfinite(got.D).all())
+    assert got.converged == want.converged
+    assert not want.converged or abs(got.E - want.E) < 1e-7
