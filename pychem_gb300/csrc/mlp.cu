@@ -15,7 +15,7 @@
 // A CTA owns a 128 x 64 tile; eight producer warps load 32 columns of K at a time (16-byte
 // loads where the operand is contiguous along k and aligned, coalesced along m or n where it
 // is contiguous there), split and store them K-major and 64-byte swizzled through three
-// stages, one thread issues the MMAs.  64 columns give 132 CTAs at 4,097 rows x 256, one
+// stages, one warp issues the MMAs.  64 columns give 132 CTAs at 4,097 rows x 256, one
 // wave of the 152 SMs; the split of A is repeated for each of the 4 column tiles, which costs
 // less than idle SMs.  The weight gradient contracts over the rows: its few output tiles
 // (8 for 256 x 256) are split along the rows into partial sums, as many as fill the GPU,
@@ -132,14 +132,14 @@ __global__ void __launch_bounds__(ML_THREADS, 2) k_gemm(const MlArgs a) {
   uint64_t* bars = (uint64_t*)(sm + ML_STAGES * Cfg::STAGE);     // full[3], empty[3], done
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * ML_STAGES + 1);
   volatile int* abort_s = (volatile int*)(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int ntn = (a.N + ML_BN - 1) / ML_BN;
   const int m0 = (int)(blockIdx.x / ntn) * ML_BM, n0 = (int)(blockIdx.x % ntn) * ML_BN;
   const int nall = (a.K + ML_BK - 1) / ML_BK;
   const int c0 = (int)((long long)nall * blockIdx.y / a.splits), c1 = (int)((long long)nall * (blockIdx.y + 1) / a.splits);
   if (threadIdx.x == 0) {
     for (int i = 0; i < ML_STAGES; ++i) {
-      mbar_init(&bars[i], ML_PROD);
+      mbar_init(&bars[i], ML_PROD / 32);
       mbar_init(&bars[ML_STAGES + i], 1);
     }
     mbar_init(&bars[2 * ML_STAGES], 1);
@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(ML_THREADS, 2) k_gemm(const MlArgs a) {
         }
       }
       fence_proxy_async_smem();
-      mbar_arrive(&bars[st]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[st]);
     }
     if (!ok) { *abort_s = 1; atomicExch(&g_mlp_err, 1); }
     if (ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s)) {
@@ -271,15 +272,19 @@ __global__ void __launch_bounds__(ML_THREADS, 2) k_gemm(const MlArgs a) {
       atomicExch(&g_mlp_err, 1);
       if (a.colsum && m0 == 0) asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
     }
-  } else if (lane == 0) {
+  } else {
     const uint32_t idesc = idesc_bf16_f32(ML_BM, ML_BN);
+    const uint32_t lead = elect_one();
+    const uint64_t xd0 = sdesc_k_sw64(smem_u32(sm));
     bool ok = true;
     unsigned have = 0;       // accumulators that hold a sum; 3: the corrections
     for (int it = 0; it < c1 - c0; ++it) {
       const int st = it % ML_STAGES;
-      if (!mbar_wait(&bars[st], (it / ML_STAGES) & 1, ML_WAIT, abort_s)) { ok = false; break; }
+      ok = mbar_wait(&bars[st], (it / ML_STAGES) & 1, ML_WAIT, abort_s);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t xa = smem_u32(sm + st * Cfg::STAGE), xb = xa + 3 * Cfg::AT;
+      const uint64_t xd = xd0 + (uint64_t)(st * (Cfg::STAGE >> 4)), yd = xd + (3 * Cfg::AT >> 4);
 #pragma unroll
       for (int kk = 0; kk < ML_BK / 16; ++kk) {
 #pragma unroll
@@ -288,20 +293,21 @@ __global__ void __launch_bounds__(ML_THREADS, 2) k_gemm(const MlArgs a) {
           for (int q = 0; q < Cfg::SB; ++q) {
             if (p + q > 3) continue;
             const int acc = p + q == 0 ? (it * (ML_BK / 16) + kk) % 3 : 3;
-            umma_bf16(tmem + acc * ML_BN, sdesc_k_sw64(xa + p * Cfg::AT + kk * 32),
-                      sdesc_k_sw64(xb + q * Cfg::BT + kk * 32), idesc, (have >> acc) & 1u);
+            umma_bf16_lead(lead, tmem + acc * ML_BN, xd + ((p * Cfg::AT + kk * 32) >> 4),
+                           yd + ((q * Cfg::BT + kk * 32) >> 4), idesc, (have >> acc) & 1u);
             have |= 1u << acc;
           }
       }
-      umma_commit(&bars[ML_STAGES + st]);
+      umma_commit_lead(lead, &bars[ML_STAGES + st]);
     }
-    umma_commit(&bars[2 * ML_STAGES]);
+    umma_commit_lead(lead, &bars[2 * ML_STAGES]);
     if (!ok) {
       *abort_s = 1;
-      atomicExch(&g_mlp_err, 2);
+      if (lead) atomicExch(&g_mlp_err, 2);
       volatile int keep_waiting = 0;
       mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, &keep_waiting);   // drain before tensor memory is freed
     }
+    __syncwarp();
   }
   tc_fence_before();
   __syncthreads();

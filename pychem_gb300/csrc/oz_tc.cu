@@ -13,16 +13,17 @@
 //    by 32-column chunk, cut it into NS digit slices and store them BF16, K-major and
 //    64-byte swizzled, straight into the shared-memory operand tiles (no BF16 copy of
 //    X in global memory).  The exponent of each row comes from a first pass over the
-//    CTA's rows (the re-read is served by L2).
+//    tile's rows, column by column beside the chunks of the tile before (the re-read is
+//    served by L2; as a pass of its own it was a third of the time).
 //  * Y, the small operand (C_occ or C_vir: a few hundred columns), is split once by
 //    k_ozt_split_y into K-major BF16 slices in the caller's workspace (slice-major,
 //    [p][n][k]) and brought into shared memory tile by tile by the tensor memory
 //    accelerator (cp.async.bulk.tensor, 64-byte swizzle, completion counted on the
 //    stage's mbarrier).
-//  * One thread issues tcgen05.mma (M = 128, N = BN, K = 16, BF16 in, FP32 out) for
+//  * One warp issues tcgen05.mma (M = 128, N = BN, K = 16, BF16 in, FP32 out) for
 //    every slice pair with p + q <= NS + 1 into NS accumulators in tensor memory, one
 //    per level (NS * BN <= 512 columns), over a two-stage mbarrier pipeline.
-//  * The producer warps then read the level accumulators (tcgen05.ld), combine them in
+//  * Eight epilogue warps then read the level accumulators (tcgen05.ld), combine them in
 //    int64, scale by 2^{eX + eY} and write FP64 C with any strides (sCm = 1 gives
 //    coalesced stores of the transposed product, which is how the MP2 transforms chain).
 //
@@ -44,7 +45,8 @@
 #define OZT_BK 32
 #define OZT_PROD_WARPS 16
 #define OZT_PROD (OZT_PROD_WARPS * 32)
-#define OZT_THREADS (OZT_PROD + 32)
+#define OZT_EPI 256                          // threads of the epilogue warps
+#define OZT_THREADS (OZT_PROD + 32 + OZT_EPI)
 #define OZT_WAIT (1u << 24)
 
 template <int NS, int BN>
@@ -52,7 +54,7 @@ struct OztCfg {
   static constexpr int XT = OZT_BM * OZT_BK * 2;  // one X slice tile (bytes)
   static constexpr int YT = BN * OZT_BK * 2;      // one Y slice tile
   static constexpr int STAGE = NS * (XT + YT);
-  static constexpr int SMEM = 2 * STAGE + 1024 + 1024;  // two stages, alignment slack, barriers and exponents
+  static constexpr int SMEM = 2 * STAGE + 1024 + 2304;  // two stages, alignment slack, barriers and exponents
   static_assert(NS * BN <= 512, "level accumulators exceed tensor memory");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "MMA N");
   static_assert(YT % 512 == 0, "Y tiles must stay 512-byte aligned");
@@ -117,6 +119,14 @@ __device__ __forceinline__ void ozt_load8(const double* __restrict__ X, long lon
   }
 }
 
+// the high words of the same values
+__device__ __forceinline__ void ozt_load_hi8(const double* __restrict__ X, long long ldx, long long m, long long M, int kb,
+                                             int K, unsigned (&h)[8]) {
+  const unsigned* src = (const unsigned*)(X + m * ldx + kb) + 1;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = (m < M && kb + j < K) ? __ldg(src + 2 * j) : 0u;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -128,6 +138,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
+// One CTA an SM works through the row tiles blockIdx.x, + gridDim.x, ...: the producers go on to
+// the next tile's exponents and digits while the tensor core finishes a tile and eight epilogue
+// warps read its accumulators; the next tile's first MMA waits for them (the levels fill tensor
+// memory, so there is one set).  With a CTA a tile each of these phases was exposed, with the
+// launch and the tensor-memory allocation: 22 us a 128-row tile of K = 104 (2.4 us of MMAs).
 template <int NS, int BN>
 __global__ void __launch_bounds__(OZT_THREADS, 1)
     k_ozt_gemm(long long M, int N, int K, int Kp, int Npad, const double* __restrict__ X, long long ldx,
@@ -137,28 +152,30 @@ __global__ void __launch_bounds__(OZT_THREADS, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = sm;                                        // [stage][X slices | Y slices]
-  uint64_t* bars = (uint64_t*)(sm + 2 * Cfg::STAGE);  // full[2], empty[2], done, drain, ycopy[2]
-  uint32_t* tmem_slot = (uint32_t*)(bars + 8);
+  uint64_t* bars = (uint64_t*)(sm + 2 * Cfg::STAGE);  // full[2], empty[2], acc full, drain, ycopy[2], acc empty
+  uint32_t* tmem_slot = (uint32_t*)(bars + 9);
   volatile int* abort_s = (volatile int*)(tmem_slot + 1);
-  int* ex_s = (int*)(tmem_slot + 4);                           // 128 row exponent fields
+  // exponent fields of a tile's 128 rows.  Four sets: while the epilogue of tile i reads its
+  // own, two stages let the producers start tile i + 3 at most
+  int* ex_s = (int*)(tmem_slot + 6);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // linear grid, the N tiles of one row tile adjacent (they share its X rows in L2)
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  // the N tiles of one row tile are adjacent (they share its X rows in L2)
   const int ntn = (N + BN - 1) / BN;
-  const long long m0 = (long long)(blockIdx.x / ntn) * OZT_BM;
-  const int n0 = (int)(blockIdx.x % ntn) * BN;
+  const long long ntile = (M + OZT_BM - 1) / OZT_BM * ntn;
   const int nchunk = Kp / OZT_BK;
 
   if (threadIdx.x == 0) {
-    // full: every producer thread; ycopy: the expect_tx arrival of the thread that issues
+    // full: one arrival a producer warp (512 on one barrier are 512 turns at its address); ycopy: the expect_tx arrival of the thread that issues
     // the Y copies, completed by their bytes
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[i], OZT_PROD);
+      mbar_init(&bars[i], OZT_PROD_WARPS);
       mbar_init(&bars[2 + i], 1);
       mbar_init(&bars[6 + i], 1);
     }
-    mbar_init(&bars[4], 1);
+    mbar_init(&bars[4], 2);
     mbar_init(&bars[5], 1);
+    mbar_init(&bars[8], OZT_EPI / 32);
     *abort_s = 0;
     mbar_fence_init();
   }
@@ -171,137 +188,174 @@ __global__ void __launch_bounds__(OZT_THREADS, 1)
   if (warp < OZT_PROD_WARPS) {
     const int t = threadIdx.x;
     const bool vec = (ldx % 2 == 0) && (((uintptr_t)X & 15) == 0);
-    // ---- exponents of the CTA's 128 rows of X: four threads per row, each over a
-    // quarter of the row (even boundaries, so 16-byte loads stay aligned)
-    {
-      const int r = t >> 2, h = t & 3;
-      const long long m = m0 + r;
-      const int kq = ((K + 3) / 4 + 1) & ~1;
-      const int klo = h * kq < K ? h * kq : K, khi = (h + 1) * kq < K ? (h + 1) * kq : K;
-      unsigned long long mx = 0;
-      if (m < M && klo < khi) {
-        const double* row = X + m * ldx;
-        int k = klo;
-        if (vec) {
-#pragma unroll 8
-          for (; k + 2 <= khi; k += 2) {
-            const double2 q = __ldg((const double2*)(row + k));
-            mx = max(mx, max(oz_absbits(q.x), oz_absbits(q.y)));
-          }
-        }
-        for (; k < khi; ++k) mx = max(mx, oz_absbits(__ldg(row + k)));
-      }
-      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      if (h == 0) ex_s[r] = (int)(mx >> 52);
-    }
-    asm volatile("bar.sync 1, %0;" ::"r"(OZT_PROD));
     // this thread's 8-column item of every chunk: row r, column group g
     const int g = t & 3, r = t >> 2;
-    const int emax = ex_s[r];
     const uint32_t off = sw64_offset(r, g);
     bool ok = true;
     int ycopies[2] = {0, 0};  // Y copies issued per stage (thread 0)
-    for (int c = 0; c < nchunk; ++c) {
-      const int st = c & 1;
-      const int k0 = c * OZT_BK;
-      double v[8];
-      ozt_load8(X, ldx, m0 + r, M, k0 + 8 * g, K, vec, v);   // issued before the wait
-      if (c >= 2 && !mbar_wait(&bars[2 + st], ((c >> 1) + 1) & 1, OZT_WAIT, abort_s)) { ok = false; break; }
-      uint8_t* xt = tiles + st * Cfg::STAGE;
-      uint8_t* yt = xt + NS * Cfg::XT;
-      if (t == 0) {  // Y slices of this chunk by TMA
-        ++ycopies[st];
-        mbar_arrive_expect_tx(&bars[6 + st], NS * Cfg::YT);
-#pragma unroll 1
-        for (int p = 0; p < NS; ++p) tma_load_2d(smem_u32(yt + p * Cfg::YT), &ymap, k0, p * Npad + n0, &bars[6 + st]);
+    unsigned cc = 0;          // chunks so far
+    int set = 0;
+    // largest high word of this thread's items; a row's four threads are neighbours
+    unsigned mx = 0;
+    {
+      const long long m = (long long)blockIdx.x / ntn * OZT_BM + r;
+      for (int c = 0; c < nchunk; ++c) {
+        unsigned h[8];
+        ozt_load_hi8(X, ldx, m, M, c * OZT_BK + 8 * g, K, h);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mx = max(mx, h[j] & 0x7fffffffu);
       }
-      unsigned w[4][NS];
+    }
+    for (long long tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x, set = (set + 1) & 3) {
+      const long long m0 = tile / ntn * OZT_BM;
+      const int n0 = (int)(tile % ntn) * BN;
+      const bool more = tile + gridDim.x < ntile;
+      const long long mnext = (tile + gridDim.x) / ntn * OZT_BM + r;
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const int emax = (int)(mx >> 20);
+      if (g == 0) ex_s[set * OZT_BM + r] = emax;
+      mx = 0;
+      double v[8], nv[8];
+      ozt_load8(X, ldx, m0 + r, M, 8 * g, K, vec, nv);
+      for (int c = 0; c < nchunk; ++c, ++cc) {
+        const int st = cc & 1;
+        const int k0 = c * OZT_BK;
 #pragma unroll
-      for (int hh = 0; hh < 4; ++hh) oz_digits_bf16x2<NS>(v[2 * hh], v[2 * hh + 1], emax, w[hh]);
+        for (int j = 0; j < 8; ++j) v[j] = nv[j];
+        // while this chunk is split: the next one's values, and the same columns of the next
+        // tile for its exponents (which also brings the tile to L2)
+        if (c + 1 < nchunk) ozt_load8(X, ldx, m0 + r, M, k0 + OZT_BK + 8 * g, K, vec, nv);
+        unsigned h[8];
+        if (more) ozt_load_hi8(X, ldx, mnext, M, k0 + 8 * g, K, h);
+        if (cc >= 2 && !mbar_wait(&bars[2 + st], ((cc >> 1) + 1) & 1, OZT_WAIT, abort_s)) ok = false;
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        uint8_t* xt = tiles + st * Cfg::STAGE;
+        uint8_t* yt = xt + NS * Cfg::XT;
+        if (t == 0) {  // Y slices of this chunk by TMA
+          ++ycopies[st];
+          mbar_arrive_expect_tx(&bars[6 + st], NS * Cfg::YT);
+#pragma unroll 1
+          for (int p = 0; p < NS; ++p) tma_load_2d(smem_u32(yt + p * Cfg::YT), &ymap, k0, p * Npad + n0, &bars[6 + st]);
+        }
+        unsigned w[4][NS];
 #pragma unroll
-      for (int p = 0; p < NS; ++p)
-        *(uint4*)(xt + p * Cfg::XT + off) = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
-      fence_proxy_async_smem();
-      mbar_arrive(&bars[st]);
+        for (int hh = 0; hh < 4; ++hh) oz_digits_bf16x2<NS>(v[2 * hh], v[2 * hh + 1], emax, w[hh]);
+#pragma unroll
+        for (int p = 0; p < NS; ++p)
+          *(uint4*)(xt + p * Cfg::XT + off) = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[st]);
+        if (more) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) mx = max(mx, h[j] & 0x7fffffffu);
+        }
+      }
     }
     if (!ok) { *abort_s = 1; atomicExch(err, 1); }
-    if (t == 0 && *abort_s) {  // let this thread's Y copies land before the CTA exits
+    // the last copies land before the CTA exits: the MMA warp has waited for them unless a
+    // wait gave up
+    if (t == 0 && *abort_s) {
       volatile int keep_waiting = 0;
       for (int i = 0; i < 2; ++i)
         if (ycopies[i]) mbar_wait(&bars[6 + i], (ycopies[i] - 1) & 1, OZT_WAIT, &keep_waiting);
     }
-    // ---- epilogue: wait for the last MMAs, combine the levels, write C
-    if (ok && mbar_wait(&bars[4], 0, OZT_WAIT, abort_s)) {
+  } else if (warp == OZT_PROD_WARPS) {
+    // ---- MMA issuer: the whole warp keeps in step, its leading lane issues
+    const uint32_t idesc = idesc_bf16_f32(OZT_BM, BN);
+    const uint32_t lead = elect_one();
+    const uint64_t xd0 = sdesc_k_sw64(smem_u32(tiles));
+    bool ok = true;
+    unsigned cc = 0, it = 0;
+    for (long long tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x, ++it) {
+      if (it && !mbar_wait(&bars[8], (it - 1) & 1, OZT_WAIT, abort_s)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
-      const int lg = warp & 3, quarter = warp >> 2;
-      const int re = 32 * lg + lane;
-      const long long m = m0 + re;
-      const int eme = ex_s[re];
+      for (int c = 0; c < nchunk && ok; ++c, ++cc) {
+        const int st = cc & 1;
+        ok = mbar_wait(&bars[st], (cc >> 1) & 1, OZT_WAIT, abort_s) &&
+             mbar_wait(&bars[6 + st], (cc >> 1) & 1, OZT_WAIT, abort_s);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        // descriptors count 16-byte units in their low bits
+        const uint64_t xd = xd0 + (uint64_t)(st * (Cfg::STAGE >> 4));
+        const uint64_t yd = xd + (NS * Cfg::XT >> 4);
+#pragma unroll
+        for (int kk = 0; kk < OZT_BK / 16; ++kk) {
+#pragma unroll
+          for (int p = 0; p < NS; ++p)
+#pragma unroll
+            for (int q = 0; q < NS - p; ++q)      // level L = p + q is first reached with p = 0
+              umma_bf16_lead(lead, tmem + (p + q) * BN, xd + ((p * Cfg::XT + kk * 32) >> 4),
+                             yd + ((q * Cfg::YT + kk * 32) >> 4), idesc, (c | kk | p) != 0);
+        }
+        umma_commit_lead(lead, &bars[2 + st]);
+      }
+      if (ok) {
+        umma_commit_lead(lead, &bars[4]);
+        if (lead) mbar_arrive(&bars[4]);      // and the producers' exponents, seen by this thread
+      }
+      __syncwarp();
+    }
+    if (!ok) {
+      *abort_s = 1;
+      if (lead) atomicExch(err, 2);
+      umma_commit_lead(lead, &bars[5]);  // drain what was issued before freeing tensor memory
+      volatile int keep_waiting = 0;
+      mbar_wait(&bars[5], 0, OZT_WAIT, &keep_waiting);
+      __syncwarp();
+    }
+  } else {
+    // ---- epilogue: wait for a tile's last MMAs, combine the levels, write C
+    const int lg = warp & 3, half = (warp - OZT_PROD_WARPS - 1) >> 2;
+    const int re = 32 * lg + lane;
+    const uint32_t trow = tmem + ((uint32_t)(32 * lg) << 16);
+    unsigned it = 0;
+    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++it) {
+      const long long m = tile / ntn * OZT_BM + re;
+      const int n0 = (int)(tile % ntn) * BN;
+      if (!mbar_wait(&bars[4], it & 1, OZT_WAIT, abort_s)) {
+        *abort_s = 1;
+        atomicExch(err, 1);
+        break;
+      }
+      tc_fence_after();
+      const int eme = ex_s[(it & 3) * OZT_BM + re];
       const int ex = (eme ? eme - 1022 : 0) - OZ_BETA * (NS + 1);
-      const uint32_t trow = tmem + ((uint32_t)(32 * lg) << 16);
 #pragma unroll 1
-      for (int cb = 8 * quarter; cb < BN; cb += 32) {
+      for (int cb = 8 * half; cb < BN; cb += 16) {
         float P[NS][8];
 #pragma unroll
         for (int L = 0; L < NS; ++L) tmem_ld8(trow + L * BN + cb, P[L]);
         tmem_wait_ld();
+        if (cb + 16 >= BN) {           // the last reads: the next tile may overwrite
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[8]);
+        }
         if (m < M) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = n0 + cb + j;
             if (n >= N) break;
-            long long acc = 0;
+            // sum of P_L 2^{7 (NS - 1 - L)}: three levels at a time by 32 x 32 + 64-bit
+            // multiply-adds
+            long long hi = 0, acc = 0;
 #pragma unroll
-            for (int L = 0; L < NS; ++L) acc += (long long)__float2int_rn(P[L][j]) << (OZ_BETA * (NS - 1 - L));
+            for (int L = 0; L < NS; ++L) {
+              const int q = __float2int_rn(P[L][j]);
+              if (L < NS - 3) hi = (long long)q * (1 << (OZ_BETA * (NS - 4 - L))) + hi;
+              else acc = (long long)q * (1 << (OZ_BETA * (NS - 1 - L))) + acc;
+            }
+            acc += hi << (3 * OZ_BETA);
             const double val = oz_ll_scaled(acc, ex + __ldg(ey + n));
             double* cp = C + m * sCm + (long long)n * sCn;
             *cp = accumulate ? *cp + val : val;
           }
         }
       }
-    } else {
-      *abort_s = 1;
-      atomicExch(err, 1);
-    }
-  } else if (lane == 0) {
-    // ---- MMA issuer
-    const uint32_t idesc = idesc_bf16_f32(OZT_BM, BN);
-    unsigned inited = 0;
-    bool ok = true;
-    for (int c = 0; c < nchunk; ++c) {
-      const int st = c & 1;
-      if (!mbar_wait(&bars[st], (c >> 1) & 1, OZT_WAIT, abort_s) ||
-          !mbar_wait(&bars[6 + st], (c >> 1) & 1, OZT_WAIT, abort_s)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t xa = smem_u32(tiles + st * Cfg::STAGE);
-      const uint32_t ya = xa + NS * Cfg::XT;
-#pragma unroll
-      for (int kk = 0; kk < OZT_BK / 16; ++kk) {
-#pragma unroll
-        for (int p = 0; p < NS; ++p)
-#pragma unroll
-          for (int q = 0; q < NS - p; ++q) {
-            const int L = p + q;
-            const uint64_t ad = sdesc_k_sw64(xa + p * Cfg::XT + kk * 32);
-            const uint64_t bd = sdesc_k_sw64(ya + q * Cfg::YT + kk * 32);
-            umma_bf16(tmem + L * BN, ad, bd, idesc, (inited >> L) & 1u);
-            inited |= 1u << L;
-          }
-      }
-      umma_commit(&bars[2 + st]);
-    }
-    if (ok) {
-      umma_commit(&bars[4]);
-    } else {
-      *abort_s = 1;
-      atomicExch(err, 2);
-      umma_commit(&bars[5]);  // drain what was issued before freeing tensor memory
-      volatile int keep_waiting = 0;
-      mbar_wait(&bars[5], 0, OZT_WAIT, &keep_waiting);
     }
   }
   tc_fence_before();
@@ -390,7 +444,10 @@ static int ozt_run(long long M, int N, int K, const double* X, long long ldx, co
     PCG_CUDA(cudaFuncSetAttribute(k_ozt_gemm<NS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
     attr_set[dev] = true;
   }
-  const long long blocks = (long long)(L.Npad / BN) * ((M + OZT_BM - 1) / OZT_BM);
+  int sms = 0;
+  PCG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const long long tiles = (long long)(L.Npad / BN) * ((M + OZT_BM - 1) / OZT_BM);
+  const long long blocks = tiles < sms ? tiles : sms;
   k_ozt_gemm<NS, BN><<<(unsigned)blocks, OZT_THREADS, Cfg::SMEM, s>>>(M, N, K, L.Kp, L.Npad, X, ldx, ymap, ey, C, sCm,
                                                                     sCn, accumulate, err);
   PCG_CUDA(cudaGetLastError());

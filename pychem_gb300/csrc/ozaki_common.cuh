@@ -55,27 +55,16 @@ __device__ __forceinline__ void oz_digits(double x, int emax, int* d) {
   }
 }
 
-// acc 2^e as a double, rounded to nearest even like an int64 -> FP64 conversion, built
-// with integer operations only (64-bit conversions run on the FP64 pipe); results
-// below the normal range are flushed to 0 (far under any tolerance here).
+// acc 2^e as a double, rounded to nearest even by the one conversion (one instruction on the FP64
+// pipe; formed from a leading-zero count and shifts it took 30 on the others) and scaled
+// by its exponent; results below the normal range are flushed to 0 (far under any tolerance
+// here).
 __device__ __forceinline__ double oz_ll_scaled(long long acc, int e) {
-  if (acc == 0) return 0.0;
-  const unsigned long long sign = acc < 0 ? 1ull : 0ull;
-  unsigned long long mag = sign ? (unsigned long long)(-acc) : (unsigned long long)acc;
-  int msb = 63 - __clzll((long long)mag);
-  unsigned long long mant;
-  if (msb <= 52) {
-    mant = mag << (52 - msb);
-  } else {
-    const int sh = msb - 52;
-    mant = mag >> sh;
-    const unsigned long long rem = mag & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-    if (rem > half || (rem == half && (mant & 1ull))) ++mant;
-    if (mant >> 53) { mant >>= 1; ++msb; }
-  }
-  const int ef = msb + 1023 + e;
-  if (ef <= 0) return 0.0;
-  return __longlong_as_double((long long)((sign << 63) | ((unsigned long long)ef << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+  const double d = __ll2double_rn(acc);
+  const int hi = __double2hiint(d);
+  const int ef = ((hi >> 20) & 0x7ff) + e;
+  const bool zero = acc == 0 || ef <= 0;
+  return __hiloint2double(zero ? 0 : ((hi & (int)0x800fffffu) | (ef << 20)), zero ? 0 : __double2loint(d));
 }
 
 // The same digits for two values at once, packed as BF16 pairs: w[p-1] holds digit p of
