@@ -404,6 +404,11 @@ int pcg_jacobi_eigh(int batch, int n, const double *A, double *w, void *V, int f
 int pcg_mlp_gemm(int M, int N, int K, const float *A, long long sam, long long sak, const void *B,
                  int b_bf16, long long sbk, long long sbn, float *C, int ldc, int accumulate,
                  const float *bias, float *Z, int act, void *stream);
+/* All layers of the forward pass, out[k] = silu(in W_k + b_k) (no activation in the last one)
+ * with dims[k] x dims[k+1] row-major BF16 weights; Z[k] (Z or its entries may be null) receives
+ * the pre-activations.  The arrays of pointers are host memory. */
+int pcg_mlp_forward(int nlayer, const int *dims, int M, const float *X, const void *const *W_bf16,
+                    const float *const *b, float *const *out, float *const *Z, void *stream);
 /* The weight gradient dW = A^T G (K x N) of a layer from its input A (M x K) and output
  * gradient G (M x N), both row-major, and the bias gradient db = column sums of G; the
  * workspace (16-byte aligned) holds partial sums over ranges of rows. */

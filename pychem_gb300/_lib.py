@@ -105,6 +105,7 @@ _SIGS = {
     "pcg_fma_probe": [c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "pcg_mlp_gemm": [c_int, c_int, c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_longlong, c_longlong,
                      c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
+    "pcg_mlp_forward": [c_int, P_INT, c_int, c_void_p] + [ctypes.POINTER(c_void_p)] * 4 + [c_void_p],
     "pcg_mlp_wgrad_workspace": [c_int, c_int, c_int],
     "pcg_mlp_wgrad": [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_size_t, c_void_p],
     "pcg_mlp_status": [c_void_p],

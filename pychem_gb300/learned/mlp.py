@@ -48,19 +48,15 @@ class PairMLP:
 
     def forward(self, X, keep=False):
         """X (M, NFEAT) float32 -> (M, NPARAM) normalised outputs."""
-        M = X.shape[0]
+        M, n = X.shape[0], self.nlayers
         A = X.contiguous()
-        cache = []
-        for k in range(self.nlayers):
-            K, N = self.dims[k], self.dims[k + 1]
-            act = 1 if k < self.nlayers - 1 else 0
-            C = torch.empty(M, N, dtype=torch.float32, device=self.dev)
-            Z = torch.empty(M, N, dtype=torch.float32, device=self.dev) if (keep and act) else None
-            _lib.call("pcg_mlp_gemm", M, N, K, _p(A), K, 1, _p(self.Wb[k]), 1, N, 1, _p(C), N, 0, _p(self.b[k]),
-                      _p(Z), act, _stream())
-            cache.append((A, Z))
-            A = C
-        return A, cache
+        outs = [torch.empty(M, N, dtype=torch.float32, device=self.dev) for N in self.dims[1:]]
+        Z = [torch.empty_like(t) if keep and k < n - 1 else None for k, t in enumerate(outs)]
+        ptrs = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else None for t in ts])
+        _lib.call("pcg_mlp_forward", n, (ctypes.c_int * (n + 1))(*self.dims), M, _p(A), ptrs(self.Wb), ptrs(self.b),
+                  ptrs(outs), ptrs(Z), _stream())
+        _lib.launch_count += n
+        return outs[-1], list(zip([A] + outs[:-1], Z))
 
     def backward(self, dY, cache):
         """Gradients (dW, db) per layer for output gradient dY (M, NPARAM)."""
