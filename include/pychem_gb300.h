@@ -192,6 +192,22 @@ int pcg_eri_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, c
 int pcg_eri_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                         int ntask, int nheavy, double *store, int fp32, void *stream);
 
+/* Packed primitive pairs for pcg_eri_class_tab: pk (npp x 8: P, K, P - A, 1/(2 zeta); 16-byte
+ * aligned), zid[i] = the index of zeta[i] among the nz ascending exponent sums zsum (-1 where it is
+ * none of them), tab (nz x nz x 6, 16-byte aligned) the factors of a primitive quartet that
+ * depend on its two sums alone.  nz = 0: no table, nz <= 4096. */
+typedef struct {
+  const double *pk;
+  const int *zid;
+  const double *tab;
+  int nz;
+} pcg_prim_t;
+int pcg_prim_pack(int npp, const double *zeta, const double *P, const double *PA, const double *K,
+                  const double *oo2z, int nz, const double *zsum, double *pk, int *zid, double *tab, void *stream);
+/* pcg_eri_class_split in double precision from the packed pairs of the same pair table. */
+int pcg_eri_class_tab(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const pcg_prim_t *prim,
+                      const int *tasks, int ntask, int nheavy, double *store, void *stream);
+
 /* Schwarz factor Q[pair] = sqrt(max (mn|mn)) from diagonal blocks of a diagonal class. */
 int pcg_schwarz_class(int cls, const int *tasks, int ntask, const double *store, double *Q,
                       void *stream);

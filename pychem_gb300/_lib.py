@@ -36,6 +36,10 @@ class PairsT(ctypes.Structure):
                 ("pf8", c_void_p)]
 
 
+class PrimT(ctypes.Structure):
+    _fields_ = [("pk", c_void_p), ("zid", c_void_p), ("tab", c_void_p), ("nz", c_int)]
+
+
 class PlanT(ctypes.Structure):
     _fields_ = [("nrow", c_longlong), ("nbucket", c_int), ("nmol", c_int), ("row0", c_void_p), ("bra_kind", c_void_p),
                 ("ket_kind", c_void_p), ("kind0", c_void_p), ("seg0", c_void_p), ("order", c_void_p),
@@ -76,6 +80,9 @@ _SIGS = {
                       c_void_p],
     "pcg_eri_class_split": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_int, c_void_p,
                             c_int, c_void_p],
+    "pcg_prim_pack": [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 5,
+    "pcg_eri_class_tab": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), ctypes.POINTER(PrimT), c_void_p, c_int,
+                          c_int, c_void_p, c_void_p],
     "pcg_schwarz_class": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "pcg_plan_count": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p],
     "pcg_plan_fill": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p, c_void_p],
@@ -144,7 +151,7 @@ _SIGS = {
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
 }
 # entry points that launch exactly one kernel of this library per call
-LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_schwarz_class", "pcg_plan_count", "pcg_plan_fill", "pcg_expand_tasks",
+LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_eri_class_tab", "pcg_schwarz_class", "pcg_plan_count", "pcg_plan_fill", "pcg_expand_tasks",
              "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_digest_lists", "pcg_digest_lists_u", "pcg_fock_build_u", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
              "pcg_dgemm", "pcg_dgemm_sym", "pcg_projector_check", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
              "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_mse_counted", "pcg_mlp_adam", "pcg_mlp_adam_all",
@@ -156,7 +163,7 @@ launch_count = 0
 _RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
              "pcg_mlp_wgrad_workspace": ctypes.c_size_t, "pcg_coulomb_exchange_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_coulomb_exchange": 4}
+MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_prim_pack": 2, "pcg_coulomb_exchange": 4}
 
 _lib = None
 

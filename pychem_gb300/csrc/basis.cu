@@ -437,3 +437,46 @@ int pcg_launch_one_electron(const DevBasis& b, const BoysTable& bt, int npair, c
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
 }
+
+// ----------------------------------------------------------------------------------
+// Packed primitive pairs (64 bytes each) with the index of their exponent sum among the
+// nz ascending sums zsum (-1: not there), and the factors of every two sums.
+// ----------------------------------------------------------------------------------
+__global__ void k_prim_pack(int npp, const double* __restrict__ zeta, const double* __restrict__ P,
+                            const double* __restrict__ PA, const double* __restrict__ K, const double* __restrict__ oo2z,
+                            int nz, const double* __restrict__ zsum, double* __restrict__ pk, int* __restrict__ zid) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npp) return;
+  double2* o = (double2*)pk + 4 * (size_t)i;
+  o[0] = make_double2(P[3 * i], P[3 * i + 1]);
+  o[1] = make_double2(P[3 * i + 2], K[i]);
+  o[2] = make_double2(PA[3 * i], PA[3 * i + 1]);
+  o[3] = make_double2(PA[3 * i + 2], oo2z[i]);
+  const double z = zeta[i];
+  int lo = 0, hi = nz;                 // first sum >= z
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(zsum + mid) < z) lo = mid + 1; else hi = mid;
+  }
+  zid[i] = lo < nz && __ldg(zsum + lo) == z ? lo : -1;
+}
+
+__global__ void k_prim_tab(int nz, const double* __restrict__ zsum, double* __restrict__ tab) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= (long long)nz * nz) return;
+  const double z = __ldg(zsum + x / nz), e = __ldg(zsum + x % nz), s = z + e;
+  const double i = 1.0 / s;
+  double2* o = (double2*)tab + 3 * x;
+  o[0] = make_double2(1.0 / sqrt(s), z * (e * i));
+  o[1] = make_double2(e * i, z * i);
+  o[2] = make_double2(0.5 * i, 0.0);
+}
+
+int pcg_launch_prim_pack(int npp, const double* zeta, const double* P, const double* PA, const double* K,
+                         const double* oo2z, int nz, const double* zsum, double* pk, int* zid, double* tab,
+                         cudaStream_t s) {
+  if (npp > 0) k_prim_pack<<<(npp + 127) / 128, 128, 0, s>>>(npp, zeta, P, PA, K, oo2z, nz, zsum, pk, zid);
+  if (nz > 0) k_prim_tab<<<(unsigned)(((long long)nz * nz + 127) / 128), 128, 0, s>>>(nz, zsum, tab);
+  PCG_CUDA(cudaGetLastError());
+  return PCG_OK;
+}

@@ -99,7 +99,7 @@ int pcg_eri_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, c
   BoysTable bt;
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
-  return pcg_launch_eri(cls, to_dev(pairs), bt, (const int2*)tasks, ntask, 0, store, fp32 ? 1 : 0,
+  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, 0, store, fp32 ? 1 : 0,
                         (cudaStream_t)stream);
 }
 
@@ -112,8 +112,32 @@ int pcg_eri_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pa
   BoysTable bt;
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
-  return pcg_launch_eri(cls, to_dev(pairs), bt, (const int2*)tasks, ntask, nheavy, store, fp32 ? 1 : 0,
+  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, nheavy, store, fp32 ? 1 : 0,
                         (cudaStream_t)stream);
+}
+
+int pcg_eri_class_tab(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const pcg_prim_t* prim,
+                      const int* tasks, int ntask, int nheavy, double* store, void* stream) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || !prim || !prim->pk || !prim->zid || (prim->nz > 0 && !prim->tab) ||
+      ((size_t)prim->pk & 15) || ((size_t)prim->tab & 15) || ntask < 0 || nheavy < 0 || nheavy > ntask) {
+    pcg_set_error("pcg_eri_class_tab: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  BoysTable bt;
+  int rc = pcg_ensure_boys(&bt);
+  if (rc) return rc;
+  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{prim->pk, prim->zid, prim->tab, prim->nz}, bt, (const int2*)tasks,
+                        ntask, nheavy, store, 0, (cudaStream_t)stream);
+}
+
+int pcg_prim_pack(int npp, const double* zeta, const double* P, const double* PA, const double* K, const double* oo2z,
+                  int nz, const double* zsum, double* pk, int* zid, double* tab, void* stream) {
+  if (npp < 0 || nz < 0 || nz > 4096 || (npp > 0 && (!zeta || !P || !PA || !K || !oo2z || !pk || !zid)) ||
+      (nz > 0 && (!zsum || !tab)) || ((size_t)pk & 15) || ((size_t)tab & 15)) {
+    pcg_set_error("pcg_prim_pack: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  return pcg_launch_prim_pack(npp, zeta, P, PA, K, oo2z, nz, zsum, pk, zid, tab, (cudaStream_t)stream);
 }
 
 int pcg_schwarz_class(int cls, const int* tasks, int ntask, const double* store, double* Q, void* stream) {

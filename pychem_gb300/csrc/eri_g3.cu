@@ -1,14 +1,14 @@
 // ERI classes 18..19 (see eri_kernels.cuh); split for parallel compilation.
 #include "eri_kernels.cuh"
 
-int pcg_launch_eri_g3(int cls, const DevPairsExt& pr, const BoysTable& bt, const int2* tasks, int ntask,
+int pcg_launch_eri_g3(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
                       int nheavy, double* store, int precision, cudaStream_t s) {
   const int threads = 128, blocks = (ntask + threads - 1) / threads;
   const EriRange rg = eri_range(ntask, nheavy);
   if (precision == 0) {
     switch (cls) {
-      case 18: k_eri<Eri2220><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, bt, tasks, rg, store); break;
-      case 19: k_eri<Eri2221><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, bt, tasks, rg, store); break;
+      case 18: k_eri<Eri2220><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, pt, bt, tasks, rg, store); break;
+      case 19: k_eri<Eri2221><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, pt, bt, tasks, rg, store); break;
       default: return PCG_ERR_ARG;
     }
   } else {

@@ -72,9 +72,14 @@ __device__ __forceinline__ void eri_lane_sum(T* acc, int lg) {
     for (int k = 0; k < N; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
 }
 
+// The factors of a primitive quartet that depend on its two exponent sums alone come from a
+// table over the molecule's distinct sums (PrimTab): 1/sqrt(zeta + eta), rho, rho/zeta, rho/eta and
+// 1/(2 (zeta + eta)), nine FP64 instructions of about 40 in (ps|ss).  A pair without an
+// entry (no table, or more sums than it takes) has them computed.  Packed pair data halve the
+// gathers: P and K, P - A and 1/(2 zeta) are two 16-byte loads each.
 template <class C>
-__global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, BoysTable bt, const int2* __restrict__ tasks, EriRange rg,
-                                             double* __restrict__ store) {
+__global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, PrimTab pt, BoysTable bt, const int2* __restrict__ tasks,
+                                             EriRange rg, double* __restrict__ store) {
   const EriLane ln = eri_lane(rg);
   const int t = ln.t;
   const int2 tk = tasks[t];
@@ -84,42 +89,75 @@ __global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, BoysTable bt, const
 #pragma unroll
   for (int k = 0; k < C::NACC; ++k) acc[k] = 0.0;
   int i = i0 - 1, jj = ln.g + nj;      // jj: ket primitive plus the bra steps not yet taken
-  double zeta = 0.0, Px = 0.0, Py = 0.0, Pz = 0.0, Kp = 0.0;
+  int zi = -1;
+  double Px = 0.0, Py = 0.0, Pz = 0.0, Kp = 0.0;
   PQd q;
   for (int n = ln.g; n < nq; n += 1 << ln.lg, jj += 1 << ln.lg) {
     if (jj >= nj) {
       do { jj -= nj; ++i; } while (jj >= nj);
-      zeta = __ldg(pr.p.zeta + i);
-      Px = __ldg(pr.p.P + 3 * i); Py = __ldg(pr.p.P + 3 * i + 1); Pz = __ldg(pr.p.P + 3 * i + 2);
-      Kp = __ldg(pr.p.K + i);
-      q.PAx = __ldg(pr.p.PA + 3 * i);
-      q.PAy = __ldg(pr.p.PA + 3 * i + 1);
-      q.PAz = __ldg(pr.p.PA + 3 * i + 2);
-      q.oo2z = __ldg(pr.oo2z + i);
+      if (pt.pk) {
+        const double2* b = (const double2*)pt.pk + 4 * (size_t)i;
+        const double2 b0 = __ldg(b), b1 = __ldg(b + 1), b2 = __ldg(b + 2), b3 = __ldg(b + 3);
+        Px = b0.x; Py = b0.y; Pz = b1.x; Kp = b1.y;
+        q.PAx = b2.x; q.PAy = b2.y; q.PAz = b3.x; q.oo2z = b3.y;
+        zi = __ldg(pt.zid + i);
+      } else {
+        Px = __ldg(pr.p.P + 3 * i); Py = __ldg(pr.p.P + 3 * i + 1); Pz = __ldg(pr.p.P + 3 * i + 2);
+        Kp = __ldg(pr.p.K + i);
+        q.PAx = __ldg(pr.p.PA + 3 * i);
+        q.PAy = __ldg(pr.p.PA + 3 * i + 1);
+        q.PAz = __ldg(pr.p.PA + 3 * i + 2);
+        q.oo2z = __ldg(pr.oo2z + i);
+      }
     }
     const int j = j0 + jj;
-    const double eta = __ldg(pr.p.zeta + j);
-    const double PQx = Px - __ldg(pr.p.P + 3 * j);
-    const double PQy = Py - __ldg(pr.p.P + 3 * j + 1);
-    const double PQz = Pz - __ldg(pr.p.P + 3 * j + 2);
-    const double rs = nr_rsqrt(zeta + eta);
-    const double izpe = rs * rs;
-    q.rz = eta * izpe;
-    const double T = zeta * q.rz * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
+    double PQx, PQy, PQz, Kq;
+    int zj = -1;
+    if (pt.pk) {
+      const double2* b = (const double2*)pt.pk + 4 * (size_t)j;
+      const double2 b0 = __ldg(b), b1 = __ldg(b + 1), b2 = __ldg(b + 2), b3 = __ldg(b + 3);
+      PQx = Px - b0.x; PQy = Py - b0.y; PQz = Pz - b1.x;
+      Kq = b1.y;
+      q.QCx = b2.x; q.QCy = b2.y; q.QCz = b3.x; q.oo2e = b3.y;
+      zj = __ldg(pt.zid + j);
+    } else {
+      PQx = Px - __ldg(pr.p.P + 3 * j);
+      PQy = Py - __ldg(pr.p.P + 3 * j + 1);
+      PQz = Pz - __ldg(pr.p.P + 3 * j + 2);
+      Kq = __ldg(pr.p.K + j);
+      q.QCx = __ldg(pr.p.PA + 3 * j);
+      q.QCy = __ldg(pr.p.PA + 3 * j + 1);
+      q.QCz = __ldg(pr.p.PA + 3 * j + 2);
+      q.oo2e = __ldg(pr.oo2z + j);
+    }
+    double rs, rho;
+    if ((zi | zj) >= 0) {
+      const double2* e = (const double2*)pt.tab + 3 * ((size_t)zi * pt.nz + zj);
+      const double2 e0 = __ldg(e), e1 = __ldg(e + 1), e2 = __ldg(e + 2);
+      rs = e0.x; rho = e0.y;
+      q.rz = e1.x; q.re = e1.y;
+      q.oo2ze = e2.x;
+    } else {
+      const double zeta = __ldg(pr.p.zeta + i), eta = __ldg(pr.p.zeta + j);
+      rs = nr_rsqrt(zeta + eta);
+      const double izpe = rs * rs;
+      q.rz = eta * izpe;
+      q.re = zeta * izpe;
+      rho = zeta * q.rz;
+      q.oo2ze = 0.5 * izpe;
+    }
     double F[C::L + 1];
-    boys_eval<C::L>(bt, T, F);
-    const double pre = Kp * __ldg(pr.p.K + j) * rs;
+    boys_eval<C::L>(bt, rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz)), F);
+    const double pre = Kp * Kq * rs;
+    if constexpr (C::L == 0) {
+      acc[0] = fma(F[0], pre, acc[0]);
+    } else {
 #pragma unroll
-    for (int m = 0; m <= C::L; ++m) F[m] *= pre;
-    q.re = zeta * izpe;
-    q.WPx = -q.rz * PQx; q.WPy = -q.rz * PQy; q.WPz = -q.rz * PQz;
-    q.WQx = q.re * PQx; q.WQy = q.re * PQy; q.WQz = q.re * PQz;
-    q.QCx = __ldg(pr.p.PA + 3 * j);
-    q.QCy = __ldg(pr.p.PA + 3 * j + 1);
-    q.QCz = __ldg(pr.p.PA + 3 * j + 2);
-    q.oo2e = __ldg(pr.oo2z + j);
-    q.oo2ze = 0.5 * izpe;
-    C::prim(q, F, acc);
+      for (int m = 0; m <= C::L; ++m) F[m] *= pre;
+      q.WPx = -q.rz * PQx; q.WPy = -q.rz * PQy; q.WPz = -q.rz * PQz;
+      q.WQx = q.re * PQx; q.WQy = q.re * PQy; q.WQz = q.re * PQz;
+      C::prim(q, F, acc);
+    }
   }
   eri_lane_sum<C::NACC>(acc, ln.lg);
   if (ln.g != 0 || !ln.on) return;

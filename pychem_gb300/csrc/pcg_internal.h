@@ -33,8 +33,20 @@ struct DevPairsExt {
   const double* oo2z;  // 1/(2 zeta) per primitive pair
 };
 
-int pcg_launch_eri(int cls, const DevPairsExt& pr, const BoysTable& bt, const int2* tasks, int ntask, int nheavy,
-                   double* store, int precision, cudaStream_t s);
+// packed primitive pairs and exponent-sum factors of the FP64 integral kernels (see
+// eri_kernels.cuh); all null: none
+struct PrimTab {
+  const double* pk;   // [npp][8]: P, K, P - A, 1/(2 zeta)
+  const int* zid;     // exponent sum of each primitive pair, -1: not in the table
+  const double* tab;  // [nz][nz][6]: 1/sqrt(z+e), z e/(z+e), e/(z+e), z/(z+e), 1/(2(z+e)), 0
+  int nz;
+};
+
+int pcg_launch_eri(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
+                   int nheavy, double* store, int precision, cudaStream_t s);
+int pcg_launch_prim_pack(int npp, const double* zeta, const double* P, const double* PA, const double* K,
+                         const double* oo2z, int nz, const double* zsum, double* pk, int* zid, double* tab,
+                         cudaStream_t s);
 int pcg_launch_pair_data_f32(int npp, const double* zeta, const double* PA, const double* oo2z, const float* Kf,
                              float* pf8, cudaStream_t s);
 int pcg_launch_pair_ao(const DevBasis& b, int npair, const int* pA, const int* pB, int* ao4, cudaStream_t s);

@@ -16,6 +16,7 @@ import torch
 from . import _lib
 from ._lib import BasisT, PairsT
 from ._stream import stream as _stream
+from .molecule import element_shells
 
 INTEGRAL_THRESHOLD = 1.0e-8   # Data/constants.py:31
 N_SPHER = [1, 3, 5]
@@ -23,6 +24,9 @@ N_SPHER = [1, 3, 5]
 # of two oxygen 1s pairs take longer than the rest of a mid-size molecule's launch, and from
 # 128 on each of 16 lanes still has eight or more to sum
 HEAVY = 128
+# distinct exponent sums up to which their factors are tabulated: 1,024^2 entries of 48 bytes stay
+# in L2 (H, C, N, O, F in 6-31G together have 990)
+MAX_EXPONENT_SUMS = 1024
 # co-density matrices by products with pair matrices: the dense tensor and the pair matrices
 # cost what the digestion of about 16 densities does, and take 1.2 GB at 96 functions
 COEXCHANGE_MIN = 16
@@ -269,7 +273,30 @@ class GpuEngine:
                   _stream())
         _lib.call("pcg_pair_data_f32", int(p["zeta"].numel()), _ptr(p["zeta"]), _ptr(p["PA"]), _ptr(p["oo2z"]),
                   _ptr(p["Kf"]), _ptr(p["pf8"]), _stream())
+        self._pack_primitives()
         self._set_pairs_t()
+
+    def _atom_kinds(self):
+        """(basis, element) of every kind of atom in the engine."""
+        return {(self.mol.Basis, a[0]) for a in self.mol.atoms}
+
+    def _pack_primitives(self):
+        """Packed primitive pairs and the table over the distinct sums of two exponents
+        (pcg_prim_pack), which the FP64 integral kernels read."""
+        p = self.pd
+        exps = np.unique(np.concatenate([e for b, sym in self._atom_kinds() for _, e, _ in element_shells(b, sym)]))
+        zsum = np.unique(exps[:, None] + exps[None, :])
+        if len(zsum) > MAX_EXPONENT_SUMS:
+            zsum = zsum[:0]
+        n, nz = p["zeta"].numel(), len(zsum)
+        zs = self._t(zsum)
+        p["pk"] = torch.empty(8 * n, dtype=torch.float64, device=self.dev)
+        p["zid"] = torch.empty(n, dtype=torch.int32, device=self.dev)
+        p["tab"] = torch.empty(6 * nz * nz, dtype=torch.float64, device=self.dev)
+        _lib.call("pcg_prim_pack", n, _ptr(p["zeta"]), _ptr(p["P"]), _ptr(p["PA"]), _ptr(p["K"]), _ptr(p["oo2z"]), nz,
+                  _ptr(zs), _ptr(p["pk"]), _ptr(p["zid"]), _ptr(p["tab"]), _stream())
+        t = self.prim_t = _lib.PrimT()
+        t.pk, t.zid, t.tab, t.nz = p["pk"].data_ptr(), p["zid"].data_ptr(), p["tab"].data_ptr() if nz else None, nz
 
     # ---------------------------------------------------------------------------------
     def one_electron(self):
@@ -293,6 +320,10 @@ class GpuEngine:
                 raise ValueError("scattering integrals are FP64 only")
             _lib.call("pcg_scattering_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
                       _ptr(factors), _ptr(tasks), ntask, nheavy, float(self.scattering), _ptr(store), _stream())
+            return
+        if not fp32:
+            _lib.call("pcg_eri_class_tab", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
+                      ctypes.byref(self.prim_t), _ptr(tasks), ntask, nheavy, _ptr(store), _stream())
             return
         _lib.call("pcg_eri_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(tasks),
                   ntask, nheavy, _ptr(store), 1 if fp32 else 0, _stream())

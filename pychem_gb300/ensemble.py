@@ -66,6 +66,9 @@ class EnsembleEngine(GpuEngine):
         self.basis_t = b
         self.nbf = self.nmax
 
+    def _atom_kinds(self):
+        return {(m.Basis, a[0]) for m in self.mols for a in m.atoms}
+
     def atom_table(self):
         if getattr(self, "_atoms", None) is None:
             self._atoms = atom_table(self.mols)

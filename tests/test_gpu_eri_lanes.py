@@ -80,3 +80,25 @@ def test_fundamentals_over_distance(S):
         ref = b.eri_dense(scattering=S) if S is not None else b.eri_dense()
         keep = np.abs(got) > 0           # the oracle leaves out what its threshold screens
         assert np.abs((got - ref)[keep & (np.abs(ref) > 0)]).max() < (1e-12 if S is None else 1e-10), r
+
+
+@pytest.mark.parametrize("most", [0, 20, 1024])
+def test_exponent_sum_table(most, monkeypatch):
+    """No table, a table that is refused for its size, and a whole one give the same blocks
+    (each factor to a few roundings: 1e-14 of the largest integral)."""
+    from pychem_gb300 import engine, workloads
+    coords = workloads.water() + [["C", 6.0, 3.0, 0.0, 0.5], ["H", 1.0, 3.0, 1.0, 0.0], ["H", 1.0, 3.5, -0.5, 0.8]]
+    ref = _engine(coords, "cc-pVDZ").prepare()
+    monkeypatch.setattr(engine, "MAX_EXPONENT_SUMS", most)
+    got = _engine(coords, "cc-pVDZ").prepare()
+    assert (got.prim_t.nz > 0) == (most == 1024)
+    for key, store in ref.stores.items():
+        assert float((got.stores[key] - store).abs().max()) < 1e-14 * max(1.0, float(store.abs().max())) * 30
+    # sums that the table lacks are computed
+    part = got.pd["zid"].clone()
+    part[::3] = -1
+    got.pd["zid"] = part
+    got.prim_t.zid = part.data_ptr()
+    got.compute_eris()
+    for key, store in ref.stores.items():
+        assert float((got.stores[key] - store).abs().max()) < 1e-14 * max(1.0, float(store.abs().max())) * 30
