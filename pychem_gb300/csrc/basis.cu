@@ -64,7 +64,7 @@ int pcg_ensure_boys(BoysTable* out) {
   DeviceState* st = pcg_state();
   if (!st) { pcg_set_error("no CUDA device"); return PCG_ERR_CUDA; }
   if (!st->boys_c) {
-    std::vector<TaylorRow> c((size_t)BOYS_M * BOYS_NP);
+    std::vector<TaylorRow> c((size_t)BOYS_M * BOYS_ROWS);
     std::vector<double> ex(BOYS_NP);
     std::vector<float> cf((size_t)BOYS_NPF * BOYS_M * BOYS_KF), exf(BOYS_NPF);
     double F[64], fact[BOYS_K];
@@ -74,7 +74,7 @@ int pcg_ensure_boys(BoysTable* out) {
       const double T = (double)p / BOYS_INV_H;
       boys_host(BOYS_M + BOYS_K, T, F);
       for (int m = 0; m < BOYS_M; ++m) {
-        TaylorRow& r = c[(size_t)m * BOYS_NP + p];
+        TaylorRow& r = c[(size_t)m * BOYS_ROWS + p];
         for (int k = 0; k < 4; ++k) r.c[k] = F[m + k] / fact[k];
         for (int k = 4; k < BOYS_K; ++k) r.t[k - 4] = (float)(F[m + k] / fact[k]);
         r.t[3] = 0.0f;
@@ -85,6 +85,20 @@ int pcg_ensure_boys(BoysTable* out) {
         for (int m = 0; m < BOYS_M; ++m)
           for (int k = 0; k < BOYS_KF; ++k) cf[((size_t)q * BOYS_M + m) * BOYS_KF + k] = (float)(F[m + k] / fact[k]);
         exf[q] = (float)ex[p];
+      }
+    }
+    for (int q = 0; q < BOYS_NLOG; ++q) {
+      // the middle of the interval whose high words start at BOYS_TMAX_HI + (q << 12)
+      const int64_t bits = ((int64_t)(BOYS_TMAX_HI + (q << 12) + 0x800)) << 32;
+      double T;
+      memcpy(&T, &bits, sizeof(T));
+      F[0] = 0.5 * sqrt(M_PI / T);
+      for (int m = 0; m < 3 + BOYS_K; ++m) F[m + 1] = (2 * m + 1) * F[m] / (2.0 * T);
+      for (int m = 0; m < 3; ++m) {
+        TaylorRow& r = c[(size_t)m * BOYS_ROWS + BOYS_NP + q];
+        for (int k = 0; k < 4; ++k) r.c[k] = F[m + k] / fact[k];
+        for (int k = 4; k < BOYS_K; ++k) r.t[k - 4] = (float)(F[m + k] / fact[k]);
+        r.t[3] = 0.0f;
       }
     }
     // j_m(z) / z^m about x_p = p / 64, x = z^2 / 2: its derivative in x is -j_{m+1}(z) / z^{m+1},

@@ -33,13 +33,19 @@ void pcg_set_error(const char* msg);
 // 5 more for the argument).  Orders up to 2 are each read from the table; above, the lower ones come
 // from the downward recursion F_{m-1} = (2T F_m + exp(-T)) / (2m - 1), exp(-T) from the
 // same grid.  Beyond BOYS_TMAX: F_0 = sqrt(pi/T)/2 and the upward recursion
-// F_{m+1} = (2m+1) F_m / (2T) (exp(-T) < 1e-20 there).
+// F_{m+1} = (2m+1) F_m / (2T) (exp(-T) < 1e-20 there).  Orders up to 2 have rows to T = 65536
+// too, 256 a binade about the middles of their intervals (|d| <= T / 512, truncation 1e-17; beyond, the
+// float terms would underflow): the lanes of a warp fall on both sides of 48 as a rule, and
+// with one evaluation for both no lane waits for the other formula.
 // The single-precision variant keeps a grid of 16 points per unit and BOYS_KF terms.
 // ----------------------------------------------------------------------------------
 #define BOYS_TMAX 48.0
 #define BOYS_TMAX_HI 0x40480000  // high word of 48.0
 #define BOYS_INV_H 64
 #define BOYS_NP (48 * BOYS_INV_H + 1)
+#define BOYS_LOG_HI 0x40F00000   // high word of 65536.0
+#define BOYS_NLOG ((BOYS_LOG_HI - BOYS_TMAX_HI) >> 12)
+#define BOYS_ROWS (BOYS_NP + BOYS_NLOG)
 #define BOYS_M (PCG_MAXLT + 1)
 #define BOYS_K 7
 #define BOYS_INV_HF 16
@@ -53,7 +59,7 @@ struct __align__(16) TaylorRow {
 };
 
 struct BoysTable {
-  const TaylorRow* c;  // [BOYS_M][BOYS_NP]
+  const TaylorRow* c;  // [BOYS_M][BOYS_ROWS] (rows from BOYS_NP on: m <= 2)
   const double* ex;    // exp(-T_p), [BOYS_NP]
   const float* cf;     // [BOYS_NPF][BOYS_M][BOYS_KF]
   const float* exf;    // [BOYS_NPF]
@@ -109,15 +115,23 @@ __device__ __forceinline__ int taylor_point(double T, double& d, float& df) {
 
 template <int L>
 __device__ __forceinline__ void boys_eval(const BoysTable& bt, double T, double* F) {
-  if (__double2hiint(T) < BOYS_TMAX_HI) {
+  const int hi = __double2hiint(T);
+  if (hi < (L <= 2 ? BOYS_LOG_HI : BOYS_TMAX_HI)) {
     double d;
     float df;
-    const int p = taylor_point(T, d, df);
+    int p;
     if (L <= 2) {
+      const float r = fmaf(bits_to_float(T), 64.0f, 12582912.0f);   // 1.5 * 2^23: rounds to an integer
+      const double lin = bits_to_double((r - 12582912.0f) * 0.015625f);
+      const bool low = hi < BOYS_TMAX_HI;
+      d = __hiloint2double(low ? __double2hiint(lin) : (hi & ~0xfff) | 0x800, low ? __double2loint(lin) : 0) - T;
+      df = bits_to_float(d);
+      p = low ? __float_as_int(r) - 0x4B400000 : BOYS_NP + ((hi - BOYS_TMAX_HI) >> 12);
 #pragma unroll
-      for (int m = 0; m <= L; ++m) F[m] = taylor_row(bt.c + m * BOYS_NP + p, d, df);
+      for (int m = 0; m <= L; ++m) F[m] = taylor_row(bt.c + m * BOYS_ROWS + p, d, df);
     } else {
-      F[L] = taylor_row(bt.c + L * BOYS_NP + p, d, df);
+      p = taylor_point(T, d, df);
+      F[L] = taylor_row(bt.c + L * BOYS_ROWS + p, d, df);
       // exp(-T) = exp(-T_p) (1 + d (1 + d/2 + d^2 (1/6 + ...)))
       const float x = df * fmaf(df, fmaf(df, 1.0f / 720.0f, 1.0f / 120.0f), 1.0f / 24.0f);
       const double u = fma(fma(1.0 / 6.0 + bits_to_double(x), d, 0.5), d, 1.0);
