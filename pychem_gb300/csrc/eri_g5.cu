@@ -2,8 +2,9 @@
 #include "eri_kernels.cuh"
 
 int pcg_launch_eri_g5(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
-                      int nheavy, double* store, int precision, cudaStream_t s) {
+                      int nheavy, int nmid, double* store, int precision, cudaStream_t s) {
   (void)nheavy;
+  (void)nmid;
   (void)pt;
   const int threads = 128, blocks = (ntask + threads - 1) / threads;
   if (cls != 20 || precision == 0) return PCG_ERR_ARG;

@@ -12,53 +12,63 @@ struct PQf {
   float PAx, PAy, PAz, WPx, WPy, WPz, QCx, QCy, QCz, WQx, WQy, WQz, oo2z, oo2e, oo2ze, rz, re;
 };
 
-// The tasks of one launch.  Tasks [0, nheavy) -- a prefix: the lists are sorted by
-// decreasing primitive-quartet count -- are shared by 2^lgh lanes each, the others by 2^lgl
-// lanes; a lane takes every 2^lg-th primitive quartet, and the partial sums are added by
+// The tasks of one launch, sorted by decreasing primitive-quartet count.  The first nheavy (128
+// or more) are shared by 16 lanes each, the next nmid (16 or more) by 2^lgm, the others have
+// one lane; a lane takes every 2^lg-th primitive quartet, and the partial sums are added by
 // shuffles.  A quartet of two oxygen 1s pairs has 36 x 36 primitive quartets, about a
 // millisecond on one lane, so without the split it ends long after the rest of its launch.
 // stride: distance of a block's elements in the store.
+#define ERI_LGH 4
 struct EriRange {
-  int ntask, nheavy, lgh, lgl, stride;
+  int ntask, nheavy, nmid, lgm, stride;
 };
 
-// heavy tasks (as counted by the caller) get 16 lanes; the others as many as leave no more
-// than about 40,000 lanes: two warps a scheduler fill the FP64 pipe
-static inline EriRange eri_range(int ntask, int nheavy) {
+// the middle part gets as many lanes as leave no more than about 40,000 in all: two warps a
+// scheduler fill the FP64 pipe.  Below 16 primitive quartets the sums over lanes cost more than
+// they save ((dd|dd): 961 accumulators).
+static inline EriRange eri_range(int ntask, int nheavy, int nmid) {
   EriRange r;
   r.ntask = r.stride = ntask;
-  r.nheavy = nheavy < 0 ? 0 : (nheavy > ntask ? ntask : nheavy);
-  r.lgh = 4;
-  r.lgl = 0;
-  while (r.lgl < 4 && ((long long)(ntask - r.nheavy) << (r.lgl + 1)) <= 40000) ++r.lgl;
+  r.nheavy = nheavy;
+  r.nmid = nmid;
+  r.lgm = 0;
+  const long long rest = ((long long)nheavy << ERI_LGH) + (ntask - nheavy - nmid);
+  while (r.lgm < ERI_LGH && ((long long)nmid << (r.lgm + 1)) + rest <= 40000) ++r.lgm;
   return r;
 }
+// lanes of the first two parts, each rounded up to whole warps
+__host__ __device__ static inline long long eri_lanes(int n, int lg) { return (((long long)n << lg) + 31) / 32 * 32; }
 static inline unsigned eri_blocks(const EriRange& r, int threads) {
-  // the heavy part is rounded up to whole warps
-  const long long heavy = (((long long)r.nheavy << r.lgh) + 31) / 32 * 32;
-  return (unsigned)((heavy + ((long long)(r.ntask - r.nheavy) << r.lgl) + threads - 1) / threads);
+  const long long n = eri_lanes(r.nheavy, ERI_LGH) + eri_lanes(r.nmid, r.lgm) + (r.ntask - r.nheavy - r.nmid);
+  return (unsigned)((n + threads - 1) / threads);
 }
 
 // This lane's task, its place among the lanes of the task, and log2 of their number; lanes
-// past the end take part in the shuffles on the last task with no primitive quartet.
+// past the end of a part take part in the shuffles on the last task with no primitive quartet.
 struct EriLane {
   int t, g, lg;
   bool on;
 };
 __device__ __forceinline__ EriLane eri_lane(const EriRange& r) {
-  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long heavy = (((long long)r.nheavy << r.lgh) + 31) / 32 * 32;
+  long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long h = eri_lanes(r.nheavy, ERI_LGH), m = eri_lanes(r.nmid, r.lgm);
   EriLane l;
   long long t;
-  if (x < heavy) {
-    l.lg = r.lgh;
+  int end;
+  if (x < h) {
+    l.lg = ERI_LGH;
     t = x >> l.lg;
-    l.on = t < r.nheavy;
+    end = r.nheavy;
+  } else if (x < h + m) {
+    l.lg = r.lgm;
+    t = r.nheavy + ((x - h) >> l.lg);
+    end = r.nheavy + r.nmid;
   } else {
-    l.lg = r.lgl;
-    t = r.nheavy + ((x - heavy) >> l.lg);
-    l.on = t < r.ntask;
+    l.lg = 0;
+    t = r.nheavy + r.nmid + (x - h - m);
+    end = r.ntask;
   }
+  l.on = t < end;
   l.g = (int)(threadIdx.x & ((1u << l.lg) - 1));
   l.t = l.on ? (int)t : r.ntask - 1;
   return l;
