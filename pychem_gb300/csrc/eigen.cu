@@ -19,34 +19,34 @@
 #include "common.cuh"
 #include "pcg_internal.h"
 
-template <typename T>
-__device__ __forceinline__ void rot_params(T app, T aqq, T apq, T& c, T& s) {
-  if (apq == (T)0) { c = (T)1; s = (T)0; return; }
-  const T tau = (aqq - app) / ((T)2 * apq);
-  T t;
-  if (fabs(tau) > (T)1e18) t = (T)0.5 / tau;
-  else t = (tau >= (T)0 ? (T)1 : (T)-1) / (fabs(tau) + sqrt((T)1 + tau * tau));
-  c = (T)1 / sqrt((T)1 + t * t);
+__device__ __forceinline__ void rot_params(float app, float aqq, float apq, float& c, float& s) {
+  if (apq == 0.0f) { c = 1.0f; s = 0.0f; return; }
+  const float tau = (aqq - app) / (2.0f * apq);
+  float t;
+  if (fabsf(tau) > 1e18f) t = 0.5f / tau;
+  else t = (tau >= 0.0f ? 1.0f : -1.0f) / (fabsf(tau) + sqrtf(1.0f + tau * tau));
+  c = 1.0f / sqrtf(1.0f + t * t);
   s = t * c;
 }
 
-// The FP64 rotation without divisions or roots on the FP64 pipe (a chain of 60 dependent
-// instructions, longer than the rest of a small matrix's round): t = tan of the angle, the
-// smaller root of a t^2 + d t - a = 0 with a = apq, d = aqq - app, both scaled to order one by
-// their exponents; an FP32 root and two Newton steps in FP64 (relative errors 1e-7, 1e-14,
-// rounding), the slope's reciprocal in FP32.  c = (1 + t^2)^-1/2 to rounding keeps c^2 + s^2 = 1.
-__device__ __forceinline__ void rot_params(double app, double aqq, double apq, double& c, double& s) {
+// The FP64 rotation: c = cos of the angle, t = tan, q = tan of its half, from a = apq and
+// d = aqq - app, scaled to order one by their exponents; t is the smaller root of
+// a t^2 + d t - a = 0: an FP32 root and one Newton step in FP64 with the FP32 slope (relative
+// error 1e-13).  No division or root on the FP64 pipe: the chain of dependent instructions is
+// what a small matrix's round takes.  The rotation is orthogonal to rounding whatever the
+// error of t (c = (1 + t^2)^-1/2); what is left of a_pq is computed, not set to zero.
+__device__ __forceinline__ void rot_params(double a0, double d0, double& c, double& t, double& q) {
   c = 1.0;
-  s = 0.0;
-  if (apq == 0.0) return;
-  double d = aqq - app, a = apq;
+  t = q = 0.0;
+  if (a0 == 0.0) return;
+  double d = d0, a = a0;
   const int ed = (__double2hiint(d) >> 20) & 0x7ff, ea = (__double2hiint(a) >> 20) & 0x7ff;
   const int e = max(ed, ea);
   if (e >= 0x7fe || e == 0) {            // infinities, NaNs and subnormal pairs: the plain form
     const double tau = d / (2.0 * a);
-    double t = fabs(tau) > 1e18 ? 0.5 / tau : (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+    t = fabs(tau) > 1e18 ? 0.5 / tau : (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
     c = 1.0 / sqrt(1.0 + t * t);
-    s = t * c;
+    q = t * c / (1.0 + c);
     return;
   }
   // exponents to [.., 1023]; what falls below 2^-1022 of the other is zero beside it
@@ -55,16 +55,17 @@ __device__ __forceinline__ void rot_params(double app, double aqq, double apq, d
   if (ea <= k) return;
   a = __hiloint2double(__double2hiint(a) - (k << 20), __double2loint(a));
   const float df = bits_to_float(d), af = bits_to_float(a);
-  float tf = 2.0f * af / (fabsf(df) + sqrtf(fmaf(df, df, 4.0f * af * af)));
-  double t = bits_to_double(df < 0.0f ? -tf : tf);
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double g = fma(a, t, d);                                  // a t + d
-    const double r = bits_to_double(1.0f / bits_to_float(fma(a, t, g)));   // 1 / (2 a t + d)
-    t = fma(-fma(g, t, -a), r, t);
-  }
+  const float w = fmaf(df, df, 4.0f * af * af), rs = rsqrtf(w);
+  const float tf = __fdividef(2.0f * af, fmaf(w, rs, fabsf(df)));
+  t = bits_to_double(df < 0.0f ? -tf : tf);
+  t = fma(-fma(fma(a, t, d), t, -a), bits_to_double(df < 0.0f ? -rs : rs), t);
   c = nr_rsqrt(fma(t, t, 1.0));
-  s = t * c;
+  // s / (1 + c): the reciprocal by a third-order step from FP32
+  const double x = 1.0 + c;
+  double y = bits_to_double(__fdividef(1.0f, bits_to_float(x)));
+  const double f = fma(-x, y, 1.0);
+  y = fma(y * f, 1.0 + f, y);
+  q = t * c * y;
 }
 
 __device__ __forceinline__ int tri(int i, int j) {  // packed lower triangle, i >= j
@@ -85,20 +86,19 @@ __device__ __forceinline__ int sym(int i, int j) { return i >= j ? tri(i, j) : t
 // is read from a table in shared memory (after V) instead of being decoded with a
 // square root per block and round.  Rotations that are the identity (a_pq = 0) skip
 // their updates.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int rows_per, const double* __restrict__ Ain,
-                                                 long long sA, T* __restrict__ Vg, long long sV,
-                                                 const T* __restrict__ V0, double* __restrict__ w, long long sw,
+__global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int rows_per, const double* __restrict__ Ain,
+                                                 long long sA, float* __restrict__ Vg, long long sV,
+                                                 const float* __restrict__ V0, double* __restrict__ w, long long sw,
                                                  int max_sweeps, double tol, int* __restrict__ info, int use_tab) {
   extern __shared__ unsigned char smem_raw[];
-  T* A = (T*)smem_raw;
+  float* A = (float*)smem_raw;
   const int ntri = m * (m + 1) / 2;
   const int b = blockIdx.x / split, part = blockIdx.x % split;
   const int r0 = part * rows_per, r1 = min(m, r0 + rows_per), nrow = max(0, r1 - r0);
-  T* V = A + ((ntri + 1) & ~1);                      // rows r0..r1 of V (nrow x m)
+  float* V = A + ((ntri + 1) & ~1);                      // rows r0..r1 of V (nrow x m)
   unsigned* tab = (unsigned*)(V + (((size_t)rows_per * m + 1) & ~(size_t)1));
   constexpr int HMAX = 176;                          // m / 2 <= 167
-  __shared__ T cs[HMAX], sn[HMAX];
+  __shared__ float cs[HMAX], sn[HMAX];
   __shared__ int pp[HMAX], qq[HMAX];
   __shared__ double red0[32], red1[32];
   __shared__ int stop;
@@ -109,11 +109,11 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
     while (tri(i + 1, 0) <= idx) ++i;
     while (tri(i, 0) > idx) --i;
     const int j = idx - tri(i, 0);
-    A[idx] = (i < n && j < n) ? (T)Ab[(size_t)i * n + j] : (T)0;
+    A[idx] = (i < n && j < n) ? (float)Ab[(size_t)i * n + j] : (float)0;
   }
   for (int idx = tid; idx < nrow * m; idx += nt) {
     const int i = r0 + idx / m, j = idx % m;
-    T v = (T)(i == j);
+    float v = (float)(i == j);
     if (V0 && i < n && j < n) v = V0[(size_t)b * sV + (size_t)i * m + j];
     V[idx] = v;
   }
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
         const int a0 = (k == 0) ? 0 : 1 + (k - 1 + r) % (m - 1);
         const int a1 = 1 + (m - 2 - k + r) % (m - 1);
         const int p = min(a0, a1), q = max(a0, a1);
-        T c, s;
+        float c, s;
         rot_params(A[tri(p, p)], A[tri(q, q)], A[tri(q, p)], c, s);
         pp[k] = p; qq[k] = q; cs[k] = c; sn[k] = s;
       }
@@ -173,20 +173,20 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
             k2 = it - k * (k + 1) / 2;
           }
           const int p = pp[k], q = qq[k], p2 = pp[k2], q2 = qq[k2];
-          const T c = cs[k], s = sn[k], c2 = cs[k2], s2 = sn[k2];
-          if (s == (T)0 && s2 == (T)0) continue;   // both rotations the identity
+          const float c = cs[k], s = sn[k], c2 = cs[k2], s2 = sn[k2];
+          if (s == (float)0 && s2 == (float)0) continue;   // both rotations the identity
           if (k == k2) {
-            const T app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
+            const float app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
             // J^T [[app, apq], [apq, aqq]] J with the rotation that zeroes apq
-            A[tri(p, p)] = c * c * app - (T)2 * c * s * apq + s * s * aqq;
-            A[tri(q, q)] = s * s * app + (T)2 * c * s * apq + c * c * aqq;
-            A[tri(q, p)] = (T)0;
+            A[tri(p, p)] = c * c * app - (float)2 * c * s * apq + s * s * aqq;
+            A[tri(q, q)] = s * s * app + (float)2 * c * s * apq + c * c * aqq;
+            A[tri(q, p)] = (float)0;
           } else {
             const int ipp = sym(p, p2), ipq = sym(p, q2), iqp = sym(q, p2), iqq = sym(q, q2);
-            const T b00 = A[ipp], b01 = A[ipq], b10 = A[iqp], b11 = A[iqq];
+            const float b00 = A[ipp], b01 = A[ipq], b10 = A[iqp], b11 = A[iqq];
             // rows: J_k^T B
-            const T r00 = c * b00 - s * b10, r01 = c * b01 - s * b11;
-            const T r10 = s * b00 + c * b10, r11 = s * b01 + c * b11;
+            const float r00 = c * b00 - s * b10, r01 = c * b01 - s * b11;
+            const float r10 = s * b00 + c * b10, r11 = s * b01 + c * b11;
             // columns: (J_k^T B) J_k2
             A[ipp] = c2 * r00 - s2 * r01;
             A[ipq] = s2 * r00 + c2 * r01;
@@ -196,10 +196,10 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
         } else {
           const int t = it - nblk;
           const int i = t / h, k = t % h;            // local row i of V
-          const T c = cs[k], s = sn[k];
-          if (s == (T)0) continue;
+          const float c = cs[k], s = sn[k];
+          if (s == (float)0) continue;
           const int p = pp[k], q = qq[k];
-          const T vp = V[i * m + p], vq = V[i * m + q];
+          const float vp = V[i * m + p], vq = V[i * m + q];
           V[i * m + p] = c * vp - s * vq;
           V[i * m + q] = s * vp + c * vq;
         }
@@ -214,16 +214,186 @@ __global__ void __launch_bounds__(1024) k_jacobi(int n, int m, int split, int ro
   for (int idx = tid; idx < nrow * m; idx += nt) Vg[(size_t)b * sV + (size_t)r0 * m + idx] = V[idx];
 }
 
+
+// FP64.  A CTA takes `per` matrices (one if split > 1): the rotations of a round fill only h
+// lanes, and an FP64 instruction takes the SM 16 cycles whether a warp's lanes are on or off.
+// The time of a round is the number of its FP64 warp instructions: 27 for the rotations (with
+// the diagonal, held apart, and what is left of a_pq), 13 for 32 blocks off the diagonal (the
+// tangents applied, then c c2), 3 for 32 pairs of V (three shears instead of two products and
+// two sums).  Each matrix stops by itself.
+// 1024 matrices, cyclic to 1e-15: n = 7 170 -> @@ us, 13 390 -> @@, 25 1840 -> @@; one matrix:
+// n = 7 105 -> @@, 13 218 -> @@, 32 908 -> @@.
+__global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int per, int split, int rows_per,
+                                                   const double* __restrict__ Ain, long long sA,
+                                                   double* __restrict__ Vg, long long sV, const double* __restrict__ V0,
+                                                   double* __restrict__ w, long long sw, int max_sweeps, double tol,
+                                                   int* __restrict__ info) {
+  extern __shared__ double smem_d[];
+  const int ntri = m * (m + 1) / 2, npad = (ntri + 1) & ~1;
+  const int h = m / 2, nblk = h * (h - 1) / 2;
+  const int b0 = blockIdx.x / split * per, part = blockIdx.x % split;
+  per = min(per, batch - b0);
+  const int r0 = part * rows_per, r1 = min(m, r0 + rows_per), nrow = max(0, r1 - r0);
+  // per matrix: the packed lower triangle (its diagonal slots zero), the diagonal, rows of V
+  const int mat = npad + m + ((rows_per * m + 1) & ~1);
+  double* rot = smem_d + per * mat;                  // c, t, s, tan of half the angle of every pair
+  unsigned* tab = (unsigned*)(rot + 4 * per * h);    // (k, k2) of a block
+  unsigned short* pq = (unsigned short*)(tab + nblk);  // p, q of pair k
+  __shared__ double red[32];
+  __shared__ int done[32], ndone;
+  const int nt = blockDim.x, tid = threadIdx.x;
+  for (int idx = tid; idx < per * m * m; idx += nt) {
+    const int g = idx / (m * m), e = idx - g * m * m, i = e / m, j = e - i * m;
+    if (j > i) continue;
+    const double a = i < n && j < n ? Ain[(size_t)(b0 + g) * sA + (size_t)i * n + j] : 0.0;
+    smem_d[g * mat + tri(i, j)] = i == j ? 0.0 : a;
+    if (i == j) smem_d[g * mat + npad + i] = a;
+  }
+  for (int idx = tid; idx < per * nrow * m; idx += nt) {
+    const int g = idx / (nrow * m), e = idx - g * nrow * m, i = r0 + e / m, j = e % m;
+    double v = (double)(i == j);
+    if (V0 && i < n && j < n) v = V0[(size_t)(b0 + g) * sV + (size_t)i * m + j];
+    smem_d[g * mat + npad + m + e] = v;
+  }
+  for (int k = tid; k < h; k += nt)
+    for (int k2 = 0; k2 < k; ++k2) tab[k * (k - 1) / 2 + k2] = ((unsigned)k << 16) | (unsigned)k2;
+  if (tid < 32) done[tid] = 0;
+  if (tid == 0) ndone = 0;
+  __syncthreads();
+  const int wpm = (nt / 32) / per, warp = tid >> 5, lane = tid & 31;   // warps per matrix
+  const int na = (per * nblk + 31) & ~31, nv = per * nrow * h;
+  double tot = 0.0;
+  int sweep = 0;
+  for (;; ++sweep) {
+    // sums of squares off the diagonal, and (unchanged by rotations) in all
+    {
+      const int g = warp / wpm, sub = (warp - g * wpm) * 32 + lane;
+      double off = 0.0, dia = 0.0;
+      if (g < per && !done[g]) {
+        const double* A = smem_d + g * mat;
+        double o1 = 0.0;
+        for (int idx = sub; idx < ntri; idx += 64 * wpm) {
+          off = fma(A[idx], A[idx], off);
+          const int i2 = idx + 32 * wpm;
+          if (i2 < ntri) o1 = fma(A[i2], A[i2], o1);
+        }
+        off = 2.0 * (off + o1);
+        if (sweep == 0)
+          for (int i = sub; i < m; i += 32 * wpm) dia = fma(A[npad + i], A[npad + i], dia);
+      }
+      for (int o = 16; o > 0; o >>= 1) off += __shfl_xor_sync(0xffffffffu, off, o);
+      if (sweep == 0) {
+        tot = dia;
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        if (lane == 0) red[warp] = tot + off;
+        __syncthreads();
+        tot = 0.0;
+        if (tid < per)
+          for (int k = 0; k < wpm; ++k) tot += red[tid * wpm + k];
+        __syncthreads();
+      }
+      if (lane == 0) red[warp] = off;
+    }
+    __syncthreads();
+    if (tid < per && !done[tid]) {
+      double o2 = 0.0;
+      for (int k = 0; k < wpm; ++k) o2 += red[tid * wpm + k];
+      if (o2 <= tol * tol * tot || sweep == max_sweeps) {
+        done[tid] = 1;
+        atomicAdd(&ndone, 1);
+        if (part == 0 && info) info[b0 + tid] = sweep;
+      }
+    }
+    __syncthreads();
+    if (ndone == per) break;
+    for (int r = 0; r < m - 1; ++r) {
+      for (int it = tid; it < per * h; it += nt) {
+        const int g = it / h, k = it - g * h;
+        // circle method: position 0 fixed, positions 1..m-1 rotate by r
+        int a0 = k - 1 + r, a1 = m - 2 - k + r;
+        a0 -= a0 >= m - 1 ? m - 1 : 0;
+        a1 -= a1 >= m - 1 ? m - 1 : 0;
+        a0 = k == 0 ? 0 : 1 + a0;
+        a1 = 1 + a1;
+        const int p = min(a0, a1), q = max(a0, a1);
+        double* A = smem_d + g * mat;
+        double* dg = A + npad;
+        const double a = done[g] ? 0.0 : A[tri(q, p)], dp = dg[p], dq = dg[q], d = dq - dp;
+        double c, t, hf;
+        rot_params(a, d, c, t, hf);
+        if (g == 0) *(unsigned*)(pq + 2 * k) = (unsigned)p | ((unsigned)q << 16);
+        double2* o = (double2*)(rot + 4 * it);
+        o[0] = make_double2(c, t);
+        o[1] = make_double2(t * c, hf);
+        if (t != 0.0) {
+          const double c2 = c * c, ch = (t * c2) * fma(-t, d, a + a);
+          dg[p] = dp - ch;
+          dg[q] = dq + ch;
+          A[tri(q, p)] = -c2 * fma(fma(a, t, d), t, -a);
+        }
+      }
+      __syncthreads();
+      for (int it = tid; it < na + nv; it += nt) {
+        if (it < na) {
+          const int g = per == 1 ? 0 : it / nblk;
+          if (g >= per || it >= per * nblk) continue;
+          const unsigned e = tab[it - g * nblk];
+          const int k = (int)(e >> 16), k2 = (int)(e & 0xFFFFu);
+          const double2 r1 = *(const double2*)(rot + 4 * (g * h + k)), r2 = *(const double2*)(rot + 4 * (g * h + k2));
+          const double t = r1.y, t2 = r2.y;
+          if (t == 0.0 && t2 == 0.0) continue;       // both rotations the identity
+          const int p = pq[2 * k], q = pq[2 * k + 1], p2 = pq[2 * k2], q2 = pq[2 * k2 + 1];
+          double* A = smem_d + g * mat;
+          const int ipp = sym(p, p2), ipq = sym(p, q2), iqp = sym(q, p2), iqq = sym(q, q2);
+          const double b00 = A[ipp], b01 = A[ipq], b10 = A[iqp], b11 = A[iqq], cc = r1.x * r2.x;
+          // rows, then columns
+          const double r00 = fma(-t, b10, b00), r01 = fma(-t, b11, b01);
+          const double r10 = fma(t, b00, b10), r11 = fma(t, b01, b11);
+          A[ipp] = cc * fma(-t2, r01, r00);
+          A[ipq] = cc * fma(t2, r00, r01);
+          A[iqp] = cc * fma(-t2, r11, r10);
+          A[iqq] = cc * fma(t2, r10, r11);
+        } else {
+          const int x = it - na, row = x / h, k = x - row * h, g = per == 1 ? 0 : row / nrow;
+          const double2 sh = *(const double2*)(rot + 4 * (g * h + k) + 2);
+          if (sh.x == 0.0) continue;
+          const unsigned e = *(const unsigned*)(pq + 2 * k);
+          double* v = smem_d + g * mat + npad + m + (row - g * nrow) * m;
+          double* vp = v + (e & 0xFFFFu);
+          double* vq = v + (e >> 16);
+          const double x0 = fma(-sh.y, *vq, *vp), y1 = fma(sh.x, x0, *vq);
+          *vp = fma(-sh.y, y1, x0);
+          *vq = y1;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int idx = tid; idx < per * m; idx += nt) {
+    const int g = idx / m, i = idx - g * m;
+    if (part == 0 && i < n) w[(size_t)(b0 + g) * sw + i] = smem_d[g * mat + npad + i];
+  }
+  for (int idx = tid; idx < per * nrow * m; idx += nt) {
+    const int g = idx / (nrow * m), e = idx - g * nrow * m;
+    Vg[(size_t)(b0 + g) * sV + (size_t)r0 * m + e] = smem_d[g * mat + npad + m + e];
+  }
+}
+
+// bytes of `per` matrices with rows_per rows of V each
+static size_t jacobi_bytes_d(int m, int per, int rows_per) {
+  const size_t h = m / 2, mat = (((size_t)m * (m + 1) / 2 + 1) & ~(size_t)1) + m + (((size_t)rows_per * m + 1) & ~(size_t)1);
+  return per * (mat + 4 * h) * 8 + h * (h - 1) / 2 * 4 + 4 * h + 16;
+}
+
 // shared-memory plan of one launch: how many CTAs share a matrix (at least `least`), rows of V
 // per CTA, whether the block table fits, and the dynamic bytes
-template <typename T>
 static bool jacobi_plan(int m, int least, int& split, int& rows_per, int& tab, size_t& bytes) {
   const size_t limit = 232448 - 5120;                // 227 KB less the static tables
-  const size_t a_bytes = (size_t)((m * (m + 1) / 2 + 1) & ~1) * sizeof(T);
+  const size_t a_bytes = (size_t)((m * (m + 1) / 2 + 1) & ~1) * sizeof(float);
   const size_t tab_bytes = (size_t)(m / 2) * (m / 2 + 1) / 2 * sizeof(unsigned);
   for (split = least; split <= m; ++split) {
     rows_per = (m + split - 1) / split;
-    const size_t v_bytes = (size_t)(((size_t)rows_per * m + 1) & ~(size_t)1) * sizeof(T);
+    const size_t v_bytes = (size_t)(((size_t)rows_per * m + 1) & ~(size_t)1) * sizeof(float);
     if (a_bytes + v_bytes <= limit) {
       tab = a_bytes + v_bytes + tab_bytes <= limit;
       bytes = a_bytes + v_bytes + (tab ? tab_bytes : 0);
@@ -258,21 +428,34 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
   int split = 1, rows_per = m, tab = 0;
   size_t bytes = 0;
   if (!fp32) {
-    if (m / 2 > 68 || !jacobi_plan<double>(m, least, split, rows_per, tab, bytes)) {
+    if (m / 2 > 68) {
       pcg_set_error("pcg_jacobi_eigh: FP64 variant needs n <= 136");
       return PCG_ERR_UNSUPPORTED;
     }
-    PCG_CUDA(cudaFuncSetAttribute(k_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_jacobi<double><<<batch * split, threads, bytes, s>>>(n, m, split, rows_per, A, sA, (double*)V, sV,
-                                                           (const double*)V0, w, sw, max_sweeps, tol, info, tab);
+    // matrices per CTA: what the rotations leave of a warp, as long as the SMs have 1.5 CTAs each
+    // (n = 13: 1024 matrices 294 us by fours, 338 by twos; 400 matrices 238 us one by one, 267 by
+    // twos)
+    int per = 1;
+    while (2 * per * (m / 2) < 32 && batch / (2 * per) >= 228) per *= 2;
+    for (split = least; jacobi_bytes_d(m, 1, (m + split - 1) / split) > 232448 - 1024; ++split) {}
+    rows_per = (m + split - 1) / split;
+    bytes = jacobi_bytes_d(m, per, rows_per);
+    const long long ctas = (long long)((batch + per - 1) / per) * split;
+    if (ctas > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
+    // 128 threads where that fills the SMs (4096 of n = 13: 691 us, 797 with 256) or a round has
+    // no more work; else 256 (one matrix of n = 32: 478 us, 526 with 128)
+    const int th = m <= 32 ? (m * per <= 8 || ctas > 608 ? 128 : 256) : threads;
+    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    k_jacobi_d<<<(unsigned)ctas, th, bytes, s>>>(n, m, batch, per, split, rows_per, A, sA, (double*)V, sV,
+                                                 (const double*)V0, w, sw, max_sweeps, tol, info);
   } else {
-    if (m / 2 > 167 || !jacobi_plan<float>(m, least, split, rows_per, tab, bytes)) {
+    if (m / 2 > 167 || !jacobi_plan(m, least, split, rows_per, tab, bytes)) {
       pcg_set_error("pcg_jacobi_eigh: FP32 variant needs n <= 334");
       return PCG_ERR_UNSUPPORTED;
     }
     if ((long long)batch * split > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
-    PCG_CUDA(cudaFuncSetAttribute(k_jacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_jacobi<float><<<batch * split, threads, bytes, s>>>(n, m, split, rows_per, A, sA, (float*)V, sV,
+    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    k_jacobi_f<<<batch * split, threads, bytes, s>>>(n, m, split, rows_per, A, sA, (float*)V, sV,
                                                           (const float*)V0, w, sw, max_sweeps, tol, info, tab);
   }
   PCG_CUDA(cudaGetLastError());
