@@ -387,6 +387,12 @@ int pcg_scf_stats(int n, int n2, const double *P, const double *D, const double 
 int pcg_projector_check(int n, int nocc, const double *S, const double *R, double *out, void *stream);
 int pcg_oa_correction(int n, int nocc, int mode, const double *delta, const double *S, const double *R, double *E,
                       double *lam, void *stream);
+/* pcg_diis_batched: the C1 systems of `batch` molecules, one warp each: Bnew (mn x mn, oldest
+ *   first) from Bold (mo x mo) and row (ldrow doubles apart: products of the newest residual with
+ *   the mo older ones, then with itself), the oldest mo + 1 - mn left out; coef: mn per
+ *   molecule.  Scaled like pcg_diis_step; the oldest are dropped while a pivot is zero. */
+int pcg_diis_batched(int batch, int mo, int mn, const double *Bold, const double *row, long long ldrow,
+                     double *Bnew, double *coef, void *stream);
 int pcg_diis_step(long long len, int cap, int *state, const double *F, const double *R, double *focks,
                   double *resids, double *Bm, double *row, double *coef, double *Fx, void *stream);
 

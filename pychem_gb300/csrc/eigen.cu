@@ -221,8 +221,9 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
 // the diagonal, held apart, and what is left of a_pq), 13 for 32 blocks off the diagonal (the
 // tangents applied, then c c2), 3 for 32 pairs of V (three shears instead of two products and
 // two sums).  Each matrix stops by itself.
-// 1024 matrices, cyclic to 1e-15: n = 7 170 -> @@ us, 13 390 -> @@, 25 1840 -> @@; one matrix:
-// n = 7 105 -> @@, 13 218 -> @@, 32 908 -> @@.
+// 1024 matrices to 1e-15, against a CTA each with two barriers' worth of rotations, 16-instruction
+// blocks and 4-instruction pairs: n = 7 170 -> 112 us, 13 390 -> 295, 25 1840 -> 1297; one
+// matrix: n = 7 105 -> 82 us, 13 218 -> 176, 32 908 -> 478.
 __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int per, int split, int rows_per,
                                                    const double* __restrict__ Ain, long long sA,
                                                    double* __restrict__ Vg, long long sV, const double* __restrict__ V0,

@@ -281,7 +281,8 @@ def rhf_batched(eng, max_iter=64, e_tol=1e-10, d_tol=1e-8, diis_size=8, guess="s
     F_fin = torch.empty_like(S)
     D_fin = torch.empty_like(S)
     focks, resids = [], []
-    Bm = np.zeros((B, 0, 0))
+    on_gpu = diis_size <= 32              # the C1 systems: a warp each
+    Bm = torch.zeros(B, 0, 0, dtype=torch.float64, device=dev) if on_gpu else np.zeros((B, 0, 0))
     E_old = D_old = None
     done_at = np.zeros(B, dtype=np.int64)
     E_at = np.zeros(B)
@@ -315,7 +316,8 @@ def rhf_batched(eng, max_iter=64, e_tol=1e-10, d_tol=1e-8, diis_size=8, guess="s
             vals.append(torch.sqrt(torch.mean((D - D_old) ** 2, dim=(1, 2))) if D_old is not None
                         else torch.zeros(len(act), dtype=torch.float64, device=dev))
             vals += [torch.sum(Rf * r.reshape(len(act), -1), dim=1) for r in resids] + [torch.sum(Rf * Rf, dim=1)]
-            host = torch.stack(vals, dim=1).cpu().numpy()
+            vals = torch.stack(vals, dim=1)
+            host = vals.cpu().numpy()
             if trace is not None:
                 now = time.perf_counter()
                 trace.append((it, len(act), int(p32.sum()), now - t_last))
@@ -343,7 +345,7 @@ def rhf_batched(eng, max_iter=64, e_tol=1e-10, d_tol=1e-8, diis_size=8, guess="s
                     Q = Q[kt] if Q is not None else None
                     focks = [f[kt] for f in focks]
                     resids = [r[kt] for r in resids]
-                    Bm = Bm[keep]
+                    Bm, vals = (Bm[kt], vals[kt]) if on_gpu else (Bm[keep], vals)
                     if len(act) <= compact * covered:
                         mask = np.zeros(B, dtype=bool)
                         mask[act] = True
@@ -364,23 +366,28 @@ def rhf_batched(eng, max_iter=64, e_tol=1e-10, d_tol=1e-8, diis_size=8, guess="s
                 # error would otherwise persist through X_prev
                 sw = torch.as_tensor(switched, device=dev)
                 Q.index_copy_(0, sw, torch.eye(n, dtype=torch.float64, device=dev).expand(len(switched), n, n))
-            row = host[:, 2:]
-            m = row.shape[1]
-            Bn = np.zeros((len(act), m, m))
-            Bn[:, :m - 1, :m - 1] = Bm
-            Bn[:, m - 1, :] = row
-            Bn[:, :, m - 1] = row
             focks.append(F)
             resids.append(R)
-            Bm = Bn
             if len(focks) > diis_size:
                 focks.pop(0); resids.pop(0)
-                Bm = Bm[:, 1:, 1:]
-            Fx = F
             k = len(focks)
-            if k > 1:
-                cw = torch.tensor(diis_coefficients_batched(Bm), dtype=torch.float64, device=dev)
-                Fx = torch.einsum("bk,kbij->bij", cw, torch.stack(focks))
+            if on_gpu:
+                Bn = torch.empty(len(act), k, k, dtype=torch.float64, device=dev)
+                cw = torch.empty(len(act), k, dtype=torch.float64, device=dev)
+                _lib.call("pcg_diis_batched", len(act), Bm.shape[1], k, _ptr(Bm), _ptr(vals[:, 2:]), vals.stride(0),
+                          _ptr(Bn), _ptr(cw), _stream())
+            else:
+                row = host[:, 2:]
+                m = row.shape[1]
+                Bn = np.zeros((len(act), m, m))
+                Bn[:, :m - 1, :m - 1] = Bm
+                Bn[:, m - 1, :] = row
+                Bn[:, :, m - 1] = row
+                Bn = Bn[:, m - k:, m - k:]
+                if k > 1:
+                    cw = torch.tensor(diis_coefficients_batched(Bn), dtype=torch.float64, device=dev)
+            Bm = Bn
+            Fx = torch.einsum("bk,kbij->bij", cw, torch.stack(focks)) if k > 1 else F
             Qn, Dn, Dpn = torch.empty_like(F), torch.empty_like(F), torch.empty_like(F)
             for rows, dt in groups(p32):
                 out = _dense_density(take(Fx, rows), take(Xa, rows), take(Xta, rows), take(occa, rows),

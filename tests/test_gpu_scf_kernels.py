@@ -5,6 +5,7 @@ Tolerances: products as sums of K terms (1e-13 K max|a| max|b|); eigenvalues and
 1e-12 of the norm and orthogonality 1e-13, the bars of test_gpu_eigen.py."""
 import ctypes
 
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -163,3 +164,45 @@ def test_rhf_without_a_gap():
     assert bool(torch.isfinite(got.eps).all()) and bool(torch.isfinite(got.D).all())
     assert got.converged == want.converged
     assert not want.converged or abs(got.E - want.E) < 1e-7
+
+
+@pytest.mark.parametrize("batch,mo,mn", [(1, 0, 1), (3, 1, 2), (5, 7, 8), (6, 8, 8), (130, 8, 8), (2, 31, 32), (2, 32, 32)])
+def test_diis_batched(batch, mo, mn):
+    """Coefficients and the moved matrix against the host's solve: 64 eps times the condition
+    of the scaled system."""
+    from pychem_gb300 import _lib
+    from pychem_gb300.engine import _ptr
+    from pychem_gb300._stream import stream
+    from pychem_gb300.scf import diis_coefficients_batched
+    rng = np.random.default_rng(mo)
+    r = rng.standard_normal((batch, mo + 1, 3 * mo + 4)) * 0.5 ** np.arange(mo + 1)[:, None]
+    G = np.einsum("bik,bjk->bij", r, r)
+    old = torch.tensor(G[:, :mo, :mo].copy(), device="cuda")
+    row = torch.zeros(batch, mo + 3, dtype=torch.float64, device="cuda")
+    row[:, 2:] = torch.tensor(G[:, mo, :].copy())
+    new = torch.empty(batch, mn, mn, dtype=torch.float64, device="cuda")
+    coef = torch.empty(batch, mn, dtype=torch.float64, device="cuda")
+    _lib.call("pcg_diis_batched", batch, mo, mn, _ptr(old), _ptr(row[:, 2:]), row.stride(0), _ptr(new), _ptr(coef), stream())
+    cut = mo + 1 - mn
+    assert np.array_equal(new.cpu().numpy(), G[:, cut:, cut:])
+    want = diis_coefficients_batched(G[:, cut:, cut:])
+    M = -np.ones((batch, mn + 1, mn + 1))
+    M[:, :mn, :mn] = G[:, cut:, cut:] / np.abs(np.diagonal(G[:, cut:, cut:], axis1=1, axis2=2)).max(1)[:, None, None]
+    M[:, mn, mn] = 0.0
+    tol = 64 * 2.2e-16 * np.linalg.cond(M)
+    assert (np.abs(coef.cpu().numpy() - want).max(1) <= tol * np.maximum(1.0, np.abs(want).max(1))).all()
+
+
+def test_diis_batched_drops_repeats():
+    """Residuals that repeat exactly: the newest alone is used."""
+    from pychem_gb300 import _lib
+    from pychem_gb300.engine import _ptr
+    from pychem_gb300._stream import stream
+    G = np.ones((2, 3, 3))
+    G[1] = 0.0
+    old = torch.tensor(G[:, :2, :2].copy(), device="cuda")
+    row = torch.tensor(G[:, 2, :].copy(), device="cuda")
+    new = torch.empty(2, 3, 3, dtype=torch.float64, device="cuda")
+    coef = torch.empty(2, 3, dtype=torch.float64, device="cuda")
+    _lib.call("pcg_diis_batched", 2, 2, 3, _ptr(old), _ptr(row), 3, _ptr(new), _ptr(coef), stream())
+    assert coef.cpu().tolist() == [[0.0, 0.0, 1.0]] * 2
