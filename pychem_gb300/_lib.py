@@ -164,7 +164,7 @@ launch_count = 0
 _RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
              "pcg_mlp_wgrad_workspace": ctypes.c_size_t, "pcg_coulomb_exchange_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_prim_pack": 2, "pcg_coulomb_exchange": 4}
+MULTI_LAUNCH = {"pcg_one_electron": 6, "pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_prim_pack": 2, "pcg_coulomb_exchange": 4}
 
 _lib = None
 

@@ -143,37 +143,64 @@ int pcg_ensure_bessel(BesselTable* out) {
 }
 
 // ----------------------------------------------------------------------------------
-// Primitive-pair data: one thread per shell pair, loop over its primitive pairs.
+// Primitive-pair data.  A warp takes the primitive pairs of `group` (1 to 32) shell pairs in a
+// row, its lanes one each whatever shell pair they belong to: an exponential, two roots and a
+// reciprocal are a chain of about a microsecond, and the 36 of an oxygen 1s pair on one
+// thread took 171 us.
 // ----------------------------------------------------------------------------------
-__global__ void k_pair_data(DevBasis b, int npair, const int* pA, const int* pB, const int* ppoff,
-                            double* AB, double* zeta, double* P, double* PA, double* K, float* Kf,
-                            double* oo2z) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npair) return;
-  const int A = pA[p], B = pB[p];
-  const double ax = b.sh_xyz[3 * A], ay = b.sh_xyz[3 * A + 1], az = b.sh_xyz[3 * A + 2];
-  const double bx = b.sh_xyz[3 * B], by = b.sh_xyz[3 * B + 1], bz = b.sh_xyz[3 * B + 2];
-  const double dx = ax - bx, dy = ay - by, dz = az - bz;
-  const double r2 = dx * dx + dy * dy + dz * dz;
-  AB[3 * p] = dx; AB[3 * p + 1] = dy; AB[3 * p + 2] = dz;
-  const int na = b.sh_nprim[A], nb = b.sh_nprim[B];
-  int k = ppoff[p];
-  for (int i = 0; i < na; ++i) {
-    const double a = b.pr_exp[b.sh_prim[A] + i], ca = b.pr_cc[b.sh_prim[A] + i];
-    for (int j = 0; j < nb; ++j, ++k) {
-      const double be = b.pr_exp[b.sh_prim[B] + j], cb = b.pr_cc[b.sh_prim[B] + j];
-      const double z = a + be, s = 1.0 / z;
-      const double U = pow(M_PI * s, 1.5) * exp(-a * be * s * r2);
-      const double px = (a * ax + be * bx) * s, py = (a * ay + be * by) * s, pz = (a * az + be * bz) * s;
-      zeta[k] = z;
-      oo2z[k] = 0.5 * s;
-      P[3 * k] = px; P[3 * k + 1] = py; P[3 * k + 2] = pz;
-      PA[3 * k] = px - ax; PA[3 * k + 1] = py - ay; PA[3 * k + 2] = pz - az;
-      // sqrt(2/sqrt(pi)) = 1.0622519320271968
-      const double kk = ca * cb * 1.0622519320271968 * U * sqrt(z);
-      K[k] = kk;
-      Kf[k] = (float)kk;
-    }
+__global__ void __launch_bounds__(128) k_pair_data(DevBasis b, int npair, int group, const int* __restrict__ pA,
+                                                   const int* __restrict__ pB, const int* __restrict__ ppoff,
+                                                   double* __restrict__ AB, double* __restrict__ zeta,
+                                                   double* __restrict__ P, double* __restrict__ PA,
+                                                   double* __restrict__ K, float* __restrict__ Kf,
+                                                   double* __restrict__ oo2z) {
+  const int lane = threadIdx.x & 31;
+  const int p0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * group;
+  if (p0 >= npair) return;
+  int A = 0, B = 0, k0 = 0, nb = 1, count = 0;       // this lane's shell pair
+  if (lane < group && p0 + lane < npair) {
+    const int p = p0 + lane;
+    A = pA[p];
+    B = pB[p];
+    k0 = ppoff[p];
+    nb = b.sh_nprim[B];
+    count = b.sh_nprim[A] * nb;
+    for (int d = 0; d < 3; ++d) AB[3 * p + d] = b.sh_xyz[3 * A + d] - b.sh_xyz[3 * B + d];
+  }
+  int end = count;                                   // primitive pairs up to and with this lane's
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += x;
+  }
+  const int total = __shfl_sync(0xffffffffu, end, 31);
+  for (int it0 = 0; it0 < total; it0 += 32) {
+    const int it = it0 + lane;
+    int src = 0;                                     // the first lane with end > it
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, end, src + o - 1) <= it) src += o;
+    src = min(src, 31);
+    const int sA = __shfl_sync(0xffffffffu, A, src), sB = __shfl_sync(0xffffffffu, B, src);
+    const int snb = __shfl_sync(0xffffffffu, nb, src), sk = __shfl_sync(0xffffffffu, k0, src);
+    const int local = it - (__shfl_sync(0xffffffffu, end, src) - __shfl_sync(0xffffffffu, count, src));
+    if (it >= total) continue;
+    const int i = local / snb, j = local - i * snb, k = sk + local;
+    const double ax = b.sh_xyz[3 * sA], ay = b.sh_xyz[3 * sA + 1], az = b.sh_xyz[3 * sA + 2];
+    const double bx = b.sh_xyz[3 * sB], by = b.sh_xyz[3 * sB + 1], bz = b.sh_xyz[3 * sB + 2];
+    const double dx = ax - bx, dy = ay - by, dz = az - bz;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double a = b.pr_exp[b.sh_prim[sA] + i], ca = b.pr_cc[b.sh_prim[sA] + i];
+    const double be = b.pr_exp[b.sh_prim[sB] + j], cb = b.pr_cc[b.sh_prim[sB] + j];
+    const double z = a + be, s = 1.0 / z, ps = M_PI * s;
+    const double U = ps * sqrt(ps) * exp(-a * be * s * r2);
+    const double px = (a * ax + be * bx) * s, py = (a * ay + be * by) * s, pz = (a * az + be * bz) * s;
+    zeta[k] = z;
+    oo2z[k] = 0.5 * s;
+    P[3 * k] = px; P[3 * k + 1] = py; P[3 * k + 2] = pz;
+    PA[3 * k] = px - ax; PA[3 * k + 1] = py - ay; PA[3 * k + 2] = pz - az;
+    // sqrt(2/sqrt(pi)) = 1.0622519320271968
+    const double kk = ca * cb * 1.0622519320271968 * U * sqrt(z);
+    K[k] = kk;
+    Kf[k] = (float)kk;
   }
 }
 
@@ -181,7 +208,10 @@ int pcg_launch_pair_data(const DevBasis& b, int npair, const int* pA, const int*
                          double* AB, double* zeta, double* P, double* PA, double* K, float* Kf, double* oo2z,
                          cudaStream_t s) {
   if (npair <= 0) return PCG_OK;
-  k_pair_data<<<(npair + 127) / 128, 128, 0, s>>>(b, npair, pA, pB, ppoff, AB, zeta, P, PA, K, Kf, oo2z);
+  int group = 1;                                     // about 16 warps on every SM
+  while (group < 32 && npair / group > 2432) group *= 2;
+  const int warps = (npair + group - 1) / group;
+  k_pair_data<<<(warps + 3) / 4, 128, 0, s>>>(b, npair, group, pA, pB, ppoff, AB, zeta, P, PA, K, Kf, oo2z);
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
 }
@@ -223,22 +253,6 @@ int pcg_launch_pair_ao(const DevBasis& b, int npair, const int* pA, const int* p
 // ----------------------------------------------------------------------------------
 // One-electron integrals
 // ----------------------------------------------------------------------------------
-__device__ __forceinline__ int d_ncart(int l) { return (l + 1) * (l + 2) / 2; }
-__device__ __forceinline__ int d_off(int l) { return l * (l + 1) * (l + 2) / 6; }
-__device__ __forceinline__ int d_gidx(int x, int y, int z) {
-  int l = x + y + z, s = y + z;
-  return d_off(l) + s * (s + 1) / 2 + z;
-}
-__device__ __forceinline__ void d_comp(int l, int k, int* c) {
-  // k-th Cartesian component of shell l (lx descending, then ly descending)
-  int idx = 0;
-  for (int lx = l; lx >= 0; --lx)
-    for (int ly = l - lx; ly >= 0; --ly) {
-      if (idx == k) { c[0] = lx; c[1] = ly; c[2] = l - lx - ly; return; }
-      ++idx;
-    }
-}
-
 // Cartesian -> spherical row coefficient times the component normalisation ratio.
 __device__ __forceinline__ double d_sph(int l, int r, int c) {
   if (l <= 1) return r == c ? 1.0 : 0.0;
@@ -253,201 +267,236 @@ __device__ __forceinline__ double d_sph(int l, int r, int c) {
   }
 }
 
-// One warp per shell pair: lanes stride over the primitive pairs for S and T and over
-// (primitive pair, nucleus) items for the nuclear attraction V (the loop that
-// dominates: nuclei x primitive pairs), the Cartesian blocks are summed across the
-// warp with shuffles, and lane 0 applies the spherical transform and stores both
-// triangles of S and H (Methods/integrals.py:220-370).
-struct OePrim {
-  double U, z, oo2z, cc, P[3], PA[3], PB[3];
-};
+// (x, y, z) of degree d is component s(s+1)/2 + z, s = y + z, of its degree
+__host__ __device__ constexpr int oe_ncart(int l) { return (l + 1) * (l + 2) / 2; }
+__host__ __device__ constexpr int oe_first(int l) { return l * (l + 1) * (l + 2) / 6; }
+__host__ __device__ constexpr int oe_k(int s, int z) { return s * (s + 1) / 2 + z; }
+__host__ __device__ constexpr int oe_up(int s, int z, int i) { return i == 0 ? oe_k(s, z) : oe_k(s + 1, z + (i == 2)); }
 
-__device__ __forceinline__ OePrim oe_prim(const DevBasis& b, int A, int B, int ia, int ib, double r2) {
-  OePrim q;
-  const double* Ax = b.sh_xyz + 3 * A;
-  const double* Bx = b.sh_xyz + 3 * B;
-  const double al = b.pr_exp[b.sh_prim[A] + ia], be = b.pr_exp[b.sh_prim[B] + ib];
-  q.cc = b.pr_cc[b.sh_prim[A] + ia] * b.pr_cc[b.sh_prim[B] + ib];
-  q.z = al + be;
-  const double s = 1.0 / q.z;
-  q.oo2z = 0.5 * s;
-  q.U = pow(M_PI * s, 1.5) * exp(-al * be * s * r2);
-  for (int i = 0; i < 3; ++i) {
-    q.P[i] = (al * Ax[i] + be * Bx[i]) * s;
-    q.PA[i] = q.P[i] - Ax[i];
-    q.PB[i] = q.P[i] - Bx[i];
-  }
-  return q;
-}
-
-__global__ void k_one_electron(DevBasis b, BoysTable bt, int npair, const int* pA, const int* pB,
-                               double* S, double* H) {
-  const int p = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (p >= npair) return;  // whole warps leave together
-  const int A = pA[p], B = pB[p];
-  const int la = b.sh_l[A], lb = b.sh_l[B];
-  const int nca = d_ncart(la), ncb = d_ncart(lb);
-  double Sc[36], Tc[36], Vc[36];
-  for (int i = 0; i < 36; ++i) { Sc[i] = 0.0; Tc[i] = 0.0; Vc[i] = 0.0; }
-  const double* Ax = b.sh_xyz + 3 * A;
-  const double* Bx = b.sh_xyz + 3 * B;
-  double r2 = 0.0;
-  for (int i = 0; i < 3; ++i) r2 += (Ax[i] - Bx[i]) * (Ax[i] - Bx[i]);
-  const int npa = b.sh_nprim[A], npb = b.sh_nprim[B];
-  for (int item = lane; item < npa * npb; item += 32) {
-    const int ia = item / npb, ib = item % npb;
-    const double be = b.pr_exp[b.sh_prim[B] + ib];
-    const OePrim q = oe_prim(b, A, B, ia, ib, r2);
-    const double U = q.U, oo2z = q.oo2z, cc = q.cc;
-    const double *PA = q.PA, *PB = q.PB;
-      // 1D overlap factors E[dir][i][j], i <= la, j <= lb + 2 (Obara-Saika)
-      double E[3][3][5];
-      for (int d = 0; d < 3; ++d) {
-        for (int i = 0; i <= la; ++i)
-          for (int j = 0; j <= lb + 2; ++j) {
-            double v;
-            if (i == 0 && j == 0) v = 1.0;
-            else if (j == 0) {
-              v = PA[d] * E[d][i - 1][0];
-              if (i > 1) v += (i - 1) * oo2z * E[d][i - 2][0];
-            } else {
-              v = PB[d] * E[d][i][j - 1];
-              if (i > 0) v += i * oo2z * E[d][i - 1][j - 1];
-              if (j > 1) v += (j - 1) * oo2z * E[d][i][j - 2];
-            }
-            E[d][i][j] = v;
-          }
-      }
-      for (int ka = 0; ka < nca; ++ka) {
-        int x[3]; d_comp(la, ka, x);
-        for (int kb = 0; kb < ncb; ++kb) {
-          int y[3]; d_comp(lb, kb, y);
-          const double sv = E[0][x[0]][y[0]] * E[1][x[1]][y[1]] * E[2][x[2]][y[2]];
-          // kinetic energy from overlaps [a|b+2], [a|b], [a|b-2] (one_electron_kinetic.c:60-64)
-          double t = be * (2 * lb + 3) * sv;
-          for (int i = 0; i < 3; ++i) {
-            int yp[3] = {y[0], y[1], y[2]};
-            yp[i] += 2;
-            t -= 2.0 * be * be * E[0][x[0]][yp[0]] * E[1][x[1]][yp[1]] * E[2][x[2]][yp[2]];
-            if (y[i] > 1) {
-              int ym[3] = {y[0], y[1], y[2]};
-              ym[i] -= 2;
-              t -= 0.5 * y[i] * (y[i] - 1) * E[0][x[0]][ym[0]] * E[1][x[1]][ym[1]] * E[2][x[2]][ym[2]];
-            }
-          }
-          Sc[ka * ncb + kb] += cc * U * sv;
-          Tc[ka * ncb + kb] += cc * U * t;
-        }
-      }
-  }
-  // nuclear attraction: Obara-Saika with auxiliary index over the molecule's nuclei
-  const int L = la + lb;
-  const int c0 = b.sh_at0 ? b.sh_at0[A] : 0;
-  const int c1 = b.sh_at0 ? c0 + b.sh_nat[A] : b.natom;
-  const int nnuc = c1 - c0;
-  for (int item = lane; item < npa * npb * nnuc; item += 32) {
-    const int c = c0 + item % nnuc, pp = item / nnuc;
-    const OePrim q = oe_prim(b, A, B, pp / npb, pp % npb, r2);
-    const double U = q.U, oo2z = q.oo2z, cc = q.cc, z = q.z;
-    const double *P = q.P, *PA = q.PA, *PB = q.PB;
-    {
-        const double* C = b.at_xyz + 3 * c;
-        double PC[3], pc2 = 0.0;
-        for (int i = 0; i < 3; ++i) { PC[i] = P[i] - C[i]; pc2 += PC[i] * PC[i]; }
-        double F[PCG_MAXLT + 1];
-        boys_eval_rt(bt, L, z * pc2, F);
-        const double pre = -b.at_z[c] * 2.0 * sqrt(z * (1.0 / M_PI)) * U * cc;
-        double V[10][10][5];  // [a global][b global][m]
-        for (int m = 0; m <= L; ++m) V[0][0][m] = pre * F[m];
-        for (int l = 1; l <= la; ++l)
-          for (int k = 0; k < d_ncart(l); ++k) {
-            int a[3]; d_comp(l, k, a);
-            int i = a[0] ? 0 : (a[1] ? 1 : 2);
-            int am[3] = {a[0], a[1], a[2]}; am[i]--;
-            int g = d_gidx(a[0], a[1], a[2]), g1 = d_gidx(am[0], am[1], am[2]);
-            int g2 = -1;
-            if (am[i] > 0) { int amm[3] = {am[0], am[1], am[2]}; amm[i]--; g2 = d_gidx(amm[0], amm[1], amm[2]); }
-            for (int m = 0; m <= L - l; ++m) {
-              double v = PA[i] * V[g1][0][m] - PC[i] * V[g1][0][m + 1];
-              if (g2 >= 0) v += am[i] * oo2z * (V[g2][0][m] - V[g2][0][m + 1]);
-              V[g][0][m] = v;
-            }
-          }
-        for (int lbb = 1; lbb <= lb; ++lbb)
-          for (int kb = 0; kb < d_ncart(lbb); ++kb) {
-            int bb[3]; d_comp(lbb, kb, bb);
-            int i = bb[0] ? 0 : (bb[1] ? 1 : 2);
-            int bm[3] = {bb[0], bb[1], bb[2]}; bm[i]--;
-            int gb = d_gidx(bb[0], bb[1], bb[2]), gb1 = d_gidx(bm[0], bm[1], bm[2]);
-            int gb2 = -1;
-            if (bm[i] > 0) { int bmm[3] = {bm[0], bm[1], bm[2]}; bmm[i]--; gb2 = d_gidx(bmm[0], bmm[1], bmm[2]); }
-            for (int laa = 0; laa <= la; ++laa)
-              for (int ka = 0; ka < d_ncart(laa); ++ka) {
-                int a[3]; d_comp(laa, ka, a);
-                int ga = d_gidx(a[0], a[1], a[2]);
-                int ga1 = -1;
-                if (a[i] > 0) { int am[3] = {a[0], a[1], a[2]}; am[i]--; ga1 = d_gidx(am[0], am[1], am[2]); }
-                for (int m = 0; m <= L - laa - lbb; ++m) {
-                  double v = PB[i] * V[ga][gb1][m] - PC[i] * V[ga][gb1][m + 1];
-                  if (ga1 >= 0) v += a[i] * oo2z * (V[ga1][gb1][m] - V[ga1][gb1][m + 1]);
-                  if (gb2 >= 0) v += bm[i] * oo2z * (V[ga][gb2][m] - V[ga][gb2][m + 1]);
-                  V[ga][gb][m] = v;
-                }
-              }
-          }
-        for (int ka = 0; ka < nca; ++ka)
-          for (int kb = 0; kb < ncb; ++kb) {
-            int x[3], y[3];
-            d_comp(la, ka, x);
-            d_comp(lb, kb, y);
-            Vc[ka * ncb + kb] += V[d_gidx(x[0], x[1], x[2])][d_gidx(y[0], y[1], y[2])][0];
-          }
-      }
-    }
-  // sum the lanes' Cartesian blocks
-  for (int i = 0; i < nca * ncb; ++i) {
-    double sv = Sc[i], tv = Tc[i], vv = Vc[i];
+// Overlap, kinetic energy and nuclear attraction of the shell pairs of one class
+// (Methods/integrals.py:220-370), a warp per pair.  32 primitive pairs at a time, a lane each
+// works out one's exponential and centre, leaves them in shared memory and adds its
+// overlap and kinetic terms; then the lanes take the (primitive pair, nucleus) items, the loop
+// that dominates: the attraction with the whole momentum on the first centre,
+// [e|0] for e = LA .. LA + LB (Obara-Saika, in registers), summed before it is shifted to the
+// second centre once per pair -- (a|b+1) = (a+1|b) + (A - B)(a|b) holds for contracted
+// functions.  FP64 instructions bound it.  C12H26/cc-pVDZ: 1760 us with run-time momenta, the
+// recursion's tables in local memory and the exponential per item; 430 us so.
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) k_one_electron(DevBasis b, BoysTable bt, int npair, const int* __restrict__ pA,
+                                                      const int* __restrict__ pB, double* __restrict__ S,
+                                                      double* __restrict__ H) {
+  constexpr int L = LA + LB, NA = oe_ncart(LA), NB = oe_ncart(LB), NE = oe_first(L + 1) - oe_first(LA);
+  __shared__ double prim[4][32][6];                  // P, exponent sum, 1 / (2 sum), factor
+  __shared__ double blk[4][2][NA * NB];              // overlap; kinetic energy, then the sum
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double(*pr)[6] = prim[warp];
+  double* sS = blk[warp][0];
+  double* sH = blk[warp][1];
+  for (int p = blockIdx.x * 4 + warp; p < npair; p += gridDim.x * 4) {
+    int A = pA[p], B = pB[p];
+    if (b.sh_l[A] < b.sh_l[B]) { const int t = A; A = B; B = t; }
+    if (b.sh_l[A] != LA || b.sh_l[B] != LB) continue;
+    double a0[3], ab[3], r2 = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sv += __shfl_xor_sync(0xffffffffu, sv, o);
-      tv += __shfl_xor_sync(0xffffffffu, tv, o);
-      vv += __shfl_xor_sync(0xffffffffu, vv, o);
+    for (int i = 0; i < 3; ++i) {
+      a0[i] = b.sh_xyz[3 * A + i];
+      ab[i] = a0[i] - b.sh_xyz[3 * B + i];
+      r2 = fma(ab[i], ab[i], r2);
     }
-    Sc[i] = sv; Tc[i] = tv; Vc[i] = vv;
-  }
-  if (lane != 0) return;
-  // spherical transform and store both triangles
-  const int nsa = 2 * la + 1, nsb = 2 * lb + 1;
-  const int oa = b.sh_ao[A], ob = b.sh_ao[B];
-  const int n = b.ld;
-  const long long o = b.sh_blk ? b.sh_blk[A] : 0ll;
-  S += o;
-  H += o;
-  for (int r = 0; r < nsa; ++r)
-    for (int q = 0; q < nsb; ++q) {
-      double s = 0.0, h = 0.0;
-      for (int ka = 0; ka < nca; ++ka) {
-        const double ca = d_sph(la, r, ka);
+    const int npb = b.sh_nprim[B], npp = b.sh_nprim[A] * npb;
+    const int c0 = b.sh_at0 ? b.sh_at0[A] : 0, nnuc = b.sh_at0 ? b.sh_nat[A] : b.natom;
+    double Sc[NA * NB], Tc[NA * NB], Vc[NE];
+#pragma unroll
+    for (int i = 0; i < NA * NB; ++i) Sc[i] = Tc[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) Vc[i] = 0.0;
+    for (int base = 0; base < npp; base += 32) {
+      const int cnt = min(32, npp - base);
+      __syncwarp();
+      if (lane < cnt) {
+        const int ia = (base + lane) / npb, ib = base + lane - ia * npb;
+        const double al = b.pr_exp[b.sh_prim[A] + ia], be = b.pr_exp[b.sh_prim[B] + ib];
+        const double cc = b.pr_cc[b.sh_prim[A] + ia] * b.pr_cc[b.sh_prim[B] + ib];
+        const double z = al + be, s = 1.0 / z, ps = M_PI * s, h = 0.5 * s;
+        const double U = ps * sqrt(ps) * exp(-al * be * s * r2) * cc;
+        double PA[3], PB[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const double P = (al * a0[i] + be * (a0[i] - ab[i])) * s;
+          PA[i] = P - a0[i];
+          PB[i] = PA[i] + ab[i];
+          pr[lane][i] = P;
+        }
+        pr[lane][3] = z;
+        pr[lane][4] = h;
+        pr[lane][5] = 2.0 * sqrt(z * (1.0 / M_PI)) * U;
+        // one-dimensional overlap factors (Obara-Saika)
+        double E[3][LA + 1][LB + 3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int i = 0; i <= LA; ++i)
+#pragma unroll
+            for (int j = 0; j <= LB + 2; ++j) {
+              double v = 1.0;
+              if (j == 0 && i > 0) {
+                v = PA[d] * E[d][i - 1][0];
+                if (i > 1) v += (i - 1) * h * E[d][i - 2][0];
+              } else if (j > 0) {
+                v = PB[d] * E[d][i][j - 1];
+                if (i > 0) v += i * h * E[d][i - 1][j - 1];
+                if (j > 1) v += (j - 1) * h * E[d][i][j - 2];
+              }
+              E[d][i][j] = v;
+            }
+        // kinetic energy from overlaps [a|b+2], [a|b], [a|b-2] (one_electron_kinetic.c:60-64)
+#pragma unroll
+        for (int sa = 0; sa <= LA; ++sa)
+#pragma unroll
+          for (int za = 0; za <= sa; ++za)
+#pragma unroll
+            for (int sb = 0; sb <= LB; ++sb)
+#pragma unroll
+              for (int zb = 0; zb <= sb; ++zb) {
+                const int x[3] = {LA - sa, sa - za, za}, y[3] = {LB - sb, sb - zb, zb};
+                double f[3], t[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                  f[d] = E[d][x[d]][y[d]];
+                  t[d] = be * E[d][x[d]][y[d] + 2];
+                  if (y[d] > 1) t[d] = fma(0.25 * y[d] * (y[d] - 1) / be, E[d][x[d]][y[d] - 2], t[d]);
+                }
+                const double sv = f[0] * f[1] * f[2];
+                const double q = t[0] * f[1] * f[2] + f[0] * t[1] * f[2] + f[0] * f[1] * t[2];
+                const int e = oe_k(sa, za) * NB + oe_k(sb, zb);
+                Sc[e] = fma(U, sv, Sc[e]);
+                Tc[e] = fma(U * be, fma(-2.0, q, (2 * LB + 3) * sv), Tc[e]);
+              }
+      }
+      __syncwarp();
+      for (int item = lane; item < cnt * nnuc; item += 32) {
+        const int pp = item / nnuc, c = c0 + item - pp * nnuc;
+        const double* q = pr[pp];
+        const double z = q[3], h = q[4];
+        double PA[3], PC[3], pc2 = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          PA[i] = q[i] - a0[i];
+          PC[i] = q[i] - b.at_xyz[3 * c + i];
+          pc2 = fma(PC[i], PC[i], pc2);
+        }
+        double F[L + 1];
+        boys_eval<L>(bt, z * pc2, F);
+        const double pre = -(double)b.at_z[c] * q[5];
+        double V[oe_first(L + 1)][L + 1];            // [component][m]
+#pragma unroll
+        for (int m = 0; m <= L; ++m) V[0][m] = pre * F[m];
+#pragma unroll
+        for (int l = 1; l <= L; ++l)
+#pragma unroll
+          for (int s = 0; s <= l; ++s)
+#pragma unroll
+            for (int zz = 0; zz <= s; ++zz) {
+              const int x = l - s, y = s - zz;
+              const int i = x ? 0 : (y ? 1 : 2), n = (i == 0 ? x : i == 1 ? y : zz) - 1;   // one down along i, then two
+              const int s1 = s - (i != 0), z1 = zz - (i == 2), s2 = s1 - (i != 0), z2 = z1 - (i == 2);
+              const int g = oe_first(l) + oe_k(s, zz), g1 = oe_first(l - 1) + oe_k(s1, z1);
+#pragma unroll
+              for (int m = 0; m <= L - l; ++m) {
+                double v = fma(PA[i], V[g1][m], -PC[i] * V[g1][m + 1]);
+                if (n > 0) {
+                  const int g2 = oe_first(l - 2) + oe_k(s2, z2);
+                  v = fma(n * h, V[g2][m] - V[g2][m + 1], v);
+                }
+                V[g][m] = v;
+              }
+            }
+#pragma unroll
+        for (int i = 0; i < NE; ++i) Vc[i] += V[oe_first(LA) + i][0];
+      }
+    }
+    auto sum = [](double v) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      return v;
+    };
+#pragma unroll
+    for (int i = 0; i < NA * NB; ++i) {
+      Sc[i] = sum(Sc[i]);
+      Tc[i] = sum(Tc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NE; ++i) Vc[i] = sum(Vc[i]);
+    // the attraction with LB units on the second centre
+#pragma unroll
+    for (int sa = 0; sa <= LA; ++sa)
+#pragma unroll
+      for (int za = 0; za <= sa; ++za)
+#pragma unroll
+        for (int sb = 0; sb <= LB; ++sb)
+#pragma unroll
+          for (int zb = 0; zb <= sb; ++zb) {
+            const int y = sb - zb;
+            const int e = oe_k(sa, za) * NB + oe_k(sb, zb);
+            const int o1 = oe_first(LA + 1) - oe_first(LA), o2 = oe_first(LA + 2) - oe_first(LA);
+            double v = Vc[oe_k(sa, za)];
+            if (LB > 0) {
+              const int i = sb < LB ? 0 : (y ? 1 : 2), s1 = sa + (i != 0), z1 = za + (i == 2);
+              v = fma(ab[i], v, Vc[o1 + oe_k(s1, z1)]);
+              if (LB > 1) {                          // one more along j
+                const int j = sb == 0 ? 0 : sb == 1 ? (zb ? 2 : 1) : (zb == 2 ? 2 : zb == 1 ? 2 : 1);
+                const int sj = sa + (j != 0), zj = za + (j == 2);
+                const double w = fma(ab[i], Vc[o1 + oe_k(sj, zj)], Vc[o2 + oe_up(s1, z1, j)]);
+                v = fma(ab[j], v, w);
+              }
+            }
+            if (lane == 0) {
+              sS[e] = Sc[e];
+              sH[e] = Tc[e] + v;
+            }
+          }
+    __syncwarp();
+    // spherical transform, both triangles
+    constexpr int SA = 2 * LA + 1, SB = 2 * LB + 1;
+    const int oa = b.sh_ao[A], ob = b.sh_ao[B], n = b.ld;
+    const long long o = b.sh_blk ? b.sh_blk[A] : 0ll;
+    if (lane < SA * SB) {
+      const int r = lane / SB, q = lane - r * SB;
+      double sv = 0.0, hv = 0.0;
+      for (int ka = 0; ka < NA; ++ka) {
+        const double ca = d_sph(LA, r, ka);
         if (ca == 0.0) continue;
-        for (int kb = 0; kb < ncb; ++kb) {
-          const double cb = d_sph(lb, q, kb);
+        for (int kb = 0; kb < NB; ++kb) {
+          const double cb = d_sph(LB, q, kb);
           if (cb == 0.0) continue;
-          s += ca * cb * Sc[ka * ncb + kb];
-          h += ca * cb * (Tc[ka * ncb + kb] + Vc[ka * ncb + kb]);
+          sv += ca * cb * sS[ka * NB + kb];
+          hv += ca * cb * sH[ka * NB + kb];
         }
       }
-      S[(size_t)(oa + r) * n + ob + q] = s;
-      S[(size_t)(ob + q) * n + oa + r] = s;
-      H[(size_t)(oa + r) * n + ob + q] = h;
-      H[(size_t)(ob + q) * n + oa + r] = h;
+      // a shell with itself: element (q, r) is the mirror of (r, q), written by one lane
+      if (A != B || r >= q) {
+        const size_t i = (size_t)(oa + r) * n + ob + q, j = (size_t)(ob + q) * n + oa + r;
+        S[o + i] = sv;
+        S[o + j] = sv;
+        H[o + i] = hv;
+        H[o + j] = hv;
+      }
     }
+  }
 }
 
 int pcg_launch_one_electron(const DevBasis& b, const BoysTable& bt, int npair, const int* pA, const int* pB,
                             double* S, double* H, cudaStream_t s) {
   if (npair <= 0) return PCG_OK;
-  k_one_electron<<<(unsigned)(((long long)npair * 32 + 127) / 128), 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  // a launch per class over all pairs: looking at a pair of another class costs little
+  const unsigned blocks = (unsigned)min((npair + 3) / 4, 152 * 8);
+  k_one_electron<0, 0><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  k_one_electron<1, 0><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  k_one_electron<1, 1><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  k_one_electron<2, 0><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  k_one_electron<2, 1><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
+  k_one_electron<2, 2><<<blocks, 128, 0, s>>>(b, bt, npair, pA, pB, S, H);
   PCG_CUDA(cudaGetLastError());
   return PCG_OK;
 }
