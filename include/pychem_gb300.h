@@ -379,12 +379,14 @@ int pcg_dgemm(int batch, int M, int N, int K, double alpha, const double *A, lon
  * pcg_scf_stats: R = P - P^T (n2 x n2), vals[0] = sum D (H + F), vals[1] = RMS(D - Dold) (n x n),
  *   vals[5] = max |R|, then Dold = D; part: 192 doubles of scratch.
  * pcg_projector_check: out = (max |R|, max |S_ij| with i < nocc <= j, max_{i<nocc} S_ii -
- *   min_{j>=nocc} S_jj), n x n; NaNs in them give NaNs. */
+ *   min_{j>=nocc} S_jj), n x n; NaNs in them give NaNs;
+ *   part: n / 2 + 4 doubles of scratch. */
 int pcg_dgemm_sym(int M, int K, double alpha, const double *A, long long sAm, long long sAk, const double *B,
                   long long sBk, long long sBn, double beta, double *C, long long sCm, long long sCn, void *stream);
 int pcg_scf_stats(int n, int n2, const double *P, const double *D, const double *H, const double *F, double *Dold,
                   double *R, double *part, double *vals, void *stream);
-int pcg_projector_check(int n, int nocc, const double *S, const double *R, double *out, void *stream);
+int pcg_projector_check(int n, int nocc, const double *S, const double *R, double *part, double *out,
+                        void *stream);
 int pcg_oa_correction(int n, int nocc, int mode, const double *delta, const double *S, const double *R, double *E,
                       double *lam, void *stream);
 /* pcg_diis_batched: the C1 systems of `batch` molecules, one warp each: Bnew (mn x mn, oldest

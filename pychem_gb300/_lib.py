@@ -138,7 +138,7 @@ _SIGS = {
     "pcg_dgemm_sym": [c_int, c_int, c_double, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong,
                       c_double, c_void_p, c_longlong, c_longlong, c_void_p],
     "pcg_scf_stats": [c_int, c_int] + [c_void_p] * 9,
-    "pcg_projector_check": [c_int, c_int] + [c_void_p] * 4,
+    "pcg_projector_check": [c_int, c_int] + [c_void_p] * 5,
     "pcg_oa_correction": [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_diis_batched": [c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p],
     "pcg_diis_step": [c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -164,7 +164,7 @@ launch_count = 0
 _RESTYPES = {"pcg_last_error": ctypes.c_char_p, "pcg_ozaki_tc_workspace": ctypes.c_size_t,
              "pcg_mlp_wgrad_workspace": ctypes.c_size_t, "pcg_coulomb_exchange_workspace": ctypes.c_size_t}
 # entry points that launch more than one kernel of this library per call
-MULTI_LAUNCH = {"pcg_one_electron": 6, "pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_prim_pack": 2, "pcg_coulomb_exchange": 4}
+MULTI_LAUNCH = {"pcg_projector_check": 2, "pcg_one_electron": 6, "pcg_ozaki_gemm_tc": 2, "pcg_diis_step": 4, "pcg_scf_stats": 2, "pcg_mlp_wgrad": 2, "pcg_prim_pack": 2, "pcg_coulomb_exchange": 4}
 
 _lib = None
 

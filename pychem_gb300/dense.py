@@ -67,7 +67,8 @@ def projector_check(S, R, nocc, out=None):
     """(max |R|, largest occupied-virtual element of S, max S_ii occupied - min S_jj
     virtual) as a device vector."""
     out = torch.empty(3, dtype=torch.float64, device=S.device) if out is None else out
-    _lib.call("pcg_projector_check", S.shape[0], nocc, _p(S), _p(R), _p(out), _stream())
+    part = torch.empty(S.shape[0] // 2 + 4, dtype=torch.float64, device=S.device)
+    _lib.call("pcg_projector_check", S.shape[0], nocc, _p(S), _p(R), _p(part), _p(out), _stream())
     return out
 
 
