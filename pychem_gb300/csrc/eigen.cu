@@ -29,16 +29,19 @@ __device__ __forceinline__ void rot_params(float app, float aqq, float apq, floa
   s = t * c;
 }
 
-// The FP64 rotation: c = cos of the angle, t = tan, q = tan of its half, from a = apq and
-// d = aqq - app, scaled to order one by their exponents; t is the smaller root of
+__device__ __forceinline__ bool is_zero(double x) {   // without the FP64 pipe
+  return ((__double2hiint(x) << 1) | __double2loint(x)) == 0;
+}
+
+// The FP64 rotation: c = cos of the angle, t = tan, from a = apq and d = aqq - app, scaled to order one by their exponents; t is the smaller root of
 // a t^2 + d t - a = 0: an FP32 root and one Newton step in FP64 with the FP32 slope (relative
 // error 1e-13).  No division or root on the FP64 pipe: the chain of dependent instructions is
 // what a small matrix's round takes.  The rotation is orthogonal to rounding whatever the
 // error of t (c = (1 + t^2)^-1/2); what is left of a_pq is computed, not set to zero.
-__device__ __forceinline__ void rot_params(double a0, double d0, double& c, double& t, double& q) {
+__device__ __forceinline__ void rot_params(double a0, double d0, double& c, double& t) {
   c = 1.0;
-  t = q = 0.0;
-  if (a0 == 0.0) return;
+  t = 0.0;
+  if (is_zero(a0)) return;
   double d = d0, a = a0;
   const int ed = (__double2hiint(d) >> 20) & 0x7ff, ea = (__double2hiint(a) >> 20) & 0x7ff;
   const int e = max(ed, ea);
@@ -46,7 +49,6 @@ __device__ __forceinline__ void rot_params(double a0, double d0, double& c, doub
     const double tau = d / (2.0 * a);
     t = fabs(tau) > 1e18 ? 0.5 / tau : (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
     c = 1.0 / sqrt(1.0 + t * t);
-    q = t * c / (1.0 + c);
     return;
   }
   // exponents to [.., 1023]; what falls below 2^-1022 of the other is zero beside it
@@ -60,12 +62,6 @@ __device__ __forceinline__ void rot_params(double a0, double d0, double& c, doub
   t = bits_to_double(df < 0.0f ? -tf : tf);
   t = fma(-fma(fma(a, t, d), t, -a), bits_to_double(df < 0.0f ? -rs : rs), t);
   c = nr_rsqrt(fma(t, t, 1.0));
-  // s / (1 + c): the reciprocal by a third-order step from FP32
-  const double x = 1.0 + c;
-  double y = bits_to_double(__fdividef(1.0f, bits_to_float(x)));
-  const double f = fma(-x, y, 1.0);
-  y = fma(y * f, 1.0 + f, y);
-  q = t * c * y;
 }
 
 __device__ __forceinline__ int tri(int i, int j) {  // packed lower triangle, i >= j
@@ -215,15 +211,16 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
 }
 
 
-// FP64.  A CTA takes `per` matrices (one if split > 1): the rotations of a round fill only h
-// lanes, and an FP64 instruction takes the SM 16 cycles whether a warp's lanes are on or off.
-// The time of a round is the number of its FP64 warp instructions: 27 for the rotations (with
-// the diagonal, held apart, and what is left of a_pq), 13 for 32 blocks off the diagonal (the
-// tangents applied, then c c2), 3 for 32 pairs of V (three shears instead of two products and
-// two sums).  Each matrix stops by itself.
-// 1024 matrices to 1e-15, against a CTA each with two barriers' worth of rotations, 16-instruction
-// blocks and 4-instruction pairs: n = 7 170 -> 112 us, 13 390 -> 295, 25 1840 -> 1297; one
-// matrix: n = 7 105 -> 82 us, 13 218 -> 176, 32 908 -> 478.
+// FP64.  A warp's FP64 instruction takes its quarter of the SM 64 cycles whatever lanes are on,
+// so the time of a round is the number of them: in its first part, one warp's as a rule, only
+// the 11 that every other lane waits for (cosine, tangent, sine); in its second part 13 for
+// 32 blocks off the diagonal (the tangents applied, then c c2), 4 for 32 pairs of V, and 10 in
+// a warp of its own for the diagonal, held apart, with what is left of a_pq.  Zeros are found by
+// their bits.  A CTA takes `per` matrices (one if split > 1), because the rotations fill only h
+// lanes; each matrix stops by itself.
+// 1024 matrices to 1e-15, against a CTA each with whole rotations in the first part,
+// 16-instruction blocks and the diagonal among them: n = 7 170 -> 86 us, 13 390 -> 268, 25 1840 ->
+// 1162; one matrix: n = 7 105 -> 60 us, 13 218 -> 123, 32 908 -> 451.
 __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int per, int split, int rows_per,
                                                    const double* __restrict__ Ain, long long sA,
                                                    double* __restrict__ Vg, long long sV, const double* __restrict__ V0,
@@ -237,7 +234,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
   const int r0 = part * rows_per, r1 = min(m, r0 + rows_per), nrow = max(0, r1 - r0);
   // per matrix: the packed lower triangle (its diagonal slots zero), the diagonal, rows of V
   const int mat = npad + m + ((rows_per * m + 1) & ~1);
-  double* rot = smem_d + per * mat;                  // c, t, s, tan of half the angle of every pair
+  double* rot = smem_d + per * mat;                  // c, t, s of every pair (and a gap)
   unsigned* tab = (unsigned*)(rot + 4 * per * h);    // (k, k2) of a block
   unsigned short* pq = (unsigned short*)(tab + nblk);  // p, q of pair k
   __shared__ double red[32];
@@ -262,7 +259,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
   if (tid == 0) ndone = 0;
   __syncthreads();
   const int wpm = (nt / 32) / per, warp = tid >> 5, lane = tid & 31;   // warps per matrix
-  const int na = (per * nblk + 31) & ~31, nv = per * nrow * h;
+  const int na = (per * nblk + 31) & ~31, nv = (per * nrow * h + 31) & ~31;
   double tot = 0.0;
   int sweep = 0;
   for (;; ++sweep) {
@@ -317,24 +314,15 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
         a0 = k == 0 ? 0 : 1 + a0;
         a1 = 1 + a1;
         const int p = min(a0, a1), q = max(a0, a1);
-        double* A = smem_d + g * mat;
-        double* dg = A + npad;
-        const double a = done[g] ? 0.0 : A[tri(q, p)], dp = dg[p], dq = dg[q], d = dq - dp;
-        double c, t, hf;
-        rot_params(a, d, c, t, hf);
+        const double* A = smem_d + g * mat;
+        double c, t;
+        rot_params(done[g] ? 0.0 : A[tri(q, p)], A[npad + q] - A[npad + p], c, t);
         if (g == 0) *(unsigned*)(pq + 2 * k) = (unsigned)p | ((unsigned)q << 16);
-        double2* o = (double2*)(rot + 4 * it);
-        o[0] = make_double2(c, t);
-        o[1] = make_double2(t * c, hf);
-        if (t != 0.0) {
-          const double c2 = c * c, ch = (t * c2) * fma(-t, d, a + a);
-          dg[p] = dp - ch;
-          dg[q] = dq + ch;
-          A[tri(q, p)] = -c2 * fma(fma(a, t, d), t, -a);
-        }
+        *(double2*)(rot + 4 * it) = make_double2(c, t);
+        rot[4 * it + 2] = t * c;
       }
       __syncthreads();
-      for (int it = tid; it < na + nv; it += nt) {
+      for (int it = tid; it < na + nv + per * h; it += nt) {
         if (it < na) {
           const int g = per == 1 ? 0 : it / nblk;
           if (g >= per || it >= per * nblk) continue;
@@ -342,7 +330,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
           const int k = (int)(e >> 16), k2 = (int)(e & 0xFFFFu);
           const double2 r1 = *(const double2*)(rot + 4 * (g * h + k)), r2 = *(const double2*)(rot + 4 * (g * h + k2));
           const double t = r1.y, t2 = r2.y;
-          if (t == 0.0 && t2 == 0.0) continue;       // both rotations the identity
+          if (is_zero(t) && is_zero(t2)) continue;   // both rotations the identity
           const int p = pq[2 * k], q = pq[2 * k + 1], p2 = pq[2 * k2], q2 = pq[2 * k2 + 1];
           double* A = smem_d + g * mat;
           const int ipp = sym(p, p2), ipq = sym(p, q2), iqp = sym(q, p2), iqq = sym(q, q2);
@@ -354,17 +342,30 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
           A[ipq] = cc * fma(t2, r00, r01);
           A[iqp] = cc * fma(-t2, r11, r10);
           A[iqq] = cc * fma(t2, r10, r11);
-        } else {
+        } else if (it < na + nv) {
           const int x = it - na, row = x / h, k = x - row * h, g = per == 1 ? 0 : row / nrow;
-          const double2 sh = *(const double2*)(rot + 4 * (g * h + k) + 2);
-          if (sh.x == 0.0) continue;
+          if (row >= per * nrow) continue;
+          const double* o = rot + 4 * (g * h + k);
+          const double c = o[0], sn = o[2];
+          if (is_zero(sn)) continue;
           const unsigned e = *(const unsigned*)(pq + 2 * k);
           double* v = smem_d + g * mat + npad + m + (row - g * nrow) * m;
           double* vp = v + (e & 0xFFFFu);
           double* vq = v + (e >> 16);
-          const double x0 = fma(-sh.y, *vq, *vp), y1 = fma(sh.x, x0, *vq);
-          *vp = fma(-sh.y, y1, x0);
-          *vq = y1;
+          const double x0 = *vp, x1 = *vq;
+          *vp = fma(c, x0, -sn * x1);
+          *vq = fma(sn, x0, c * x1);
+        } else {
+          const int x = it - na - nv, g = x / h, k = x - g * h;
+          const double c = rot[4 * x], t = rot[4 * x + 1];
+          if (is_zero(t)) continue;
+          const int p = pq[2 * k], q = pq[2 * k + 1];
+          double* A = smem_d + g * mat;
+          const double dp = A[npad + p], dq = A[npad + q], a = A[tri(q, p)], d = dq - dp;
+          const double c2 = c * c, f = fma(a, t, d), ch = (t * c2) * fma(-t, d, a + a);
+          A[npad + p] = dp - ch;
+          A[npad + q] = dq + ch;
+          A[tri(q, p)] = -c2 * fma(f, t, -a);
         }
       }
       __syncthreads();
@@ -434,8 +435,8 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
       return PCG_ERR_UNSUPPORTED;
     }
     // matrices per CTA: what the rotations leave of a warp, as long as the SMs have 1.5 CTAs each
-    // (n = 13: 1024 matrices 294 us by fours, 338 by twos; 400 matrices 238 us one by one, 267 by
-    // twos)
+    // (n = 13, whole rotations in the first part: 1024 matrices 294 us by fours, 338 by twos; 400
+    // matrices 238 us one by one, 267 by twos)
     int per = 1;
     while (2 * per * (m / 2) < 32 && batch / (2 * per) >= 228) per *= 2;
     for (split = least; jacobi_bytes_d(m, 1, (m + split - 1) / split) > 232448 - 1024; ++split) {}
@@ -443,8 +444,8 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
     bytes = jacobi_bytes_d(m, per, rows_per);
     const long long ctas = (long long)((batch + per - 1) / per) * split;
     if (ctas > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
-    // 128 threads where that fills the SMs (4096 of n = 13: 691 us, 797 with 256) or a round has
-    // no more work; else 256 (one matrix of n = 32: 478 us, 526 with 128)
+    // 128 threads where that fills the SMs (4096 of n = 13: 621 us) or a round has no more work;
+    // else 256 (one matrix of n = 32: 451 us; 478 and 526 with 128 before the diagonal had its warp)
     const int th = m <= 32 ? (m * per <= 8 || ctas > 608 ? 128 : 256) : threads;
     PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     k_jacobi_d<<<(unsigned)ctas, th, bytes, s>>>(n, m, batch, per, split, rows_per, A, sA, (double*)V, sV,
