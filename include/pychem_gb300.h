@@ -321,6 +321,11 @@ int pcg_dense_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs,
  * (pairmap NULL: row = pair(a, b), nbf(nbf+1)/2 rows); E: rows x nbf x nbf doubles. */
 int pcg_dense_pairs_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                           int ntask, const double *store, const int *pairmap, double *E, void *stream);
+/* flag[k] = Q[sp[k]] * (largest Q of the other shell pairs) > threshold, for nk AO pairs with
+ * their shell pairs sp (Q >= 0; false where there is no other pair). */
+int pcg_pair_flags(int npair, const double *Q, double threshold, int nk, const long long *sp, int *flag,
+                   void *stream);
+
 /* The symmetric pair matrix of the compact rows: M[pairmap[pair(a, b)]][pairmap[pair(c, d)]]
  * = (ab|cd) (both triangles; rows x rows doubles, zeroed by the caller), for the
  * elements whose bra and ket pairs both have rows; with pcg_unpack_pairs(rows, nbf, rows,

@@ -126,6 +126,7 @@ _SIGS = {
                      ctypes.c_float, ctypes.c_float, c_int, c_void_p],
     "pcg_jacobi_eigh": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_double, c_void_p,
                         c_void_p],
+    "pcg_pair_flags": [c_int, c_void_p, ctypes.c_double, c_int, c_void_p, c_void_p, c_void_p],
     "pcg_dense_pairs_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
                               c_void_p, c_void_p, c_void_p],
     "pcg_sym_pairs_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
@@ -153,7 +154,7 @@ _SIGS = {
 }
 # entry points that launch exactly one kernel of this library per call
 LAUNCHERS = {"pcg_pair_data", "pcg_pair_data_f32", "pcg_pair_ao", "pcg_one_electron", "pcg_eri_class", "pcg_eri_class_split", "pcg_eri_class_tab", "pcg_schwarz_class", "pcg_plan_count", "pcg_plan_fill", "pcg_expand_tasks",
-             "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_digest_lists", "pcg_digest_lists_u", "pcg_fock_build_u", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_diis_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
+             "pcg_digest_class", "pcg_digest_class_u", "pcg_digest_class_co", "pcg_digest_lists", "pcg_digest_lists_u", "pcg_fock_build_u", "pcg_scattering_class", "pcg_scattering_factors", "pcg_scattering_class_split", "pcg_fock_build", "pcg_fock_build_batched", "pcg_pair_flags", "pcg_diis_batched", "pcg_dense_class", "pcg_fma_probe", "pcg_jacobi_eigh", "pcg_dense_pairs_class", "pcg_sym_pairs_class", "pcg_mark_pairs", "pcg_pair_colmap", "pcg_unpack_pairs",
              "pcg_dgemm", "pcg_dgemm_sym", "pcg_projector_check", "pcg_oa_correction", "pcg_mp2_pair_sums", "pcg_mlp_gemm", "pcg_mlp_dsilu",
              "pcg_mlp_colsum", "pcg_mlp_mse", "pcg_mlp_mse_counted", "pcg_mlp_adam", "pcg_mlp_adam_all",
              "pcg_shellpair_quantities", "pcg_two_electron_bound", "pcg_two_electron_fundamentals",

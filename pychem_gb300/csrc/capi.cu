@@ -268,6 +268,14 @@ int pcg_dense_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs,
                           (cudaStream_t)stream);
 }
 
+int pcg_pair_flags(int npair, const double* Q, double threshold, int nk, const long long* sp, int* flag, void* stream) {
+  if (npair < 0 || nk < 0 || (nk > 0 && (npair < 1 || !Q || !sp || !flag))) {
+    pcg_set_error("pcg_pair_flags: bad arguments");
+    return PCG_ERR_ARG;
+  }
+  return nk == 0 ? PCG_OK : pcg_launch_pair_flags(npair, Q, threshold, nk, sp, flag, (cudaStream_t)stream);
+}
+
 int pcg_dense_pairs_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const int* tasks, int ntask,
                           const double* store, const int* pairmap, double* E, void* stream) {
   if (cls < 0 || cls > 20 || !basis || !pairs || !E) {

@@ -109,6 +109,47 @@ __global__ void k_sym_pairs(DevBasis b, DevPairsExt pr, const int2* __restrict__
     }
 }
 
+// flag[k] = 1 for the AO pairs k whose shell pair sp[k] passes the screen with the largest
+// Schwarz factor of the other pairs.  Every block finds the two largest of Q by itself (a few
+// thousand numbers; selecting them took 55 us of sorting kernels, this 8 us).
+__global__ void __launch_bounds__(1024) k_pair_flags(int npair, const double* __restrict__ Q, double thr, int nk,
+                                                     const long long* __restrict__ sp, int* __restrict__ flag) {
+  __shared__ double s1[32], s2[32];
+  double t1 = -__longlong_as_double(0x7ff0000000000000ll), t2 = t1;   // the two largest (with repeats)
+  for (int p = threadIdx.x; p < npair; p += 1024) {
+    const double q = __ldg(Q + p);
+    t2 = fmax(t2, fmin(t1, q));
+    t1 = fmax(t1, q);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double u1 = __shfl_xor_sync(0xffffffffu, t1, o), u2 = __shfl_xor_sync(0xffffffffu, t2, o);
+    t2 = fmax(fmax(t2, u2), fmin(t1, u1));
+    t1 = fmax(t1, u1);
+  }
+  if ((threadIdx.x & 31) == 0) { s1[threadIdx.x >> 5] = t1; s2[threadIdx.x >> 5] = t2; }
+  __syncthreads();
+  t1 = s1[threadIdx.x & 31];
+  t2 = s2[threadIdx.x & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double u1 = __shfl_xor_sync(0xffffffffu, t1, o), u2 = __shfl_xor_sync(0xffffffffu, t2, o);
+    t2 = fmax(fmax(t2, u2), fmin(t1, u1));
+    t1 = fmax(t1, u1);
+  }
+  for (int k = blockIdx.x * 1024 + threadIdx.x; k < nk; k += gridDim.x * 1024) {
+    const double q = __ldg(Q + __ldg(sp + k));
+    flag[k] = q * (q == t1 ? t2 : t1) > thr;       // of equal largest ones t2 = t1
+  }
+}
+
+int pcg_launch_pair_flags(int npair, const double* Q, double thr, int nk, const long long* sp, int* flag, cudaStream_t s) {
+  const int blocks = min((nk + 1023) / 1024, 152);
+  k_pair_flags<<<blocks, 1024, 0, s>>>(npair, Q, thr, nk, sp, flag);
+  PCG_CUDA(cudaGetLastError());
+  return PCG_OK;
+}
+
 // used[p] = 1 for both pairs of every task (x, y) with x != y; a byte is read before it
 // is written, so the many tasks of one pair store it once or a few times
 __global__ void k_mark_pairs(const int2* __restrict__ tasks, int ntask, unsigned char* __restrict__ used) {

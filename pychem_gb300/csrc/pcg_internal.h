@@ -78,6 +78,7 @@ int pcg_launch_digest_co(int cls, const DevBasis& b, const DevPairsExt& pr, cons
                          const double* store, int nd, const double* W, double* GJ, double* GK, cudaStream_t s);
 int pcg_launch_dense_pairs(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                            const double* store, const int* pmap, double* E, cudaStream_t s);
+int pcg_launch_pair_flags(int npair, const double* Q, double thr, int nk, const long long* sp, int* flag, cudaStream_t s);
 int pcg_launch_sym_pairs(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                          const double* store, const int* pmap, long long rows, double* M, cudaStream_t s);
 int pcg_launch_mark_pairs(const int2* tasks, int ntask, unsigned char* used, cudaStream_t s);

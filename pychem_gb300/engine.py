@@ -576,15 +576,11 @@ class GpuEngine:
             self._ao_shell_pair = (self.h_pairs, torch.as_tensor(sp, device=self.dev))
         # a pair is in some off-diagonal stored quartet when its product with the largest
         # Schwarz factor of the other pairs passes the screen (products are monotone)
-        if self.npair > 1:
-            top, at = torch.topk(self.Q, 2)
-            other = torch.where(torch.arange(self.npair, device=self.dev) == at[0], top[1], top[0])
-            used = self.Q * other > float(self.threshold)
-        else:
-            used = torch.zeros(1, dtype=torch.bool, device=self.dev)
-        flag = used[self._ao_shell_pair[1]]
+        flag = torch.empty(nao2, dtype=torch.int32, device=self.dev)
+        _lib.call("pcg_pair_flags", self.npair, _ptr(self.Q), float(self.threshold), nao2, _ptr(self._ao_shell_pair[1]),
+                  _ptr(flag), _stream())
         rank = torch.cumsum(flag, 0, dtype=torch.int32)
-        pmap = torch.where(flag, rank - 1, -1).to(torch.int32)
+        pmap = torch.where(flag > 0, rank - 1, -1).to(torch.int32)
         return pmap, int(rank[-1])
 
     def dense_eri_pairs(self, compact=False):

@@ -70,3 +70,26 @@ def test_one_electron_pair_order(basis):
     assert float((S2 - S0).abs().max()) <= 1e-12
     assert float((H2 - H0).abs().max()) <= 1e-12 * float(H0.abs().max())
     assert torch.equal(S2, S2.T) and torch.equal(H2, H2.T)
+
+
+@pytest.mark.parametrize("npair", [1, 2, 31, 1025, 40000])
+def test_pair_flags(npair):
+    """Against the definition, exactly: one pair (no other), repeated and zero factors."""
+    from pychem_gb300 import _lib
+    from pychem_gb300.engine import _ptr, _stream
+    rng = np.random.default_rng(npair)
+    for kind in range(3):
+        Q = rng.random(npair) ** 8
+        if kind == 1:
+            Q[rng.integers(npair, size=2)] = 2.0
+        if kind == 2:
+            Q[:] = np.where(rng.random(npair) < 0.5, 0.0, 1.0)
+        sp = rng.integers(npair, size=2 * npair + 3)
+        best = np.argmax(Q)
+        rest = np.delete(Q, best)
+        for thr in (0.0, 0.1, -1.0):
+            want = np.zeros(npair, dtype=bool) if npair == 1 else Q * np.where(np.arange(npair) == best, rest.max(), Q[best]) > thr
+            flag = torch.full((len(sp),), -7, dtype=torch.int32, device="cuda")
+            Qd, spd = torch.tensor(Q, device="cuda"), torch.tensor(sp, device="cuda")
+            _lib.call("pcg_pair_flags", npair, _ptr(Qd), thr, len(sp), _ptr(spd), _ptr(flag), _stream())
+            assert np.array_equal(flag.cpu().numpy(), want[sp].astype(np.int32)), (kind, thr)
