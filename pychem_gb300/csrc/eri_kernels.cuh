@@ -161,6 +161,16 @@ __global__ void __launch_bounds__(128) k_eri(DevPairsExt pr, PrimTab pt, BoysTab
     const double pre = Kp * Kq * rs;
     if constexpr (C::L == 0) {
       acc[0] = fma(F[0], pre, acc[0]);
+    } else if constexpr (C::LC + C::LD == 0 && C::L <= 2) {
+      // all momentum on the bra: rz^m goes with F_m, so that W - P = -rz (P - Q) and the rz of the
+      // recursion need no products of their own (27 FP64 instructions instead of 29 for (ps|ss))
+      double f = pre;
+      F[0] *= f;
+#pragma unroll
+      for (int m = 1; m <= C::L; ++m) F[m] *= f *= q.rz;
+      q.WPx = -PQx; q.WPy = -PQy; q.WPz = -PQz;
+      q.rz = 1.0;
+      C::prim(q, F, acc);
     } else {
 #pragma unroll
       for (int m = 0; m <= C::L; ++m) F[m] *= pre;
