@@ -271,12 +271,13 @@ def count_flops(lines):
 
 
 def overhead_flops(L):
-    """Per primitive quartet, outside the VRR (see k_eri in eri_kernels.cuh): P-Q (3),
-    zeta+eta (1), Newton rsqrt (9), 1/(zeta+eta) (1), rho (2), T (6), Boys top order
-    (2 + 7 FMA), prefactor (2), scaling F_0..F_L (L+1); for L > 0 also exp(-T) (7 FMA
-    + 2), downward recursion (3 per order) and the W-P, W-Q, 1/2(zeta+eta), rho/zeta,
-    rho/eta factors (11)."""
-    return 41 + L if L == 0 else 68 + 4 * L
+    """FP64 operations per primitive quartet outside the VRR (k_eri in eri_kernels.cuh, with the
+    exponent sums' factors read from their table): P-Q (3), its square (5), T (1), prefactor (2),
+    the distance to the grid point (1); Boys rows of one sum and three FMA (7 each: every order
+    up to L = 2, the top one above, with exp(-T) 9 and the downward recursion 3 per order);
+    L = 0: one FMA into the sum (2), else scaling F_0..F_L (L+1) and W-P, W-Q (6)."""
+    boys = 7 * (L + 1) if L <= 2 else 16 + 3 * L
+    return 12 + boys + (2 if L == 0 else L + 7)
 
 
 def gen_class(la, lb, lc, ld, ctype="double", suffix=""):
