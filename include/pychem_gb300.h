@@ -185,12 +185,12 @@ int pcg_eri_class_nout(int cls);
  * single precision (for quartets below the mixed-precision Schwarz threshold). */
 int pcg_eri_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                   int ntask, double *store, int fp32, void *stream);
-/* The same for a list ordered by decreasing primitive-quartet count, its first nheavy tasks
- * spread over 16 lanes each and the next nmid over as many as the GPU has room for: quartets of
- * many primitives would outlast the launch on one lane.  The blocks are the same up to the
- * order of their primitive sums; fp32 != 0 ignores both. */
+/* The same for a list ordered by decreasing primitive-quartet count, more[0..5] (host) of its
+ * tasks having 256, 128, 64, 32, 16 and 8 or more (NULL: none said to): these are spread over as many
+ * lanes as balance the launch.  The blocks are the same up to the order of their primitive sums;
+ * fp32 != 0 ignores it. */
 int pcg_eri_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
-                        int ntask, int nheavy, int nmid, double *store, int fp32, void *stream);
+                        int ntask, const int *more, double *store, int fp32, void *stream);
 
 /* Packed primitive pairs for pcg_eri_class_tab: pk (npp x 8: P, K, P - A, 1/(2 zeta); 16-byte
  * aligned), zid[i] = the index of zeta[i] among the nz ascending exponent sums zsum (-1 where it is
@@ -206,7 +206,7 @@ int pcg_prim_pack(int npp, const double *zeta, const double *P, const double *PA
                   const double *oo2z, int nz, const double *zsum, double *pk, int *zid, double *tab, void *stream);
 /* pcg_eri_class_split in double precision from the packed pairs of the same pair table. */
 int pcg_eri_class_tab(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const pcg_prim_t *prim,
-                      const int *tasks, int ntask, int nheavy, int nmid, double *store, void *stream);
+                      const int *tasks, int ntask, const int *more, double *store, void *stream);
 
 /* Schwarz factor Q[pair] = sqrt(max (mn|mn)) from diagonal blocks of a diagonal class. */
 int pcg_schwarz_class(int cls, const int *tasks, int ntask, const double *store, double *Q,
@@ -270,9 +270,9 @@ int pcg_scattering_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *p
 /* fac[i] for every primitive pair: what it contributes to each scattering integral's
  * prefactor, K (sqrt(pi)/(2 zeta))^{1/2} exp(-S^2/(4 zeta)); formed once per S. */
 int pcg_scattering_factors(int npp, const double *zeta, const double *K, double S, double *fac, void *stream);
-/* pcg_scattering_class from those factors, with nheavy and nmid as in pcg_eri_class_split. */
+/* pcg_scattering_class from those factors, with `more` as in pcg_eri_class_split. */
 int pcg_scattering_class_split(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const double *fac,
-                               const int *tasks, int ntask, int nheavy, int nmid, double S, double *store, void *stream);
+                               const int *tasks, int ntask, const int *more, double S, double *store, void *stream);
 /* Co-density digestion for non-orthogonal CI (Methods/noci.py:243-300 evaluates
  * hartree_fock.py:345-347 on the non-symmetric co-densities of Lowdin-paired
  * determinants): nd densities W, consecutive nbf x nbf row-major blocks; per density

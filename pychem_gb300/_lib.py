@@ -78,11 +78,11 @@ _SIGS = {
     "pcg_eri_class_nout": [c_int],
     "pcg_eri_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p, c_int,
                       c_void_p],
-    "pcg_eri_class_split": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_int, c_int,
+    "pcg_eri_class_split": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
                             c_void_p, c_int, c_void_p],
     "pcg_prim_pack": [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 5,
     "pcg_eri_class_tab": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), ctypes.POINTER(PrimT), c_void_p, c_int,
-                          c_int, c_int, c_void_p, c_void_p],
+                          c_void_p, c_void_p, c_void_p],
     "pcg_schwarz_class": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "pcg_plan_count": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p],
     "pcg_plan_fill": [ctypes.POINTER(PlanT), c_void_p, c_double, c_double, c_void_p, c_void_p, c_void_p],
@@ -100,7 +100,7 @@ _SIGS = {
                              ctypes.c_double, c_void_p, c_void_p],
     "pcg_scattering_factors": [c_int, c_void_p, c_void_p, ctypes.c_double, c_void_p, c_void_p],
     "pcg_scattering_class_split": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_void_p, c_int,
-                                   c_int, c_int, ctypes.c_double, c_void_p, c_void_p],
+                                   c_void_p, ctypes.c_double, c_void_p, c_void_p],
     "pcg_digest_class_co": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_void_p],
     "pcg_coulomb_exchange_workspace": [c_int, c_int],

@@ -99,27 +99,35 @@ int pcg_eri_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, c
   BoysTable bt;
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
-  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, 0, 0, store, fp32 ? 1 : 0,
+  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, nullptr, store, fp32 ? 1 : 0,
                         (cudaStream_t)stream);
 }
 
+// six ascending counts of at most ntask tasks, or none
+static bool parts_ok(int ntask, const int* more) {
+  if (!more) return true;
+  for (int i = 0, prev = 0; i < 6; prev = more[i++])
+    if (more[i] < prev || more[i] > ntask) return false;
+  return true;
+}
+
 int pcg_eri_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const int* tasks, int ntask,
-                        int nheavy, int nmid, double* store, int fp32, void* stream) {
-  if (cls < 0 || cls > 20 || !basis || !pairs || ntask < 0 || nheavy < 0 || nmid < 0 || nmid > ntask - nheavy) {
+                        const int* more, double* store, int fp32, void* stream) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || ntask < 0 || !parts_ok(ntask, more)) {
     pcg_set_error("pcg_eri_class_split: bad arguments");
     return PCG_ERR_ARG;
   }
   BoysTable bt;
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
-  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, nheavy, nmid, store, fp32 ? 1 : 0,
+  return pcg_launch_eri(cls, to_dev(pairs), PrimTab{nullptr, nullptr, nullptr, 0}, bt, (const int2*)tasks, ntask, more, store, fp32 ? 1 : 0,
                         (cudaStream_t)stream);
 }
 
 int pcg_eri_class_tab(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const pcg_prim_t* prim,
-                      const int* tasks, int ntask, int nheavy, int nmid, double* store, void* stream) {
+                      const int* tasks, int ntask, const int* more, double* store, void* stream) {
   if (cls < 0 || cls > 20 || !basis || !pairs || !prim || !prim->pk || !prim->zid || (prim->nz > 0 && !prim->tab) ||
-      ((size_t)prim->pk & 15) || ((size_t)prim->tab & 15) || ntask < 0 || nheavy < 0 || nmid < 0 || nmid > ntask - nheavy) {
+      ((size_t)prim->pk & 15) || ((size_t)prim->tab & 15) || ntask < 0 || !parts_ok(ntask, more)) {
     pcg_set_error("pcg_eri_class_tab: bad arguments");
     return PCG_ERR_ARG;
   }
@@ -127,7 +135,7 @@ int pcg_eri_class_tab(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pair
   int rc = pcg_ensure_boys(&bt);
   if (rc) return rc;
   return pcg_launch_eri(cls, to_dev(pairs), PrimTab{prim->pk, prim->zid, prim->tab, prim->nz}, bt, (const int2*)tasks,
-                        ntask, nheavy, nmid, store, 0, (cudaStream_t)stream);
+                        ntask, more, store, 0, (cudaStream_t)stream);
 }
 
 int pcg_prim_pack(int npp, const double* zeta, const double* P, const double* PA, const double* K, const double* oo2z,
@@ -216,7 +224,7 @@ int pcg_scattering_class(int cls, const pcg_basis_t* basis, const pcg_pairs_t* p
   }
   BesselTable bt;
   if (int rc = pcg_ensure_bessel(&bt)) return rc;
-  return pcg_launch_scattering(cls, to_dev(pairs), bt, nullptr, (const int2*)tasks, ntask, 0, 0, S, store,
+  return pcg_launch_scattering(cls, to_dev(pairs), bt, nullptr, (const int2*)tasks, ntask, nullptr, S, store,
                                (cudaStream_t)stream);
 }
 
@@ -229,14 +237,14 @@ int pcg_scattering_factors(int npp, const double* zeta, const double* K, double 
 }
 
 int pcg_scattering_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const double* fac,
-                               const int* tasks, int ntask, int nheavy, int nmid, double S, double* store, void* stream) {
-  if (cls < 0 || cls > 20 || !basis || !pairs || !fac || ntask < 0 || nheavy < 0 || nmid < 0 || nmid > ntask - nheavy || !(S >= 0.0)) {
+                               const int* tasks, int ntask, const int* more, double S, double* store, void* stream) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || !fac || ntask < 0 || !parts_ok(ntask, more) || !(S >= 0.0)) {
     pcg_set_error("pcg_scattering_class_split: bad arguments");
     return PCG_ERR_ARG;
   }
   BesselTable bt;
   if (int rc = pcg_ensure_bessel(&bt)) return rc;
-  return pcg_launch_scattering(cls, to_dev(pairs), bt, fac, (const int2*)tasks, ntask, nheavy, nmid, S, store,
+  return pcg_launch_scattering(cls, to_dev(pairs), bt, fac, (const int2*)tasks, ntask, more, S, store,
                                (cudaStream_t)stream);
 }
 

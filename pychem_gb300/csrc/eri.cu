@@ -301,39 +301,39 @@ int pcg_class_nout(int cls) {
   return (2 * l[0] + 1) * (2 * l[1] + 1) * (2 * l[2] + 1) * (2 * l[3] + 1);
 }
 
-int pcg_launch_eri_g0(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g0(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
-int pcg_launch_eri_g1(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g1(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
-int pcg_launch_eri_g2(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g2(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
-int pcg_launch_eri_g3(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g3(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
-int pcg_launch_eri_g4(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g4(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
-int pcg_launch_eri_g5(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, int, int, double*, int,
+int pcg_launch_eri_g5(int, const DevPairsExt&, const PrimTab&, const BoysTable&, const int2*, int, const int*, double*, int,
                       cudaStream_t);
 
 int pcg_launch_eri(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
-                   int nheavy, int nmid, double* store, int precision, cudaStream_t s) {
+                   const int* more, double* store, int precision, cudaStream_t s) {
   if (ntask <= 0) return PCG_OK;
   if (cls < 0 || cls > 20) return PCG_ERR_ARG;
-  if (cls <= 5) return pcg_launch_eri_g0(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
-  if (cls <= 13) return pcg_launch_eri_g1(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
-  if (cls <= 17) return pcg_launch_eri_g2(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
-  if (cls <= 19) return pcg_launch_eri_g3(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
-  if (precision == 0) return pcg_launch_eri_g4(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
-  return pcg_launch_eri_g5(cls, pr, pt, bt, tasks, ntask, nheavy, nmid, store, precision, s);
+  if (cls <= 5) return pcg_launch_eri_g0(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
+  if (cls <= 13) return pcg_launch_eri_g1(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
+  if (cls <= 17) return pcg_launch_eri_g2(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
+  if (cls <= 19) return pcg_launch_eri_g3(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
+  if (precision == 0) return pcg_launch_eri_g4(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
+  return pcg_launch_eri_g5(cls, pr, pt, bt, tasks, ntask, more, store, precision, s);
 }
 
 int pcg_launch_scattering(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                          int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s) {
+                          int ntask, const int* more, double S, double* store, cudaStream_t s) {
   if (ntask <= 0) return PCG_OK;
   if (cls < 0 || cls > 20) return PCG_ERR_ARG;
-  if (cls <= 13) return pcg_launch_eri_s0(cls, pr, bt, fac, tasks, ntask, nheavy, nmid, S, store, s);
-  if (cls <= 17) return pcg_launch_eri_s1(cls, pr, bt, fac, tasks, ntask, nheavy, nmid, S, store, s);
-  if (cls <= 19) return pcg_launch_eri_s2(cls, pr, bt, fac, tasks, ntask, nheavy, nmid, S, store, s);
-  return pcg_launch_eri_s3(cls, pr, bt, fac, tasks, ntask, nheavy, nmid, S, store, s);
+  if (cls <= 13) return pcg_launch_eri_s0(cls, pr, bt, fac, tasks, ntask, more, S, store, s);
+  if (cls <= 17) return pcg_launch_eri_s1(cls, pr, bt, fac, tasks, ntask, more, S, store, s);
+  if (cls <= 19) return pcg_launch_eri_s2(cls, pr, bt, fac, tasks, ntask, more, S, store, s);
+  return pcg_launch_eri_s3(cls, pr, bt, fac, tasks, ntask, more, S, store, s);
 }
 
 int pcg_launch_dense(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,

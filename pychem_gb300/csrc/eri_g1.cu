@@ -2,9 +2,9 @@
 #include "eri_kernels.cuh"
 
 int pcg_launch_eri_g1(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
-                      int nheavy, int nmid, double* store, int precision, cudaStream_t s) {
+                      const int* more, double* store, int precision, cudaStream_t s) {
   const int threads = 128, blocks = (ntask + threads - 1) / threads;
-  const EriRange rg = eri_range(ntask, nheavy, nmid);
+  const EriRange rg = eri_range(ntask, more);
   if (precision == 0) {
     switch (cls) {
       case 6: k_eri<Eri2000><<<eri_blocks(rg, threads), threads, 0, s>>>(pr, pt, bt, tasks, rg, store); break;

@@ -2,9 +2,8 @@
 #include "eri_kernels.cuh"
 
 int pcg_launch_eri_g5(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
-                      int nheavy, int nmid, double* store, int precision, cudaStream_t s) {
-  (void)nheavy;
-  (void)nmid;
+                      const int* more, double* store, int precision, cudaStream_t s) {
+  (void)more;
   (void)pt;
   const int threads = 128, blocks = (ntask + threads - 1) / threads;
   if (cls != 20 || precision == 0) return PCG_ERR_ARG;

@@ -1,6 +1,7 @@
 // ERI kernel templates (one thread per shell quartet) -- included by the eri_g*.cu
 // translation units, each of which instantiates a group of classes.
 #pragma once
+#include <math.h>
 #include "common.cuh"
 #include "pcg_internal.h"
 #include "eri_gen.cuh"
@@ -12,34 +13,43 @@ struct PQf {
   float PAx, PAy, PAz, WPx, WPy, WPz, QCx, QCy, QCz, WQx, WQy, WQz, oo2z, oo2e, oo2ze, rz, re;
 };
 
-// The tasks of one launch, sorted by decreasing primitive-quartet count.  The first nheavy (128
-// or more) are shared by 16 lanes each, the next nmid (16 or more) by 2^lgm, the others have
-// one lane; a lane takes every 2^lg-th primitive quartet, and the partial sums are added by
-// shuffles.  A quartet of two oxygen 1s pairs has 36 x 36 primitive quartets, about a
-// millisecond on one lane, so without the split it ends long after the rest of its launch.
+// The tasks of one launch, sorted by decreasing primitive-quartet count: end[i] of them have
+// 256, 128, 64, 32, 16, 8 or more (and end[6] = ntask all).  Part i is shared by 2^lg[i] lanes a
+// task; a lane takes every 2^lg-th primitive quartet, the partial sums are added by shuffles.
 // stride: distance of a block's elements in the store.
-#define ERI_LGH 4
+#define ERI_PARTS 7
 struct EriRange {
-  int ntask, nheavy, nmid, lgm, stride;
+  int stride, end[ERI_PARTS], lg[ERI_PARTS];
 };
 
-// the middle part gets as many lanes as leave no more than about 40,000 in all: two warps a
-// scheduler fill the FP64 pipe.  Below 16 primitive quartets the sums over lanes cost more than
-// they save ((dd|dd): 961 accumulators).
-static inline EriRange eri_range(int ntask, int nheavy, int nmid) {
+// One warp's FP64 instruction takes its quarter of an SM 64 cycles whatever runs beside it, and a
+// quarter's resident warps take turns: a lane with a few times the average share of a quarter
+// (mean = all primitive quartets / (608 quarters x 32 lanes)) ends alone, after the launch.  So
+// a lane gets at most a twelfth of that share, but not fewer than 4 to 8 primitive quartets: a
+// step of the sums over lanes costs a third of one ((dd|dd): 961 accumulators).  (H2O)8, 6-31G,
+// FP64 part of a mixed pass: (pp|ps) 188 us with one lane up to 127 primitive quartets, 117 us so;
+// C12H26/cc-pVDZ with a half, a quarter, an eighth, a 16th, a 32nd of the share: 62.3, 59.8, 58.8,
+// 59.0, 59.5 ms; with at least 2, 4, 8, 16 in a lane 60.8, 58.8, 58.1, 58.9 ms.
+static inline EriRange eri_range(int ntask, const int* more) {
+  static const int from[ERI_PARTS] = {256, 128, 64, 32, 16, 8, 1}, most[ERI_PARTS] = {1296, 256, 128, 64, 32, 16, 8};
   EriRange r;
-  r.ntask = r.stride = ntask;
-  r.nheavy = nheavy;
-  r.nmid = nmid;
-  r.lgm = 0;
-  const long long rest = ((long long)nheavy << ERI_LGH) + (ntask - nheavy - nmid);
-  while (r.lgm < ERI_LGH && ((long long)nmid << (r.lgm + 1)) + rest <= 40000) ++r.lgm;
+  r.stride = ntask;
+  double all = 0.0;
+  for (int i = 0, prev = 0; i < ERI_PARTS; ++i) {
+    r.end[i] = i + 1 < ERI_PARTS ? (more ? more[i] : 0) : ntask;
+    all += 1.4 * from[i] * (r.end[i] - prev);
+    prev = r.end[i];
+  }
+  const double share = fmax(8.0, all / (608 * 32 * 12));
+  for (int i = 0; i < ERI_PARTS; ++i)
+    for (r.lg[i] = 0; i + 1 < ERI_PARTS && r.lg[i] < 5 && most[i] > share * (1 << r.lg[i]);) ++r.lg[i];
   return r;
 }
-// lanes of the first two parts, each rounded up to whole warps
+// lanes of a part, rounded up to whole warps
 __host__ __device__ static inline long long eri_lanes(int n, int lg) { return (((long long)n << lg) + 31) / 32 * 32; }
 static inline unsigned eri_blocks(const EriRange& r, int threads) {
-  const long long n = eri_lanes(r.nheavy, ERI_LGH) + eri_lanes(r.nmid, r.lgm) + (r.ntask - r.nheavy - r.nmid);
+  long long n = 0;
+  for (int i = 0; i < ERI_PARTS; ++i) n += eri_lanes(r.end[i] - (i ? r.end[i - 1] : 0), r.lg[i]);
   return (unsigned)((n + threads - 1) / threads);
 }
 
@@ -51,26 +61,22 @@ struct EriLane {
 };
 __device__ __forceinline__ EriLane eri_lane(const EriRange& r) {
   long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long h = eri_lanes(r.nheavy, ERI_LGH), m = eri_lanes(r.nmid, r.lgm);
-  EriLane l;
-  long long t;
-  int end;
-  if (x < h) {
-    l.lg = ERI_LGH;
-    t = x >> l.lg;
-    end = r.nheavy;
-  } else if (x < h + m) {
-    l.lg = r.lgm;
-    t = r.nheavy + ((x - h) >> l.lg);
-    end = r.nheavy + r.nmid;
-  } else {
-    l.lg = 0;
-    t = r.nheavy + r.nmid + (x - h - m);
-    end = r.ntask;
+  int lo = 0, hi = r.end[0], lg = r.lg[0];
+#pragma unroll
+  for (int i = 1; i < ERI_PARTS; ++i) {
+    const long long n = eri_lanes(hi - lo, lg);
+    if (x < n || hi == r.end[ERI_PARTS - 1]) break;
+    x -= n;
+    lo = hi;
+    hi = r.end[i];
+    lg = r.lg[i];
   }
-  l.on = t < end;
-  l.g = (int)(threadIdx.x & ((1u << l.lg) - 1));
-  l.t = l.on ? (int)t : r.ntask - 1;
+  EriLane l;
+  l.lg = lg;
+  const long long t = lo + (x >> lg);
+  l.on = t < hi;
+  l.g = (int)(threadIdx.x & ((1u << lg) - 1));
+  l.t = l.on ? (int)t : r.end[ERI_PARTS - 1] - 1;
   return l;
 }
 

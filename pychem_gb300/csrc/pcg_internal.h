@@ -43,7 +43,7 @@ struct PrimTab {
 };
 
 int pcg_launch_eri(int cls, const DevPairsExt& pr, const PrimTab& pt, const BoysTable& bt, const int2* tasks, int ntask,
-                   int nheavy, int nmid, double* store, int precision, cudaStream_t s);
+                   const int* more, double* store, int precision, cudaStream_t s);
 int pcg_launch_prim_pack(int npp, const double* zeta, const double* P, const double* PA, const double* K,
                          const double* oo2z, int nz, const double* zsum, double* pk, int* zid, double* tab,
                          cudaStream_t s);
@@ -51,15 +51,15 @@ int pcg_launch_pair_data_f32(int npp, const double* zeta, const double* PA, cons
                              float* pf8, cudaStream_t s);
 int pcg_launch_pair_ao(const DevBasis& b, int npair, const int* pA, const int* pB, int* ao4, cudaStream_t s);
 int pcg_launch_eri_s0(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                      int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s);
+                      int ntask, const int* more, double S, double* store, cudaStream_t s);
 int pcg_launch_eri_s1(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                      int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s);
+                      int ntask, const int* more, double S, double* store, cudaStream_t s);
 int pcg_launch_eri_s2(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                      int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s);
+                      int ntask, const int* more, double S, double* store, cudaStream_t s);
 int pcg_launch_eri_s3(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                      int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s);
+                      int ntask, const int* more, double S, double* store, cudaStream_t s);
 int pcg_launch_scattering(int cls, const DevPairsExt& pr, const BesselTable& bt, const double* fac, const int2* tasks,
-                          int ntask, int nheavy, int nmid, double S, double* store, cudaStream_t s);
+                          int ntask, const int* more, double S, double* store, cudaStream_t s);
 int pcg_launch_scattering_factors(int npp, const double* zeta, const double* K, double S, double* fac, cudaStream_t s);
 int pcg_launch_digest(int cls, const DevBasis& b, const DevPairsExt& pr, const int2* tasks, int ntask,
                       const double* store, const double* D, double* G, cudaStream_t s);

@@ -20,11 +20,14 @@ from .molecule import element_shells
 
 INTEGRAL_THRESHOLD = 1.0e-8   # Data/constants.py:31
 N_SPHER = [1, 3, 5]
-# primitive quartets from which a shell quartet is shared by 16 lanes, and by several lanes where
-# the GPU has room: with one lane the 1,296 of two oxygen 1s pairs take longer than the rest of
-# a mid-size molecule's launch; from 128 on each of 16 lanes still has eight or more to sum, and
-# below 16 the sums over lanes cost more than they save
-HEAVY, MIDDLE = 128, 16
+# the ERI kernels are told how many shell quartets of a list have at least so many primitive
+# quartets, and spread these over several lanes where one would outlast the launch
+PARTS = (256, 128, 64, 32, 16, 8)
+
+
+def _parts(counts):
+    return (ctypes.c_int * len(PARTS))(*counts)
+
 # distinct exponent sums up to which their factors are tabulated: 1,024^2 entries of 48 bytes stay
 # in L2 (H, C, N, O, F in 6-31G together have 990)
 MAX_EXPONENT_SUMS = 1024
@@ -313,21 +316,22 @@ class GpuEngine:
     # Methods/properties.py:20-23); schwarz(), build_tasks() and compute_eris() follow it
     scattering = None
 
-    def _eri(self, cls, tasks, ntask, store, fp32, split=(0, 0), factors=None):
-        """Blocks of one task list; split: how many of its tasks, first ones, have HEAVY or
-        more primitive quartets, and how many next ones MIDDLE or more.  factors: _scattering_factors() of this pass (scattering operator)."""
+    def _eri(self, cls, tasks, ntask, store, fp32, more=None, factors=None):
+        """Blocks of one task list; more: how many of its tasks, first ones, have the primitive
+        quartets of PARTS (_parts).  factors: _scattering_factors() of this pass (scattering
+        operator)."""
         if self.scattering is not None:
             if fp32:
                 raise ValueError("scattering integrals are FP64 only")
             _lib.call("pcg_scattering_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
-                      _ptr(factors), _ptr(tasks), ntask, *split, float(self.scattering), _ptr(store), _stream())
+                      _ptr(factors), _ptr(tasks), ntask, more, float(self.scattering), _ptr(store), _stream())
             return
         if not fp32:
             _lib.call("pcg_eri_class_tab", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t),
-                      ctypes.byref(self.prim_t), _ptr(tasks), ntask, *split, _ptr(store), _stream())
+                      ctypes.byref(self.prim_t), _ptr(tasks), ntask, more, _ptr(store), _stream())
             return
         _lib.call("pcg_eri_class_split", cls, ctypes.byref(self.basis_t), ctypes.byref(self.pairs_t), _ptr(tasks),
-                  ntask, 0, 0, _ptr(store), 1 if fp32 else 0, _stream())
+                  ntask, None, _ptr(store), 1 if fp32 else 0, _stream())
 
     def _scattering_factors(self):
         if self.scattering is None:
@@ -339,8 +343,8 @@ class GpuEngine:
 
     def schwarz(self):
         """Q[pair] = sqrt(max (mn|mn)) over the diagonal quartets (ab|ab), the pairs of
-        each class in decreasing order of their kept primitives: the quartets of HEAVY or
-        more primitive quartets (an oxygen 1s pair has 36 x 36) get several lanes each."""
+        each class in decreasing order of their kept primitives: those with many (an
+        oxygen 1s pair has 36 x 36 primitive quartets) get several lanes each."""
         Q = torch.zeros(self.npair, dtype=torch.float64, device=self.dev)
         pc = pair_class(self.h_pairs["lA"], self.h_pairs["lB"])
         factors = self._scattering_factors()
@@ -359,8 +363,7 @@ class GpuEngine:
             part = tasks[2 * lo:2 * hi]
             store = torch.empty(lib.pcg_eri_class_nout(cls) * (hi - lo), dtype=torch.float64, device=self.dev)
             n = npp[order[lo:hi]]
-            heavy, some = (int(np.count_nonzero(n * n >= k)) for k in (HEAVY, MIDDLE))
-            self._eri(cls, part, hi - lo, store, False, (heavy, some - heavy), factors)
+            self._eri(cls, part, hi - lo, store, False, _parts(int(np.count_nonzero(n * n >= k)) for k in PARTS), factors)
             _lib.call("pcg_schwarz_class", cls, _ptr(part), hi - lo, _ptr(store), _ptr(Q), _stream())
         self.Q = Q
         return Q
@@ -375,7 +378,7 @@ class GpuEngine:
         A, B), and the buckets (bra kind, ket kind <= it) sorted by (class, decreasing
         primitive quartets per task, bra kind, ket kind).  They follow from the pairs and
         their kept primitives, not from the Schwarz factors.  Returns the struct and per
-        class its rows (first, end of the tasks of HEAVY or more, of MIDDLE or more, end)."""
+        class its rows (first, ends of the tasks with the primitive quartets of PARTS, end)."""
         if self._plan_tables is not None:
             return self._plan_tables
         nk = len(self.kinds)
@@ -395,7 +398,7 @@ class GpuEngine:
         rows = {}
         for c in np.unique(cls):
             lo, hi = np.searchsorted(cls, [c, c + 1])
-            rows[int(c)] = (int(row0[lo]), *(int(row0[lo + np.count_nonzero(work[lo:hi] >= k)]) for k in (HEAVY, MIDDLE)),
+            rows[int(c)] = (int(row0[lo]), *(int(row0[lo + np.count_nonzero(work[lo:hi] >= k)]) for k in PARTS),
                             int(row0[hi]))
         if row0[-1] > 0x7fffffff:
             raise _lib.PcgError("too many rows for the quartet planner")
@@ -424,15 +427,15 @@ class GpuEngine:
         off = torch.cumsum(cnt, 0)
         at = np.array([[p * n + r for r in rows[c]] for p in range(parts) for c in rows])
         ends = off[self._t(at)].tolist()
-        total = ends[-1][3]
+        total = ends[-1][-1]
         tasks = torch.empty(2 * total, dtype=torch.int32, device=self.dev)
         _lib.call("pcg_plan_fill", ctypes.byref(plan), _ptr(Qs), thr, thr32, _ptr(off), _ptr(tasks), _stream())
         self.classes, self.heavy = {}, {}
         for part, lists in zip(("64", "32"), (ends[:len(rows)], ends[len(rows):])):
-            for cls, (lo, heavy, some, hi) in zip(rows, lists):
+            for cls, (lo, *some, hi) in zip(rows, lists):
                 if hi > lo:
                     self.classes.setdefault(cls, {})[part] = (tasks[2 * lo:2 * hi], hi - lo)
-                    self.heavy[(cls, part)] = (heavy - lo, some - heavy)
+                    self.heavy[(cls, part)] = tuple(k - lo for k in some)
         self._task_stats()
         return self.classes
 
@@ -467,10 +470,10 @@ class GpuEngine:
             nout = _lib.load().pcg_eri_class_nout(cls)
             for part, (tasks, n) in rec.items():
                 store = torch.empty(nout * n, dtype=torch.float64, device=self.dev)
-                split = self.heavy.get((cls, part), (0, 0))
-                if sum(split) > n:       # a list cut down since
-                    split = (0, 0)
-                self._eri(cls, tasks, n, store, part == "32", split, factors)
+                more = self.heavy.get((cls, part))
+                if more is not None and more[-1] > n:       # a list cut down since
+                    more = None
+                self._eri(cls, tasks, n, store, part == "32", _parts(more) if more else None, factors)
                 self.stores[(cls, part)] = store
         return self.stores
 

@@ -26,18 +26,18 @@ def _engine(coords, basis):
     return eng
 
 
-def _blocks(eng, cls, tasks, n, nheavy, nmid, S):
+def _blocks(eng, cls, tasks, n, more, S):
     from pychem_gb300 import _lib
     from pychem_gb300.engine import _ptr, _stream
     store = torch.full((_lib.load().pcg_eri_class_nout(cls) * n,), float("nan"), dtype=torch.float64, device="cuda")
     b, p = ctypes.byref(eng.basis_t), ctypes.byref(eng.pairs_t)
     if S is None:
-        _lib.call("pcg_eri_class_split", cls, b, p, _ptr(tasks), n, nheavy, nmid, _ptr(store), 0, _stream())
+        _lib.call("pcg_eri_class_split", cls, b, p, _ptr(tasks), n, (ctypes.c_int * 6)(*more), _ptr(store), 0, _stream())
     else:
         eng.scattering = S
         fac = eng._scattering_factors()
         eng.scattering = None
-        _lib.call("pcg_scattering_class_split", cls, b, p, _ptr(fac), _ptr(tasks), n, nheavy, nmid, S, _ptr(store), _stream())
+        _lib.call("pcg_scattering_class_split", cls, b, p, _ptr(fac), _ptr(tasks), n, (ctypes.c_int * 6)(*more), S, _ptr(store), _stream())
     return store.view(-1, n)
 
 
@@ -53,14 +53,13 @@ def test_lanes_of_a_quartet(basis, S):
     for cls, rec in eng.classes.items():
         tasks, n = rec["64"]
         many = tasks.view(n, 2).repeat(-(-45000 // n), 1).contiguous().view(-1)   # > 40,000: one lane each
-        ref = _blocks(eng, cls, many, many.numel() // 2, 0, 0, S)[:, :n]
+        ref = _blocks(eng, cls, many, many.numel() // 2, (0,) * 6, S)[:, :n]
         scale = float(ref.abs().max())
         for k in sorted({1, min(2, n), min(33, n), n}):
-            for nheavy, nmid in sorted({(0, 0), (1, 0), (0, 1), (k // 2, k - k // 2), (k, 0), (0, k)}):
-                if nheavy + nmid > k:
-                    continue
-                got = _blocks(eng, cls, tasks, k, nheavy, nmid, S)
-                assert float((got - ref[:, :k]).abs().max()) <= 2e-12 * max(1.0, scale), (cls, k, nheavy, nmid)
+            for more in sorted({tuple(min(k, x) for x in m) for m in ((0, 0, 0, 0, 0, 0), (1, 1, 1, 1, 1, 1), (0, 0, 0, 0, 0, 1),
+                                (0, 0, k // 2, k, k, k), (k // 2, k // 2, k, k, k, k), (1, 2, 3, 4, 5, 6), (k, k, k, k, k, k))}):
+                got = _blocks(eng, cls, tasks, k, more, S)
+                assert float((got - ref[:, :k]).abs().max()) <= 2e-12 * max(1.0, scale), (cls, k, more)
 
 
 @pytest.mark.parametrize("S", [None, 0.0, 0.5, 6.0, 40.0])

@@ -25,7 +25,7 @@ def _engine(name):
 @pytest.mark.parametrize("thr,thr32", [(1e-8, 0.0), (1e-8, 1e-4), (1e-3, 1e-2), (0.0, 0.0), (10.0, 0.0), (1e30, 1e31)])
 @pytest.mark.parametrize("name", ["atom", "water6", "alkane", "ensemble"])
 def test_plan(name, thr, thr32):
-    from pychem_gb300.engine import HEAVY, MIDDLE, plan_quartets
+    from pychem_gb300.engine import PARTS, plan_quartets
     eng = _engine(name)
     eng.one_electron()
     eng.schwarz()
@@ -54,6 +54,5 @@ def test_plan(name, thr, thr32):
         assert canon(tasks.tolist()) == canon(want[key])
         work = npp[tasks[:, 0]] * npp[tasks[:, 1]]
         assert (np.diff(work) <= 0).all()
-        heavy = np.count_nonzero(work >= HEAVY)
-        assert eng.heavy[key] == (heavy, np.count_nonzero(work >= MIDDLE) - heavy)
+        assert eng.heavy[key] == tuple(np.count_nonzero(work >= k) for k in PARTS)
         assert classes[key[0]][key[1]][1] == len(tasks)
