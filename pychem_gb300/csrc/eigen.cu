@@ -1,4 +1,4 @@
-// Batched symmetric eigensolver: parallel cyclic Jacobi, one CTA per matrix.
+// Batched symmetric eigensolver: parallel cyclic Jacobi.
 //
 // Method: two-sided Jacobi rotations B = J^T A J (Golub & Van Loan, Matrix
 // Computations, 4th ed., Alg. 8.5.2 sym.schur2 for the rotation), applied to n/2
@@ -7,10 +7,9 @@
 // pairs, then columns of A and of V; the sweep loop stops when the off-diagonal
 // Frobenius norm falls below tol times the total norm.
 //
-// T = double keeps A (packed) and V in shared memory (n <= 136; used by the batched
-// small-molecule SCF).  T = float (n <= 334) keeps packed A and V in shared memory
-// too, V's rows spread over as many CTAs per matrix as that takes (two at n = 208,
-// eight at n = 298); the caller refines the float result in FP64 (Ogita-Aishima
+// FP64 (n <= 136; the batched small-molecule SCF): up to four matrices to a CTA, or one over
+// several CTAs.  FP32 (n <= 334): packed A and V in shared memory too, V's rows spread
+// over as many CTAs per matrix as that takes and the GPU has free; the caller refines the float result in FP64 (Ogita-Aishima
 // iteration, pychem_gb300/eigen.py), so the O(n^3) rotation work runs on the FP32
 // pipe.
 #include <math.h>
