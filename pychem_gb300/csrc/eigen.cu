@@ -9,9 +9,9 @@
 //
 // FP64 (n <= 136; the batched small-molecule SCF): up to four matrices to a CTA, or one over
 // several CTAs.  FP32 (n <= 334): packed A and V in shared memory too, V's rows spread
-// over as many CTAs per matrix as that takes and the GPU has free; the caller refines the float result in FP64 (Ogita-Aishima
-// iteration, pychem_gb300/eigen.py), so the O(n^3) rotation work runs on the FP32
-// pipe.
+// over as many CTAs per matrix as that takes and the GPU has free; the caller refines the
+// float result in FP64 (Ogita-Aishima iteration, pychem_gb300/eigen.py), so the O(n^3)
+// rotation work runs on the FP32 pipe.
 #include <math.h>
 
 #include "../../include/pychem_gb300.h"
@@ -80,7 +80,10 @@ __device__ __forceinline__ int sym(int i, int j) { return i >= j ? tri(i, j) : t
 // memory for n up to 334 in FP32.  With use_tab, the (k, k2) pair of every 2x2 block
 // is read from a table in shared memory (after V) instead of being decoded with a
 // square root per block and round.  Rotations that are the identity (a_pq = 0) skip
-// their updates.
+// their updates.  Instructions bound a round (n = 208: 5,460 blocks on every CTA); a pair's
+// indices with the starts of their rows are one 16-byte word, its cosine and sine one of 8:
+// n = 208 0.835 -> 0.800 ms a sweep, 298 2.57 -> 2.28.  A in square storage with odd rows, free
+// of bank conflicts, gave 4 % more at 208 and lost 2 % at 64.
 __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int rows_per, const double* __restrict__ Ain,
                                                  long long sA, float* __restrict__ Vg, long long sV,
                                                  const float* __restrict__ V0, double* __restrict__ w, long long sw,
@@ -93,8 +96,8 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
   float* V = A + ((ntri + 1) & ~1);                      // rows r0..r1 of V (nrow x m)
   unsigned* tab = (unsigned*)(V + (((size_t)rows_per * m + 1) & ~(size_t)1));
   constexpr int HMAX = 176;                          // m / 2 <= 167
-  __shared__ float cs[HMAX], sn[HMAX];
-  __shared__ int pp[HMAX], qq[HMAX];
+  __shared__ float2 cs[HMAX];                        // c, s of pair k
+  __shared__ int4 pq[HMAX];                          // p, q and the starts of their rows
   __shared__ double red0[32], red1[32];
   __shared__ int stop;
   const double* Ab = Ain + (size_t)b * sA;
@@ -152,7 +155,8 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
         const int p = min(a0, a1), q = max(a0, a1);
         float c, s;
         rot_params(A[tri(p, p)], A[tri(q, q)], A[tri(q, p)], c, s);
-        pp[k] = p; qq[k] = q; cs[k] = c; sn[k] = s;
+        cs[k] = make_float2(c, s);
+        pq[k] = make_int4(p, q, tri(p, 0), tri(q, 0));
       }
       __syncthreads();
       for (int it = tid; it < nblk + nrow * h; it += nt) {
@@ -167,17 +171,21 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
             while (k * (k + 1) / 2 > it) --k;
             k2 = it - k * (k + 1) / 2;
           }
-          const int p = pp[k], q = qq[k], p2 = pp[k2], q2 = qq[k2];
-          const float c = cs[k], s = sn[k], c2 = cs[k2], s2 = sn[k2];
+          const float2 r1 = cs[k], r2 = cs[k2];
+          const float c = r1.x, s = r1.y, c2 = r2.x, s2 = r2.y;
           if (s == (float)0 && s2 == (float)0) continue;   // both rotations the identity
+          const int4 e1 = pq[k], e2 = pq[k2];
+          const int p = e1.x, q = e1.y;
           if (k == k2) {
-            const float app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
+            const int ip = e1.z + p, iq = e1.w + q, iqp = e1.w + p;
+            const float app = A[ip], aqq = A[iq], apq = A[iqp];
             // J^T [[app, apq], [apq, aqq]] J with the rotation that zeroes apq
-            A[tri(p, p)] = c * c * app - (float)2 * c * s * apq + s * s * aqq;
-            A[tri(q, q)] = s * s * app + (float)2 * c * s * apq + c * c * aqq;
-            A[tri(q, p)] = (float)0;
+            A[ip] = c * c * app - (float)2 * c * s * apq + s * s * aqq;
+            A[iq] = s * s * app + (float)2 * c * s * apq + c * c * aqq;
+            A[iqp] = (float)0;
           } else {
-            const int ipp = sym(p, p2), ipq = sym(p, q2), iqp = sym(q, p2), iqq = sym(q, q2);
+            const int ipp = p >= e2.x ? e1.z + e2.x : e2.z + p, ipq = p >= e2.y ? e1.z + e2.y : e2.w + p;
+            const int iqp = q >= e2.x ? e1.w + e2.x : e2.z + q, iqq = q >= e2.y ? e1.w + e2.y : e2.w + q;
             const float b00 = A[ipp], b01 = A[ipq], b10 = A[iqp], b11 = A[iqq];
             // rows: J_k^T B
             const float r00 = c * b00 - s * b10, r01 = c * b01 - s * b11;
@@ -191,9 +199,9 @@ __global__ void __launch_bounds__(1024) k_jacobi_f(int n, int m, int split, int 
         } else {
           const int t = it - nblk;
           const int i = t / h, k = t % h;            // local row i of V
-          const float c = cs[k], s = sn[k];
+          const float c = cs[k].x, s = cs[k].y;
           if (s == (float)0) continue;
-          const int p = pp[k], q = qq[k];
+          const int p = pq[k].x, q = pq[k].y;
           const float vp = V[i * m + p], vq = V[i * m + q];
           V[i * m + p] = c * vp - s * vq;
           V[i * m + q] = s * vp + c * vq;

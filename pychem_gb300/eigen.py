@@ -2,7 +2,7 @@
 ``Methods/hartree_fock.py:172-175,226``), on the library's own kernels only:
 
 * batches with n <= 136, and single matrices of n <= 32: parallel cyclic Jacobi in FP64
-  (pcg_jacobi_eigh), one CTA per matrix in a batch.
+  (pcg_jacobi_eigh), up to four matrices to a CTA in a batch.
 * single matrices of larger n: the FP32 variant of the Jacobi kernel (FP32-accurate vectors, n <= 334),
   then FP64 iterative refinement (T. Ogita and K. Aishima, "Iterative refinement for
   symmetric eigenvalue decomposition", Japan J. Indust. Appl. Math. 35 (2018)
