@@ -157,6 +157,26 @@ def refine_projector(A, X, nocc, steps=2, check=False, ortho_steps=1):
     return lam, X, dense.projector_check(S, R, nocc)
 
 
+def occupied_space(A, X_prev, nocc):
+    """Orthonormal columns, the first nocc of which span the lowest nocc eigenvectors of
+    symmetric A to FP64 rounding, each within FP32 accuracy of an eigenvector: the FP32
+    Jacobi kernel on X_prev^T A X_prev, whose order is the spectrum's, then the refined
+    projector.  No host round trip.  Also returns a device vector (orthogonality error,
+    largest occupied-virtual coupling, largest occupied minus smallest virtual level) of
+    the result; the levels are the ends of the rows' Gershgorin discs, so below zero the
+    first nocc columns do hold the lowest levels."""
+    # off-diagonal norm 2e-6 of the whole: couplings of 1e-4 at levels of -20, which three
+    # steps bring to rounding (each squares them or multiplies them by 1e-4 over the gap)
+    _, V = eigh32_own(A, X_prev, tol=2e-6)
+    _, V = refine_projector(A, V, nocc, steps=3)
+    R, S = _rs(A, V)
+    chk = dense.projector_check(S, R, nocc)
+    d = torch.diagonal(S)
+    radius = S.abs().sum(dim=1) - d.abs()
+    chk[2] = (d + radius)[:nocc].amax() - (d - radius)[nocc:].amin()
+    return V, chk
+
+
 EXACT_BLOCK = 64    # exact_eigh finishes blocks up to this size with the FP64 Jacobi kernel
 
 

@@ -108,11 +108,14 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     Fock matrices are kept in the orthonormal basis, F' = X^T F X; the DIIS residual
     is D'F' - F'D' (= X^T (S D F - F D S) X for D = X D' X^T) and DIIS extrapolates F'
     with its Pulay system solved on the GPU.  Every step runs on the library's
-    kernels: Fock digestion, FP64 GEMMs (pcg_dgemm), the eigenvectors (Jacobi for the
-    first exact_iters iterations, then refinement of the previous vectors that
+    kernels: Fock digestion, FP64 GEMMs (pcg_dgemm), the eigenvectors, the density
+    C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc, n > 136).  The eigenvectors come
+    from the FP64 Jacobi kernel (n <= 32); from the FP32 one with the occupied space
+    refined to rounding, checked, and the FP64 kernel where the check fails (n <= 136:
+    the density of every iteration is the FP64 kernel's); or, above, from FP32 Jacobi in the
+    first exact_iters iterations and then by refinement of the previous vectors that
     decouples the occupied space, checked, with the Jacobi route when the check
-    fails; for n <= 32 the FP64 Jacobi kernel in every iteration), the density
-    C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc, n > 136).  With graph None or
+    fails.  With graph None or
     True every iteration after the first exact_iters is one CUDA graph replay followed
     by one read of six numbers (energy, density change, refinement checks, commutator
     size): an iteration is 50 to 60 launches, which for a small molecule take 1 ms of
@@ -129,8 +132,10 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     use_graph = graph is None or graph
     X = orthogonaliser(S)
     n2 = X.shape[1]
-    # refined vectors instead of a Jacobi solve an iteration (with both spaces to decouple)
-    big = n > eigen.FP64_JACOBI_ONE_N and 0 < nocc < n2
+    # refined vectors instead of an FP64 Jacobi solve an iteration: to rounding (mid), or
+    # as far as the SCF has come (big)
+    big = n > eigen.FP64_JACOBI_MAX_N and 0 < nocc < n2
+    mid = eigen.FP64_JACOBI_ONE_N < n <= eigen.FP64_JACOBI_MAX_N and 0 < nocc < n2
     mm = dense.mm
 
     # static buffers (the CUDA graph reads and writes these addresses)
@@ -183,13 +188,22 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
             # a few FP32 Jacobi sweeps put the occupied space well inside the HOMO-LUMO
             # gap; the projector refinement does the rest in FP64
             _, V = eigen.eigh32_own(Fx, Q if have_q[0] else None, tol=1e-4, max_sweeps=5)
-            _, V, chk = eigen.refine_projector(Fx, V, nocc, steps=3, check=True)
-            vals[2:5] = chk
+            _, V = eigen.refine_projector(Fx, V, nocc, steps=3)
         else:
             _, V = eigen.eigh(Fx, X_prev=Q if have_q[0] else None)
-            vals[2:5] = 0.0
         Q.copy_(V)
         have_q[0] = True
+        vals[2:5] = 0.0
+
+    def diag_mid():
+        V, chk = eigen.occupied_space(Fx, Q, nocc)
+        Q.copy_(V)
+        vals[2:5] = chk
+
+    def mid_ok(c):
+        # a coupling of 1e-12 of the largest element over the gap is what an exact solve's
+        # rounding leaves in the density
+        return bool(c[0] <= 1e-12 and c[1] <= 1e-12 * scale and c[2] < 0.0)
 
     def diag_refine():
         _, V, chk = eigen.refine_projector(Fx, Q, nocc, steps=2, check=True)
@@ -210,13 +224,11 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     it = 0
     scale = None
     for it in range(1, max_iter + 1):
-        exact = it <= exact_iters or not big
+        exact = not mid and (it <= exact_iters or not big)
+        diag = diag_mid if mid else diag_exact if exact else diag_refine
         if it <= max(exact_iters, diis_start) or not use_graph:
             fock_and_diis(it > diis_start)
-            if exact:
-                diag_exact()
-            else:
-                diag_refine()
+            diag()
             density()
         else:
             if g is None:
@@ -233,10 +245,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
                     g.capture_begin(pool=pool, capture_error_mode="thread_local")
                     try:
                         fock_and_diis(True)
-                        if exact:
-                            diag_exact()
-                        else:
-                            diag_refine()
+                        diag()
                         density()
                     finally:
                         g.capture_end()
@@ -253,9 +262,21 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
         if record and it <= 2:
             phases["iteration%d" % it] = time.perf_counter()
         E = float(host[0]) + e_nuc
-        if not exact or (big and n <= eigen.FP64_JACOBI_MAX_N):
-            if scale is None:
-                scale = max(float(Fx.abs().amax()), 1.0)
+        if not exact and scale is None:
+            scale = max(float(Fx.abs().amax()), 1.0)
+        if mid and not mid_ok(host[2:5]):
+            # no gap between the spaces, or more steps to go
+            fallbacks += 1
+            c = host[2:5]
+            if np.isfinite(c).all() and c[2] < 0.0:
+                V, chk = eigen.occupied_space(Fx, Q, nocc)
+                c = chk.cpu().numpy()
+            if mid_ok(c):
+                Q.copy_(V)
+            else:
+                Q.copy_(eigen.eigh(Fx.unsqueeze(0))[1][0])
+            density()
+        elif big and not exact:
             # the refined occupied space need only be as good as the SCF itself: Q stays
             # orthonormal, so D is a valid (idempotent) density, and its coupling to the
             # virtual space must be small against this iteration's commutator; near
@@ -264,21 +285,16 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
             ok = host[2] <= 1e-10 and host[3] <= ov_tol and host[4] < 0.0
             if not ok:
                 # refinement not yet converged (a large step early on): more steps from
-                # where it stopped, then the Jacobi route (for n <= 136 the FP64 kernel, at
-                # once when there is no gap between the spaces)
+                # where it stopped, then the Jacobi route
                 fallbacks += 1
-                jacobi64 = n <= eigen.FP64_JACOBI_MAX_N
-                rounds = 0 if jacobi64 and not (np.isfinite(host[2:5]).all() and host[4] < 0.0) else 4
-                for _ in range(rounds):
+                for _ in range(4):
                     _, V, chk = eigen.refine_projector(Fx, Q, nocc, steps=3, check=True, ortho_steps=2)
                     Q.copy_(V)
                     c = chk.cpu().numpy()
                     if c[0] <= 1e-10 and c[1] <= ov_tol and c[2] < 0.0:
                         ok = True
                         break
-                if not ok and jacobi64:
-                    Q.copy_(eigen.eigh(Fx.unsqueeze(0))[1][0])
-                elif not ok:
+                if not ok:
                     diag_exact()
                 density()
         if E_old is not None:
@@ -302,10 +318,12 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     Ff = mm(X, mm(F, X), ta=True)
     split = big
     if big:
-        _, V, chk = eigen.refine_projector(Ff, Q, nocc, steps=2, check=True)
-        if n <= eigen.FP64_JACOBI_MAX_N:
-            c = chk.cpu().numpy()
-            split = c[0] <= 1e-10 and c[1] <= 1e-8 * max(scale or 1.0, 1.0) and c[2] < 0.0
+        _, V = eigen.refine_projector(Ff, Q, nocc, steps=2)
+    elif mid:
+        V, chk = eigen.occupied_space(Ff, Q, nocc)
+        if scale is None:
+            scale = max(float(Ff.abs().amax()), 1.0)
+        split = mid_ok(chk.cpu().numpy())
     if split:
         blks = (V[:, :nocc], V[:, nocc:])
         Abs = [mm(blk, mm(Ff, blk), ta=True) for blk in blks]
