@@ -232,7 +232,8 @@ def exact_eigh_many(As, X_prevs=None, steps=4):
       in the FP32 vectors' basis, its diagonal ordering the part's spectrum -- is
       split the same way while above 64;
     * every part of at most 64 is finished by the FP64 Jacobi kernel, which needs
-      few sweeps from nearly diagonal, all parts in one batched launch.
+      few sweeps from nearly diagonal, all parts in one batched launch; so is a part of
+      at most 136 that cannot be sliced to rounding.
 
     Near-degenerate clusters end up inside one part, where Jacobi resolves them.
     Returns [(w ascending, V)] in the order of As."""
@@ -260,6 +261,11 @@ def exact_eigh_many(As, X_prevs=None, steps=4):
         V = orthonormalize(V)           # FP32-orthonormal -> FP64
         todo.append((r, a, B, w32[r, :n], V))
     leaves = []
+
+    def whole(r, a, B, V):
+        Ap = dense.mm(V, dense.mm(a, V), ta=True)
+        leaves.append((r, 0.5 * (Ap + Ap.T), V if B is None else dense.mm(B, V)))
+
     while todo:
         r, a, B, w, V = todo.pop()
         n = a.shape[0]
@@ -267,10 +273,20 @@ def exact_eigh_many(As, X_prevs=None, steps=4):
         if n <= EXACT_BLOCK or (n <= FP64_JACOBI_MAX_N and not _gap(w, s)):
             # the part in the basis V, where it is nearly diagonal; a cluster that leaves no gap
             # to slice at stays whole where the FP64 kernel takes it
-            Ap = dense.mm(V, dense.mm(a, V), ta=True)
-            leaves.append((r, 0.5 * (Ap + Ap.T), V if B is None else dense.mm(B, V)))
+            whole(r, a, B, V)
             continue
-        _, V = refine_projector(a, V, s, steps=steps)
+        if n <= FP64_JACOBI_MAX_N:
+            # what still couples the two subspaces is dropped from here on: rounding of the
+            # projected matrix at most (spectra of 65 to 136 levels 5e-6 to 1e-3 of the
+            # largest apart, or graded over 12 decades, refine to 1e-9 or not at all)
+            _, Vs, chk = refine_projector(a, V, s, steps=steps, check=True)
+            orth, coupling, _, size = torch.cat([chk, w.abs().amax().unsqueeze(0)]).tolist()
+            if not (orth <= 1e-13 and coupling <= 0.25 * 2.3e-16 * n * size):
+                whole(r, a, B, V)
+                continue
+            V = Vs
+        else:
+            _, V = refine_projector(a, V, s, steps=steps)
         for blk in (V[:, :s], V[:, s:]):
             Ab = dense.mm(blk, dense.mm(a, blk), ta=True)
             Ab = 0.5 * (Ab + Ab.T)
