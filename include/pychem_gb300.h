@@ -421,6 +421,9 @@ int pcg_mp2_pair_sums(int o, int v, const double *X, const double *eo, const dou
  * for the identity.  info (optional): sweeps used per matrix. */
 int pcg_jacobi_eigh(int batch, int n, const double *A, double *w, void *V, int fp32, const void *V0,
                     int max_sweeps, double tol, int *info, void *stream);
+/* The launch of the FP64 variant (host only): matrices a CTA, CTAs a matrix, rows of V a CTA,
+ * threads and bytes of dynamic shared memory.  Each matrix of a CTA has at least a warp. */
+int pcg_jacobi_plan(int batch, int n, int *plan);
 
 /* Learned initial guess (no upstream counterpart; upstream's guesses are the core
  * Hamiltonian and MO files, Methods/hartree_fock.py:35-57).  Dense-layer kernels:

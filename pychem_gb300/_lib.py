@@ -126,6 +126,7 @@ _SIGS = {
                      ctypes.c_float, ctypes.c_float, c_int, c_void_p],
     "pcg_jacobi_eigh": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_double, c_void_p,
                         c_void_p],
+    "pcg_jacobi_plan": [c_int, c_int, P_INT],
     "pcg_pair_flags": [c_int, c_void_p, ctypes.c_double, c_int, c_void_p, c_void_p, c_void_p],
     "pcg_dense_pairs_class": [c_int, ctypes.POINTER(BasisT), ctypes.POINTER(PairsT), c_void_p, c_int, c_void_p,
                               c_void_p, c_void_p, c_void_p],

@@ -394,7 +394,48 @@ static size_t jacobi_bytes_d(int m, int per, int rows_per) {
   return per * (mat + 4 * h) * 8 + h * (h - 1) / 2 * 4 + 4 * h + 16;
 }
 
-// shared-memory plan of one launch: how many CTAs share a matrix (at least `least`), rows of V
+// A round updates m^2 / 8 blocks of A, in every CTA, and m^2 / 2 elements of V: while SMs are
+// free, V's rows are shared by up to 16 CTAs (n = 208, FP32: 0.84 ms a sweep with 2 CTAs)
+static int jacobi_least(int batch, int m) {
+  const int k = 152 / batch < 16 ? 152 / batch : 16;
+  return k > m / 8 ? (m / 8 > 1 ? m / 8 : 1) : (k > 1 ? k : 1);
+}
+
+struct JacobiPlanD {
+  int per, split, rows_per, threads;
+  size_t bytes;
+};
+static JacobiPlanD jacobi_plan_d(int batch, int m, int least) {
+  JacobiPlanD p;
+  // matrices per CTA: what the rotations leave of a warp, as long as the SMs have 1.5 CTAs each
+  // (n = 13, whole rotations in the first part: 1024 matrices 294 us by fours, 338 by twos; 400
+  // matrices 238 us one by one, 267 by twos), and at most four: each matrix has a warp of the
+  // smallest CTA to itself for its sums
+  p.per = 1;
+  while (p.per < 4 && 2 * p.per * (m / 2) < 32 && batch / (2 * p.per) >= 228) p.per *= 2;
+  for (p.split = least; jacobi_bytes_d(m, 1, (m + p.split - 1) / p.split) > 232448 - 1024; ++p.split) {}
+  p.rows_per = (m + p.split - 1) / p.split;
+  p.bytes = jacobi_bytes_d(m, p.per, p.rows_per);
+  const long long ctas = (long long)((batch + p.per - 1) / p.per) * p.split;
+  // above n = 64 one CTA per SM is resident anyway (shared memory): 1024 threads.  Up to 32, 128
+  // threads where that fills the SMs (4096 of n = 13: 621 us) or a round has no more work; else
+  // 256 (one matrix of n = 32: 451 us; 478 and 526 with 128 before the diagonal had its warp)
+  p.threads = m <= 32 ? (m * p.per <= 8 || ctas > 608 ? 128 : 256) : (m <= 64 ? 256 : 1024);
+  return p;
+}
+
+extern "C" int pcg_jacobi_plan(int batch, int n, int* plan) {
+  if (batch < 1 || n < 1 || n > 136 || !plan) {
+    pcg_set_error("pcg_jacobi_plan: bad arguments (n <= 136)");
+    return PCG_ERR_ARG;
+  }
+  const int m = n + (n & 1);
+  const JacobiPlanD p = jacobi_plan_d(batch, m, jacobi_least(batch, m));
+  plan[0] = p.per; plan[1] = p.split; plan[2] = p.rows_per; plan[3] = p.threads; plan[4] = (int)p.bytes;
+  return PCG_OK;
+}
+
+// shared-memory plan of one FP32 launch: how many CTAs share a matrix (at least `least`), rows of V
 // per CTA, whether the block table fits, and the dynamic bytes
 static bool jacobi_plan(int m, int least, int& split, int& rows_per, int& tab, size_t& bytes) {
   const size_t limit = 232448 - 5120;                // 227 KB less the static tables
@@ -431,9 +472,7 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
   const long long sA = (long long)n * n, sV = (long long)m * m, sw = n;
   // above n = 64 one CTA per SM is resident anyway (shared memory): 1024 threads
   const int threads = m <= 32 ? 128 : (m <= 64 ? 256 : 1024);
-  // A round updates m^2 / 8 blocks of A, in every CTA, and m^2 / 2 elements of V: while SMs are
-  // free, V's rows are shared by up to 16 CTAs (n = 208, FP32: 0.84 ms a sweep with 2 CTAs)
-  const int least = max(1, min(min(16, 152 / batch), m / 8));
+  const int least = jacobi_least(batch, m);
   int split = 1, rows_per = m, tab = 0;
   size_t bytes = 0;
   if (!fp32) {
@@ -441,21 +480,12 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
       pcg_set_error("pcg_jacobi_eigh: FP64 variant needs n <= 136");
       return PCG_ERR_UNSUPPORTED;
     }
-    // matrices per CTA: what the rotations leave of a warp, as long as the SMs have 1.5 CTAs each
-    // (n = 13, whole rotations in the first part: 1024 matrices 294 us by fours, 338 by twos; 400
-    // matrices 238 us one by one, 267 by twos)
-    int per = 1;
-    while (2 * per * (m / 2) < 32 && batch / (2 * per) >= 228) per *= 2;
-    for (split = least; jacobi_bytes_d(m, 1, (m + split - 1) / split) > 232448 - 1024; ++split) {}
-    rows_per = (m + split - 1) / split;
-    bytes = jacobi_bytes_d(m, per, rows_per);
-    const long long ctas = (long long)((batch + per - 1) / per) * split;
+    const JacobiPlanD p = jacobi_plan_d(batch, m, least);
+    const long long ctas = (long long)((batch + p.per - 1) / p.per) * p.split;
     if (ctas > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
-    // 128 threads where that fills the SMs (4096 of n = 13: 621 us) or a round has no more work;
-    // else 256 (one matrix of n = 32: 451 us; 478 and 526 with 128 before the diagonal had its warp)
-    const int th = m <= 32 ? (m * per <= 8 || ctas > 608 ? 128 : 256) : threads;
-    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_jacobi_d<<<(unsigned)ctas, th, bytes, s>>>(n, m, batch, per, split, rows_per, A, sA, (double*)V, sV,
+    if (32 * p.per > p.threads) { pcg_set_error("pcg_jacobi_eigh: a CTA with more matrices than warps"); return PCG_ERR_UNSUPPORTED; }
+    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes));
+    k_jacobi_d<<<(unsigned)ctas, p.threads, p.bytes, s>>>(n, m, batch, p.per, p.split, p.rows_per, A, sA, (double*)V, sV,
                                                  (const double*)V0, w, sw, max_sweeps, tol, info);
   } else {
     if (m / 2 > 167 || !jacobi_plan(m, least, split, rows_per, tab, bytes)) {
