@@ -37,6 +37,8 @@ void pcg_set_error(const char* msg);
 // too, 256 a binade about the middles of their intervals (|d| <= T / 512, truncation 1e-17; beyond, the
 // float terms would underflow): the lanes of a warp fall on both sides of 48 as a rule, and
 // with one evaluation for both no lane waits for the other formula.
+// The range test is on the high word, unsigned: a NaN of either sign (and a negative T) goes past
+// the table to the formula for large T.
 // The single-precision variant keeps a grid of 16 points per unit and BOYS_KF terms.
 // ----------------------------------------------------------------------------------
 #define BOYS_TMAX 48.0
@@ -116,7 +118,7 @@ __device__ __forceinline__ int taylor_point(double T, double& d, float& df) {
 template <int L>
 __device__ __forceinline__ void boys_eval(const BoysTable& bt, double T, double* F) {
   const int hi = __double2hiint(T);
-  if (hi < (L <= 2 ? BOYS_LOG_HI : BOYS_TMAX_HI)) {
+  if ((unsigned)hi < (unsigned)(L <= 2 ? BOYS_LOG_HI : BOYS_TMAX_HI)) {
     double d;
     float df;
     int p;

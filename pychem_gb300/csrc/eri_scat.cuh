@@ -18,7 +18,7 @@
 template <int L>
 __device__ __forceinline__ void bessel_eval(const BesselTable& bt, double S, double iS, double R2, double* f) {
   const double x = 0.5 * S * S * R2;
-  if (__double2hiint(x) < 0x40490000) {   // x < 50
+  if ((unsigned)__double2hiint(x) < 0x40490000u) {   // 0 <= x < 50, and no NaN
     double d;
     float df;
     const int p = taylor_point(x, d, df);
