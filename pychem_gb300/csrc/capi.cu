@@ -126,7 +126,8 @@ int pcg_eri_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pa
 
 int pcg_eri_class_tab(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const pcg_prim_t* prim,
                       const int* tasks, int ntask, const int* more, double* store, void* stream) {
-  if (cls < 0 || cls > 20 || !basis || !pairs || !prim || !prim->pk || !prim->zid || (prim->nz > 0 && !prim->tab) ||
+  if (cls < 0 || cls > 20 || !basis || !pairs || !prim || (pairs->npp > 0 && (!prim->pk || !prim->zid)) ||
+      (prim->nz > 0 && !prim->tab) ||
       ((size_t)prim->pk & 15) || ((size_t)prim->tab & 15) || ntask < 0 || !parts_ok(ntask, more)) {
     pcg_set_error("pcg_eri_class_tab: bad arguments");
     return PCG_ERR_ARG;
@@ -238,7 +239,8 @@ int pcg_scattering_factors(int npp, const double* zeta, const double* K, double 
 
 int pcg_scattering_class_split(int cls, const pcg_basis_t* basis, const pcg_pairs_t* pairs, const double* fac,
                                const int* tasks, int ntask, const int* more, double S, double* store, void* stream) {
-  if (cls < 0 || cls > 20 || !basis || !pairs || !fac || ntask < 0 || !parts_ok(ntask, more) || !(S >= 0.0)) {
+  if (cls < 0 || cls > 20 || !basis || !pairs || (pairs->npp > 0 && !fac) || ntask < 0 || !parts_ok(ntask, more) ||
+      !(S >= 0.0)) {
     pcg_set_error("pcg_scattering_class_split: bad arguments");
     return PCG_ERR_ARG;
   }

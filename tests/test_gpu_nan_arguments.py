@@ -41,3 +41,19 @@ def test_one_electron(nan, basis):
     n = GpuEngine(Molecule(coords[:2], basis)).nbf
     assert bool(torch.isfinite(S[:n, :n]).all()) and bool(torch.isnan(H[:n, :n]).all())
     assert bool(torch.isnan(S[:n, n:]).any())
+
+
+@pytest.mark.parametrize("nan", NANS, ids=["+", "-"])
+@pytest.mark.parametrize("basis", ["STO-3G", "cc-pVDZ"])
+def test_engine_without_primitive_pairs(nan, basis):
+    """The largest primitive-pair factor is then a NaN and no pair is kept: integrals are zeros,
+    Fock matrices NaNs."""
+    from pychem_gb300.engine import GpuEngine
+    from pychem_gb300.molecule import Molecule
+    coords = [["HE", 2.0, 0.0, 0.0, 0.0], ["HE", 2.0, 1.5, nan, 0.0]]
+    for precision in ("fp64", "mixed"):
+        eng = GpuEngine(Molecule(coords, basis), precision=precision).prepare()
+        assert eng.pd["zeta"].numel() == 0 and float(eng.Q.abs().max()) == 0.0
+        assert bool(torch.isnan(eng.fock(torch.eye(eng.nbf, dtype=torch.float64, device="cuda"))).all())
+    eng.scattering = 1.3
+    assert float(eng.schwarz().abs().max()) == 0.0
