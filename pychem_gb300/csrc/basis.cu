@@ -15,18 +15,24 @@
 // ----------------------------------------------------------------------------------
 // Boys table (host build once per device)
 // ----------------------------------------------------------------------------------
+// In extended precision: the error of a row would otherwise be that of this series, 2e-15 of
+// the value, ten times what the evaluation from the row adds.
 static void boys_host(int mmax, double T, double* F) {
   // positive series for the top order, downward recursion (stable for all T here,
   // T <= 48 keeps exp(T) finite)
-  double e = exp(-T);
-  double term = 1.0 / (2 * mmax + 1), acc = term;
+  const long double t2 = 2.0L * T, e = expl(-(long double)T);
+  long double term = 1.0L / (2 * mmax + 1), acc = term;
   for (int k = 1; k < 10000; ++k) {
-    term *= 2.0 * T / (2 * mmax + 2 * k + 1);
+    term *= t2 / (2 * mmax + 2 * k + 1);
     acc += term;
-    if (k > 10 && term < 1e-18 * acc) break;
+    if (k > 10 && term < 1e-20L * acc) break;
   }
-  F[mmax] = e * acc;
-  for (int m = mmax; m > 0; --m) F[m - 1] = (2.0 * T * F[m] + e) / (2 * m - 1);
+  long double f = e * acc;
+  F[mmax] = (double)f;
+  for (int m = mmax; m > 0; --m) {
+    f = (t2 * f + e) / (2 * m - 1);
+    F[m - 1] = (double)f;
+  }
 }
 
 // z^-m j_m(z), m = 0 .. mmax (z <= 10 < mmax): the power series for the two highest
@@ -79,7 +85,7 @@ int pcg_ensure_boys(BoysTable* out) {
         for (int k = 4; k < BOYS_K; ++k) r.t[k - 4] = (float)(F[m + k] / fact[k]);
         r.t[3] = 0.0f;
       }
-      ex[p] = exp(-T);
+      ex[p] = (double)expl(-(long double)T);
       if (p % (BOYS_INV_H / BOYS_INV_HF) == 0) {
         const int q = p / (BOYS_INV_H / BOYS_INV_HF);
         for (int m = 0; m < BOYS_M; ++m)
