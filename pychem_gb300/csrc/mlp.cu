@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
       if (lane == 0) mbar_arrive(&bars[st]);
     }
     if (!ok) { *abort_s = 1; atomicExch(&g_mlp_err, 1); }
-    if (ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s)) {
+    if (warp_all(ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s))) {
       tc_fence_after();
       const int m = m0 + 32 * (warp & 3) + lane;
       const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
         // the accumulators in use: three only from three K steps of 16 on
         const int lead = min(3, (c1 - c0) * (ML_BK / 16));
         float v[8], w[8], u[8], x3[8];
+        if (m0 + ML_BM > a.M) __syncwarp();   // the loads want every lane, also those past the last row
         tmem_ld8(trow + cb, v);
         tmem_ld8(trow + BN + cb, u);
         tmem_ld8(trow + 2 * BN + cb, x3);

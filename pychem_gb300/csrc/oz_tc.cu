@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(OZT_THREADS, 1)
     for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++it) {
       const long long m = tile / ntn * OZT_BM + re;
       const int n0 = (int)(tile % ntn) * BN;
-      if (!mbar_wait(&bars[4], it & 1, OZT_WAIT, abort_s)) {
+      if (!warp_all(mbar_wait(&bars[4], it & 1, OZT_WAIT, abort_s))) {
         *abort_s = 1;
         atomicExch(err, 1);
         break;
@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(OZT_THREADS, 1)
 #pragma unroll 1
       for (int cb = 8 * half; cb < BN; cb += 16) {
         float P[NS][8];
+        __syncwarp();                  // the loads want every lane, also those past the last row
 #pragma unroll
         for (int L = 0; L < NS; ++L) tmem_ld8(trow + L * BN + cb, P[L]);
         tmem_wait_ld();

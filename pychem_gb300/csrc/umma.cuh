@@ -45,6 +45,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
+// Whether x holds in every lane of the warp.  A vote of its own: after __all_sync the compiler
+// takes what follows for converged and keeps addresses of a later loop in registers, which spilled
+// the network GEMM's epilogue (367 -> 371 us a training step).
+__device__ __forceinline__ bool warp_all(bool x) {
+  uint32_t m;
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %1, 0;\n vote.sync.ballot.b32 %0, p, 0xffffffff;\n}" : "=r"(m) : "r"((int)x));
+  return m == 0xffffffffu;
+}
+
 // make generic-proxy shared-memory writes visible to the tensor core (async proxy)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

@@ -91,3 +91,11 @@ def test_infinities_and_nans():
     ref = A @ B.float()
     assert torch.equal(torch.isnan(C), torch.isnan(ref))
     assert torch.equal(C[torch.isinf(ref)], ref[torch.isinf(ref)])
+
+
+@pytest.mark.parametrize("N,K", [(256, 40), (250, 47)])
+@pytest.mark.parametrize("layout", ["nn", "nt"])
+@pytest.mark.parametrize("bf16", [True, False])
+def test_gemm_wide_tiles(N, K, layout, bf16):
+    """Tiles of 128 columns (more than 152 of 64), with rows and columns past the last tile."""
+    test_gemm(5001, N, K, layout, bf16)
