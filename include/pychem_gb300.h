@@ -447,7 +447,8 @@ int pcg_mlp_forward(int nlayer, const int *dims, int M, const float *X, const vo
 size_t pcg_mlp_wgrad_workspace(int M, int K, int N);
 int pcg_mlp_wgrad(int M, int K, int N, const float *A, const float *G, float *dW, float *db, void *workspace,
                   size_t ws_bytes, void *stream);
-/* Nonzero once a GEMM's wait has given up on this device; synchronises the stream. */
+/* Nonzero when a GEMM's wait has given up on this device since the last call (what the tile
+ * would have stored is then NaNs); synchronises the stream. */
 int pcg_mlp_status(void *stream);
 int pcg_mlp_dsilu(long long n, float *dY, const float *Z, void *stream);
 int pcg_mlp_colsum(int M, int N, const float *G, float *db, void *stream);

@@ -36,7 +36,7 @@
 #define ML_STAGES 3
 #define ML_WAIT (1u << 24)
 
-// set when a wait of the GEMM gave up (its tile is then not written); read by
+// set when a wait of the GEMM gave up (its part of the tile is then NaNs); read and cleared by
 // pcg_mlp_status
 static __device__ int g_mlp_err;
 
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
       if (lane == 0) mbar_arrive(&bars[st]);
     }
     if (!ok) { *abort_s = 1; atomicExch(&g_mlp_err, 1); }
-    if (warp_all(ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s))) {
+    if (warp_all(ok && mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, abort_s) && !*abort_s)) {
       tc_fence_after();
       const int m = m0 + 32 * (warp & 3) + lane;
       const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
@@ -285,19 +285,26 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
             }
         }
       }
-      if (a.colsum && m0 == 0) {
-        // the MMAs have read the last tiles, so the stages are free for the four groups' sums
-        float* red = (float*)sm;
-        if (has_b) red[gb * BN + rb] = csum;
-        asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
-        if (t < BN && n0 + t < a.N)
-          a.colsum[(long long)blockIdx.y * a.N + n0 + t] =
-              (red[t] + red[BN + t]) + (red[2 * BN + t] + red[3 * BN + t]);
-      }
+      // the MMAs have read the last tiles, so the stages are free for the four groups' sums
+      if (a.colsum && m0 == 0 && has_b) ((float*)sm)[gb * BN + rb] = csum;
     } else {
+      // given up: NaNs for what this warp would have stored
       *abort_s = 1;
       atomicExch(&g_mlp_err, 1);
-      if (a.colsum && m0 == 0) asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
+      const int m = m0 + 32 * (warp & 3) + lane;
+      float* C = a.C + (a.splits > 1 ? (long long)blockIdx.y * a.M * a.N : 0ll);
+      for (int cb = 8 * (warp >> 2); cb < BN; cb += 32)
+        for (int n = n0 + cb; m < a.M && n < min(a.N, n0 + cb + 8); ++n) {
+          C[(long long)m * a.ldc + n] = __int_as_float(0x7fffffff);
+          if (a.Z && a.act != 2) a.Z[(long long)m * a.ldc + n] = __int_as_float(0x7fffffff);
+        }
+    }
+    if (a.colsum && m0 == 0) {
+      const float* red = (const float*)sm;
+      asm volatile("bar.sync 1, %0;" ::"r"(ML_PROD) : "memory");
+      if (t < BN && n0 + t < a.N)
+        a.colsum[(long long)blockIdx.y * a.N + n0 + t] =
+            *abort_s ? __int_as_float(0x7fffffff) : (red[t] + red[BN + t]) + (red[2 * BN + t] + red[3 * BN + t]);
     }
   } else {
     const uint32_t idesc = idesc_bf16_f32(ML_BM, BN);
@@ -327,10 +334,14 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
       }
       umma_commit_lead(lead, &bars[ML_STAGES + st]);
     }
+    if (!ok) {               // before the commit: the epilogue looks at the flag after its wait
+      *abort_s = 1;
+      __threadfence_block();
+      if (lead) atomicExch(&g_mlp_err, 2);
+      __syncwarp();
+    }
     umma_commit_lead(lead, &bars[2 * ML_STAGES]);
     if (!ok) {
-      *abort_s = 1;
-      if (lead) atomicExch(&g_mlp_err, 2);
       volatile int keep_waiting = 0;
       mbar_wait(&bars[2 * ML_STAGES], 0, ML_WAIT, &keep_waiting);   // drain before tensor memory is freed
     }
@@ -504,6 +515,11 @@ extern "C" int pcg_mlp_status(void* stream) {
   int h = 0;
   PCG_CUDA(cudaMemcpyFromSymbolAsync(&h, g_mlp_err, sizeof(int), 0, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   PCG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  if (h) {
+    const int zero = 0;
+    PCG_CUDA(cudaMemcpyToSymbolAsync(g_mlp_err, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, (cudaStream_t)stream));
+    PCG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  }
   return h;
 }
 

@@ -108,6 +108,13 @@ class PairMLP:
         Y, _ = self.forward(X)
         return torch.addcmul(self.mean, Y, self.std)
 
+    def check(self):
+        """Raises if a tensor-core wait gave up since the last check (its outputs are NaNs);
+        synchronises."""
+        rc = _lib.load().pcg_mlp_status(_stream())
+        if rc:
+            raise _lib.PcgError("a wait of the network's GEMM gave up (status %d)" % rc)
+
     def state(self):
         d = {"dims": np.array(self.dims), "mean": self.mean.cpu().numpy(), "std": self.std.cpu().numpy()}
         for k in range(self.nlayers):

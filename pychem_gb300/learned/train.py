@@ -231,6 +231,7 @@ def train(pairs, atoms, nmol, epochs=8, mols_per_batch=96, lr=1e-3, seed=0, log=
             tot_o += float(lo)
             tot_d += float(ld)
             step += 1
+        net.check()
         hist.append([tot_o / nb, tot_d / nb])
         if log:
             log("epoch %d loss off-diagonal %.5f diagonal %.5f" % (ep, tot_o / nb, tot_d / nb))
