@@ -142,6 +142,18 @@ struct MlArgs {
   float* colsum;           // partial sums of B over k per split (wgrad), or null
 };
 
+// one element of the product over k0 <= k < k1 in FP32
+template <bool BF>
+__device__ __forceinline__ float plain_dot(const MlArgs& a, int m, int n, int k0, int k1) {
+  float s = 0.0f;
+  for (int k = k0; k < k1; ++k) {
+    const float x = __ldg(a.A + m * a.sam + k * a.sak);
+    const float y = BF ? __bfloat162float(((const __nv_bfloat16*)a.B)[k * a.sbk + n * a.sbn]) : __ldg((const float*)a.B + k * a.sbk + n * a.sbn);
+    s = fmaf(x, y, s);
+  }
+  return s;
+}
+
 template <bool BF, int BN>
 __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlArgs a) {
   using Cfg = MlCfg<BF, BN>;
@@ -259,10 +271,31 @@ __global__ void __launch_bounds__(ML_THREADS, BN == 64 ? 2 : 1) k_gemm(const MlA
 #pragma unroll
           for (int j = 0; j < 8; ++j) z[j] = n + j < a.N ? a.Z[o + j] : 0.0f;
         }
+        unsigned top = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[j] += w[j];
+          top = max(top, __float_as_uint(v[j]) & 0x7fffffffu);
+        }
+        // a second or third term of zero times an infinity of the other operand is a NaN that the
+        // FP32 product does not have: such elements are summed plainly (the test costs 1.3 % of a
+        // 256 x 256 layer; beside the splits, for BF16 weights, it would cost the producers more)
+        if (top > 0x7f800000u) {
+#pragma unroll 1
+          for (int j = 0; j < 8; ++j) {
+            float x = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x = i == j ? v[i] : x;
+            if (x == x || n + j >= a.N) continue;
+            x = plain_dot<BF>(a, m, n + j, c0 * ML_BK, min(a.K, c1 * ML_BK));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = i == j ? x : v[i];
+          }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const bool in = n + j < a.N;
-          float x = v[j] + w[j];
+          float x = v[j];
           if (a.accumulate && in) x += C[o + j];
           if (a.bias && in) x += __ldg(a.bias + n + j);
           if (a.act == 2) x *= dsilu(z[j]);

@@ -99,3 +99,35 @@ def test_infinities_and_nans():
 def test_gemm_wide_tiles(N, K, layout, bf16):
     """Tiles of 128 columns (more than 152 of 64), with rows and columns past the last tile."""
     test_gemm(5001, N, K, layout, bf16)
+
+
+@pytest.mark.parametrize("M", [130, 5001])
+@pytest.mark.parametrize("bf16", [True, False])
+def test_infinite_weights(M, bf16):
+    """Infinities in the other operand, against activations that are exact in one and in two BF16
+    terms: infinities and NaNs where FP32 products have them."""
+    from pychem_gb300 import _lib
+    g = torch.Generator(device="cuda").manual_seed(M)
+    N, K = 200, 40
+    A = torch.randint(1, 9, (M, K), device="cuda", generator=g).float()
+    A[::3] = A[::3] + 1.0 / 1024
+    A[5, 7], A[6, 2] = 0.0, -1.5                       # 0 times an infinity is a NaN
+    B = (_rand(g, K, N).abs() + 0.5)
+    B[3, 11], B[39, 199], B[7, 64], B[2, 5] = float("inf"), float("-inf"), float("inf"), float("nan")
+    B[0, 20], B[1, 20] = float("inf"), float("-inf")
+    B = B.to(torch.bfloat16) if bf16 else B
+    ref = A @ B.float()
+    C = torch.empty(M, N, device="cuda")
+    _call("pcg_mlp_gemm", M, N, K, A, K, 1, B, int(bf16), N, 1, C, N, 0, None, None, 0)
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(C), torch.isnan(ref)) and torch.equal(C[torch.isinf(ref)], ref[torch.isinf(ref)])
+    assert ((C - ref)[fin].abs() <= 4e-6 * (A.abs() @ B.float().abs())[fin]).all()
+    G = _rand(g, M, N).abs()
+    G[1, 3], G[M - 1, 199] = float("inf"), float("-inf")
+    dW, db = torch.empty(K, N, device="cuda"), torch.empty(N, device="cuda")
+    ws = torch.empty(_lib.load().pcg_mlp_wgrad_workspace(M, K, N), dtype=torch.uint8, device="cuda")
+    _call("pcg_mlp_wgrad", M, K, N, A, G, dW, db, ws, ws.numel())
+    ref = A.T @ G
+    assert torch.equal(torch.isnan(dW), torch.isnan(ref)) and torch.equal(dW[torch.isinf(ref)], ref[torch.isinf(ref)])
+    assert torch.equal(torch.isinf(db), torch.isinf(G.sum(0)))
+    assert _status() == 0
