@@ -377,28 +377,28 @@ def _lib_add_launches(k):
     _lib.launch_count += k
 
 
-_TC_WS = {}
+class _LastWorkspace(threading.local):
+    """This thread's last pcg_ozaki_gemm_tc workspace by device index, for ozaki_tc_status."""
+
+    def __init__(self):
+        self.by_device = {}
 
 
-def _tc_workspace(dev, nbytes):
-    """A cached device workspace for pcg_ozaki_gemm_tc (grown on demand)."""
-    ws = _TC_WS.get(dev)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
-        _TC_WS[dev] = ws
-    return ws
+_TC_LAST = _LastWorkspace()
 
 
 def ozaki_gemm_tc(X, Y, C, M, N, K, ldx, sY, sC, nslice=6, accumulate=False):
     """C[m*sC[0] + n*sC[1]] (+)= sum_k X[m*ldx + k] Y[k*sY[0] + n*sY[1]] in FP64 accuracy
     with every Ozaki level in one tcgen05 tensor-core kernel (pcg_ozaki_gemm_tc); X is
     split into BF16 digit slices on the fly.  Element offsets are relative to the
-    tensors' data pointers."""
+    tensors' data pointers.  The workspace (Y's slices, half a megabyte) is the call's own, from
+    the caching allocator: threads and streams share none, and a captured call's lives with
+    the graph's pool."""
     import ctypes
     from . import _lib
     lib = _lib.load()
-    nbytes = lib.pcg_ozaki_tc_workspace(N, K, nslice)
-    ws = _tc_workspace(C.device, nbytes)
+    ws = torch.empty(lib.pcg_ozaki_tc_workspace(N, K, nslice), dtype=torch.uint8, device=C.device)
+    _TC_LAST.by_device[C.device.index] = ws
     _lib.call("pcg_ozaki_gemm_tc", M, N, K, ctypes.c_void_p(X.data_ptr()), ldx, ctypes.c_void_p(Y.data_ptr()),
               sY[0], sY[1], ctypes.c_void_p(C.data_ptr()), sC[0], sC[1], nslice, 1 if accumulate else 0,
               ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream())
@@ -406,14 +406,14 @@ def ozaki_gemm_tc(X, Y, C, M, N, K, ldx, sY, sC, nslice=6, accumulate=False):
 
 
 def ozaki_tc_status(dev):
-    """Error flag of the last pcg_ozaki_gemm_tc on this device (0 = every wait ended)."""
+    """Error flag of this thread's last pcg_ozaki_gemm_tc on this device (0 = every wait ended)."""
     import ctypes
     from . import _lib
-    ws = _TC_WS.get(torch.device(dev) if not isinstance(dev, torch.device) else dev)
+    dev = torch.device(dev)
+    ws = _TC_LAST.by_device.get(torch.cuda.current_device() if dev.index is None else dev.index)
     if ws is None:
         return 0
-    return _lib.load().pcg_ozaki_tc_status(ctypes.c_void_p(ws.data_ptr()),
-                                           _stream())
+    return _lib.load().pcg_ozaki_tc_status(ctypes.c_void_p(ws.data_ptr()), _stream())
 
 
 def _pair_rows(n, dev):
