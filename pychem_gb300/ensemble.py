@@ -281,7 +281,7 @@ def rhf_batched(eng, max_iter=64, e_tol=1e-10, d_tol=1e-8, diis_size=8, guess="s
     F_fin = torch.empty_like(S)
     D_fin = torch.empty_like(S)
     focks, resids = [], []
-    on_gpu = diis_size <= 32              # the C1 systems: a warp each
+    on_gpu = 0 < diis_size <= 32          # the C1 systems: a warp each
     Bm = torch.zeros(B, 0, 0, dtype=torch.float64, device=dev) if on_gpu else np.zeros((B, 0, 0))
     E_old = D_old = None
     done_at = np.zeros(B, dtype=np.int64)
