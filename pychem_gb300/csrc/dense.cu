@@ -22,7 +22,10 @@
 
 // 8 x 8 output tiles (one thread per element), K in steps of 32: at n = 208 that is
 // 676 CTAs, 4-5 per SM, so the FP64 work is spread evenly over the 152 SMs (with
-// 16 x 16 tiles the 169 CTAs left 17 SMs with twice the work of the others).
+// 16 x 16 tiles the 169 CTAs left 17 SMs with twice the work of the others).  Larger products and
+// batches run at the FP64 rate too (3 x 756 x 406 x 406: 639 us, 1.17 TFLOP/s; 1500^3: 1.22);
+// 32 x 32 tiles of 4 x 4 outputs a thread were slower at every shape (858 us and 1.12 TFLOP/s; 64 x 104^3
+// 237 us against 153).
 #define DG_T 8
 #define DG_K 32
 
@@ -92,76 +95,6 @@ __global__ void __launch_bounds__(DG_T* DG_T)
   }
 }
 
-// The same product with 32 x 32 tiles and 4 x 4 outputs a thread, for products of many tiles
-// (a batch, or the co-density products): a quarter of the shared-memory reads and a
-// sixteenth of the CTAs; each output is still summed in order of k.  3 x 756 x 406 x 406:
-// 2.0 ms with 8 x 8 tiles.
-#define DT_T 32
-#define DT_K 16
-__global__ void __launch_bounds__(64)
-    k_dgemm_tile(int M, int N, int K, double alpha, const double* __restrict__ A, long long sAb, long long sAm,
-                 long long sAk, const double* __restrict__ B, long long sBb, long long sBk, long long sBn, double beta,
-                 double* __restrict__ C, long long sCb, long long sCm, long long sCn) {
-  __shared__ double As[2][DT_K][DT_T + 1], Bs[2][DT_K][DT_T + 1];
-  constexpr int PER = DT_T * DT_K / 64;
-  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
-  const long long b = blockIdx.z;
-  const int m0 = blockIdx.y * DT_T, n0 = blockIdx.x * DT_T;
-  A += b * sAb;
-  B += b * sBb;
-  const bool a_k = sAk == 1, b_k = sBk == 1;       // consecutive threads along the contiguous index
-  double ra[PER], rb[PER];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int e = tid + u * 64;
-      const int ka = a_k ? e % DT_K : e / DT_T, ma = a_k ? e / DT_K : e % DT_T;
-      const int kb = b_k ? e % DT_K : e / DT_T, nb = b_k ? e / DT_K : e % DT_T;
-      ra[u] = (m0 + ma < M && k0 + ka < K) ? __ldg(A + (m0 + ma) * sAm + (k0 + ka) * sAk) : 0.0;
-      rb[u] = (n0 + nb < N && k0 + kb < K) ? __ldg(B + (k0 + kb) * sBk + (n0 + nb) * sBn) : 0.0;
-    }
-  };
-  auto store = [&](int st) {
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int e = tid + u * 64;
-      As[st][a_k ? e % DT_K : e / DT_T][a_k ? e / DT_K : e % DT_T] = ra[u];
-      Bs[st][b_k ? e % DT_K : e / DT_T][b_k ? e / DT_K : e % DT_T] = rb[u];
-    }
-  };
-  double acc[4][4] = {};
-  load(0);
-  store(0);
-  __syncthreads();
-  int st = 0;
-  for (int k0 = 0; k0 < K; k0 += DT_K) {
-    const bool more = k0 + DT_K < K;
-    if (more) load(k0 + DT_K);
-#pragma unroll
-    for (int kk = 0; kk < DT_K; ++kk) {
-      double x[4], y[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { x[i] = As[st][kk][ty + 8 * i]; y[i] = Bs[st][kk][tx + 8 * i]; }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(x[i], y[j], acc[i][j]);
-    }
-    if (more) store(st ^ 1);
-    __syncthreads();
-    st ^= 1;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty + 8 * i, n = n0 + tx + 8 * j;
-      if (m >= M || n >= N) continue;
-      double* c = C + b * sCb + m * sCm + n * sCn;
-      *c = beta == 0.0 ? alpha * acc[i][j] : fma(alpha, acc[i][j], beta * *c);
-    }
-}
-
 extern "C" int pcg_dgemm(int batch, int M, int N, int K, double alpha, const double* A, long long sAb, long long sAm,
                          long long sAk, const double* B, long long sBb, long long sBk, long long sBn, double beta,
                          double* C, long long sCb, long long sCm, long long sCn, void* stream) {
@@ -170,17 +103,12 @@ extern "C" int pcg_dgemm(int batch, int M, int N, int K, double alpha, const dou
     return PCG_ERR_ARG;
   }
   if (M == 0 || N == 0) return PCG_OK;
-  // 32 x 32 tiles from two a SM on, for products long enough to fill their pipeline (a batch
-  // of 1,024 x 30 x 30 x 30: 77 us against 47 with 8 x 8 tiles)
-  const long long tn = (N + DT_T - 1) / DT_T, tm = (M + DT_T - 1) / DT_T;
-  if (batch * tn * tm >= 304 && tm <= 65535 && M >= 64 && N >= 64 && K >= 64) {
-    k_dgemm_tile<<<dim3((unsigned)tn, (unsigned)tm, batch), 64, 0, (cudaStream_t)stream>>>(
-        M, N, K, alpha, A, sAb, sAm, sAk, B, sBb, sBk, sBn, beta, C, sCb, sCm, sCn);
-    PCG_CUDA(cudaGetLastError());
-    return PCG_OK;
-  }
   dim3 grid((N + DG_T - 1) / DG_T, (M + DG_T - 1) / DG_T, batch);
-  if (grid.y > 65535) { pcg_set_error("pcg_dgemm: M too large"); return PCG_ERR_UNSUPPORTED; }
+  if (grid.y > 65535) {
+    if (grid.x > 65535) { pcg_set_error("pcg_dgemm: M too large"); return PCG_ERR_UNSUPPORTED; }
+    // C^T = B^T A^T: the long side along grid.x
+    return pcg_dgemm(batch, N, M, K, alpha, B, sBb, sBn, sBk, A, sAb, sAk, sAm, beta, C, sCb, sCn, sCm, stream);
+  }
   k_dgemm<false><<<grid, DG_T * DG_T, 0, (cudaStream_t)stream>>>(M, N, K, alpha, A, sAb, sAm, sAk, B, sBb, sBk, sBn, beta,
                                                           C, sCb, sCm, sCn);
   PCG_CUDA(cudaGetLastError());
