@@ -1,6 +1,6 @@
-// Fock digestion kernels (closed shell and unrestricted) -- included by digest.cu and
-// digest_u.cu, one translation unit each so that the class instantiations compile in
-// parallel.
+// Fock digestion kernels (closed shell, unrestricted, co-densities) -- included by digest.cu,
+// digest_u.cu and digest_co.cu, one translation unit each so that the class instantiations
+// compile in parallel.
 //
 // For every stored quartet block, with the shell-level degeneracy d = (A!=B ? 2:1)
 // (C!=D ? 2:1)(AB!=CD ? 2:1) and v' = d (ab|cd),
@@ -13,7 +13,10 @@
 // (Methods/noci.py:243-300, hartree_fock.py:345-347 for non-symmetric densities) are the
 // unrestricted case with D_a = W and D_b = W^T, the D_a exchange blocks written transposed:
 // GK then holds G[W^T] + G[W]^T, J[W] = (GJ + GJ^T)/4 and K[W] = -GK/2 with K_ad = sum_bc
-// (ab|cd) W_cb; blockIdx.y selects the density.
+// (ab|cd) W_cb; blockIdx.y selects the density.  They are instances of their own (CO): with both
+// in one kernel each address was a choice of two ((dd|dd): 39 KB of stack instead of 8), and an
+// unrestricted build of C10H22 / cc-pVDZ took 5.80 ms instead of 5.47, of four waters 1.61 instead
+// of 1.40.
 //
 // Bound: the FP64 pipe, six instructions an integral (0.48 ms for the 42 M integrals of
 // (H2O)16 / 6-31G), and the load/store queue, which one gather and one reduction a density
@@ -35,7 +38,6 @@ struct DigestArgs {
   const double* D[2];
   double* GJ;
   double* GK[2];
-  bool co;                     // co-densities: D[1] is D[0] transposed, GK[0] is written transposed
   unsigned d0;                 // first density of the launch
 };
 
@@ -72,15 +74,14 @@ __device__ __forceinline__ void dg_add(double* __restrict__ M, int r0, int c0, i
 }
 
 // the quartets of block blk: 128 threads of a.run consecutive ones
-template <int NA, int NB, int NC, int ND, int S>
+template <int NA, int NB, int NC, int ND, int S, bool CO>
 __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) {
   const long long first = ((long long)blk * blockDim.x + threadIdx.x) * a.run;
   if (first >= a.ntask) return;
   const int t1 = (int)(first + a.run < a.ntask ? first + a.run : a.ntask);
   constexpr int JK = S == 2 ? -1 : 0;      // the J density is the sum of both spins: half of it
   const int n = a.b.ld;
-  const bool co = S == 2 && a.co;
-  const long long dens = co ? (long long)(a.d0 + blockIdx.y) * n * n : 0;
+  const long long dens = CO ? (long long)(a.d0 + blockIdx.y) * n * n : 0;
   int bra = -1, oa = 0, ob = 0, oc = -1;
   long long o = dens;
   bool sab = false;
@@ -90,8 +91,8 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
     if (oc < 0) return;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      dg_add(a.GK[s] + o, oa, oc, n, -2, true, gac[s], co && s == 0);
-      dg_add(a.GK[s] + o, ob, oc, n, -2, true, gbc[s], co && s == 0);
+      dg_add(a.GK[s] + o, oa, oc, n, -2, true, gac[s], CO && s == 0);
+      dg_add(a.GK[s] + o, ob, oc, n, -2, true, gbc[s], CO && s == 0);
     }
   };
   auto load_j = [&](int r0, int c0, auto& v) {
@@ -101,7 +102,7 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
 #pragma unroll
       for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int j = 0; j < C; ++j) v[i][j] += __ldg(a.D[1] + o + (co ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j));
+        for (int j = 0; j < C; ++j) v[i][j] += __ldg(a.D[1] + o + (CO ? (size_t)(c0 + j) * n + r0 + i : (size_t)(r0 + i) * n + c0 + j));
     }
   };
   // the next quartet and its ket (AO of C | (C == D) << 30, AO of D, block offset) are loaded
@@ -144,8 +145,8 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
       oc = c;
 #pragma unroll
       for (int s = 0; s < S; ++s) {
-        dg_load(a.D[s] + o, oa, oc, n, Dac[s], co && s == 1);
-        dg_load(a.D[s] + o, ob, oc, n, Dbc[s], co && s == 1);
+        dg_load(a.D[s] + o, oa, oc, n, Dac[s], CO && s == 1);
+        dg_load(a.D[s] + o, ob, oc, n, Dbc[s], CO && s == 1);
       }
     }
     const int deg = !sab + !scd + (tk.x != tk.y);      // log2 of the degeneracy
@@ -154,8 +155,8 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
     load_j(oc, d, Jcd);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      dg_load(a.D[s] + o, oa, d, n, Dad[s], co && s == 1);
-      dg_load(a.D[s] + o, ob, d, n, Dbd[s], co && s == 1);
+      dg_load(a.D[s] + o, oa, d, n, Dad[s], CO && s == 1);
+      dg_load(a.D[s] + o, ob, d, n, Dbd[s], CO && s == 1);
     }
     const double* st = a.store + t;
 #pragma unroll
@@ -180,35 +181,36 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
     dg_add(a.GJ + o, oc, d, n, JK, false, gcd);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      dg_add(a.GK[s] + o, ob, d, n, -2, true, gbd[s], co && s == 0);
-      dg_add(a.GK[s] + o, oa, d, n, -2, true, gad[s], co && s == 0);
+      dg_add(a.GK[s] + o, ob, d, n, -2, true, gbd[s], CO && s == 0);
+      dg_add(a.GK[s] + o, oa, d, n, -2, true, gad[s], CO && s == 0);
     }
   }
   flush_c();
   dg_add(a.GJ + o, oa, ob, n, JK, false, gab);
 }
 
-template <int NA, int NB, int NC, int ND, int S>
+template <int NA, int NB, int NC, int ND, int S, bool CO>
 __global__ void __launch_bounds__(128) k_digest(const DigestArgs a) {
-  digest_block<NA, NB, NC, ND, S>(a, blockIdx.x);
+  digest_block<NA, NB, NC, ND, S, CO>(a, blockIdx.x);
 }
 
 // consecutive quartets per thread: up to 4, fewer where that would leave less than 1,024
-// threads an SM
-static inline int digest_run(int ntask) {
-  const int r = ntask / (152 * 1024);
-  return r < 1 ? 1 : (r > 4 ? 4 : r);
+// threads an SM, over all densities of the launch (six waters in 6-31G, 15 co-densities: 1.27 ms, 2.02
+// one by one; one co-density 0.26 against 0.38 with four)
+static inline int digest_run(long long quartets) {
+  const long long r = quartets / (152 * 1024);
+  return r < 1 ? 1 : (r > 4 ? 4 : (int)r);
 }
 
-template <int S>
+template <int S, bool CO = false>
 static int launch_digest(int cls, DigestArgs a, cudaStream_t s, unsigned ndens = 1) {
   if (a.ntask <= 0) return PCG_OK;
-  a.run = digest_run(a.ntask);
+  a.run = digest_run((long long)a.ntask * ndens);
   const int threads = 128;
   const unsigned blocks = (unsigned)(((long long)a.ntask + (long long)threads * a.run - 1) / ((long long)threads * a.run));
   switch (cls) {
 #define X(id, na, nb, nc, nd) \
-  case id: k_digest<na, nb, nc, nd, S><<<dim3(blocks, ndens), threads, 0, s>>>(a); break;
+  case id: k_digest<na, nb, nc, nd, S, CO><<<dim3(blocks, ndens), threads, 0, s>>>(a); break;
     PCG_SHAPE_CASES(X)
 #undef X
     default: pcg_set_error("digestion: class id out of range"); return PCG_ERR_ARG;

@@ -5,5 +5,5 @@ int pcg_launch_digest_lists(int nlist, const int* cls, const int* const* tasks, 
                             const double* const* stores, const DevBasis& b, const DevPairsExt& pr, const double* D,
                             double* G, cudaStream_t s) {
   return launch_digest_lists<1>(nlist, cls, tasks, ntask, stores,
-                                DigestArgs{b, pr, nullptr, 0, 1, nullptr, {D, nullptr}, G, {G, nullptr}, false, 0}, s);
+                                DigestArgs{b, pr, nullptr, 0, 1, nullptr, {D, nullptr}, G, {G, nullptr}, 0}, s);
 }

@@ -5,7 +5,7 @@ int pcg_launch_digest_lists_u(int nlist, const int* cls, const int* const* tasks
                               const double* const* stores, const DevBasis& b, const DevPairsExt& pr, const double* Da,
                               const double* Db, double* GJ, double* GKa, double* GKb, cudaStream_t s) {
   return launch_digest_lists<2>(nlist, cls, tasks, ntask, stores,
-                                DigestArgs{b, pr, nullptr, 0, 1, nullptr, {Da, Db}, GJ, {GKa, GKb}, false, 0}, s);
+                                DigestArgs{b, pr, nullptr, 0, 1, nullptr, {Da, Db}, GJ, {GKa, GKb}, 0}, s);
 }
 
 // F_s = H + (GJ + GK_s + its transpose) / 2 for both spins
