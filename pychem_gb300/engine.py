@@ -31,10 +31,22 @@ def _parts(counts):
 # distinct exponent sums up to which their factors are tabulated: 1,024^2 entries of 48 bytes stay
 # in L2 (H, C, N, O, F in 6-31G together have 990)
 MAX_EXPONENT_SUMS = 1024
-# co-density matrices by products with pair matrices: the dense tensor and the pair matrices
-# cost what the digestion of about 16 densities does, and take 1.2 GB at 96 functions
+# co-density matrices by products with pair matrices from COEXCHANGE_MIN densities on, up to
+# COEXCHANGE_MAX_N functions (1.2 GB of tensor and pair matrices); one density counts for more where
+# the digestion is dear beside the n^4 of the products (_density_weight)
 COEXCHANGE_MIN = 16
 COEXCHANGE_MAX_N = 96
+
+
+def _density_weight(n, has_d):
+    """How many of COEXCHANGE_MIN densities one density stands for.  Measured, digestion against
+    products, us: (dd|..) classes make a digestion last 1,200 us whatever the molecule: 28
+    functions 1,217 / 181 for one density, 82 1,580 / 1,370, but 96 1,670 / 2,230 and 2,460 / 2,230
+    for four.  Without d shells: 52 functions 186 / 196 for one density, 235 / 195 for two; 69 in a line
+    1,190 / 780 for ten, 65 in a chain of waters 410 / 570 for ten, 84 900 / 1,460."""
+    if has_d:
+        return 16 if n <= 88 else 4
+    return 8 if n <= 56 else 1
 
 
 def _ptr(t):
@@ -526,8 +538,8 @@ class GpuEngine:
         (nd, nbf, nbf): J_ab = sum_cd (ab|cd) W_cd, K_ad = sum_bc (ab|cd) W_cb
         (Methods/hartree_fock.py:345-347, applied by Methods/noci.py:261-318).
 
-        From COEXCHANGE_MIN densities on, for molecules whose dense tensor is small, three
-        matrix products of the packed densities with pair matrices (pcg_coulomb_exchange).
+        For enough densities (COEXCHANGE_MIN, _density_weight) of a molecule whose dense tensor
+        is small, three matrix products of the packed densities with pair matrices (pcg_coulomb_exchange).
         Otherwise one pcg_digest_class_co launch per class part digests every density
         (blockIdx.y selects it): per unique quartet the digestion accumulates one
         orientation of each exchange block (G[M]_ad from M_bc and so on); the kernel adds
@@ -536,7 +548,7 @@ class GpuEngine:
         GJ^T)/4."""
         W = W.contiguous()
         nd, n = W.shape[0], self.nbf
-        if nd >= COEXCHANGE_MIN and n <= COEXCHANGE_MAX_N:
+        if nd * _density_weight(n, int(self.h_pairs["lA"].max()) > 1) >= COEXCHANGE_MIN and n <= COEXCHANGE_MAX_N:
             lib = _lib.load()
             eri = self.dense_eri()
             J, K = torch.empty_like(W), torch.empty_like(W)
