@@ -1,6 +1,6 @@
 // Fock digestion kernels (closed shell, unrestricted, co-densities) -- included by digest.cu,
-// digest_u.cu and digest_co.cu, one translation unit each so that the class instantiations
-// compile in parallel.
+// digest_u.cu, digest_co.cu and digest_co1.cu, one translation unit each so that the class
+// instantiations compile in parallel.
 //
 // For every stored quartet block, with the shell-level degeneracy d = (A!=B ? 2:1)
 // (C!=D ? 2:1)(AB!=CD ? 2:1) and v' = d (ab|cd),
@@ -73,12 +73,13 @@ __device__ __forceinline__ void dg_add(double* __restrict__ M, int r0, int c0, i
     }
 }
 
-// the quartets of block blk: 128 threads of a.run consecutive ones
-template <int NA, int NB, int NC, int ND, int S, bool CO>
+// the quartets of block blk: 128 threads of a.run consecutive ones, or of one (ONE)
+template <int NA, int NB, int NC, int ND, int S, bool CO, bool ONE>
 __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) {
-  const long long first = ((long long)blk * blockDim.x + threadIdx.x) * a.run;
+  const int run = ONE ? 1 : a.run;
+  const long long first = ((long long)blk * blockDim.x + threadIdx.x) * run;
   if (first >= a.ntask) return;
-  const int t1 = (int)(first + a.run < a.ntask ? first + a.run : a.ntask);
+  const int t1 = ONE ? (int)first + 1 : (int)(first + run < a.ntask ? first + run : a.ntask);
   constexpr int JK = S == 2 ? -1 : 0;      // the J density is the sum of both spins: half of it
   const int n = a.b.ld;
   const long long dens = CO ? (long long)(a.d0 + blockIdx.y) * n * n : 0;
@@ -189,9 +190,9 @@ __device__ __forceinline__ void digest_block(const DigestArgs& a, unsigned blk) 
   dg_add(a.GJ + o, oa, ob, n, JK, false, gab);
 }
 
-template <int NA, int NB, int NC, int ND, int S, bool CO>
+template <int NA, int NB, int NC, int ND, int S, bool CO, bool ONE>
 __global__ void __launch_bounds__(128) k_digest(const DigestArgs a) {
-  digest_block<NA, NB, NC, ND, S, CO>(a, blockIdx.x);
+  digest_block<NA, NB, NC, ND, S, CO, ONE>(a, blockIdx.x);
 }
 
 // consecutive quartets per thread: up to 4, fewer where that would leave less than 1,024
@@ -202,15 +203,15 @@ static inline int digest_run(long long quartets) {
   return r < 1 ? 1 : (r > 4 ? 4 : (int)r);
 }
 
-template <int S, bool CO = false>
+template <int S, bool CO = false, bool ONE = false>
 static int launch_digest(int cls, DigestArgs a, cudaStream_t s, unsigned ndens = 1) {
   if (a.ntask <= 0) return PCG_OK;
-  a.run = digest_run((long long)a.ntask * ndens);
+  a.run = ONE ? 1 : digest_run((long long)a.ntask * ndens);
   const int threads = 128;
   const unsigned blocks = (unsigned)(((long long)a.ntask + (long long)threads * a.run - 1) / ((long long)threads * a.run));
   switch (cls) {
 #define X(id, na, nb, nc, nd) \
-  case id: k_digest<na, nb, nc, nd, S, CO><<<dim3(blocks, ndens), threads, 0, s>>>(a); break;
+  case id: k_digest<na, nb, nc, nd, S, CO, ONE><<<dim3(blocks, ndens), threads, 0, s>>>(a); break;
     PCG_SHAPE_CASES(X)
 #undef X
     default: pcg_set_error("digestion: class id out of range"); return PCG_ERR_ARG;

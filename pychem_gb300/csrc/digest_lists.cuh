@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(128) k_digest_lists(const __grid_constant__ Di
   const unsigned blk = blockIdx.x - ls.first[q];
   switch (ls.cls[q]) {
 #define X(id, na, nb, nc, nd) \
-  case id: if constexpr (id < DIGEST_SHARED) digest_block<na, nb, nc, nd, S, false>(a, blk); break;
+  case id: if constexpr (id < DIGEST_SHARED) digest_block<na, nb, nc, nd, S, false, false>(a, blk); break;
     PCG_SHAPE_CASES(X)
 #undef X
   }

@@ -40,12 +40,12 @@ COEXCHANGE_MAX_N = 96
 
 def _density_weight(n, has_d):
     """How many of COEXCHANGE_MIN densities one density stands for.  Measured, digestion against
-    products, us: (dd|..) classes make a digestion last 1,200 us whatever the molecule: 28
-    functions 1,217 / 181 for one density, 82 1,580 / 1,370, but 96 1,670 / 2,230 and 2,460 / 2,230
-    for four.  Without d shells: 52 functions 186 / 196 for one density, 235 / 195 for two; 69 in a line
-    1,190 / 780 for ten, 65 in a chain of waters 410 / 570 for ten, 84 900 / 1,460."""
+    products, us.  (dd|..) classes make a digestion last 1,000 us whatever the molecule: 28
+    functions 998 / 211 for one density, 72 1,118 / 666, 82 1,281 / 1,375 (two: 1,562 / 1,373), 96 1,302 /
+    2,240 (eight: 2,777 / 2,238).  Without d shells: 52 functions 178 / 197 for one density, 235 / 198
+    for two; 65 in a chain of waters 484 / 571 for fifteen, 78 1,266 / 1,165, 95 3,614 / 2,944."""
     if has_d:
-        return 16 if n <= 88 else 4
+        return 16 if n <= 76 else 8 if n <= 88 else 3
     return 8 if n <= 56 else 1
 
 
