@@ -41,13 +41,13 @@ struct DigestArgs {
   unsigned d0;                 // first density of the launch
 };
 
-// x 2^k, |k| <= 7, by its exponent; zero, infinities and NaNs stay what they are, below 2^-1015
-// is zero and beyond 2^1008 unscaled.  Selects, no branch: a branch an integral would keep the
+// x 2^k, |k| <= 3, by its exponent; zero, infinities and NaNs stay what they are, below 2^-1015
+// is zero and from 2^1021 on unscaled.  Selects, no branch: a branch an integral would keep the
 // loads of a block from being in flight together (1.6 times the time).
 __device__ __forceinline__ double dg_scale(double x, int k) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  const bool small = e < 8u, usual = e - 8u < 0x7e8u;
+  const bool small = e < 8u, usual = e - 8u < 0x7f4u;
   return __hiloint2double(small ? 0 : (usual ? hi + (k << 20) : hi), small ? 0 : lo);
 }
 
