@@ -7,6 +7,7 @@
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -69,6 +70,9 @@ DeviceState* pcg_state() {
 int pcg_ensure_boys(BoysTable* out) {
   DeviceState* st = pcg_state();
   if (!st) { pcg_set_error("no CUDA device"); return PCG_ERR_CUDA; }
+  // threads may make their first calls at the same time: none sees some of the tables
+  static std::mutex building;
+  std::lock_guard<std::mutex> hold(building);
   if (!st->boys_c) {
     std::vector<TaylorRow> c((size_t)BOYS_M * BOYS_ROWS);
     std::vector<double> ex(BOYS_NP);

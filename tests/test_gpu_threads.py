@@ -1,0 +1,36 @@
+"""First calls and solves from several threads at the same time."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+FIRST = """
+import threading, torch
+from pychem_gb300.engine import GpuEngine
+from pychem_gb300.molecule import Molecule
+torch.zeros(1, device="cuda"); torch.cuda.synchronize()
+mol = Molecule([["H", 1.0, 0.0, 0.0, 0.0], ["F", 9.0, 0.0, 0.0, 0.92]], "6-31G")
+start, out = threading.Barrier(8), [None] * 8
+def work(k):
+    start.wait()
+    eng = GpuEngine(mol).prepare()
+    out[k] = (eng.H.cpu(), eng.Q.cpu())
+threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+[t.start() for t in threads]; [t.join() for t in threads]
+want = GpuEngine(mol).prepare()
+for H, Q in out:
+    assert torch.equal(H, want.H.cpu()) and torch.equal(Q, want.Q.cpu())
+print("ok")
+"""
+
+
+def test_first_calls_of_threads():
+    """The tables that the first call of a process makes, from eight threads at once."""
+    r = subprocess.run([sys.executable, "-c", FIRST], cwd=REPO, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
