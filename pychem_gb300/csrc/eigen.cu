@@ -388,6 +388,11 @@ __global__ void __launch_bounds__(1024) k_jacobi_d(int n, int m, int batch, int 
   }
 }
 
+// 227 KB less the static tables.  The launches ask for this limit whatever they use: the attribute
+// is the process's, and a thread with a smaller matrix would take it from another's launch.
+#define JACOBI_D_SMEM (232448 - 1024)
+#define JACOBI_F_SMEM (232448 - 5120)
+
 // bytes of `per` matrices with rows_per rows of V each
 static size_t jacobi_bytes_d(int m, int per, int rows_per) {
   const size_t h = m / 2, mat = (((size_t)m * (m + 1) / 2 + 1) & ~(size_t)1) + m + (((size_t)rows_per * m + 1) & ~(size_t)1);
@@ -413,7 +418,7 @@ static JacobiPlanD jacobi_plan_d(int batch, int m, int least) {
   // smallest CTA to itself for its sums
   p.per = 1;
   while (p.per < 4 && 2 * p.per * (m / 2) < 32 && batch / (2 * p.per) >= 228) p.per *= 2;
-  for (p.split = least; jacobi_bytes_d(m, 1, (m + p.split - 1) / p.split) > 232448 - 1024; ++p.split) {}
+  for (p.split = least; jacobi_bytes_d(m, 1, (m + p.split - 1) / p.split) > JACOBI_D_SMEM; ++p.split) {}
   p.rows_per = (m + p.split - 1) / p.split;
   p.bytes = jacobi_bytes_d(m, p.per, p.rows_per);
   const long long ctas = (long long)((batch + p.per - 1) / p.per) * p.split;
@@ -438,7 +443,7 @@ extern "C" int pcg_jacobi_plan(int batch, int n, int* plan) {
 // shared-memory plan of one FP32 launch: how many CTAs share a matrix (at least `least`), rows of V
 // per CTA, whether the block table fits, and the dynamic bytes
 static bool jacobi_plan(int m, int least, int& split, int& rows_per, int& tab, size_t& bytes) {
-  const size_t limit = 232448 - 5120;                // 227 KB less the static tables
+  const size_t limit = JACOBI_F_SMEM;
   const size_t a_bytes = (size_t)((m * (m + 1) / 2 + 1) & ~1) * sizeof(float);
   const size_t tab_bytes = (size_t)(m / 2) * (m / 2 + 1) / 2 * sizeof(unsigned);
   for (split = least; split <= m; ++split) {
@@ -484,7 +489,7 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
     const long long ctas = (long long)((batch + p.per - 1) / p.per) * p.split;
     if (ctas > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
     if (32 * p.per > p.threads) { pcg_set_error("pcg_jacobi_eigh: a CTA with more matrices than warps"); return PCG_ERR_UNSUPPORTED; }
-    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes));
+    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_d, cudaFuncAttributeMaxDynamicSharedMemorySize, JACOBI_D_SMEM));
     k_jacobi_d<<<(unsigned)ctas, p.threads, p.bytes, s>>>(n, m, batch, p.per, p.split, p.rows_per, A, sA, (double*)V, sV,
                                                  (const double*)V0, w, sw, max_sweeps, tol, info);
   } else {
@@ -493,7 +498,7 @@ extern "C" int pcg_jacobi_eigh(int batch, int n, const double* A, double* w, voi
       return PCG_ERR_UNSUPPORTED;
     }
     if ((long long)batch * split > 0x7fffffffLL) { pcg_set_error("pcg_jacobi_eigh: batch too large"); return PCG_ERR_ARG; }
-    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    PCG_CUDA(cudaFuncSetAttribute(k_jacobi_f, cudaFuncAttributeMaxDynamicSharedMemorySize, JACOBI_F_SMEM));
     k_jacobi_f<<<batch * split, threads, bytes, s>>>(n, m, split, rows_per, A, sA, (float*)V, sV,
                                                           (const float*)V0, w, sw, max_sweeps, tol, info, tab);
   }

@@ -34,3 +34,27 @@ def test_first_calls_of_threads():
     """The tables that the first call of a process makes, from eight threads at once."""
     r = subprocess.run([sys.executable, "-c", FIRST], cwd=REPO, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
+
+
+def test_eigensolvers_of_two_threads():
+    """Large and small matrices at once, each kernel with its shared memory."""
+    import threading
+    from pychem_gb300 import eigen
+    failed = []
+
+    def work(n, fp32):
+        M = torch.randn(2, n, n, dtype=torch.float64, device="cuda")
+        A = M + M.transpose(1, 2)
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(200):
+                    w, _ = eigen.jacobi(A, fp32=fp32, max_sweeps=1, tol=1e-1)
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:
+            failed.append((n, fp32, e))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=a) for a in ((136, False), (6, False), (300, True), (12, True))]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not failed
