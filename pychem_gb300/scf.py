@@ -115,10 +115,10 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     the density of every iteration is the FP64 kernel's); or, above, from FP32 Jacobi in the
     first exact_iters iterations and then by refinement of the previous vectors that
     decouples the occupied space, checked, with the Jacobi route when the check
-    fails.  With graph None or
-    True every iteration after the first exact_iters is one CUDA graph replay followed
-    by one read of six numbers (energy, density change, refinement checks, commutator
-    size): an iteration is 50 to 60 launches, which for a small molecule take 1 ms of
+    fails.  With graph True (None: for n > 136, or in a program of one thread) every
+    iteration after the first exact_iters is one CUDA graph replay followed by one read
+    of six numbers (energy, density change, refinement checks, commutator size): an
+    iteration is 50 to 60 launches, which for a small molecule take 1 ms of
     host time against 0.3 ms replayed."""
     from . import dense
     mol = engine.mol
@@ -130,6 +130,9 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     e_nuc = mol.nuclear_repulsion()
     n = engine.nbf
     use_graph = graph is None or graph
+    # CUDA refuses another thread's device synchronisation while a stream is captured: a program
+    # with several threads gets graphs by itself only where an iteration is long
+    if_alone = graph is None and n <= eigen.FP64_JACOBI_MAX_N
     X = orthogonaliser(S)
     n2 = X.shape[1]
     # refined vectors instead of an FP64 Jacobi solve an iteration: to rounding (mid), or
@@ -226,13 +229,15 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     for it in range(1, max_iter + 1):
         exact = not mid and (it <= exact_iters or not big)
         diag = diag_mid if mid else diag_exact if exact else diag_refine
+        if g is None and if_alone and threading.active_count() > 1:
+            use_graph = False
         if it <= max(exact_iters, diis_start) or not use_graph:
             fock_and_diis(it > diis_start)
             diag()
             density()
         else:
             if g is None:
-                torch.cuda.synchronize()
+                torch.cuda.current_stream().synchronize()
                 g = torch.cuda.CUDAGraph()
                 c0 = _lib_launches()
                 # captured on a side stream with the graph pool, without the

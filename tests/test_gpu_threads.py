@@ -58,3 +58,31 @@ def test_eigensolvers_of_two_threads():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not failed
+
+
+def test_solves_of_three_threads():
+    """RHF with iteration graphs on streams of their own, one size for each way to the orbitals."""
+    import threading
+    from pychem_gb300 import workloads
+    from pychem_gb300.engine import GpuEngine
+    from pychem_gb300.molecule import Molecule
+    from pychem_gb300.scf import rhf
+    water = lambda nx, ny, nz: workloads.water_cluster(nx=nx, ny=ny, nz=nz, seed=2)
+    mols = [Molecule(water(1, 1, 1), "6-31G"), Molecule(water(2, 2, 1), "6-31G"), Molecule(water(3, 2, 2), "6-31G")]
+    want = [rhf(GpuEngine(m).prepare()) for m in mols]
+    got = [[], [], []]
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(4):
+                got[k].append(rhf(GpuEngine(mols[k]).prepare()))
+            torch.cuda.current_stream().synchronize()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    for rs, w in zip(got, want):
+        assert len(rs) == 4
+        for r in rs:
+            assert r.converged and abs(r.E - w.E) < 1e-8 and float((r.D - w.D).abs().max()) < 1e-6
