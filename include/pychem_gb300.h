@@ -232,7 +232,8 @@ int pcg_plan_fill(const pcg_plan_t *plan, const double *Qs, double thr, double t
                   void *stream);
 /* Expand screened quartet rows into task pairs: row r pairs bra pair bra[r] with the
  * kets ket[qstart[r] + q] for q < off[r+1] - off[r] - diag[r], and with itself last
- * when diag[r]; its tasks are written at [off[r], off[r+1]) of out_tasks (int2). */
+ * when diag[r]; its tasks are written at [off[r], off[r+1]) of out_tasks (int2).  For lists
+ * planned elsewhere; the engine's come from pcg_plan_fill. */
 int pcg_expand_tasks(int nbra, const int *bra, const int *ket, const long long *off,
                      const int *qstart, const int *diag, long long ntask, int *out_tasks,
                      void *stream);
@@ -261,10 +262,10 @@ int pcg_fock_build_u(int n, const double *H, const double *GJ, const double *GKa
                      double *Fb, void *stream);
 /* Electron-scattering integrals (ab|j0(S r12)|cd) of one class for a task list, same
  * store layout as pcg_eri_class (FP64): the operator of Methods/properties.py:20-23,
- * fundamentals of Methods/c_ints/two_electron_scattering.c:6-81 with z^-m j_m(z) by
- * the regimes of spherical_bessel_j.c:5-81.  S >= 0 is the momentum transfer in the
- * reference's units (inverse bohr).  Used for the Schwarz pass (diagonal tasks) and
- * the screened store of each grid value. */
+ * fundamentals of Methods/c_ints/two_electron_scattering.c:6-81 with z^-m j_m(z) from tables up to
+ * z = 100 and by the two terms of spherical_bessel_j.c:5-81 beyond.  S >= 0 is the momentum transfer in the
+ * reference's units (inverse bohr).  The engine's passes call pcg_scattering_class_split with
+ * the factors of each grid value instead. */
 int pcg_scattering_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pairs, const int *tasks,
                          int ntask, double S, double *store, void *stream);
 /* fac[i] for every primitive pair: what it contributes to each scattering integral's
@@ -335,7 +336,7 @@ int pcg_sym_pairs_class(int cls, const pcg_basis_t *basis, const pcg_pairs_t *pa
                         const double *store, const int *pairmap, long long rows, double *M, void *stream);
 /* used[p] = 1 (bytes, zeroed by the caller, one per shell pair) for both shell pairs of
  * every task (x, y) of a class list with x != y: the pairs that some off-diagonal
- * stored quartet contains (the rows of the compact pair tensor). */
+ * stored quartet contains.  The engine's compact rows come from pcg_pair_flags. */
 int pcg_mark_pairs(const int *tasks, int ntask, unsigned char *used, void *stream);
 /* colmap[a*n + b] = pairmap[pair(a, b)] (pairmap NULL: pair(a, b) itself), n x n ints:
  * where each (a, b) sits in a pair-packed row, -1 for nowhere. */
@@ -450,6 +451,8 @@ int pcg_mlp_wgrad(int M, int K, int N, const float *A, const float *G, float *dW
 /* Nonzero when a GEMM's wait has given up on this device since the last call (what the tile
  * would have stored is then NaNs); synchronises the stream. */
 int pcg_mlp_status(void *stream);
+/* Single steps of the same, for networks put together elsewhere: the package's passes use the
+ * fused forms (act = 2, pcg_mlp_wgrad, pcg_mlp_mse_counted, pcg_mlp_adam_all). */
 int pcg_mlp_dsilu(long long n, float *dY, const float *Z, void *stream);
 int pcg_mlp_colsum(int M, int N, const float *G, float *db, void *stream);
 int pcg_mlp_mse(long long n, const float *Y, const float *T, const float *mask, float inv_count,
