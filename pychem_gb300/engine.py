@@ -219,6 +219,7 @@ class GpuEngine:
         ppoff = np.concatenate([[0], np.cumsum(npp)[:-1]]).astype(np.int32)
         self.h_pairs = dict(A=A, B=B, npp=npp, ppoff=ppoff, lA=a["sh_l"][A], lB=a["sh_l"][B], nA=nA, nB=nB)
         self.npair = len(A)
+        self.has_d = bool((a["sh_l"] > 1).any())
         tot = int(npp.sum())
         dv = self.dev
         # every primitive pair (pcg_pair_data writes these) ...
@@ -548,7 +549,7 @@ class GpuEngine:
         GJ^T)/4."""
         W = W.contiguous()
         nd, n = W.shape[0], self.nbf
-        if nd * _density_weight(n, int(self.h_pairs["lA"].max()) > 1) >= COEXCHANGE_MIN and n <= COEXCHANGE_MAX_N:
+        if nd * _density_weight(n, self.has_d) >= COEXCHANGE_MIN and n <= COEXCHANGE_MAX_N:
             lib = _lib.load()
             eri = self.dense_eri()
             J, K = torch.empty_like(W), torch.empty_like(W)
