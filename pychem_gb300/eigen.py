@@ -1,7 +1,7 @@
 """Symmetric eigensolver for the SCF on the GPU (replaces numpy.linalg.eigh of
 ``Methods/hartree_fock.py:172-175,226``), on the library's own kernels only:
 
-* batches with n <= 136, and single matrices of n <= 32: parallel cyclic Jacobi in FP64
+* batches with n <= 136, and single matrices of n <= 80: parallel cyclic Jacobi in FP64
   (pcg_jacobi_eigh), up to four matrices to a CTA in a batch.
 * single matrices of larger n: the FP32 variant of the Jacobi kernel (FP32-accurate vectors, n <= 334),
   then FP64 iterative refinement (T. Ogita and K. Aishima, "Iterative refinement for
@@ -21,10 +21,16 @@ from . import _lib, dense
 from ._stream import stream as _stream
 
 FP64_JACOBI_MAX_N = 136
-# single matrices above this size go through FP32 Jacobi and FP64 refinement: an FP64 sweep of
-# one matrix is n - 1 rounds bound by one SM's FP64 pipe (an SCF iteration of 104 functions
-# took 3 to 6 ms in it, 0.9 ms refined)
+# above this size a symmetric orthogonaliser is tried before the eigenvectors of S
 FP64_JACOBI_ONE_N = 32
+# single matrices above this size are sliced (FP32 Jacobi, FP64 refinement): an FP64 sweep of one
+# matrix is n - 1 rounds bound by one SM's FP64 pipe.  Sliced against the FP64 kernel: n = 40 1.04 / 0.73
+# ms, 65 3.08 / 1.82, 80 3.35 / 3.23, 100 3.73 / 5.33
+SLICED_MIN_N = 80
+# RHF iterations above this size refine the occupied space from FP32 vectors (occupied_space).  A
+# solve, refined against the FP64 kernel in every iteration: 39 functions 12.9 / 8.6 ms, 52 13.8 / 13.5, 56
+# 13.0 / 13.6 and 14.3 / 13.8, 65 14.8 / 18.9, 78 17.4 / 28.8, 104 23.5 / 52.7
+REFINED_MIN_N = 56
 
 # counts of eigh calls by route (exact library solve, refinement, refinement rejected)
 stats = {"exact": 0, "refined": 0, "fallback": 0}
@@ -315,7 +321,7 @@ def _eigh_scaled(A, X_prev):
 def eigh(A, X_prev=None, refine_steps=2, exact=True, check_tol=1e-10, nocc=None):
     """Ascending eigenvalues and eigenvectors of symmetric FP64 A (..., n, n).
 
-    n <= 136 in a batch, n <= 32 alone or while the stream is captured: FP64 Jacobi
+    n <= 136 in a batch, n <= 80 alone or while the stream is captured: FP64 Jacobi
     (exact to rounding).  One matrix of n <= 136: spectrum slicing (exact_eigh) on the matrix
     scaled to order one.  Larger n (one matrix): exact=True or no X_prev -- spectrum slicing (exact_eigh);
     otherwise refinement from X_prev (consecutive SCF iterations): with nocc, only the
@@ -323,7 +329,7 @@ def eigh(A, X_prev=None, refine_steps=2, exact=True, check_tol=1e-10, nocc=None)
     else the exact route); without nocc, full refinement (checked for orthogonality,
     else the exact route)."""
     n = A.shape[-1]
-    if FP64_JACOBI_ONE_N < n <= FP64_JACOBI_MAX_N and A.dim() == 2 and not torch.cuda.is_current_stream_capturing():
+    if max(FP64_JACOBI_ONE_N, SLICED_MIN_N) < n <= FP64_JACOBI_MAX_N and A.dim() == 2 and not torch.cuda.is_current_stream_capturing():
         return _eigh_scaled(A, X_prev)
     if n <= FP64_JACOBI_MAX_N:
         if X_prev is not None:

@@ -110,7 +110,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     with its Pulay system solved on the GPU.  Every step runs on the library's
     kernels: Fock digestion, FP64 GEMMs (pcg_dgemm), the eigenvectors, the density
     C_occ C_occ^T on the tensor cores (pcg_ozaki_gemm_tc, n > 136).  The eigenvectors come
-    from the FP64 Jacobi kernel (n <= 32); from the FP32 one with the occupied space
+    from the FP64 Jacobi kernel (n <= 56); from the FP32 one with the occupied space
     refined to rounding, checked, and the FP64 kernel where the check fails (n <= 136:
     the density of every iteration is the FP64 kernel's); or, above, from FP32 Jacobi in the
     first exact_iters iterations and then by refinement of the previous vectors that
@@ -138,7 +138,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
     # refined vectors instead of an FP64 Jacobi solve an iteration: to rounding (mid), or
     # as far as the SCF has come (big)
     big = n > eigen.FP64_JACOBI_MAX_N and 0 < nocc < n2
-    mid = eigen.FP64_JACOBI_ONE_N < n <= eigen.FP64_JACOBI_MAX_N and 0 < nocc < n2
+    mid = max(eigen.FP64_JACOBI_ONE_N, eigen.REFINED_MIN_N) < n <= eigen.FP64_JACOBI_MAX_N and 0 < nocc < n2
     mm = dense.mm
 
     # static buffers (the CUDA graph reads and writes these addresses)
@@ -314,7 +314,7 @@ def rhf(engine, max_iter=128, e_tol=1e-10, d_tol=1e-8, diis_size=10, diis_start=
                 break
         E_old = E
     # orbitals of the final Fock matrix, exact (including inside near-degenerate
-    # clusters) for MP2's denominators: for n > 32 the occupied and virtual blocks of
+    # clusters) for MP2's denominators: for n > 56 the occupied and virtual blocks of
     # the refined vectors are decoupled once more and each block is diagonalised
     # exactly (spectrum slicing inside blocks above 64)
     if record:

@@ -30,3 +30,19 @@ def test_exact_whatever_the_gaps(n):
             assert float((w - lam).abs().max()) < 1e-12 * size
             assert float((A @ V - V * w).abs().max()) < 1e-12 * size
             assert float((V.T @ V - torch.eye(n, dtype=torch.float64, device="cuda")).abs().max()) < 1e-13
+
+
+@pytest.mark.parametrize("n", [33, 64, 65, 80, 81])
+def test_slicing_itself(n):
+    """Below the size from which single matrices are sliced by themselves, too."""
+    from pychem_gb300 import eigen
+    Q = torch.tensor(np.linalg.qr(np.random.default_rng(n).standard_normal((n, n)))[0], device="cuda")
+    for lam in spectra(n):
+        lam = torch.tensor(lam, device="cuda")
+        A = (Q * lam) @ Q.T
+        A = 0.5 * (A + A.T)
+        for w, V in (eigen.exact_eigh(A), eigen.eigh(A)):
+            size = float(lam.abs().max())
+            assert float((w - lam).abs().max()) < 1e-12 * size
+            assert float((A @ V - V * w).abs().max()) < 1e-12 * size
+            assert float((V.T @ V - torch.eye(n, dtype=torch.float64, device="cuda")).abs().max()) < 1e-13

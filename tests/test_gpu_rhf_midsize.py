@@ -38,3 +38,26 @@ def test_same_as_jacobi_route(system, units, basis, n, graph):
     for key in ("D", "eps"):
         a, b = got[key], want[key]
         assert float((a - b).norm() / b.norm()) < 5e-10
+
+
+@pytest.mark.parametrize("gap", [True, False])
+def test_refined_below_its_sizes(gap, monkeypatch):
+    """36 functions with refined vectors, which go to the FP64 kernel by themselves: helium atoms, and
+    with a square of hydrogen atoms whose frontier orbitals are degenerate."""
+    from pychem_gb300 import eigen
+    from pychem_gb300.engine import GpuEngine
+    from pychem_gb300.molecule import Molecule
+    from pychem_gb300.scf import rhf
+    coords = [["H", 1.0, x, y if gap else 1.2 * (y > 0), 0.0] for x in (0.0, 1.2) for y in (0.0, 0.8)]
+    coords += [["HE", 2.0, 6.0 + 3.0 * k, 0.0, 0.0] for k in range(14)]
+    eng = GpuEngine(Molecule(coords, "6-31G")).prepare()
+    want = rhf(eng, max_iter=60)
+    monkeypatch.setattr(eigen, "REFINED_MIN_N", 0)
+    got = rhf(eng, max_iter=60)
+    assert eng.nbf == 36 and got.converged == want.converged
+    assert bool(torch.isfinite(got.eps).all()) and bool(torch.isfinite(got.D).all())
+    if gap:
+        assert want.converged and got.iterations == want.iterations
+        assert float((got.D - want.D).norm() / want.D.norm()) < 5e-10
+    elif want.converged:
+        assert abs(got.E - want.E) < 1e-7
